@@ -246,15 +246,16 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_ml + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // a CTA that starts after another one of this or an earlier launch has recorded a failed wait leaves at once: one stuck tile
   // must not make every later tile sit out its own time limit
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int*>(p.status) != 0)) return;
   // heavy tiles first: inside a sequence the late query tiles see the most keys, and the host lists tiles in ascending order
   const int tile = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
-  const int seq = p.tile_seq[tile], q0 = p.tile_q0[tile], h = blockIdx.y;
+  auto uniform = [](int v) { return __shfl_sync(0xffffffffu, v, 0); };  // (one value for the CTA, told to the compiler)
+  const int seq = uniform(p.tile_seq[tile]), q0 = uniform(p.tile_q0[tile]), h = blockIdx.y;
   const int kvh = h / (p.H / p.KV);
-  const int qs = p.q_start[seq], ql = p.q_len[seq], ctx = p.ctx_lens[seq];
+  const int qs = uniform(p.q_start[seq]), ql = uniform(p.q_len[seq]), ctx = uniform(p.ctx_lens[seq]);
   const int pos0 = ctx - ql;  // position of the sequence's first query row
   constexpr bool SPLIT = PIECES && QT == 2;  // one query tile, its key tiles alternate between the softmax groups
   const int rows_all = min((SPLIT ? 1 : QT) * kAtBM, ql - q0);
@@ -456,12 +457,14 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
       const int j = tile_at(u), a = q == 0 ? a0 : a1;
       return j < kept_tiles ? j : j - max(a, kept_tiles) + kept_tiles;
     };
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
+      auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abort_flag, p.status)) != 0; };
       bool ok = true;
       int u = 0, q = 0;
       if (n_tiles > 0 && !valid(u, q)) advance(u, q);
       if (warp != kIssuerPV) {
-        if (KM != 2) ok = mbar_wait(smem_u32(bar_q), 0, abort_flag, p.status);
+        if (KM != 2) ok = wait(bar_q, 0);
         if (warp == kIssuer2) {
           u = 1;
           q = 1;
@@ -474,32 +477,32 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
           const int t = count_at(u, q);
           const int s = u % NS;
           const uint32_t slot = q * 2 + (t & 1);
-          if (t >= 2) ok = mbar_wait(smem_u32(&bar_pv_done[slot]), ((t >> 1) - 1) & 1, abort_flag, p.status);
+          if (t >= 2) ok = wait(&bar_pv_done[slot], ((t >> 1) - 1) & 1);
           if constexpr (PIECES) {
             const uint32_t d_w = tmem_base + kColS + slot * kAtBN;
             for (int pc = 0; ok && pc < pieces; ++pc, ++piece) {
               const int st = (SPLIT ? q * NSK : 0) + piece % NSK;
-              ok = mbar_wait(smem_u32(&bar_k_full[st]), (piece / NSK) & 1, abort_flag, p.status);
+              ok = wait(&bar_k_full[st], (piece / NSK) & 1);
               if (!ok) break;
               tc_fence_after();
               const uint64_t desc_q = umma_desc_k_sw128(smem_u32(smem + (KM == 1 ? pc * L::kTileQ : L::kOffK + st * L::kTileK)));
               const uint64_t desc_k = umma_desc_k_sw128(smem_u32(smem + L::kOffK + st * L::kTileK + L::kOffKeys));
               const int subs = min(kAtPiece, p.k_subs - pc * kAtPiece);
-              for (int c = 0; c < subs; ++c)
+              for (int c = 0; leader && c < subs; ++c)
 #pragma unroll
                 for (int k16 = 0; k16 < 4; ++k16)
                   umma_bf16(d_w, desc_q + static_cast<uint64_t>((c * (kAtBM * 128) + k16 * 32) >> 4), desc_k + static_cast<uint64_t>((c * (kAtBN * 128) + k16 * 32) >> 4),
                             idesc_s, (pc > 0 || c > 0 || k16 > 0) ? 1u : 0u);
-              umma_commit(smem_u32(&bar_k_empty[st]));
+              if (leader) umma_commit(smem_u32(&bar_k_empty[st]));
             }
             if (!ok) break;
-            umma_commit(smem_u32(&bar_s_full[slot]));
+            if (leader) umma_commit(smem_u32(&bar_s_full[slot]));
             if (SPLIT) u += 2;
             else advance(u, q);
             continue;
           }
           if (ok && u > k_seen) {
-            ok = mbar_wait(smem_u32(&bar_k_full[s]), (u / NS) & 1, abort_flag, p.status);
+            ok = wait(&bar_k_full[s], (u / NS) & 1);
             k_seen = u;
           }
           if (!ok) break;
@@ -507,14 +510,15 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
           const uint64_t desc_q = desc_q0 + static_cast<uint64_t>((q * L::kTileQ) >> 4);
           const uint64_t desc_k = desc_k0 + static_cast<uint64_t>((s * L::kTileK) >> 4);
           const uint32_t d_s = tmem_base + kColS + slot * kAtBN;
+          if (leader)
 #pragma unroll
           for (int k16 = 0; k16 < DK / 16; ++k16) {
             const uint64_t adv_q = static_cast<uint64_t>(((k16 >> 2) * (kAtBM * 128) + (k16 & 3) * 32) >> 4);
             const uint64_t adv_k = static_cast<uint64_t>(((k16 >> 2) * (kAtBN * 128) + (k16 & 3) * 32) >> 4);
             umma_bf16(d_s, desc_q + adv_q, desc_k + adv_k, idesc_s, k16 > 0 ? 1u : 0u);
           }
-          if (last_of_tile(u, q)) umma_commit(smem_u32(&bar_k_empty[s]));
-          umma_commit(smem_u32(&bar_s_full[slot]));
+          if (leader && last_of_tile(u, q)) umma_commit(smem_u32(&bar_k_empty[s]));
+          if (leader) umma_commit(smem_u32(&bar_s_full[slot]));
           advance(u, q);
         }
       } else {
@@ -523,25 +527,26 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
           const int t = count_at(u, q);
           const int s = u % NSV;
           const uint32_t slot = q * 2 + (t & 1);
-          ok = mbar_wait(smem_u32(&bar_p_full[slot]), (t >> 1) & 1, abort_flag, p.status) &&
-               mbar_wait(smem_u32(&bar_v_full[s]), (u / NSV) & 1, abort_flag, p.status);
+          ok = wait(&bar_p_full[slot], (t >> 1) & 1) &&
+               wait(&bar_v_full[s], (u / NSV) & 1);
           if (!ok) break;
           tc_fence_after();
           const uint32_t tmem_p = tmem_base + kColS + slot * kAtBN, d_o = tmem_base + kColO + q * DV;
           const uint64_t desc_v0 = umma_desc_mn_sw128(v_base + s * L::kTileV, kAtBN * 128, 1024);
+          if (leader)
 #pragma unroll
           for (int k16 = 0; k16 < kAtBN / 16; ++k16) {
             // 16 keys = two 8-row swizzle atoms (2048 bytes) further down the V tile; the 64-column blocks of D are kAtBN * 128 bytes apart
             umma_bf16_ts(d_o, tmem_p + k16 * 8, desc_v0 + static_cast<uint64_t>((k16 * 2048) >> 4), idesc_o, (t == 0 && k16 == 0) ? 0u : 1u);
           }
-          if (last_of_tile(u, q)) umma_commit(smem_u32(&bar_v_empty[s]));
-          umma_commit(smem_u32(&bar_pv_done[slot]));
+          if (leader && last_of_tile(u, q)) umma_commit(smem_u32(&bar_v_empty[s]));
+          if (leader) umma_commit(smem_u32(&bar_pv_done[slot]));
           advance(u, q);
-          if (u >= n_tiles) umma_commit(smem_u32(bar_o_final));
+          if (leader && u >= n_tiles) umma_commit(smem_u32(bar_o_final));
         }
-        if (n_tiles == 0) umma_commit(smem_u32(bar_o_final));
+        if (leader && n_tiles == 0) umma_commit(smem_u32(bar_o_final));
       }
-      if (!ok) {
+      if (!ok && leader) {
         // a wait ran out: let this thread's outstanding MMAs retire (bounded) before tensor memory is released
         uint64_t* drain = &bar_drain[warp == kIssuer ? 0 : (warp == kIssuerPV ? 1 : 2)];
         umma_commit(smem_u32(drain));

@@ -203,7 +203,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
   int* s_last = const_cast<int*>(abort_flag) + 1;
   constexpr int NAS = Q4 ? NA : NW;  // depth of the A-operand ring
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   int n_tile = blockIdx.x, split = blockIdx.z;
   const int m_tile = blockIdx.y;
   int splits = p.splits, kb_per_split = p.kb_per_split, ws_tile = m_tile * p.n_tiles + blockIdx.x;
@@ -377,6 +377,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
       const uint64_t desc_w0 = umma_desc_k_sw128(smem_u32(smem));
       const uint64_t desc_x0 = umma_desc_k_sw128(smem_u32(smem + L::kOffX));
       const uint32_t tmem_acc = tmem_base + (L::kSharedAcc ? 0 : issuer * BN);
+      const bool leader = elect_one();
       bool ok = true;
       for (int i = issuer; i < nkb; i += NI) {
         const int sa = i % NAS, sx = i % NX;
@@ -387,7 +388,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        if (lane == 0) {
+        if (leader) {
           // descriptor start-address field counts 16-byte units: stage strides and the 32-byte k-step are added there
           const uint64_t dx = desc_x0 + static_cast<uint64_t>((sx * L::kXStage) >> 4);
 #pragma unroll
@@ -408,7 +409,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
         }
         __syncwarp();
       }
-      if (lane == 0) {
+      if (leader) {  // (the thread that issued: a commit covers its own MMAs)
         umma_commit(smem_u32(bar_acc));  // one arrival per issuer
         if (!ok) {
           // outstanding MMAs must retire before TMEM is released
