@@ -174,9 +174,11 @@ def _experts_cuda(st, lw, x, logits, E, k, mode, renorm, act, e0, ne):
         if hmid is None:
             with st("moe.gate_up"):
                 xs = gathered()
-                gu = gu_w.run(xs, items, bn, k_splits(gu_w))
-            with st("moe.activation_multiply"):
-                hmid = ops.act_mul(gu, act)
+                hmid = gu_w.run_gated(xs, items, act) if bn == 256 else None
+                gu = gu_w.run(xs, items, bn, k_splits(gu_w)) if hmid is None else None
+            if hmid is None:
+                with st("moe.activation_multiply"):
+                    hmid = ops.act_mul(gu, act)
     with st("moe.down"):
         ys = down_w.run(hmid, items, bn, k_splits(down_w))
     return ys, pos, w, offsets

@@ -266,14 +266,18 @@ def interleave_gate_up(gate, up, block: int = 64):
 
 def linear_gated(x: torch.Tensor, w: LinearWeight, act: str) -> torch.Tensor:
     """``act(x @ Wg^T) * (x @ Wu^T)`` for a weight that holds the gate rows followed by the up rows (plain order). One kernel for
-    1..8 rows of a JQ4 weight on CUDA (the small-batch GEMV's epilogue), projection + activation kernel otherwise."""
-    if _cuda(x) and w.q4 and x.shape[0] <= GEMV_MAX_ROWS:
+    1..8 rows of a JQ4 weight on CUDA (the small-batch GEMV's epilogue) and for prompt-size batches (the pair kernel's), projection +
+    activation kernel otherwise."""
+    if _cuda(x) and x.dtype == torch.bfloat16 and w.bias is None:
         kind = fused_act_kind(act)
-        if kind:
+        out = None
+        if kind and x.shape[0] > GEMV_MAX_ROWS:
+            out = w.handle().run_gated(x, kind)
+        elif kind and w.q4:
             out = w.handle().run_gemv_act(x, kind)
-            if out is not None:
-                _count()
-                return out
+        if out is not None:
+            _count()
+            return out
     return act_mul(linear(x, w), act)
 
 
@@ -668,6 +672,14 @@ class GroupedLinearWeight:
         if out is None:
             return None
         _count()
+        return out
+
+    def run_gated(self, xs: torch.Tensor, items: torch.Tensor, act: str) -> Optional[torch.Tensor]:
+        """Prompt-size work items (256 rows): gate|up projection of plain-order rows with ``act(gate) * up`` in the epilogue, or ``None``."""
+        kind = fused_act_kind(act)
+        out = self.handle.run_grouped_gated(xs, items, self.N, kind) if kind and self.handle is not None else None
+        if out is not None:
+            _count()
         return out
 
     def run_act(self, xs: torch.Tensor, items: torch.Tensor, bn: int, splits: int, act: str) -> torch.Tensor:

@@ -240,7 +240,14 @@ class GemmWeight {
     dlv::gemm_weight_init(&desc_);
   }
 
-  // out[m, :] = x[m, :] @ W^T (+ bias). impl: 0 = auto, 1 = tcgen05, 2 = CUDA-core GEMV
+  // room for the bf16 form of a JQ4 weight in front of a prompt-size product; it belongs to this call and goes back to the allocator
+  // behind it in stream order
+  Tensor expanded() const {
+    const size_t bytes = dlv::gemm_pair_expanded_bytes(&desc_);
+    return bytes > 0 ? at::empty({static_cast<int64_t>(bytes)}, w_.options().dtype(at::kByte)) : Tensor();
+  }
+
+  // out[m, :] = x[m, :] @ W^T (+ bias). impl: 0 = auto, 1 = tcgen05, 2 = CUDA-core GEMV, 3 = tcgen05 on pairs of SMs
   Tensor run(const Tensor& x, c10::optional<Tensor> out_opt, c10::optional<Tensor> bias, bool out_f32, int64_t impl,
              int64_t force_splits) {
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2, "x must be bf16 [M, K] on CUDA");
@@ -264,6 +271,16 @@ class GemmWeight {
       bptr = b.data_ptr<float>();
     }
     if (M == 0) return out;
+    const bool pair = impl == 3 || (impl == 0 && force_splits == 0 && !dlv::g_gemm_persist && dlv::g_gemm_force_bn == 0 &&
+                                    dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0));
+    if (pair && !out_f32 && dlv::gemm_pair_supported(&desc_, desc_.N, out.data_ptr(), static_cast<int>(out.stride(0)))) {
+      Tensor room = expanded();
+      dlv::gemm_pair_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), bptr,
+                         room.defined() ? room.data_ptr() : nullptr, scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
+      check_last_error("pair gemm launch");
+      return out;
+    }
+    TORCH_CHECK(impl != 3, "shape outside the pair kernel");
     const bool simt = impl == 2 || (impl == 0 && M <= 1 && !desc_.is_q4);
     if (simt) {
       dlv::gemv_simt_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), out_f32,
@@ -306,6 +323,41 @@ class GemmWeight {
     dlv::gemv_dense_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), false, nullptr,
                         static_cast<int>(act), cur_stream());
     check_last_error("gemv (gated activation) launch");
+    return out;
+  }
+  // Prefill-size batches: act(gate) * up in the epilogue of the pair kernel, gate | up rows in plain order. Undefined where that kernel is
+  // not the faster one or does not take the shape.
+  Tensor run_gated(const Tensor& x, int64_t act) {
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.size(1) == desc_.K && x.stride(1) == 1, "x must be bf16 [M, K]");
+    TORCH_CHECK(x.device() == w_.device(), "x and weight live on different devices");
+    const int M = static_cast<int>(x.size(0));
+    if ((act != 1 && act != 2) || desc_.N % 16 != 0 || !dlv::gemm_pair_preferred(&desc_, M, desc_.N, 3 * desc_.N / 2) || x.stride(0) % 8 != 0 ||
+        (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) != 0 || !dlv::gemm_pair_act_supported(&desc_, desc_.N, nullptr, desc_.N / 2))
+      return Tensor();
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor out = new_out({M, desc_.N / 2}, x.options());
+    Tensor room = expanded();
+    dlv::gemm_pair_run_act(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), static_cast<int>(act),
+                           room.defined() ? room.data_ptr() : nullptr, scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
+    check_last_error("pair gemm (gated activation) launch");
+    return out;
+  }
+  // The same for experts (items of 256 rows): [rows, n / 2], or undefined.
+  Tensor run_grouped_gated(const Tensor& xs, const Tensor& items, int64_t n_per_expert, int64_t act) {
+    TORCH_CHECK(xs.is_cuda() && xs.scalar_type() == at::kBFloat16 && xs.dim() == 2 && xs.size(1) == desc_.K && xs.stride(1) == 1, "xs must be bf16 [rows, K]");
+    TORCH_CHECK(xs.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(xs.data_ptr()) & 15) == 0, "xs rows must be 16-byte aligned");
+    TORCH_CHECK(items.is_cuda() && items.scalar_type() == at::kInt && items.dim() == 2 && items.size(1) == 4 && items.is_contiguous(), "items must be int32 [n, 4]");
+    const int64_t per = desc_.is_q4 ? ((n_per_expert + 127) / 128) * 128 : n_per_expert;
+    TORCH_CHECK(n_per_expert > 0 && desc_.N % per == 0, "stacked weight rows are not a multiple of the per-expert rows");
+    if ((act != 1 && act != 2) || n_per_expert % 16 != 0 || !dlv::gemm_pair_act_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2)))
+      return Tensor();
+    c10::cuda::CUDAGuard guard(xs.device());
+    Tensor out = new_out({xs.size(0), n_per_expert / 2}, xs.options());
+    if (xs.size(0) == 0 || items.size(0) == 0) return out;
+    dlv::gemm_pair_run_grouped(&desc_, static_cast<int>(n_per_expert), xs.data_ptr(), static_cast<int>(xs.size(0)), static_cast<int>(xs.stride(0)),
+                               out.data_ptr(), static_cast<int>(out.stride(0)), items.data_ptr<int>(), static_cast<int>(items.size(0)),
+                               static_cast<int>(act), scratch_for(xs.device().index()).status.data_ptr<int>(), cur_stream());
+    check_last_error("pair gemm (grouped, gated activation) launch");
     return out;
   }
   bool gemv_ok(int64_t M, int64_t ldx) const { return dlv::gemv_dense_supported(&desc_, static_cast<int>(M), static_cast<int>(ldx)); }
@@ -413,6 +465,14 @@ class GemmWeight {
     Tensor q = new_out({M, H * 128}, x.options());
     if (M == 0) return q;
     DeviceScratch& s = scratch_for(x.device().index());
+    if (dlv::g_gemm_force_bn == 0 && dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0) && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
+        desc_.N == (a.heads + 2 * a.kv_heads) * 128 && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a)) {
+      Tensor room = expanded();
+      dlv::gemm_pair_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
+                             room.defined() ? room.data_ptr() : nullptr, s.status.data_ptr<int>(), cur_stream());
+      check_last_error("pair gemm (fused q/k/v epilogue) launch");
+      return q;
+    }
     dlv::gemm_tc_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
                          s.ws.data_ptr<float>(), static_cast<size_t>(s.ws.numel()), s.counters.data_ptr<int>(),
                          static_cast<int>(s.counters.numel()), s.status.data_ptr<int>(), cur_stream());
@@ -1527,6 +1587,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("run_gathered", &GemmWeight::run_gathered, py::arg("x_own"), py::arg("M"), py::arg("out"), py::arg("comm"), py::arg("bias") = py::none())
       .def("run_act", &GemmWeight::run_act, py::arg("x"), py::arg("act"))
       .def("run_qkv", &GemmWeight::run_qkv)
+      .def("run_gated", &GemmWeight::run_gated, py::arg("x"), py::arg("act"))
+      .def("run_grouped_gated", &GemmWeight::run_grouped_gated, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("act"))
       .def("run_grouped_act", &GemmWeight::run_grouped_act, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("bn"), py::arg("splits"),
            py::arg("act"))
       .def("run_grouped_gemv_act", &GemmWeight::run_grouped_gemv_act, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("act"),

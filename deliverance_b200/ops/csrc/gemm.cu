@@ -80,6 +80,7 @@ void gemm_weight_init(GemmWeightDesc* w) {
     w->w3d = w->K % 64 == 0;
     if (w->w3d) encode_map_kchunks(&w->map_w, w->data, w->N, w->K, static_cast<uint64_t>(w->K) * 2, kGemmBM);
     else encode_map_2d(&w->map_w, 0, w->data, w->N, w->K, static_cast<uint64_t>(w->K) * 2, kGemmBM, 64, 128);
+    encode_map_2d(&w->map_w64, 0, w->data, w->N, w->K, static_cast<uint64_t>(w->K) * 2, 128, 64, 128);
   }
 }
 
@@ -497,6 +498,10 @@ void gemm_tc_run_grouped(const GemmWeightDesc* w, int n_per_expert, const void* 
   if (rows <= 0 || max_items <= 0) return;
   if (ldx % 8 != 0) throw std::runtime_error("activation row pitch must be a multiple of 8 elements");
   if (max_items > 65535) throw std::runtime_error("grouped gemm: work list too long");
+  if (bn == 256 && splits <= 1 && gemm_pair_supported(w, n_per_expert, out, ldo)) {
+    gemm_pair_run_grouped(w, n_per_expert, x, rows, ldx, out, ldo, items, max_items, 0, status, st);
+    return;
+  }
   GemmParams p = {};
   p.M = rows;
   p.N = n_per_expert;

@@ -19,6 +19,7 @@ struct GemmWeightDesc {
   const void* data = nullptr;  // bf16 [N, K] or the tile-packed JQ4 bytes
   CUtensorMap map_w;           // dense: [N, K] (3-D chunked form when w3d); JQ4: the packed stages as rows of 1 KB
   bool w3d = false;
+  CUtensorMap map_w64;         // dense: [N, K] in boxes of 128 rows x 64 k (gemm_pair.cu)
 };
 
 // Peer-memory state of the fused GEMM + all-reduce epilogue (all pointers are device addresses mapped in this process).
@@ -107,6 +108,18 @@ bool gemm_gathered_supported(const GemmWeightDesc* w, int M, const GemmScatterAr
 void launch_gather_push(const GemmScatterArgs* a, const GemmScatterPlan* plan, const void* x_own, int M, int K, int* status, cudaStream_t st);
 void gemm_tc_run_gathered(const GemmWeightDesc* w, int M, const GemmScatterArgs* a, const unsigned* group_targets, void* out, int ldo,
                           const float* bias, float* ws, size_t ws_floats, int* counters, int n_counters, int* status, cudaStream_t st);
+// gemm_pair.cu: prefill-size products on pairs of SMs. `expanded`: device room of gemm_pair_expanded_bytes() for a JQ4 weight's bf16 form.
+bool gemm_pair_preferred(const GemmWeightDesc* w, int M, int n, int merged);  // faster than the one-tile kernel
+bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ldo);
+bool gemm_pair_act_supported(const GemmWeightDesc* w, int n, const void* out, int ldo);
+size_t gemm_pair_expanded_bytes(const GemmWeightDesc* w);
+void gemm_pair_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, const float* bias, void* expanded, int* status, cudaStream_t st);
+void gemm_pair_run_act(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, int act, void* expanded, int* status, cudaStream_t st);
+void gemm_pair_run_qkv(const GemmWeightDesc* w, const void* x, int M, int ldx, void* q_out, int ldo, const float* bias, const GemmQkvArgs* a, void* expanded,
+                       int* status, cudaStream_t st);
+bool gemm_pair_qkv_supported(const GemmWeightDesc* w, const void* q_out, int ldo, const GemmQkvArgs* a);
+void gemm_pair_run_grouped(const GemmWeightDesc* w, int n_per_expert, const void* x, int rows, int ldx, void* out, int ldo, const int* items, int max_items,
+                           int act, int* status, cudaStream_t st);
 // true when the fused all-reduce epilogue can take this problem (one wave of CTAs, rows and columns inside the slab)
 bool gemm_tp_supported(const GemmWeightDesc* w, int M, const GemmTpArgs* tp);
 void gemv_simt_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, bool out_f32, const float* bias,

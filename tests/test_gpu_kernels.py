@@ -702,3 +702,78 @@ def test_persistent_prefill_gemm(N, K, M):
     ref_y = x.float() @ wd.t()
     assert _rel(y.cpu().float(), ref_y) < 1e-2 and _rel(y32.cpu(), ref_y + bias) < 1e-2
     assert _rel(y.cpu().float(), y0.cpu().float()) < 1e-2
+
+
+# The pair kernel rounds its fp32 sums to bf16 once: 2^-9 per value at most, about 1.7e-3 in the 2-norm; JQ4 weights are products rounded to
+# bf16 twice on top (scale, then nibble times scale): another 1.4e-3. 4e-3 holds both.
+@pytest.mark.parametrize("M,N,K", [(1, 256, 64), (255, 264, 64), (257, 520, 192), (300, 512, 2592), (1030, 1096, 416), (2049, 512, 1280)])
+@pytest.mark.parametrize("q4", [True, False])
+def test_pair_gemm_edges(M, N, K, q4):
+    """One row, ragged last token and weight tiles, one k step, k that ends inside a step, more tiles than pairs of SMs; bias; repeatable."""
+    qt, wd = _q4_weight(N, K, seed=N + K)
+    lw = (LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16)
+    lw.bias = torch.randn(N, device=DEV) if M % 2 else None
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    y, again = ops.linear(x, lw, impl=3), ops.linear(x, lw, impl=3)
+    torch.cuda.synchronize()
+    ops.check_status()
+    yr = x.double().cpu() @ (wd if q4 else wd.to(torch.bfloat16)).double().t() + (lw.bias.double().cpu() if lw.bias is not None else 0.0)
+    assert torch.equal(y, again) and _rel(y.cpu(), yr) < 4e-3
+
+
+@pytest.mark.parametrize("M,inter,K,act", [(2048, 256, 128, "silu"), (2100, 1408, 512, "gelu_pytorch_tanh"), (4097, 640, 320, "silu")])
+@pytest.mark.parametrize("q4", [True, False])
+def test_pair_gemm_gated(M, inter, K, act, q4):
+    qt, wd = _q4_weight(2 * inter, K, seed=inter)
+    lw = (LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16)
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    h = ops.linear_gated(x, lw, act)
+    torch.cuda.synchronize()
+    ops.check_status()
+    f = x.double().cpu() @ (wd if q4 else wd.to(torch.bfloat16)).double().t()
+    assert _rel(h.cpu(), ref.act_fn(act)(f[:, :inter]) * f[:, inter:]) < 6e-3  # (without the epilogue the projection is rounded once more)
+
+
+@pytest.mark.parametrize("heads,kv,norm,rope", [(4, 1, True, True), (6, 3, False, True), (3, 1, True, False)])
+@pytest.mark.parametrize("q4", [True, False])
+def test_pair_gemm_heads(heads, kv, norm, rope, q4):
+    """q | k | v epilogue: an odd number of heads (half a tile at the end), rows without a cache slot, positions behind a prefix."""
+    M, K, D = 2310, 512, 128
+    qt, wd = _q4_weight((heads + 2 * kv) * D, K, seed=heads)
+    lw = (LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16)
+    assert ops.require_ext() is not None
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    pages = M // 32 + 2
+    slots = torch.randperm(pages * 32)[:M].to(DEV)
+    pos = torch.arange(M, dtype=torch.int32, device=DEV) + 37
+    cos, sin = (t.to(DEV) for t in ref.rope_tables(D, 4096, 10000.0)) if rope else (None, None)
+    qn, kn = ((1 + 0.1 * torch.randn(D)).to(torch.bfloat16).to(DEV) for _ in range(2)) if norm else (None, None)
+    kc, vc = (torch.zeros(pages, kv, 32, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    q = ops.linear_rope_kv(x, lw, pos, slots, qn, kn, cos, sin, kc, vc, heads, kv, D, 1e-6)
+    torch.cuda.synchronize()
+    ops.check_status()
+    f = x.float() @ (wd if q4 else wd.to(torch.bfloat16).float()).to(DEV).t()
+    k2, v2 = (torch.zeros(pages, kv, 32, D, device=DEV) for _ in range(2))
+    qr = ref.qk_prepare_and_cache(f, pos.long(), slots.long(), heads, kv, D, qn, kn, 1e-6, 0.0, cos, sin, k2, v2)
+    assert _rel(q, qr.reshape(M, -1)) < 6e-3 and _rel(kc, k2) < 6e-3 and _rel(vc, v2) < 4e-3
+
+
+@pytest.mark.parametrize("E,n,K,T,k", [(4, 512, 256, 700, 2), (3, 768, 1216, 1500, 1)])
+@pytest.mark.parametrize("q4", [True, False])
+def test_pair_gemm_experts(E, n, K, T, k, q4):
+    """Work items of 256 rows that end inside a tile, unused ones at the end of the list; plain store and gated activation."""
+    e = ops.require_ext()
+    made = [_q4_weight(n, K, seed=i) for i in range(E)]
+    g = ops.GroupedLinearWeight([(LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16) for qt, wd in made])
+    x = (torch.randn(T, K) * 0.5).to(torch.bfloat16).to(DEV)
+    w, idx, counts, offsets, perm, pos = e.moe_route(torch.randn(T, E, device=DEV), k, 0, True)
+    items = e.moe_items(offsets, 0, E, 256, (T * k + 255) // 256 + E)
+    xs = e.moe_gather(x, perm, k, None, 0, 0)
+    y, h = g.run(xs, items, 256), g.run_gated(xs, items, "silu")
+    torch.cuda.synchronize()
+    ops.check_status()
+    off = offsets.tolist()
+    for i, (_, wd) in enumerate(made):
+        f = xs[off[i]:off[i + 1]].double().cpu() @ (wd if q4 else wd.to(torch.bfloat16)).double().t()
+        assert _rel(y[off[i]:off[i + 1]].cpu(), f) < 4e-3
+        assert h is not None and _rel(h[off[i]:off[i + 1]].cpu(), torch.nn.functional.silu(f[:, : n // 2]) * f[:, n // 2:]) < 6e-3
