@@ -411,20 +411,51 @@ __device__ __forceinline__ uint32_t swz(int row, int chunk) {
 // The CUDA-core decode kernel above needs one FMA per (key, dim, head) and is issue bound long before the KV stream reaches
 // the HBM rate. Here the G query heads that share a KV head are the rows of a 16 x D MMA A-operand (rows >= G are zero), so a
 // 16-key slice of K / V costs 2 * D / 8 mma.sync instead of 16 * D * G FMAs.
-//   grid (num_seqs, KV, splits), 4 warps. The warps work independently: warp w takes the 16-key slices w, w + 4, ... of the
-//   CTA's key range through its own three-stage cp.async ring (no CTA-wide barrier in the loop) and keeps its own online-
-//   softmax state; the four states are merged through shared memory at the end. A slice never straddles a page
-//   (page_size % 16 == 0), so it needs one block-table lookup.
-template <int D>
+//   grid (num_seqs, KV, splits), NW warps. The warps work independently: warp w takes the 16-key slices w, w + NW, ... of the
+//   CTA's key range through its own cp.async ring (no CTA-wide barrier in the loop) and keeps its own online-softmax state; the
+//   states are merged through shared memory at the end. A slice never straddles a page (page_size % 16 == 0); lanes look up the
+//   rows of the next 32 slices at once, so that no copy waits for the block table.
+// What bounds it: the K / V stream. NW 4 with three stages and two CTAs per SM for heads up to 128; 6 warps with two stages for 256-wide heads
+// (192 KB of rings; with four warps and three stages the chain of one slice set the pace: 128 x 1920 keys x 8 heads 617 us, now 333, of
+// 303 at the copy rate). (The splits as a thread-block cluster that merges through distributed shared memory, instead of a second launch:
+// 106 us against 101 at 64 x 2176 keys, 10 against 6 at one sequence, because the CTAs of a cluster start and leave together. Not kept.)
+template <int D, int NW>
 struct DecodeMma {
-  static constexpr int kStages = 3;
+  static constexpr int kStages = D > 128 ? 2 : 3;
   static constexpr int kSliceBytes = 16 * D * 2;                 // K or V of one slice
   static constexpr int kWarpBytes = kStages * 2 * kSliceBytes;   // ring of one warp
   static constexpr int kQBytes = 16 * D * 2;                     // D > 128: the query tile stays in shared memory
-  static constexpr int kRing = 4 * kWarpBytes;
-  static constexpr int kMerge = 4 * 16 * (D + 2) * 4;            // per warp: 16 rows x (D + m + l) fp32 (aliases the rings)
+  static constexpr int kRing = NW * kWarpBytes;
+  static constexpr int kMerge = NW * 16 * (D + 2) * 4;           // per warp: 16 rows x (D + m + l) fp32 (aliases the rings)
   static constexpr int kBytes = (kRing > kMerge ? kRing : kMerge) + (D > 128 ? kQBytes : 0);
 };
+
+// cap * tanh(s / cap) of a lane's eight scores: the series up to x^11 where all of the warp's arguments are small, 1 - 2 / (e^2x + 1) otherwise
+// (tanhf's division and branch per score were a third of the slice's instructions)
+__device__ __forceinline__ void softcap_slice(float (&f)[2][4], float cap) {
+  const float inv = 1.f / cap;
+  float mx = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(f[i >> 2][i & 3]));
+  if (__all_sync(0xffffffffu, mx * inv < 0.35f)) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float x = f[i >> 2][i & 3] * inv, x2 = x * x;
+      float p = fmaf(x2, -1382.f / 155925.f, 62.f / 2835.f);
+      p = fmaf(x2, p, -17.f / 315.f);
+      p = fmaf(x2, p, 2.f / 15.f);
+      p = fmaf(x2, p, -1.f / 3.f);
+      p = fmaf(x2, p, 1.f);
+      f[i >> 2][i & 3] = f[i >> 2][i & 3] * p;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float e = __expf(2.f * f[i >> 2][i & 3] * inv);
+      f[i >> 2][i & 3] = cap - __fdividef(2.f * cap, e + 1.f);
+    }
+  }
+}
 
 // EXT 1: head widths below the tile width D, groups of more than 16 heads, kept first keys. Without it those are compile-time constants (as
 // run-time values they cost the plain kernel a tenth of its speed: the loop is paced by its address arithmetic). EXT 1 and 2: the options
@@ -436,15 +467,15 @@ struct DecodeOptions {
 };
 template <>
 struct DecodeOptions<0> {};
-template <int D, int EXT>
-__global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kernel(
+template <int D, int EXT, int NW>
+__global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode_attn_mma_kernel(
     const __nv_bfloat16* __restrict__ q, long long q_stride, const __nv_bfloat16* __restrict__ k_cache,
     const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_tables, int bt_stride,
     const int* __restrict__ ctx_lens, __nv_bfloat16* __restrict__ out, float* part_o, float* part_ml, int* __restrict__ arrivals,
     int H, int KV, int page_size, float scale, float softcap, int window, int splits, const DecodeOptions<EXT> opt) {
   pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
   pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
-  using L = DecodeMma<D>;
+  using L = DecodeMma<D, NW>;
   constexpr int CPR = D / 8;  // 16-byte chunks per row
   extern __shared__ __align__(128) uint8_t msm[];
   int dk = D, dv = D, keep_first = 0;
@@ -474,7 +505,7 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
 
   // ---- query A-fragments: registers (D <= 128) or a swizzled shared tile read with ldmatrix (D = 256)
   uint32_t qa[D <= 128 ? D / 16 : 1][4];
-  uint8_t* sQ = msm + (L::kRing > L::kMerge ? L::kRing : L::kMerge);
+  uint8_t* sQ = msm + (L::kBytes - L::kQBytes);
   if constexpr (D <= 128) {
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) {
@@ -485,7 +516,7 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
       qa[ks][3] = g + 8 < G && d0 + 8 < dk ? *reinterpret_cast<const uint32_t*>(qrow + (g + 8) * dk + d0 + 8) : 0u;
     }
   } else {
-    for (int c = tid; c < 16 * CPR; c += 128) {
+    for (int c = tid; c < 16 * CPR; c += NW * 32) {
       const int r = c / CPR, cc = c % CPR;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < G && cc * 8 < dk) v = *reinterpret_cast<const uint4*>(qrow + r * dk + cc * 8);
@@ -495,11 +526,18 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
   }
 
   auto slice_at = [&](int i) { return EXT == 1 && i < sl_kept ? i : i + sl_skip; };
-  auto load_slice = [&](int i, int stage) {
+  const int first = s0 + warp;
+  const int n_mine = first < s1 ? (s1 - first + NW - 1) / NW : 0;
+  const int per_page = page_size / 16;
+  int my_row = 0;  // cache row of slice (j & ~31) + lane of this warp
+  auto load_slice = [&](int j, int stage) {
     // 16 keys x D of K and V: 2 * 16 * CPR chunks over 32 lanes (zeros behind the real widths)
-    const int key0 = slice_at(i) * 16;
-    const int page = block_tables[static_cast<long long>(b) * bt_stride + key0 / page_size];
-    const long long row0 = (static_cast<long long>(page) * KV + kvh) * page_size + key0 % page_size;
+    if ((j & 31) == 0 && j + lane < n_mine) {
+      const int sl = slice_at(first + NW * (j + lane));
+      my_row = (block_tables[static_cast<long long>(b) * bt_stride + sl / per_page] * KV + kvh) * page_size + sl % per_page * 16;
+    }
+    const int key0 = slice_at(first + NW * j) * 16;
+    const long long row0 = __shfl_sync(0xffffffffu, my_row, j & 31);
     const __nv_bfloat16 *kb = k_cache + row0 * dk, *vb = v_cache + row0 * dv;
     const uint32_t kdst = ring_u + stage * 2 * L::kSliceBytes, vdst = kdst + L::kSliceBytes;
 #pragma unroll
@@ -523,39 +561,44 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
 #pragma unroll
   for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-  const int first = s0 + warp;
-  const int n_mine = first < s1 ? (s1 - first + 3) / 4 : 0;
 #pragma unroll
   for (int j = 0; j < L::kStages - 1; ++j) {
-    if (j < n_mine) load_slice(first + 4 * j, j);
+    if (j < n_mine) load_slice(j, j);
     cp_async_commit();
   }
   for (int j = 0; j < n_mine; ++j) {
     const int stage = j % L::kStages;
-    if (j + L::kStages - 1 < n_mine) load_slice(first + 4 * (j + L::kStages - 1), (j + L::kStages - 1) % L::kStages);
+    if (j + L::kStages - 1 < n_mine) load_slice(j + L::kStages - 1, (j + L::kStages - 1) % L::kStages);
     cp_async_commit();
     cp_async_wait<L::kStages - 1>();
     __syncwarp();
-    const int key0 = slice_at(first + 4 * j) * 16;
+    const int key0 = slice_at(first + NW * j) * 16;
     const uint32_t kbase = ring_u + stage * 2 * L::kSliceBytes, vbase = kbase + L::kSliceBytes;
     // S (16 heads x 16 keys) = Q K^T
-    float sc[2][4];
+    float sc[2][4], sd[2][4];  // (two chains of products: one of D / 16 dependent MMAs is what a warp would wait for)
 #pragma unroll
-    for (int i = 0; i < 2; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
+    for (int i = 0; i < 2; ++i) {
+      sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
+      sd[i][0] = sd[i][1] = sd[i][2] = sd[i][3] = 0.f;
+    }
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) {
       uint32_t b0, b1, b2, b3;
       ldmatrix_x4(kbase + swz<D>((lane & 7) + (lane >> 4) * 8, ks * 2 + ((lane >> 3) & 1)), b0, b1, b2, b3);
+      float(&acc)[2][4] = (ks & 1) ? sd : sc;
       if constexpr (D <= 128) {
-        mma_bf16_16816(sc[0], qa[ks], b0, b1);
-        mma_bf16_16816(sc[1], qa[ks], b2, b3);
+        mma_bf16_16816(acc[0], qa[ks], b0, b1);
+        mma_bf16_16816(acc[1], qa[ks], b2, b3);
       } else {
         uint32_t a[4];
         ldmatrix_x4(smem_u32(sQ) + swz<D>((lane & 7) + ((lane >> 3) & 1) * 8, ks * 2 + (lane >> 4)), a[0], a[1], a[2], a[3]);
-        mma_bf16_16816(sc[0], a, b0, b1);
-        mma_bf16_16816(sc[1], a, b2, b3);
+        mma_bf16_16816(acc[0], a, b0, b1);
+        mma_bf16_16816(acc[1], a, b2, b3);
       }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sc[i >> 2][i & 3] = (sc[i >> 2][i & 3] + sd[i >> 2][i & 3]) * scale;
+    if (softcap > 0.f) softcap_slice(sc, softcap);
     // scale, softcap, mask (keys outside [first_key, ctx)), online softmax per head row
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -563,7 +606,7 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int key = key0 + nt * 8 + 2 * t4 + (e & 1);
-        float v = softcap_apply(sc[nt][e] * scale, softcap);
+        float v = sc[nt][e];
         v = (key < ctx && (key >= first_key || (EXT == 1 && key < kept))) ? v : -INFINITY;
         sc[nt][e] = v;
         mx[e >> 1] = fmaxf(mx[e >> 1], v);
@@ -621,7 +664,7 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
   cp_async_wait<0>();
   __syncthreads();  // every warp is done with its ring: the merge area aliases the rings
 
-  // ---- merge the four warps: each stores its rows < G as [row][D + 2] = O (unnormalised), m, l
+  // ---- merge the warps: each stores its rows < G as [row][D + 2] = O (unnormalised), m, l
   float* mg = reinterpret_cast<float*>(msm);
   {
     float* mine = mg + static_cast<size_t>(warp) * 16 * (D + 2);
@@ -644,38 +687,42 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
   }
   __syncthreads();
   const int dv2 = dv / 2;
-  for (int idx = tid; idx < G * dv2; idx += 128) {
+  // row r, columns d and d + 1 of the output from the weighted sums of all keys
+  auto finish = [&](int r, int d, float m, float n0, float n1, float den) {
+    const int h = h0 + r;
+    if constexpr (EXT != 0) {
+      if (opt.x.sink != nullptr) den += __expf(opt.x.sink[h] - m);  // relative to the maximum
+    }
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+    if constexpr (EXT != 0) {
+      const AttnExtra& x = opt.x;
+      const __nv_bfloat16* gate = static_cast<const __nv_bfloat16*>(x.gate);
+      n0 *= attn_gate(x, gate, b, h, h * dv + d);
+      n1 *= attn_gate(x, gate, b, h, h * dv + d + 1);
+      const long long pitch = x.out_pitch > 0 ? x.out_pitch : static_cast<long long>(H) * dv;
+      *reinterpret_cast<uint32_t*>(out + b * pitch + h * dv + d) = pack_bf162(n0 * inv, n1 * inv);
+    } else {
+      *reinterpret_cast<uint32_t*>(out + (static_cast<long long>(b) * H + h) * dv + d) = pack_bf162(n0 * inv, n1 * inv);
+    }
+  };
+  for (int idx = tid; idx < G * dv2; idx += NW * 32) {
     const int r = idx / dv2, d = (idx % dv2) * 2;
     float m = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) m = fmaxf(m, mg[(w * 16 + r) * (D + 2) + D]);
+    for (int w = 0; w < NW; ++w) m = fmaxf(m, mg[(w * 16 + r) * (D + 2) + D]);
     float n0 = 0.f, n1 = 0.f, den = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
+    for (int w = 0; w < NW; ++w) {
       const float* row = mg + (w * 16 + r) * (D + 2);
       const float wt = (row[D] == -INFINITY) ? 0.f : __expf(row[D] - m);
       n0 += wt * row[d];
       n1 += wt * row[d + 1];
       den += wt * row[D + 1];
     }
-    const int h = h0 + r;
     if (splits == 1) {
-      if constexpr (EXT != 0) {
-        if (opt.x.sink != nullptr) den += __expf(opt.x.sink[h] - m);  // relative to the maximum
-      }
-      const float inv = den > 0.f ? 1.f / den : 0.f;
-      if constexpr (EXT != 0) {
-        const AttnExtra& x = opt.x;
-        const __nv_bfloat16* gate = static_cast<const __nv_bfloat16*>(x.gate);
-        n0 *= attn_gate(x, gate, b, h, h * dv + d);
-        n1 *= attn_gate(x, gate, b, h, h * dv + d + 1);
-        const long long pitch = x.out_pitch > 0 ? x.out_pitch : static_cast<long long>(H) * dv;
-        *reinterpret_cast<uint32_t*>(out + b * pitch + h * dv + d) = pack_bf162(n0 * inv, n1 * inv);
-      } else {
-        *reinterpret_cast<uint32_t*>(out + (static_cast<long long>(b) * H + h) * dv + d) = pack_bf162(n0 * inv, n1 * inv);
-      }
+      finish(r, d, m, n0, n1, den);
     } else {
-      const long long base = (static_cast<long long>(b) * H + h) * splits + sp;
+      const long long base = (static_cast<long long>(b) * H + h0 + r) * splits + sp;
       *reinterpret_cast<float2*>(part_o + base * dv + d) = make_float2(n0, n1);
       if (d == 0) {
         part_ml[base * 2] = m;
@@ -704,7 +751,7 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
   float* w_s = mg;  // [G][splits] weights, then [G] denominators (the warp-merge area is free again)
   float* den_s = mg + G * splits;
   if (G * (splits + 1) <= L::kMerge / 4) {
-    for (int r = warp; r < G; r += 4) {
+    for (int r = warp; r < G; r += NW) {
       const long long base = (static_cast<long long>(b) * H + kvh * G + r) * splits;
       float m = -INFINITY;
       for (int s2 = lane; s2 < splits; s2 += 32) m = fmaxf(m, __ldcg(part_ml + (base + s2) * 2));
@@ -720,7 +767,7 @@ __global__ void __launch_bounds__(128, (D <= 128 ? 2 : 1)) decode_attn_mma_kerne
       if (lane == 0) den_s[r] = den;
     }
     __syncthreads();
-    for (int idx = tid; idx < G * (D / 2); idx += 128) {
+    for (int idx = tid; idx < G * (D / 2); idx += NW * 32) {
       const int r = idx / (D / 2), d = (idx % (D / 2)) * 2;
       const int h = kvh * G + r;
       const long long base = (static_cast<long long>(b) * H + h) * splits;
@@ -743,17 +790,18 @@ template <int D, int EXT>
 static int launch_decode_mma_t(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride,
                                const int* ctx, void* out, float* po, float* pml, int* arrivals, int B, int H, int KV, int page,
                                float scale, float cap, int window, int splits, cudaStream_t st, int dk = D, int dv = D, AttnExtra x = {}) {
-  using L = DecodeMma<D>;
+  constexpr int NW = D > 128 ? 6 : 4;
+  using L = DecodeMma<D, NW>;
   // the in-kernel merge keeps its weights in the warp-merge area of shared memory
   if (splits > 1 && (H / KV) * (splits + 1) > L::kMerge / 4) arrivals = nullptr;
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
-    cudaFuncSetAttribute(decode_attn_mma_kernel<D, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+    cudaFuncSetAttribute(decode_attn_mma_kernel<D, EXT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
   }
   dim3 grid(B, KV * ((H / KV + 15) / 16), splits);
   DecodeOptions<EXT> opt;
   if constexpr (EXT != 0) opt = {dk, dv, x};
-  launch_pdl(decode_attn_mma_kernel<D, EXT>, dim3(grid), dim3(128), L::kBytes, st, static_cast<const __nv_bfloat16*>(q), q_stride,
+  launch_pdl(decode_attn_mma_kernel<D, EXT, NW>, dim3(grid), dim3(NW * 32), L::kBytes, st, static_cast<const __nv_bfloat16*>(q), q_stride,
                                                           static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(vc), bt,
                                                           bt_stride, ctx, static_cast<__nv_bfloat16*>(out), po, pml, arrivals, H, KV, page, scale,
                                                           cap, window, splits, opt);
@@ -819,8 +867,8 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(const TIO* __restrict__ 
                                                         const TIO* __restrict__ v_cache, const int* __restrict__ bt, int bt_stride,
                                                         const int* __restrict__ row_seq, const int* __restrict__ positions, TIO* __restrict__ out, int H, int KV,
                                                         int dk, int dv, int page, float scale, float softcap, int window, bool wide, const AttnExtra x) {
-  pdl_wait();
-  pdl_trigger();
+  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
+  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
   extern __shared__ float rsm[];  // q [dk] | accumulators [4][dv]
   __shared__ float ml[4][2];
   const int t = blockIdx.x, h = blockIdx.y, kvh = h / (H / KV);
