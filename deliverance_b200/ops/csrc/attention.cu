@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(
     float* __restrict__ part_o,               // [num_seqs, H, splits, D]
     float* __restrict__ part_ml,              // [num_seqs, H, splits, 2]
     int H, int KV, int page_size, float scale, float softcap, int window, int splits) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   constexpr int PARTS0 = D * GP / 64;
   constexpr int PARTS = PARTS0 < 8 ? 8 : (PARTS0 > 32 ? 32 : PARTS0);  // threads that share one key
   constexpr int EPT = D / PARTS;                                       // query elements per thread and head
@@ -263,8 +263,8 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
                                     const std::conditional_t<EXT, AttnExtra, NoExtra> x) {
   __shared__ float w_s[256];
   __shared__ float red[2][8];
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x, lane = d & 31, wp = d >> 5, nw = (blockDim.x + 31) >> 5;
   const long long base = (static_cast<long long>(b) * H + h) * splits;
   float logit = 0.f, sink = -INFINITY;  // (read here: their latency passes under the reductions)
@@ -473,8 +473,8 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
     const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_tables, int bt_stride,
     const int* __restrict__ ctx_lens, __nv_bfloat16* __restrict__ out, float* part_o, float* part_ml, int* __restrict__ arrivals,
     int H, int KV, int page_size, float scale, float softcap, int window, int splits, const DecodeOptions<EXT> opt) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   using L = DecodeMma<D, NW>;
   constexpr int CPR = D / 8;  // 16-byte chunks per row
   extern __shared__ __align__(128) uint8_t msm[];
@@ -867,8 +867,8 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(const TIO* __restrict__ 
                                                         const TIO* __restrict__ v_cache, const int* __restrict__ bt, int bt_stride,
                                                         const int* __restrict__ row_seq, const int* __restrict__ positions, TIO* __restrict__ out, int H, int KV,
                                                         int dk, int dv, int page, float scale, float softcap, int window, bool wide, const AttnExtra x) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   extern __shared__ float rsm[];  // q [dk] | accumulators [4][dv]
   __shared__ float ml[4][2];
   const int t = blockIdx.x, h = blockIdx.y, kvh = h / (H / KV);
@@ -941,8 +941,8 @@ __global__ void __launch_bounds__(128) prefill_attn_kernel(
     const int* __restrict__ q_start, const int* __restrict__ q_len, const int* __restrict__ ctx_lens,
     const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, __nv_bfloat16* __restrict__ out,  // [T, H, D]
     int H, int KV, int page_size, float scale, float softcap, int window, int causal) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   constexpr int BM = 64, BN = 64, CPR = D / 8;
   extern __shared__ __align__(128) uint8_t psm[];
   uint8_t* sQ = psm;                       // BM * D * 2

@@ -16,8 +16,8 @@ namespace dlv {
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* residual,
                                                       const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                                       int H, float eps, float offset, float res_mult) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   extern __shared__ float row[];  // H floats
   __shared__ float red[32];
   const size_t base = static_cast<size_t>(blockIdx.x) * H;
@@ -74,8 +74,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __res
 __global__ void __launch_bounds__(256) layernorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                         const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y, int H,
                                                         float eps) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   extern __shared__ float row[];
   __shared__ float red[32];
   const size_t base = static_cast<size_t>(blockIdx.x) * H;
@@ -113,8 +113,8 @@ __device__ __forceinline__ float act_apply(float g, int act) {
 // in: [T, 2*I] (gate | up), out: [T, I]; I % 8 == 0
 __global__ void __launch_bounds__(256) act_mul_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int I,
                                                       int act, long long total_vec) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total_vec) return;
   const int per_row = I / 8;
@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(256) act_mul_kernel(const __nv_bfloat16* __res
 // unary activation (MLPs without an up projection): a thread takes eight elements
 template <typename TIO>
 __global__ void __launch_bounds__(256) act_kernel(const TIO* __restrict__ in, TIO* __restrict__ out, int act, long long n) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i + 8 <= n) {
     float v[8];
@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(128) embedding_kernel(const __nv_bfloat16* __r
                                                         const __nv_bfloat16* __restrict__ pos_table, const int* __restrict__ pos,
                                                         const __nv_bfloat16* __restrict__ type_table, const int* __restrict__ types,
                                                         __nv_bfloat16* __restrict__ out, int H, int vocab, float scale) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= vocab) id = 0;  // host validates ids; never read out of the table
@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(256) rope_kv_kernel(__nv_bfloat16* __restrict_
                                                       const float* __restrict__ sin_t, __nv_bfloat16* __restrict__ k_cache,
                                                       __nv_bfloat16* __restrict__ v_cache, int T, int H, int KV, int block_size,
                                                       int rot_half, float eps, float norm_offset, int max_pos) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const int warp_global = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const int heads = H + 2 * KV;
@@ -309,8 +309,8 @@ __global__ void __launch_bounds__(128) bigram_embedding_kernel(const TIO* __rest
                                                                const int* __restrict__ prev, float* __restrict__ out, int W, int vocab, int buckets,
                                                                long long mul_prev, long long mul_cur, float scale, TIO* __restrict__ out2,
                                                                long long ld2) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= vocab) id = 0;  // host validates ids; never read out of the table
@@ -335,8 +335,8 @@ template <typename TIO>
 __global__ void __launch_bounds__(256) add_layernorm_kernel(float* __restrict__ residual, const float* __restrict__ delta, const float* __restrict__ w1,
                                                             const float* __restrict__ b1, TIO* __restrict__ y1, const float* __restrict__ w2,
                                                             const float* __restrict__ b2, TIO* __restrict__ y2, int W, int y_pitch, float eps) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   extern __shared__ __align__(16) float row[];
   __shared__ float red[32];
   const size_t base = static_cast<size_t>(blockIdx.x) * W, yb = static_cast<size_t>(blockIdx.x) * y_pitch;
@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(256) add_layernorm_kernel(float* __restrict__ 
 template <typename TIO>
 __global__ void __launch_bounds__(256) gated_act_kernel(const TIO* __restrict__ in, long long ld_in, TIO* __restrict__ out, long long ld_out, int I, int act,
                                                         long long total) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const int per_row = I / 8;
@@ -461,8 +461,8 @@ __global__ void __launch_bounds__(NT) sandwich_norm_kernel(const SandwichArgs a)
   const TSUB* sub = static_cast<const TSUB*>(a.sub);
   float v[NV][4];
   auto col = [&](int n) { return (n * NT + static_cast<int>(threadIdx.x)) * 4; };
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   auto load = [&](auto* p, int c, float* o) {
     if (a.vec) {
       if (c < W) io_ld4(p + c, o);
@@ -574,8 +574,8 @@ __global__ void __launch_bounds__(256) rope_pairs_kv_kernel(TIO* __restrict__ qk
                                                             const long long* __restrict__ slots, const float* __restrict__ cos_t,
                                                             const float* __restrict__ sin_t, TIO* __restrict__ k_cache, TIO* __restrict__ v_cache, int T, int H,
                                                             int KV, int dk, int dv, int page, int half, int max_pos) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   const int rot = (2 * half + 7) / 8, ck = dk / 8, cv = dv / 8;
   const int nq = H * rot, nk = KV * ck, per = nq + nk + KV * cv;
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -637,8 +637,8 @@ __global__ void __launch_bounds__(256) rope_pairs_kv_kernel(TIO* __restrict__ qk
 // registers when `half` is a multiple of eight and the head is one step wide (LANES); otherwise the head passes through shared memory.
 template <typename TIO, int LPH, bool LANES>
 __global__ void __launch_bounds__(256) rope_heads_kv_kernel(const RopeHeadsArgs a) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   extern __shared__ __align__(16) float hsm[];
   const bool tied = a.off_v == a.off_k;
   const int heads = a.H + a.KV + (tied ? 0 : a.KV);

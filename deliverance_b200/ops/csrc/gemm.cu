@@ -611,6 +611,57 @@ void gemm_tc_run_grouped_act(const GemmWeightDesc* w, int n_per_expert, const vo
 #undef DLV_LAUNCH
 }
 
+__device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// ------------------------------------------------------------------------------------------------ one row of bf16 weights
+// One token row against a dense weight: a warp per weight row, 16 bytes per lane and chunk of 256 elements. Bound by the weight stream, and at
+// a few megabytes by how early and how widely it starts: eight chunks per lane are in flight, the first eight (and L2 prefetches of the rest)
+// from before the wait for the kernel in front. gemv_simt_kernel, which it replaces here, had one or two chunks in flight behind an
+// ordinary launch (tinyllama's 22 layers at one token: 638 us of GEMVs for 2.07 GB).
+constexpr int kGemvChunks = 8;
+template <bool OUTF>
+__global__ void __launch_bounds__(128) gemv_bf16_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x, void* __restrict__ out,
+                                                        const float* __restrict__ bias, int N, int K) {
+  pdl_trigger();
+  const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const __nv_bfloat16* row = w + static_cast<size_t>(min(n, N - 1)) * K;
+  uint4 wv[kGemvChunks];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < kGemvChunks; ++i) {
+      const int k = k0 + i * 256 + lane * 8;
+      wv[i] = k < K ? __ldg(reinterpret_cast<const uint4*>(row + k)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  fetch(0);
+  for (int k = kGemvChunks * 256 + lane * 8; k < K; k += 256) l2_prefetch(row + k);
+  pdl_wait();
+  if (n >= N) return;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int k0 = 0; k0 < K; k0 += kGemvChunks * 256) {
+    if (k0 > 0) fetch(k0);
+#pragma unroll
+    for (int i = 0; i < kGemvChunks; ++i) {
+      const int k = k0 + i * 256 + lane * 8;
+      if (k < K) {
+        const uint4 xv = *reinterpret_cast<const uint4*>(x + k);
+        const uint32_t wu[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w}, xu[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 a = unpack_bf162(wu[e]), b = unpack_bf162(xu[e]);
+          acc[e] += a.x * b.x + a.y * b.y;
+        }
+      }
+    }
+  }
+  const float sum = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+  if (lane == 0) {
+    const float v = sum + (bias != nullptr ? bias[n] : 0.f);
+    if (OUTF) static_cast<float*>(out)[n] = v;
+    else static_cast<__nv_bfloat16*>(out)[n] = f2bf(v);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ CUDA-core GEMV
 // One warp per weight row, MT tokens. fp32 accumulation; JQ4 blocks are expanded in registers.
 template <int MT, bool Q4>
@@ -705,8 +756,8 @@ template <int MT, bool Q4>
 __global__ void __launch_bounds__(128) gemv_grouped_kernel(const void* __restrict__ wdata, const __nv_bfloat16* __restrict__ x, int ldx,
                                                            __nv_bfloat16* __restrict__ out, int ldo, int N, int K,
                                                            const int4* __restrict__ items) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   const int4 it = items[blockIdx.y];
   if (it.x < 0) return;
   const int lane = threadIdx.x & 31;
@@ -825,8 +876,8 @@ __global__ void __launch_bounds__(kGemvMmaWarps * 32) gemv_grouped_mma_kernel(co
                                                                                int row_div) {
   // row_map (optional): grouped row r reads the token row row_map[r] / row_div of x instead of row r, i.e. x is the ungathered
   // [tokens, K] activation and row_map the grouping permutation (the copy into expert order never happens)
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   const int4 it = items[blockIdx.y];
   if (it.x < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
@@ -920,7 +971,6 @@ __global__ void __launch_bounds__(S * 32, gemv_resident<S, TG>()) gemv_dense_mma
                                                                                          const float* __restrict__ bias, int M, int N, int K) {
   constexpr int kGemvSplit = S;
   __shared__ float part[kGemvSplit][TG][32][4];
-  pdl_wait();
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   constexpr int RW = ACT > 0 ? 8 : 16;
@@ -933,6 +983,17 @@ __global__ void __launch_bounds__(S * 32, gemv_resident<S, TG>()) gemv_dense_mma
   const uint8_t* baseB = wdata + static_cast<size_t>(nB >> 7) * kb_total * kQ4StageBytes;
   const uint32_t offA = rA * 64 + ((c ^ ((rA >> 1) & 3)) << 4), offB = rB * 64 + ((c ^ ((rB >> 1) & 3)) << 4);
   const uint32_t scA = 8192 + rA * 16 + c * 4, scB = 8192 + rB * 16 + c * 4;
+  // The weights do not depend on the kernel in front: the CTA's share (16 rows) is on its way to L2 while that kernel finishes.
+  for (int kb = warp; kb < kb_total; kb += kGemvSplit) {
+    const size_t so = static_cast<size_t>(kb) * kQ4StageBytes;
+    l2_prefetch(baseA + so + offA);
+    l2_prefetch(baseB + so + offB);
+    if (c == 0) {
+      l2_prefetch(baseA + so + scA);
+      l2_prefetch(baseB + so + scB);
+    }
+  }
+  pdl_wait();
   bool tok[TG];
   const __nv_bfloat16* xrow[TG];
   float acc[TG][4];
@@ -1119,6 +1180,12 @@ bool gemv_grouped_act_run(const GemmWeightDesc* w, int n_per_expert, const void*
 void gemv_simt_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, bool out_f32, const float* bias,
                    cudaStream_t st) {
   const unsigned grid = (w->N + 3) / 4;
+  if (M == 1 && !w->is_q4 && (reinterpret_cast<uintptr_t>(w->data) & 15) == 0) {  // (K % 8 == 0 and aligned x rows: checked at the entry points)
+    const __nv_bfloat16 *wp = static_cast<const __nv_bfloat16*>(w->data), *xp = static_cast<const __nv_bfloat16*>(x);
+    if (out_f32) launch_pdl(gemv_bf16_kernel<true>, dim3(grid), dim3(128), 0, st, wp, xp, out, bias, w->N, w->K);
+    else launch_pdl(gemv_bf16_kernel<false>, dim3(grid), dim3(128), 0, st, wp, xp, out, bias, w->N, w->K);
+    return;
+  }
   for (int m0 = 0; m0 < M; m0 += 4) {
     const int mt = M - m0 < 4 ? M - m0 : 4;
     const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x) + static_cast<size_t>(m0) * ldx;

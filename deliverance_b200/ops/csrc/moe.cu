@@ -142,8 +142,8 @@ __device__ __forceinline__ void moe_topk_token(const float* __restrict__ row, in
 // one warp per token
 __global__ void __launch_bounds__(256) moe_topk_kernel(const float* __restrict__ logits, int T, int E, int k, const MoeRouting rt,
                                                        float* __restrict__ w_out, int* __restrict__ idx_out, int* __restrict__ counts) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const float* __re
                                                                float* __restrict__ w_out, int* __restrict__ idx_out, int* __restrict__ counts,
                                                                int* __restrict__ offsets, int* __restrict__ perm, int* __restrict__ pos, int e0,
                                                                int ne, int bn, int max_items, int4* __restrict__ items) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   extern __shared__ int rs[];
   const int P = T * k;
   int* idx_s = rs;              // [P] expert of every (token, slot) pair
@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const float* __re
 // pos[t * k + j] = row of that pair in the grouped order; perm[row] = t * k + j.
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ idx, const int* __restrict__ counts, int T, int E, int k,
                                                         int* __restrict__ offsets, int* __restrict__ perm, int* __restrict__ pos) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   extern __shared__ int sh[];  // E + 1 offsets
   if (threadIdx.x == 0) {
     int acc = 0;
@@ -277,8 +277,8 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
 constexpr int kSortChunk = 1024;
 constexpr int kSortSerialMaxPairs = 1024;  // up to here the single-CTA kernel is used
 __global__ void __launch_bounds__(256) moe_chunk_hist_kernel(const int* __restrict__ idx, int P, int E, int* __restrict__ chunk_hist) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   extern __shared__ int hs[];  // [E]
   for (int e = threadIdx.x; e < E; e += blockDim.x) hs[e] = 0;
   __syncthreads();
@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(256) moe_chunk_hist_kernel(const int* __restri
 // chunk_hist [C, E]: counts on entry, first grouped row of the (chunk, expert) on exit
 __global__ void __launch_bounds__(1024) moe_chunk_scan_kernel(const int* __restrict__ counts, int E, int C, int* __restrict__ offsets,
                                                               int* __restrict__ chunk_hist) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   extern __shared__ int sh[];  // [E + 1]
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 32) {
@@ -319,8 +319,8 @@ __global__ void __launch_bounds__(1024) moe_chunk_scan_kernel(const int* __restr
 }
 __global__ void __launch_bounds__(32) moe_chunk_rank_kernel(const int* __restrict__ idx, int P, int E, const int* __restrict__ chunk_base,
                                                             int* __restrict__ perm, int* __restrict__ pos) {
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  pdl_trigger();
   extern __shared__ int rk[];  // [E] running row per expert, then [kSortChunk] the chunk's expert ids
   int* run_s = rk;
   int* idx_s = rk + E;
@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(32) moe_chunk_rank_kernel(const int* __restric
 
 __global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ perm, int k, int row_vecs,
                                                          uint4* __restrict__ xs, const int* __restrict__ offsets, int e0, int ne) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const int row = blockIdx.x;
   if (offsets != nullptr && (row < offsets[e0] || row >= offsets[e0 + ne])) return;  // another rank's expert
   const int t = perm[row] / k;
@@ -361,8 +361,8 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict
 __global__ void __launch_bounds__(128) moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const int* __restrict__ pos,
                                                           const float* __restrict__ w, int k, int H, __nv_bfloat16* __restrict__ out,
                                                           const int* __restrict__ offsets, int e0, int ne) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   const int t = blockIdx.x;
   const int lo = offsets != nullptr ? offsets[e0] : 0, hi = offsets != nullptr ? offsets[e0 + ne] : 0x7fffffff;
   for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
@@ -436,8 +436,8 @@ void launch_moe_combine(const void* ys, const int* pos, const float* w, int T, i
 // rows, in expert order; the rest of the `max_items` slots get expert = -1. Single CTA (at most a few hundred items).
 __global__ void __launch_bounds__(256) moe_items_kernel(const int* __restrict__ offsets, int e0, int ne, int bn, int max_items,
                                                         int4* __restrict__ items) {
-  pdl_wait();     // no-op unless launched with programmatic stream serialization: the kernel in front has completed
-  pdl_trigger();  // the next kernel may start its prologue (and a GEMM its weight prefetch) under this kernel's tail
+  pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
+  pdl_wait();
   __shared__ int first[1025];
   if (threadIdx.x == 0) {
     int acc = 0;
