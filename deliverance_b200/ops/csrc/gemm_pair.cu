@@ -131,11 +131,6 @@ __global__ void __launch_bounds__(256) q4_expand_kernel(const uint8_t* __restric
   }
 }
 
-// Barrier of both CTAs, every thread for itself: the copy loops and the drain leave warps in pieces, which the .aligned form does not allow.
-__device__ __forceinline__ void pair_sync() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
 struct Tile {
   int m0, m_lim, n_tile, expert;  // m0 < 0: nothing to do
 };
@@ -185,7 +180,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == 2) tmem_alloc_pair(smem_u32(tmem_slot), 512);
   tc_fence_before();
   __syncthreads();
-  pair_sync();  // the peer's barriers exist before anything arrives on them
+  cluster_sync_all();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   pdl_trigger();  // (behind the set-up: the next kernel's blocks are not to come between the two CTAs of a pair and their tensor memory)
   const uint32_t tmem_base = *tmem_slot;
@@ -474,6 +469,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           pos = pos < 0 ? 0 : (pos >= a.max_pos ? a.max_pos - 1 : pos);
           slot = a.slots != nullptr ? a.slots[m] : -1;
         }
+        __syncwarp();
         const size_t cache_row = slot >= 0 ? static_cast<size_t>(slot / a.block_size) * a.kv_heads * a.block_size + static_cast<size_t>(slot % a.block_size) : 0;
 #pragma unroll 1
         for (int hh = 0; hh < 2; ++hh) {
@@ -563,7 +559,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
 
   // ---------------- teardown ----------------
-  __syncwarp();  // single lanes ran the copy loops; the barriers below want whole warps
+  __syncwarp();  // single lanes ran the copy loops
   if (*abort_flag) {
     // a wait ran out: copies that are still in flight get time to land before their shared memory goes away
     const unsigned long long t0 = globaltimer_ns();
@@ -572,13 +568,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  pair_sync();  // no CTA leaves while the pair's MMAs or arrivals may still touch its shared memory
+  cluster_sync_all();  // no CTA leaves while the pair's MMAs or arrivals may still touch its shared memory
   if (warp == 2) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, 512);
   }
   __syncwarp();
-  pair_sync();  // the release of a pair's tensor memory involves both CTAs: neither leaves before both have asked for it
+  cluster_sync_all();  // the release of a pair's tensor memory involves both CTAs: neither leaves before both have asked for it
 }
 
 template <bool Q4, int EPI>
@@ -636,11 +632,8 @@ void launch_pair(const GemmWeightDesc* w, const void* x, int ldx, int rows, Pair
   cfg.blockDim = dim3(PairSmem<Q4>::kThreads);
   cfg.dynamicSmemBytes = PairSmem<Q4>::kBytes;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = g_pdl_enabled ? 1 : 0;
-  cfg.attrs = attr;
-  cfg.numAttrs = expanded != nullptr ? 0 : 1;  // behind an expansion there is nothing to start early on
+  // In ordinary stream order: pairs of CTAs that started under the kernel in front did not always come to an end (and a prompt-size product has
+  // little to gain from its first microseconds).
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<Q4, EPI>, map_w, map_x, p);
   if (e != cudaSuccess) throw std::runtime_error(std::string("pair gemm launch: ") + cudaGetErrorString(e));
 }

@@ -161,8 +161,15 @@ __device__ __forceinline__ uint32_t q4_pair_to_bf162(uint32_t nib4, uint32_t sel
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Role code leaves warps in pieces (single lanes copy, every lane polls a barrier for itself), and with a uniform warp index nothing joins them
+// again by itself: the .aligned barriers would count such a warp wrongly and never open. So the cluster barrier is the form that every thread
+// executes for itself, and the named barrier of the epilogue warps comes behind a __syncwarp.
 __device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void epilogue_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 1, 512;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -213,7 +220,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
     split = j % p.tail_splits;
     splits = p.tail_splits;
     kb_per_split = p.tail_kb_per_split;
-    ws_tile = j / p.tail_splits;
+    ws_tile = (j / p.tail_splits) * p.m_tiles + m_tile;
   }
   const int n0 = n_tile * kGemmBM;
   int m0 = m_tile * BN, m_lim = p.M, w_tile = n_tile, w_row0 = n0;
@@ -444,6 +451,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
         // the tensor-memory stage is free once the MMAs of k-block i - NA have retired
         if (!mbar_wait(smem_u32(&bar_a_empty[sa]), ((i / NA) & 1) ^ 1, abort_flag, p.status)) { ok = false; break; }
         tc_fence_after();
+        __syncwarp();  // (every lane polled for itself; the stores below are warp-wide)
         const uint32_t tdst = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + L::kTmemA + sa * kGemmTmemAStage;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
@@ -475,7 +483,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
     if (ok) ok = mbar_wait(smem_u32(bar_acc), 0, abort_flag, p.status);
     // All 512 threads reach this barrier; afterwards the abort flag gives a CTA-uniform decision (it is only ever
     // raised before the accumulator barrier can complete), so the named barriers below never miss a thread.
-    asm volatile("bar.sync 1, 512;" ::: "memory");
+    epilogue_sync();
     ok = (*abort_flag == 0);
     if (ok) {
       tc_fence_after();
@@ -505,8 +513,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
         }
       }
     }
-    if (splits == 1 || !p.cluster_reduce) asm volatile("bar.sync 1, 512;" ::: "memory");
+    if (splits == 1 || !p.cluster_reduce) epilogue_sync();
   }
+  __syncwarp();
   // ---------------- reduce over the split-K cluster (distributed shared memory) and store ----------------
   const bool clustered = splits > 1 && p.cluster_reduce;
   if (clustered) cluster_sync_all();  // every CTA of the cluster has its partial tile in shared memory (or is aborting)
@@ -523,12 +532,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
       for (int col = csel; col < BN; col += 16)
         *reinterpret_cast<float4*>(part + col * kGemmBM + row4) = *reinterpret_cast<const float4*>(stage + col * kGemmBM + row4);
       __threadfence();
-      asm volatile("bar.sync 1, 512;" ::: "memory");
+      epilogue_sync();
       if (t == 0) {
         const int old = atomicAdd(&p.counters[tile_id], 1);
         *s_last = (old == splits - 1) ? 1 : 0;
       }
-      asm volatile("bar.sync 1, 512;" ::: "memory");
+      epilogue_sync();
       if (*s_last) __threadfence();
     }
     const bool do_store = splits == 1 || p.cluster_reduce || *s_last;
@@ -717,7 +726,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
         }
       }
       __threadfence_system();
-      asm volatile("bar.sync 1, 512;" ::: "memory");
+      epilogue_sync();
       // every CTA of the tile (all splits of a cluster) counts once at every rank that owns some of the tile's rows: an owner
       // expects n_tiles * (m-tiles that overlap its rows) * splits publications per source and launch
       const int o_lo = m0 / p.tp_rows, o_hi = (min(m0 + BN, m_lim) - 1) / p.tp_rows;
@@ -757,7 +766,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
         }
       }
       __threadfence_system();
-      asm volatile("bar.sync 1, 512;" ::: "memory");
+      epilogue_sync();
       if (t < 32) {
         // One lane per peer: the release-adds (each carries a system-scope fence) and the flag waits of the tp_size peers run
         // side by side; issued by a single thread they cost tp_size serial fence round trips (measured: 8 ranks, +20 us).
@@ -776,7 +785,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
           *s_last = (all && p.tp_mode == 0) ? 1 : 0;
         }
       }
-      asm volatile("bar.sync 1, 512;" ::: "memory");
+      epilogue_sync();
       if (*s_last && n + 3 < p.N) {
         const __nv_bfloat16* rbase = reinterpret_cast<const __nv_bfloat16*>(p.tp_recv[p.tp_rank]) + par_off;
         for (int col = static_cast<int>(me) + stride * csel; col < BN; col += stride * 16) {
@@ -792,7 +801,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
         }
       }
       // launch bookkeeping: the last CTA of the grid to get here advances the launch counter (flips the parity)
-      asm volatile("bar.sync 1, 512;" ::: "memory");
+      epilogue_sync();
       if (t == 0) {
         const unsigned total = gridDim.x * gridDim.y * gridDim.z;
         if (atomicAdd(p.tp_call + 1, 1u) == total - 1u) {
@@ -805,6 +814,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
   }
   if (clustered) cluster_sync_all();  // no CTA leaves while a peer may still read its shared memory
   // ---------------- teardown ----------------
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
