@@ -244,6 +244,23 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(
   }
 }
 
+// The 16-key slices of a context: those that hold kept first tokens in front of the window, then [first_key, ctx). List position i is slice i or,
+// behind the kept ones, i + skip.
+struct DecodeSlices {
+  int first_key, kept, lo, hi, n_kept, skip;
+  __device__ DecodeSlices(int ctx, int window, int keep_first) {
+    first_key = (window > 0 && ctx > window) ? ctx - window : 0;
+    kept = min(keep_first, first_key);
+    lo = first_key / 16;
+    hi = (ctx + 15) / 16;
+    n_kept = min((kept + 15) / 16, lo);
+    skip = lo - n_kept;
+  }
+  __device__ int count() const { return hi - skip; }
+};
+// Of `splits` CTAs per (sequence, KV head) as many work as have min_slices slices each: a short context is not worth a merge.
+__device__ __forceinline__ int decode_used_splits(int slices, int splits, int min_slices) { return max(1, min(splits, slices / min_slices)); }
+
 // factor of one output column: out_mult, times sigmoid of the row's gate logit for the head or the column
 template <typename TIO>
 __device__ __forceinline__ float attn_gate(const AttnExtra& x, const TIO* gate, long long row, int h, int col) {
@@ -257,10 +274,11 @@ __device__ __forceinline__ float attn_gate(const AttnExtra& x, const TIO* gate, 
 // all splits twice with dependent loads: 12 us at 64 splits, more than the attention kernel it follows.)
 // EXT: with the options of AttnExtra.
 struct NoExtra {};
+// ctx_lens (nullptr: all splits were used): the attention kernel has used decode_used_splits() of them, one of which writes the output itself.
 template <bool EXT>
 __global__ void decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                    __nv_bfloat16* __restrict__ out, int H, int D, int splits,
-                                    const std::conditional_t<EXT, AttnExtra, NoExtra> x) {
+                                    __nv_bfloat16* __restrict__ out, int H, int D, int splits, const int* __restrict__ ctx_lens, int window, int keep_first,
+                                    int min_slices, const std::conditional_t<EXT, AttnExtra, NoExtra> x) {
   __shared__ float w_s[256];
   __shared__ float red[2][8];
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
@@ -281,9 +299,15 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
     for (int j = 0; j < BATCH; ++j) v[j] = d < D && s0 + j < splits ? po[static_cast<long long>(s0 + j) * D] : 0.f;
   };
   fetch(0);
+  float2 ml = d < splits ? *reinterpret_cast<const float2*>(part_ml + (base + d) * 2) : make_float2(-INFINITY, 0.f);
+  if (ctx_lens != nullptr) {  // (the loads above are in flight with this one; what they bring from unused splits is not looked at)
+    splits = decode_used_splits(DecodeSlices(ctx_lens[b], window, keep_first).count(), splits, min_slices);
+    if (splits == 1) return;
+    if (d >= splits) ml = make_float2(-INFINITY, 0.f);
+  }
   // maximum over the splits
-  float m = -INFINITY;
-  for (int s = d; s < splits; s += blockDim.x) m = fmaxf(m, part_ml[(base + s) * 2]);
+  float m = ml.x;
+  for (int s = d + blockDim.x; s < splits; s += blockDim.x) m = fmaxf(m, part_ml[(base + s) * 2]);
   m = warp_max(m);
   if (lane == 0) red[0][wp] = m;
   __syncthreads();
@@ -292,10 +316,10 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
   // weights and the denominator
   float den = 0.f;
   for (int s = d; s < splits; s += blockDim.x) {
-    const float ms = part_ml[(base + s) * 2];
-    const float w = (ms == -INFINITY) ? 0.f : __expf(ms - m);
+    if (s != d) ml = *reinterpret_cast<const float2*>(part_ml + (base + s) * 2);
+    const float w = (ml.x == -INFINITY) ? 0.f : __expf(ml.x - m);
     if (s < 256) w_s[s] = w;
-    den += w * part_ml[(base + s) * 2 + 1];
+    den += w * ml.y;
   }
   den = warp_sum(den);
   if (lane == 0) red[1][wp] = den;
@@ -349,7 +373,8 @@ static int launch_decode_t(const void* q, long long q_stride, const void* kc, co
                                                       scale, cap, window, splits);
   if (splits > 1) {
     dim3 g2(B, H);
-    launch_pdl(decode_merge_kernel<false>, dim3(g2), dim3(D), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, D, splits, NoExtra{});
+    launch_pdl(decode_merge_kernel<false>, dim3(g2), dim3(D), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, D, splits,
+               static_cast<const int*>(nullptr), 0, 0, 1, NoExtra{});
   }
   return 0;
 }
@@ -472,7 +497,7 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
     const __nv_bfloat16* __restrict__ q, long long q_stride, const __nv_bfloat16* __restrict__ k_cache,
     const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_tables, int bt_stride,
     const int* __restrict__ ctx_lens, __nv_bfloat16* __restrict__ out, float* part_o, float* part_ml, int* __restrict__ arrivals,
-    int H, int KV, int page_size, float scale, float softcap, int window, int splits, const DecodeOptions<EXT> opt) {
+    int H, int KV, int page_size, float scale, float softcap, int window, int splits, int min_slices, const DecodeOptions<EXT> opt) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
   using L = DecodeMma<D, NW>;
@@ -492,13 +517,12 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
   const int h0 = kvh * heads_per_kv + (EXT == 1 ? (blockIdx.y % groups) * 16 : 0);  // first query head of this CTA
   const int G = EXT == 1 ? min(16, (kvh + 1) * heads_per_kv - h0) : heads_per_kv;
   const int ctx = ctx_lens[b];
-  const int first_key = (window > 0 && ctx > window) ? ctx - window : 0;
-  // slices of 16 keys: those that hold kept first tokens in front of the window, then [first_key, ctx); the CTA's share of that list
-  const int kept = min(keep_first, first_key);  // keys [0, kept) are visible beside the window
-  const int sl_lo = first_key / 16, sl_hi = (ctx + 15) / 16;
-  const int sl_kept = EXT == 1 ? min((kept + 15) / 16, sl_lo) : 0, sl_skip = sl_lo - sl_kept;  // list position i is slice i or, behind the kept ones, i + sl_skip
-  const int per = (sl_hi - sl_skip + splits - 1) / splits;
-  const int s0 = sp * per, s1 = min(sl_hi - sl_skip, s0 + per);
+  const DecodeSlices list(ctx, window, EXT == 1 ? keep_first : 0);
+  const int first_key = list.first_key, kept = list.kept, sl_kept = list.n_kept, sl_skip = list.skip;
+  const int used = arrivals == nullptr ? decode_used_splits(list.count(), splits, min_slices) : splits;
+  if (sp >= used) return;
+  const int per = (list.count() + used - 1) / used;
+  const int s0 = sp * per, s1 = min(list.count(), s0 + per);
   uint8_t* ring = msm + warp * L::kWarpBytes;
   const uint32_t ring_u = smem_u32(ring);
   const __nv_bfloat16* qrow = q + static_cast<long long>(b) * q_stride + static_cast<long long>(h0) * dk;
@@ -719,7 +743,7 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
       n1 += wt * row[d + 1];
       den += wt * row[D + 1];
     }
-    if (splits == 1) {
+    if (used == 1) {
       finish(r, d, m, n0, n1, den);
     } else {
       const long long base = (static_cast<long long>(b) * H + h0 + r) * splits + sp;
@@ -730,7 +754,7 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
       }
     }
   }
-  if (splits == 1 || arrivals == nullptr) return;  // (no arrival counters: decode_merge_kernel follows)
+  if (used == 1 || arrivals == nullptr) return;  // (no arrival counters: decode_merge_kernel follows)
 
   // ---- (opt-in; measured slower than decode_merge_kernel) merge of the splits by the CTA that finishes last for this
   // (sequence, KV head): no second launch.
@@ -794,6 +818,13 @@ static int launch_decode_mma_t(const void* q, long long q_stride, const void* kc
   using L = DecodeMma<D, NW>;
   // the in-kernel merge keeps its weights in the warp-merge area of shared memory
   if (splits > 1 && (H / KV) * (splits + 1) > L::kMerge / 4) arrivals = nullptr;
+  // `splits` is an upper bound. Where (sequence, KV head) pairs alone fill 0.7 of the resident CTAs, splitting them only adds a merge (us, unsplit
+  // against what the engine asks for: 512 pairs x 2176 keys 88 / 100, 1024 pairs of 256-wide heads 310 / 331, 128 of those 42 / 63); fewer pairs
+  // are split to at most two waves (128 pairs of 300..3000 keys: 4 splits 26.6, 9 splits 26.9, 2 splits 29.0), and no CTA takes less than 16
+  // slices (128 pairs x 576 keys: 13.5 / 21.0), or 3 where a few sequences have the GPU to themselves (8 pairs x 777 keys: 16 splits 5.4, 32 splits 6.6).
+  const long long pairs = static_cast<long long>(B) * KV * ((H / KV + 15) / 16), room = static_cast<long long>(gemm_num_sms()) * (D > 128 ? 1 : 2);
+  if (arrivals == nullptr) splits = pairs * 10 >= room * 7 ? 1 : static_cast<int>(splits < 2 * room / pairs ? splits : 2 * room / pairs);
+  const int min_slices = pairs >= 64 ? 16 : 3;
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
     cudaFuncSetAttribute(decode_attn_mma_kernel<D, EXT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
@@ -804,18 +835,21 @@ static int launch_decode_mma_t(const void* q, long long q_stride, const void* kc
   launch_pdl(decode_attn_mma_kernel<D, EXT, NW>, dim3(grid), dim3(NW * 32), L::kBytes, st, static_cast<const __nv_bfloat16*>(q), q_stride,
                                                           static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(vc), bt,
                                                           bt_stride, ctx, static_cast<__nv_bfloat16*>(out), po, pml, arrivals, H, KV, page, scale,
-                                                          cap, window, splits, opt);
+                                                          cap, window, splits, min_slices, opt);
   if (splits > 1 && arrivals == nullptr) {
     dim3 g2(B, H);
     const dim3 block((dv + 31) / 32 * 32);
-    if constexpr (EXT != 0) launch_pdl(decode_merge_kernel<true>, g2, block, 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, x);
-    else launch_pdl(decode_merge_kernel<false>, g2, block, 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, NoExtra{});
+    const int keep = EXT == 1 ? x.keep_first : 0;
+    if constexpr (EXT != 0) launch_pdl(decode_merge_kernel<true>, g2, block, 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, ctx, window, keep,
+                                       min_slices, x);
+    else launch_pdl(decode_merge_kernel<false>, g2, block, 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, ctx, window, keep, min_slices, NoExtra{});
   }
   return 0;
 }
 
 void launch_decode_merge(const float* po, const float* pml, void* out, int B, int H, int dv, int splits, AttnExtra x, cudaStream_t st) {
-  launch_pdl(decode_merge_kernel<true>, dim3(B, H), dim3((dv + 31) / 32 * 32), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, x);
+  launch_pdl(decode_merge_kernel<true>, dim3(B, H), dim3((dv + 31) / 32 * 32), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits,
+             static_cast<const int*>(nullptr), 0, 0, 1, x);
 }
 
 // impl: 0 = tensor-core kernel when it applies (group <= 16, page_size % 16 == 0), 1 = CUDA-core kernel

@@ -777,3 +777,50 @@ def test_pair_gemm_experts(E, n, K, T, k, q4):
         f = xs[off[i]:off[i + 1]].double().cpu() @ (wd if q4 else wd.to(torch.bfloat16)).double().t()
         assert _rel(y[off[i]:off[i + 1]].cpu(), f) < 4e-3
         assert h is not None and _rel(h[off[i]:off[i + 1]].cpu(), torch.nn.functional.silu(f[:, : n // 2]) * f[:, n // 2:]) < 6e-3
+
+
+@pytest.mark.parametrize("B,H,KV,D", [(1, 8, 4, 64), (2, 32, 8, 128), (9, 16, 8, 256), (40, 16, 4, 128), (64, 8, 8, 64)])
+@pytest.mark.parametrize("window,cap", [(0, 0.0), (100, 30.0)])
+def test_decode_attention_used_splits(B, H, KV, D, window, cap):
+    """Contexts around the lengths at which one more split is used (3 and 16 slices of 16 keys), for few and many (sequence, KV head) pairs; a batch
+    mixes sequences that write their output alone with ones that are merged. bf16 probabilities and output: 2^-9 each."""
+    lens = [1, 15, 16, 17, 47, 48, 49, 95, 97, 255, 257, 511, 513, 700, 1500]
+    ctx = torch.tensor([lens[(7 * i) % len(lens)] for i in range(B)], dtype=torch.int32)
+    per = [(int(c) + 31) // 32 for c in ctx]
+    bt = torch.zeros(B, max(per), dtype=torch.int32)
+    order = torch.randperm(sum(per)) + 1
+    for i, n in enumerate(per):
+        bt[i, :n] = order[sum(per[:i]):sum(per[:i]) + n]
+    kc, vc = (torch.randn(sum(per) + 1, KV, 32, D).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(B, H * D).to(torch.bfloat16)
+    r = ref.paged_attention(q.reshape(B, H, D).float(), kc.float(), vc.float(), bt, torch.arange(B), torch.ones(B, dtype=torch.long), ctx, D**-0.5, cap, window)
+    for splits in (1, 2, 9, 32):
+        o = ops.decode_attention(q.to(DEV), kc.to(DEV), vc.to(DEV), bt.to(DEV), ctx.to(DEV), H, D**-0.5, cap, window, splits)
+        torch.cuda.synchronize()
+        d = (o.cpu().float() - r.reshape(B, -1)).reshape(B, -1).norm(dim=1) / r.reshape(B, -1).norm(dim=1)
+        assert d.max().item() < 6e-3, (splits, d)
+
+
+@pytest.mark.parametrize("T", [1, 7, 1183, 1185])
+@pytest.mark.parametrize("H", [8, 1024, 2048, 2056, 2560, 3584, 4096, 4104, 8192, 8200])
+def test_rmsnorm_widths(T, H):
+    """Both register forms and the loop behind them at the widths where they take over, with and without the residual."""
+    x, res = ((torch.randn(T, H) * s).to(torch.bfloat16) for s in (1.0, 3.0))
+    w = (torch.randn(H) * 0.1).to(torch.bfloat16)
+    y = ops.rmsnorm(x.to(DEV), w.to(DEV), 1e-6, 1.0)
+    got_res = res.to(DEV).clone()
+    z = ops.add_rmsnorm(x.to(DEV), got_res, w.to(DEV), 1e-6, 0.0, 0.5)
+    torch.cuda.synchronize()
+    want_res = (res.float() + 0.5 * x.float()).to(torch.bfloat16)
+    assert torch.equal(got_res.cpu(), want_res)
+    assert _rel(y.cpu(), ref.rmsnorm(x.double(), w.double(), 1e-6, 1.0)) < 3e-3 and _rel(z.cpu(), ref.rmsnorm(want_res.double(), w.double(), 1e-6)) < 3e-3
+
+
+@pytest.mark.parametrize("N,K", [(5, 8), (130, 2040), (64, 2048), (33, 2056), (3, 5632)])
+@pytest.mark.parametrize("f32", [True, False])
+def test_gemv_bf16_row(N, K, f32):
+    w, x = (torch.randn(N, K) * 0.05).to(torch.bfloat16), torch.randn(1, K).to(torch.bfloat16)
+    bias = torch.randn(N)
+    y = ops.linear(x.to(DEV), LinearWeight(w, bias).to(DEV, torch.bfloat16), out_f32=f32)
+    torch.cuda.synchronize()
+    assert _rel(y.cpu(), x.double() @ w.double().t() + bias.double()) < (1e-5 if f32 else 4e-3)
