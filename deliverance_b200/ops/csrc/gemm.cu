@@ -209,17 +209,16 @@ static void run_tc(const GemmWeightDesc* w, const void* x, int M, int ldx, GemmP
   p.x3d = w->K % 64 == 0 ? 1 : 0;
   if (p.x3d) encode_map_kchunks(&map_x, x, static_cast<uint64_t>(M), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, BN);
   else encode_map_2d(&map_x, 0, x, static_cast<uint64_t>(M), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, BN, 64, 128);
-  // Tail split: a single-split grid that is a few tiles larger than the SM count would run a full second wave for those few
-  // tiles. They are cut into up to 8 k-ranges each (reduced through the workspace), so the second wave is a short one.
+  // Tail split: a single-split grid that is a few tiles larger than a whole number of waves would run one more for those few tiles. The last
+  // weight tiles (of every token tile) are cut into up to 8 k-ranges each (reduced through the workspace), so that wave is a short one.
   int grid_x = p.n_tiles;
-  if ((tp == nullptr || tp->size <= 1) && splits == 1 && p.m_tiles == 1 && force_splits == 0 && ws != nullptr && counters != nullptr &&
-      p.kb_total >= 8) {
+  if (EPI <= 2 && (tp == nullptr || tp->size <= 1) && splits == 1 && force_splits == 0 && ws != nullptr && counters != nullptr && p.kb_total >= 8) {
     const int cap = gemm_num_sms();
-    const int rem = p.n_tiles % cap;
-    if (p.n_tiles > cap && rem > 0 && rem * 8 <= cap) {
+    const int over = tiles % cap, rem = (over + p.m_tiles - 1) / p.m_tiles;  // weight tiles to cut
+    if (tiles > cap && over > 0 && rem < p.n_tiles && rem * p.m_tiles * 8 <= cap) {
       const int kb_per = (p.kb_total + 7) / 8;
       const int s_eff = (p.kb_total + kb_per - 1) / kb_per;
-      if (s_eff > 1 && static_cast<size_t>(rem) * s_eff * BN * kGemmBM <= ws_floats && rem <= n_counters) {
+      if (s_eff > 1 && static_cast<size_t>(rem) * p.m_tiles * s_eff * BN * kGemmBM <= ws_floats && rem * p.m_tiles <= n_counters) {
         p.tail_tile0 = p.n_tiles - rem;
         p.tail_splits = s_eff;
         p.tail_kb_per_split = kb_per;
@@ -615,8 +614,8 @@ __device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefe
 
 // ------------------------------------------------------------------------------------------------ one row of bf16 weights
 // One token row against a dense weight: a warp per weight row, 16 bytes per lane and chunk of 256 elements. Bound by the weight stream, and at
-// a few megabytes by how early and how widely it starts: eight chunks per lane are in flight, the first eight (and L2 prefetches of the rest)
-// from before the wait for the kernel in front. gemv_simt_kernel, which it replaces here, had one or two chunks in flight behind an
+// a few megabytes by how early and how widely it starts: the row is on its way to L2 while the kernel in front finishes, and eight chunks per
+// lane are in flight behind the wait. gemv_simt_kernel, which it replaces here, had one or two chunks in flight behind an
 // ordinary launch (tinyllama's 22 layers at one token: 638 us of GEMVs for 2.07 GB).
 constexpr int kGemvChunks = 8;
 template <bool OUTF>
@@ -633,10 +632,10 @@ __global__ void __launch_bounds__(128) gemv_bf16_kernel(const __nv_bfloat16* __r
       wv[i] = k < K ? __ldg(reinterpret_cast<const uint4*>(row + k)) : make_uint4(0u, 0u, 0u, 0u);
     }
   };
-  fetch(0);
-  for (int k = kGemvChunks * 256 + lane * 8; k < K; k += 256) l2_prefetch(row + k);
+  for (int k = lane * 8; k < K; k += 256) l2_prefetch(row + k);
   pdl_wait();
   if (n >= N) return;
+  fetch(0);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (int k0 = 0; k0 < K; k0 += kGemvChunks * 256) {
     if (k0 > 0) fetch(k0);
