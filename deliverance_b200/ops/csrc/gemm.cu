@@ -209,16 +209,17 @@ static void run_tc(const GemmWeightDesc* w, const void* x, int M, int ldx, GemmP
   p.x3d = w->K % 64 == 0 ? 1 : 0;
   if (p.x3d) encode_map_kchunks(&map_x, x, static_cast<uint64_t>(M), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, BN);
   else encode_map_2d(&map_x, 0, x, static_cast<uint64_t>(M), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, BN, 64, 128);
-  // Tail split: a single-split grid that is a few tiles larger than a whole number of waves would run one more for those few tiles. The last
-  // weight tiles (of every token tile) are cut into up to 8 k-ranges each (reduced through the workspace), so that wave is a short one.
+  // Tail split: a single-split grid that is a few tiles larger than the SM count would run a full second wave for those few
+  // tiles. They are cut into up to 8 k-ranges each (reduced through the workspace), so the second wave is a short one.
   int grid_x = p.n_tiles;
-  if (EPI <= 2 && (tp == nullptr || tp->size <= 1) && splits == 1 && force_splits == 0 && ws != nullptr && counters != nullptr && p.kb_total >= 8) {
+  if ((tp == nullptr || tp->size <= 1) && splits == 1 && p.m_tiles == 1 && force_splits == 0 && ws != nullptr && counters != nullptr &&
+      p.kb_total >= 8) {
     const int cap = gemm_num_sms();
-    const int over = tiles % cap, rem = (over + p.m_tiles - 1) / p.m_tiles;  // weight tiles to cut
-    if (tiles > cap && over > 0 && rem < p.n_tiles && rem * p.m_tiles * 8 <= cap) {
+    const int rem = p.n_tiles % cap;
+    if (p.n_tiles > cap && rem > 0 && rem * 8 <= cap) {
       const int kb_per = (p.kb_total + 7) / 8;
       const int s_eff = (p.kb_total + kb_per - 1) / kb_per;
-      if (s_eff > 1 && static_cast<size_t>(rem) * p.m_tiles * s_eff * BN * kGemmBM <= ws_floats && rem * p.m_tiles <= n_counters) {
+      if (s_eff > 1 && static_cast<size_t>(rem) * s_eff * BN * kGemmBM <= ws_floats && rem <= n_counters) {
         p.tail_tile0 = p.n_tiles - rem;
         p.tail_splits = s_eff;
         p.tail_kb_per_split = kb_per;

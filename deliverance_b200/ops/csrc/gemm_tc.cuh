@@ -220,7 +220,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
     split = j % p.tail_splits;
     splits = p.tail_splits;
     kb_per_split = p.tail_kb_per_split;
-    ws_tile = (j / p.tail_splits) * p.m_tiles + m_tile;
+    ws_tile = j / p.tail_splits;
   }
   const int n0 = n_tile * kGemmBM;
   int m0 = m_tile * BN, m_lim = p.M, w_tile = n_tile, w_row0 = n0;
