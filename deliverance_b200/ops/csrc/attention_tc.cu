@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
     if (LATENT) tma_prefetch_desc(&map_r);
   }
   constexpr uint32_t kTmemCols = 512;
+  __syncwarp();  // (one lane set the barriers up)
   if (warp == kIssuer) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
   tc_fence_before();
   __syncthreads();
@@ -705,6 +706,7 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
           for (int i = 0; i < 4; ++i)
             if (c0 + i * 8 < p.dv) gv[i] = *reinterpret_cast<const uint4*>(grow + c0 + i * 8);
         }
+        __syncwarp();  // (rows behind the last one store nothing; the loads below are warp-wide)
         uint32_t v[32];
         if (my_tiles > 0) {
           tmem_ld_x32(lane_addr + kColO + q * DV + c0, v);
@@ -758,6 +760,7 @@ __global__ void __launch_bounds__(AttnTcLayout<DK, DV, QT, KM>::T::kThreads, 1)
       }
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == kIssuer) {

@@ -166,6 +166,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) decode_chain_kernel(const __g
     for (int g = 0; g < p.n_ops; ++g) tma_prefetch_desc(&p.maps[g]);
   }
   pdl_trigger();
+  __syncwarp();
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), kGemmTmemCols);
   tc_fence_before();
   __syncthreads();
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) decode_chain_kernel(const __g
         if (u == u0 || kb == 0) seg_i0 = i;
         if ((i & 3) == grp4) {
           const int sr = i % NR, sa = i & 3;
-          if (!mbar_wait(smem_u32(&bar_r_full[sr]), (i / NR) & 1, abort_flag, p.status)) { ok = false; break; }
+          ok = mbar_wait(smem_u32(&bar_r_full[sr]), (i / NR) & 1, abort_flag, p.status);
           uint4 wq[4];
 #pragma unroll
           for (int b = 0; b < 4; ++b) wq[b] = *reinterpret_cast<const uint4*>(raw_tile(sr) + r * 64 + ((b ^ ((r >> 1) & 3)) << 4));
@@ -344,7 +345,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) decode_chain_kernel(const __g
 #pragma unroll
           for (int b = 0; b < 4; ++b) {
             if ((b & 1) == 0) {  // a half stage (64 k) is free once the MMAs that read it for unit i - 4 have retired
-              if (!mbar_wait(smem_u32(&bar_a_empty[2 * sa + (b >> 1)]), ((i / NA) & 1) ^ 1, abort_flag, p.status)) { ok = false; break; }
+              // (every lane polls for itself; the stores below are warp-wide, so the warp goes on or leaves as a whole)
+              ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bar_a_empty[2 * sa + (b >> 1)]), ((i / NA) & 1) ^ 1, abort_flag, p.status));
+              if (!ok) break;
               tc_fence_after();
             }
             const __nv_bfloat162 s2 = __float2bfloat162_rn(sc[b]);
@@ -375,7 +378,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) decode_chain_kernel(const __g
         if (u == u1 - 1 || kb == o.kbt - 1) {
           // ---- segment epilogue: accumulators -> fp32 partial tile in the workspace slot of (tile, this segment) ----
           const int len = i + 1 - seg_i0;
-          if (!mbar_wait(smem_u32(bar_acc_full), segn & 1, abort_flag, p.status)) { ok = false; break; }
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar_acc_full), segn & 1, abort_flag, p.status));
+          if (!ok) break;
           tc_fence_after();
           constexpr int GROUPS = BN >= 32 ? 4 : BN / 8;
           constexpr int COLS = BN / GROUPS;
@@ -402,7 +406,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) decode_chain_kernel(const __g
             }
           }
           tc_fence_before();
-          asm volatile("bar.sync 1, 512;" ::: "memory");
+          epilogue_sync();
           if (t == 0) {
             mbar_arrive(smem_u32(bar_acc_empty));
             red_release_gpu_add(p.sync + o.off_cnt + tile, 1u);  // cumulative over the stores of all 512 threads (ordered by the barrier)
@@ -436,7 +440,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) decode_chain_kernel(const __g
             got = __all_sync(0xffffffffu, got);
             if (t == 0) *s_flag = got ? 1 : 0;
           }
-          asm volatile("bar.sync 1, 512;" ::: "memory");
+          epilogue_sync();
           if (*s_flag == 0) {
             *abort_flag = 1;
             ok = false;
@@ -551,13 +555,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) decode_chain_kernel(const __g
               }
             }
           }
-          asm volatile("bar.sync 1, 512;" ::: "memory");
+          epilogue_sync();
           if (t == 0) red_release_gpu_add(p.sync + o.off_done, 1u);
         }
       }
     }
   }
   // ---------------- teardown ----------------
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

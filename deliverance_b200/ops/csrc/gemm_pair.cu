@@ -325,7 +325,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           if ((j & 1) != (grp >> 1)) continue;
           const int sr = j % NR;
           ok = mbar_wait(smem_u32(&bar_raw_full[sr]), (j / NR) & 1, abort_flag, p.status);
-          if (!ok) break;
           const uint8_t* raw = smem + L::kOffRaw + sr * kRawBytes;
           uint4 w[2];
           float sc[2];
@@ -353,7 +352,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           // A last stage of 64 k has one half only; its other group waits for the same operand stage and writes nothing: parities tell
           // the right phase only while a group is less than two rounds of the ring behind.
           const int g = g0 + min(k, p.nk - 1), s = g % NS;
-          ok = mbar_wait(smem_u32(&bar_empty[s]), ((g / NS) & 1) ^ 1, abort_flag, p.status);
+          ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bar_empty[s]), ((g / NS) & 1) ^ 1, abort_flag, p.status));  // (the warp stays whole)
           if (!ok) break;
           if (k < p.nk) {
             uint8_t* dst = smem + s * kStageBytes + kOpBytes + r * 128;
@@ -566,6 +565,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     while (globaltimer_ns() - t0 < 20000000ull) {
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // no CTA leaves while the pair's MMAs or arrivals may still touch its shared memory
@@ -573,7 +573,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, 512);
   }
-  __syncwarp();
   cluster_sync_all();  // the release of a pair's tensor memory involves both CTAs: neither leaves before both have asked for it
 }
 

@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_persist_kernel(const __grid
     tma_prefetch_desc(&map_x);
   }
   pdl_trigger();
+  __syncwarp();
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), kGemmTmemCols);
   tc_fence_before();
   __syncthreads();
@@ -242,14 +243,16 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_persist_kernel(const __grid
     const int r = q * 32 + lane;
     for (int g = grp; g < total_kb; g += 4) {
       const int sr = g % kPNR, sa = g % kPNA;
-      if (!mbar_wait(smem_u32(&bar_r_full[sr]), static_cast<uint32_t>(g / kPNR) & 1, abort_flag, p.status)) break;
+      bool ok = mbar_wait(smem_u32(&bar_r_full[sr]), static_cast<uint32_t>(g / kPNR) & 1, abort_flag, p.status);
       uint4 wq[4];
 #pragma unroll
       for (int blk = 0; blk < 4; ++blk) wq[blk] = *reinterpret_cast<const uint4*>(raw_tile(sr) + r * 64 + ((blk ^ ((r >> 1) & 3)) << 4));
       const float4 sc4 = *reinterpret_cast<const float4*>(raw_tile(sr) + kGemmBM * 64 + r * 16);
       const float sc[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
       // the tensor-memory stage is free once the MMAs of k-block g - 4 have retired
-      if (!mbar_wait(smem_u32(&bar_a_empty[sa]), (static_cast<uint32_t>(g / kPNA) & 1) ^ 1, abort_flag, p.status)) break;
+      // (every lane polls for itself; the stores below are warp-wide, so the warp goes on or leaves as a whole)
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bar_a_empty[sa]), (static_cast<uint32_t>(g / kPNA) & 1) ^ 1, abort_flag, p.status));
+      if (!ok) break;
       tc_fence_after();
       const uint32_t tdst = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + kPTmemA + sa * kGemmTmemAStage;
 #pragma unroll
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_persist_kernel(const __grid
       tc_fence_after();
       const int n = n_tile * kGemmBM + q * 32 + lane;  // output column of this thread
       const float bv = (p.bias != nullptr && n < p.N) ? p.bias[n] : 0.f;
+      __syncwarp();
       const int m0 = m_tile * kPT;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + b * kPT;
 #pragma unroll 1
@@ -308,12 +312,14 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_persist_kernel(const __grid
             }
           }
         }
+        __syncwarp();  // (the next load is warp-wide)
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[b]));
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

@@ -163,9 +163,13 @@ __device__ __forceinline__ uint32_t q4_pair_to_bf162(uint32_t nib4, uint32_t sel
 
 // Role code leaves warps in pieces (single lanes copy, every lane polls a barrier for itself), and with a uniform warp index nothing joins them
 // again by itself: the .aligned barriers would count such a warp wrongly and never open. So the cluster barrier is the form that every thread
-// executes for itself, and the named barrier of the epilogue warps comes behind a __syncwarp.
+// executes for itself, and the named barrier of the epilogue warps comes behind a __syncwarp. That form lets the lanes of a warp go one by one,
+// and what follows it (tcgen05.alloc, tcgen05.dealloc) wants the whole warp at once: it joins them again. The same holds wherever a .sync.aligned
+// instruction follows a poll that every lane makes for itself or a branch that single lanes take.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  __syncwarp();
 }
 __device__ __forceinline__ void epilogue_sync() {
   __syncwarp();
@@ -269,6 +273,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
     tma_prefetch_desc(&map_x);
   }
   pdl_trigger();  // kernels behind this one may be scheduled as soon as every CTA of this grid has started
+  __syncwarp();
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
   tc_fence_before();
   __syncthreads();
@@ -442,16 +447,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
       const int r = q * 32 + lane;
       for (int i = grp4; i < nkb; i += 4) {
         const int sr = i % NR, sa = i % NA;
-        if (!mbar_wait(smem_u32(&bar_r_full[sr]), (i / NR) & 1, abort_flag, p.status)) { ok = false; break; }
+        ok = mbar_wait(smem_u32(&bar_r_full[sr]), (i / NR) & 1, abort_flag, p.status);
         uint4 wq[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) wq[b] = *reinterpret_cast<const uint4*>(raw_tile(sr) + r * 64 + ((b ^ ((r >> 1) & 3)) << 4));
         const float4 sc4 = *reinterpret_cast<const float4*>(sc_tile(sr) + r * 16);
         const float sc[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
         // the tensor-memory stage is free once the MMAs of k-block i - NA have retired
-        if (!mbar_wait(smem_u32(&bar_a_empty[sa]), ((i / NA) & 1) ^ 1, abort_flag, p.status)) { ok = false; break; }
+        // (every lane polls for itself; the stores below are warp-wide, so the warp goes on or leaves as a whole)
+        ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bar_a_empty[sa]), ((i / NA) & 1) ^ 1, abort_flag, p.status));
+        if (!ok) break;
         tc_fence_after();
-        __syncwarp();  // (every lane polled for itself; the stores below are warp-wide)
         const uint32_t tdst = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + L::kTmemA + sa * kGemmTmemAStage;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
@@ -485,6 +491,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,   // dense: bf16 [N, K
     // raised before the accumulator barrier can complete), so the named barriers below never miss a thread.
     epilogue_sync();
     ok = (*abort_flag == 0);
+    __syncwarp();
     if (ok) {
       tc_fence_after();
       constexpr int GROUPS = BN >= 32 ? 4 : BN / 8;  // warps that share a quarter split the columns
