@@ -52,7 +52,8 @@ struct PairSmem {
 
 struct PairParams {
   int M, N, K;       // N: weight rows (per expert in grouped mode)
-  int nk;            // 64-k steps
+  int nk;            // 64-k steps; JQ4: two for every packed stage, also where K ends in the first half of the last one (the padding holds zero
+                     // scales, the copies bring zero tokens), because a group that waits for a step must also be waited for in that step
   int kq;            // JQ4: 128-k stages of a tile row
   int n_tiles, m_tiles;
   int w_rows;        // weight rows of one expert in the stacked weight (dense) / 128-row tiles of one expert (JQ4)
@@ -348,20 +349,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bar_raw_empty[sr]));
-          const int k = 2 * q + h;
-          // A last stage of 64 k has one half only; its other group waits for the same operand stage and writes nothing: parities tell
-          // the right phase only while a group is less than two rounds of the ring behind.
-          const int g = g0 + min(k, p.nk - 1), s = g % NS;
+          const int g = g0 + 2 * q + h, s = g % NS;
           ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bar_empty[s]), ((g / NS) & 1) ^ 1, abort_flag, p.status));  // (the warp stays whole)
           if (!ok) break;
-          if (k < p.nk) {
-            uint8_t* dst = smem + s * kStageBytes + kOpBytes + r * 128;
+          uint8_t* dst = smem + s * kStageBytes + kOpBytes + r * 128;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dst + ((c ^ (r & 7)) << 4)) = o[c];
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(&bar_full[s]), 0));
-          }
+          for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dst + ((c ^ (r & 7)) << 4)) = o[c];
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(&bar_full[s]), 0));
         }
         g0 += p.nk;
       }
@@ -622,8 +618,8 @@ void launch_pair(const GemmWeightDesc* w, const void* x, int ldx, int rows, Pair
   }
   encode_map_2d(&map_x, 0, x, static_cast<uint64_t>(rows), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, 128, 64, 128);
   p.K = w->K;
-  p.nk = (w->K + 63) / 64;
   p.kq = (w->K + 127) / 128;
+  p.nk = Q4 ? 2 * p.kq : (w->K + 63) / 64;
   const int total = p.n_tiles * p.m_tiles;
   const int pairs = total < cap ? total : cap;
   cudaLaunchConfig_t cfg = {};

@@ -758,10 +758,11 @@ def test_pair_gemm_heads(heads, kv, norm, rope, q4):
     assert _rel(q, qr.reshape(M, -1)) < 6e-3 and _rel(kc, k2) < 6e-3 and _rel(vc, v2) < 4e-3
 
 
-@pytest.mark.parametrize("E,n,K,T,k", [(4, 512, 256, 700, 2), (3, 768, 1216, 1500, 1)])
+@pytest.mark.parametrize("E,n,K,T,k", [(4, 512, 256, 700, 2), (3, 768, 1216, 1500, 1), (3, 512, 64, 900, 2), (40, 1280, 160, 9000, 2)])
 @pytest.mark.parametrize("q4", [True, False])
 def test_pair_gemm_experts(E, n, K, T, k, q4):
-    """Work items of 256 rows that end inside a tile, unused ones at the end of the list; plain store and gated activation."""
+    """Work items of 256 rows that end inside a tile, unused ones at the end of the list; plain store and gated activation. K that ends in the
+    first half of a packed stage, also with several tiles per pair of SMs and the step ring at every phase."""
     e = ops.require_ext()
     made = [_q4_weight(n, K, seed=i) for i in range(E)]
     g = ops.GroupedLinearWeight([(LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16) for qt, wd in made])
