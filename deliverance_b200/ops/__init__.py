@@ -40,6 +40,8 @@ def ext():
         persist = os.environ.get("DLV_GEMM_PERSIST", "0")
         if _ext is not None and persist in ("1", "race"):
             _ext.gemm_persist(True, False, persist != "race")
+        if _ext is not None and os.environ.get("DLV_GEMM_PAIR", "1") == "0":
+            set_gemm_pairs(0)
         if _ext is not None and os.environ.get("DLV_DECODE_MERGE", "launch") == "kernel":
             _MERGE_IN_KERNEL[0] = True
             _ext.decode_merge_in_kernel(True)
@@ -53,6 +55,12 @@ def ext():
 def set_gemm_pdl(on: bool) -> None:
     """Programmatic dependent launch of the GEMM kernels (their prologue and weight prefetch overlap the previous kernel's tail)."""
     require_ext().gemm_pdl(bool(on))
+
+
+def set_gemm_pairs(n: int = -1) -> None:
+    """Most pairs of SMs that a prompt-size product takes (default: as many as the GPU holds). 0 switches the pair kernel off, as ``DLV_GEMM_PAIR=0`` does:
+    every product then runs on the one-tile kernel, which also takes over where no pair fits."""
+    require_ext().gemm_pairs(int(n))
 
 
 def require_ext():

@@ -271,9 +271,8 @@ class GemmWeight {
       bptr = b.data_ptr<float>();
     }
     if (M == 0) return out;
-    const bool pair = impl == 3 || (impl == 0 && force_splits == 0 && !dlv::g_gemm_persist && dlv::g_gemm_force_bn == 0 &&
-                                    dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0));
-    if (pair && !out_f32 && dlv::gemm_pair_supported(&desc_, desc_.N, out.data_ptr(), static_cast<int>(out.stride(0)))) {
+    const bool pair = impl == 3 || (impl == 0 && force_splits == 0 && dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0));
+    if (pair && !out_f32 && dlv::gemm_pair_supported(&desc_, desc_.N, out.data_ptr(), static_cast<int>(out.stride(0)), false, 0)) {
       Tensor room = expanded();
       dlv::gemm_pair_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), bptr,
                          room.defined() ? room.data_ptr() : nullptr, scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
@@ -332,7 +331,7 @@ class GemmWeight {
     TORCH_CHECK(x.device() == w_.device(), "x and weight live on different devices");
     const int M = static_cast<int>(x.size(0));
     if ((act != 1 && act != 2) || desc_.N % 16 != 0 || !dlv::gemm_pair_preferred(&desc_, M, desc_.N, 3 * desc_.N / 2) || x.stride(0) % 8 != 0 ||
-        (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) != 0 || !dlv::gemm_pair_act_supported(&desc_, desc_.N, nullptr, desc_.N / 2))
+        (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) != 0 || !dlv::gemm_pair_act_supported(&desc_, desc_.N, nullptr, desc_.N / 2, false))
       return Tensor();
     c10::cuda::CUDAGuard guard(x.device());
     Tensor out = new_out({M, desc_.N / 2}, x.options());
@@ -349,7 +348,7 @@ class GemmWeight {
     TORCH_CHECK(items.is_cuda() && items.scalar_type() == at::kInt && items.dim() == 2 && items.size(1) == 4 && items.is_contiguous(), "items must be int32 [n, 4]");
     const int64_t per = desc_.is_q4 ? ((n_per_expert + 127) / 128) * 128 : n_per_expert;
     TORCH_CHECK(n_per_expert > 0 && desc_.N % per == 0, "stacked weight rows are not a multiple of the per-expert rows");
-    if ((act != 1 && act != 2) || n_per_expert % 16 != 0 || !dlv::gemm_pair_act_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2)))
+    if ((act != 1 && act != 2) || n_per_expert % 16 != 0 || !dlv::gemm_pair_act_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2), true))
       return Tensor();
     c10::cuda::CUDAGuard guard(xs.device());
     Tensor out = new_out({xs.size(0), n_per_expert / 2}, xs.options());
@@ -465,7 +464,7 @@ class GemmWeight {
     Tensor q = new_out({M, H * 128}, x.options());
     if (M == 0) return q;
     DeviceScratch& s = scratch_for(x.device().index());
-    if (dlv::g_gemm_force_bn == 0 && dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0) && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
+    if (dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0) && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
         desc_.N == (a.heads + 2 * a.kv_heads) * 128 && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a)) {
       Tensor room = expanded();
       dlv::gemm_pair_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
@@ -1658,6 +1657,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         dlv::g_gemm_persist_ordered = ordered;
       },
       py::arg("on"), py::arg("all") = false, py::arg("ordered") = true);
+  m.def("gemm_pairs", [](int64_t n) { dlv::g_gemm_pairs = static_cast<int>(n); });
   m.def("decode_merge_in_kernel", [](bool on) { g_decode_merge_in_kernel = on; });
   m.def("gemv_max_rows", [](int64_t n) { dlv::g_gemv_max_rows = static_cast<int>(n); });
   m.def("gemv_force_split", [](int64_t s) { dlv::g_gemv_force_split = static_cast<int>(s); });

@@ -110,8 +110,9 @@ void gemm_tc_run_gathered(const GemmWeightDesc* w, int M, const GemmScatterArgs*
                           const float* bias, float* ws, size_t ws_floats, int* counters, int n_counters, int* status, cudaStream_t st);
 // gemm_pair.cu: prefill-size products on pairs of SMs. `expanded`: device room of gemm_pair_expanded_bytes() for a JQ4 weight's bf16 form.
 bool gemm_pair_preferred(const GemmWeightDesc* w, int M, int n, int merged);  // faster than the one-tile kernel
-bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ldo);
-bool gemm_pair_act_supported(const GemmWeightDesc* w, int n, const void* out, int ldo);
+extern int g_gemm_pairs;  // most pairs of SMs that a launch takes; 0: the pair kernel is off, < 0: as many as the GPU holds
+bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ldo, bool grouped, int epi);
+bool gemm_pair_act_supported(const GemmWeightDesc* w, int n, const void* out, int ldo, bool grouped);
 size_t gemm_pair_expanded_bytes(const GemmWeightDesc* w);
 void gemm_pair_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, const float* bias, void* expanded, int* status, cudaStream_t st);
 void gemm_pair_run_act(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, int act, void* expanded, int* status, cudaStream_t st);

@@ -27,6 +27,8 @@
 
 namespace dlv {
 
+int g_gemm_pairs = -1;
+
 void encode_map_2d(CUtensorMap* map, int dtype_code, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows,
                    uint32_t box_cols, int swizzle_code);
 
@@ -572,33 +574,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   cluster_sync_all();  // the release of a pair's tensor memory involves both CTAs: neither leaves before both have asked for it
 }
 
+// Pairs of SMs that can hold the kernel at one time on the current GPU, within the limit that is set; 0: none (a GPU or a share of one on
+// which no cluster of this size fits), so that products take the one-tile kernel.
 template <bool Q4, int EPI>
 int pair_capacity() {
-  using L = PairSmem<Q4>;
-  static PerDeviceOnce attr_once;
-  static int cap = -1;  // the GPUs of one process are the same model
-  if (attr_once.first()) {
+  static int caps[64];  // per GPU; 0: not asked yet, -1: none
+  int dev = 0;
+  if (g_gemm_pairs == 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (caps[dev] == 0) {
+    using L = PairSmem<Q4>;
     cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<Q4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
-    if (e != cudaSuccess) throw std::runtime_error(std::string("pair gemm: cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-  }
-  if (cap < 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2);
-    cfg.blockDim = dim3(L::kThreads);
-    cfg.dynamicSmemBytes = L::kBytes;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     int n = 0;
-    cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<Q4, EPI>, &cfg);
-    (void)cudaGetLastError();
-    cap = (e == cudaSuccess && n > 0) ? n : 0;
+    if (e == cudaSuccess) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(2);
+      cfg.blockDim = dim3(L::kThreads);
+      cfg.dynamicSmemBytes = L::kBytes;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      e = cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<Q4, EPI>, &cfg);
+    }
+    if (e != cudaSuccess) (void)cudaGetLastError();  // (this query's own error; nothing was launched)
+    caps[dev] = e == cudaSuccess && n > 0 ? n : -1;
   }
-  return cap;
+  const int cap = caps[dev] < 0 ? 0 : caps[dev];
+  return g_gemm_pairs > 0 && g_gemm_pairs < cap ? g_gemm_pairs : cap;
+}
+
+int pair_capacity_of(bool q4, int epi) {
+  if (q4) return epi == 1 ? pair_capacity<true, 1>() : pair_capacity<true, 0>();
+  return epi == 2 ? pair_capacity<false, 2>() : (epi == 1 ? pair_capacity<false, 1>() : pair_capacity<false, 0>());
 }
 
 // `expanded`: bf16 [N, K] room for a JQ4 weight that is expanded in front of the product (nullptr: expanded inside the kernel, stage by stage)
@@ -635,9 +645,11 @@ void launch_pair(const GemmWeightDesc* w, const void* x, int ldx, int rows, Pair
 
 }  // namespace
 
-// Shapes the pair kernel takes: 16-byte output chunks, a weight of at least one tile.
-bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ldo) {
-  return n % 8 == 0 && n >= 256 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && w->K >= 64;
+// Shapes the pair kernel takes: 16-byte output chunks, a weight of at least one tile; and a GPU that can hold a pair of it.
+// `grouped`: JQ4 weights are expanded inside the kernel. `epi`: its epilogue.
+bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ldo, bool grouped, int epi) {
+  return n % 8 == 0 && n >= 256 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && w->K >= 64 &&
+         pair_capacity_of(grouped && w->is_q4, epi) > 0;
 }
 
 // Whether the pair kernel is faster than the one-tile kernel (gemm_tc.cuh) for M rows of this weight. Both times in microseconds, by whole
@@ -646,7 +658,7 @@ bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ld
 // that push others out of L2: 36 us for 19456 x 2560, so that 4-bit weights come here from about 1500 rows on. `merged`: outputs per row that
 // the epilogue saves a later kernel from reading and writing.
 bool gemm_pair_preferred(const GemmWeightDesc* w, int M, int n, int merged) {
-  if (M < 192 || n < kWRows) return false;
+  if (M < 192 || n < kWRows || g_gemm_persist || g_gemm_force_bn != 0) return false;  // (the last two: another kernel or tile was asked for)
   const double nk = (w->K + 63) / 64;
   const int m_tiles = (M + kTokens - 1) / kTokens, sms = gemm_num_sms();
   auto waves = [](long long tiles, long long room) { return static_cast<double>((tiles + room - 1) / room); };
@@ -678,8 +690,8 @@ void gemm_pair_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void*
 }
 
 // gate rows [0, N / 2) and up rows [N / 2, N) in plain order; out [M, N / 2]. JQ4 experts: whole weight tiles of either (N / 2 % 128 == 0).
-bool gemm_pair_act_supported(const GemmWeightDesc* w, int n, const void* out, int ldo) {
-  return n % 16 == 0 && gemm_pair_supported(w, n / 2, out, ldo) && (!w->is_q4 || n % 256 == 0);
+bool gemm_pair_act_supported(const GemmWeightDesc* w, int n, const void* out, int ldo, bool grouped) {
+  return n % 16 == 0 && (!w->is_q4 || n % 256 == 0) && gemm_pair_supported(w, n / 2, out, ldo, grouped, 1);
 }
 
 void gemm_pair_run_act(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, int act, void* expanded, int* status, cudaStream_t st) {
@@ -698,7 +710,7 @@ void gemm_pair_run_act(const GemmWeightDesc* w, const void* x, int M, int ldx, v
 
 bool gemm_pair_qkv_supported(const GemmWeightDesc* w, const void* q_out, int ldo, const GemmQkvArgs* a) {
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  return gemm_pair_supported(w, w->N, q_out, ldo) && (a->cos_t == nullptr || a->rot_half == 64) && aligned(a->k_cache) && aligned(a->v_cache) && aligned(a->cos_t) &&
+  return gemm_pair_supported(w, w->N, q_out, ldo, false, 2) && (a->cos_t == nullptr || a->rot_half == 64) && aligned(a->k_cache) && aligned(a->v_cache) && aligned(a->cos_t) &&
          aligned(a->sin_t);
 }
 

@@ -780,6 +780,42 @@ def test_pair_gemm_experts(E, n, K, T, k, q4):
         assert h is not None and _rel(h[off[i]:off[i + 1]].cpu(), torch.nn.functional.silu(f[:, : n // 2]) * f[:, n // 2:]) < 6e-3
 
 
+@pytest.mark.parametrize("q4", [True, False])
+def test_pair_gemm_limits(q4):
+    """Products that the pair kernel is preferred for, with no pair (the one-tile kernel takes them all), with three, and with all of the GPU."""
+    M, K, I, H, KV, E = 4096, 512, 1024, 16, 8, 3
+    gate_up, heads = [_q4_weight(n, K, seed=n) for n in (2 * I, (H + 2 * KV) * 128)]
+    a, b = [(LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16) for qt, wd in (gate_up, heads)]
+    experts = [_q4_weight(2 * I, K, seed=i) for i in range(E)]
+    g = ops.GroupedLinearWeight([(LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16) for qt, wd in experts])
+    e = ops.require_ext()
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    w, idx, counts, offsets, perm, pos = e.moe_route(torch.randn(M, E, device=DEV), 1, 0, True)
+    items, xs = e.moe_items(offsets, 0, E, 256, M // 256 + E), e.moe_gather(x, perm, 1, None, 0, 0)
+    cos, sin = (t.to(DEV) for t in ref.rope_tables(128, M, 10000.0))
+    got = {}
+    try:
+        for n in (0, 3, -1):
+            ops.set_gemm_pairs(n)
+            kc, vc = (torch.zeros(M // 32, KV, 32, 128, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+            at = torch.arange(M, device=DEV)
+            q = ops.linear_rope_kv(x, b, at.int(), at, None, None, cos, sin, kc, vc, H, KV, 128, 1e-6)
+            gated, grouped = a.handle().run_gated(x, 1), g.run_gated(xs, items, "silu")
+            assert (gated is None) == (grouped is None) == (n == 0)
+            got[n] = [ops.linear(x, a), ops.linear_gated(x, a, "silu"), q, kc, vc, g.run(xs, items, 256)] + ([gated, grouped] if n else [])
+            if n == 0:
+                with pytest.raises(RuntimeError):
+                    ops.linear(x, a, impl=3)
+        torch.cuda.synchronize()
+        ops.check_status()
+    finally:
+        ops.set_gemm_pairs(-1)
+    for u, v in zip(got[3], got[-1]):
+        assert torch.equal(u, v)
+    for u, v in zip(got[0], got[-1]):  # (sums in another order, rounded to bf16 once or twice: 2^-9 each)
+        assert _rel(u, v) < 6e-3
+
+
 @pytest.mark.parametrize("B,H,KV,D", [(1, 8, 4, 64), (2, 32, 8, 128), (9, 16, 8, 256), (40, 16, 4, 128), (64, 8, 8, 64)])
 @pytest.mark.parametrize("window,cap", [(0, 0.0), (100, 30.0)])
 def test_decode_attention_used_splits(B, H, KV, D, window, cap):
