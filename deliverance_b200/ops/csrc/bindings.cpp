@@ -325,12 +325,12 @@ class GemmWeight {
     return out;
   }
   // Prefill-size batches: act(gate) * up in the epilogue of the pair kernel, gate | up rows in plain order. Undefined where that kernel is
-  // not the faster one or does not take the shape.
-  Tensor run_gated(const Tensor& x, int64_t act) {
+  // not the faster one or does not take the shape. impl 3 (as in run): that kernel wherever it takes the shape.
+  Tensor run_gated(const Tensor& x, int64_t act, int64_t impl) {
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.size(1) == desc_.K && x.stride(1) == 1, "x must be bf16 [M, K]");
     TORCH_CHECK(x.device() == w_.device(), "x and weight live on different devices");
     const int M = static_cast<int>(x.size(0));
-    if ((act != 1 && act != 2) || desc_.N % 16 != 0 || !dlv::gemm_pair_preferred(&desc_, M, desc_.N, 3 * desc_.N / 2) || x.stride(0) % 8 != 0 ||
+    if ((act != 1 && act != 2) || desc_.N % 16 != 0 || M == 0 || (impl != 3 && !dlv::gemm_pair_preferred(&desc_, M, desc_.N, 3 * desc_.N / 2)) || x.stride(0) % 8 != 0 ||
         (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) != 0 || !dlv::gemm_pair_act_supported(&desc_, desc_.N, nullptr, desc_.N / 2, false))
       return Tensor();
     c10::cuda::CUDAGuard guard(x.device());
@@ -415,7 +415,7 @@ class GemmWeight {
   // query heads [M, H * 128]; K and V go straight into the cache rows `slots`.
   Tensor run_qkv(const Tensor& x, const Tensor& positions, const Tensor& slots, c10::optional<Tensor> q_norm_w, c10::optional<Tensor> k_norm_w,
                  c10::optional<Tensor> cos_t, c10::optional<Tensor> sin_t, Tensor& k_cache, Tensor& v_cache, int64_t H, int64_t KV, double eps,
-                 double norm_offset, c10::optional<Tensor> bias) {
+                 double norm_offset, c10::optional<Tensor> bias, int64_t impl) {
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.size(1) == desc_.K && x.stride(1) == 1, "x must be bf16 [M, K]");
     TORCH_CHECK(x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0, "x rows must be 16-byte aligned");
     TORCH_CHECK(desc_.N == (H + 2 * KV) * 128, "weight rows must be (H + 2 KV) * 128 (head_dim 128)");
@@ -464,14 +464,14 @@ class GemmWeight {
     Tensor q = new_out({M, H * 128}, x.options());
     if (M == 0) return q;
     DeviceScratch& s = scratch_for(x.device().index());
-    if (dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0) && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
-        desc_.N == (a.heads + 2 * a.kv_heads) * 128 && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a)) {
+    if ((impl == 3 || dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0)) && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a)) {
       Tensor room = expanded();
       dlv::gemm_pair_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
                              room.defined() ? room.data_ptr() : nullptr, s.status.data_ptr<int>(), cur_stream());
       check_last_error("pair gemm (fused q/k/v epilogue) launch");
       return q;
     }
+    TORCH_CHECK(impl != 3, "shape outside the pair kernel");
     dlv::gemm_tc_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
                          s.ws.data_ptr<float>(), static_cast<size_t>(s.ws.numel()), s.counters.data_ptr<int>(),
                          static_cast<int>(s.counters.numel()), s.status.data_ptr<int>(), cur_stream());
@@ -1585,8 +1585,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("gather") = true)
       .def("run_gathered", &GemmWeight::run_gathered, py::arg("x_own"), py::arg("M"), py::arg("out"), py::arg("comm"), py::arg("bias") = py::none())
       .def("run_act", &GemmWeight::run_act, py::arg("x"), py::arg("act"))
-      .def("run_qkv", &GemmWeight::run_qkv)
-      .def("run_gated", &GemmWeight::run_gated, py::arg("x"), py::arg("act"))
+      .def("run_qkv", &GemmWeight::run_qkv, py::arg("x"), py::arg("positions"), py::arg("slots"), py::arg("q_norm_w"), py::arg("k_norm_w"), py::arg("cos_t"),
+           py::arg("sin_t"), py::arg("k_cache"), py::arg("v_cache"), py::arg("H"), py::arg("KV"), py::arg("eps"), py::arg("norm_offset"), py::arg("bias"),
+           py::arg("impl") = 0)
+      .def("run_gated", &GemmWeight::run_gated, py::arg("x"), py::arg("act"), py::arg("impl") = 0)
       .def("run_grouped_gated", &GemmWeight::run_grouped_gated, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("act"))
       .def("run_grouped_act", &GemmWeight::run_grouped_act, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("bn"), py::arg("splits"),
            py::arg("act"))

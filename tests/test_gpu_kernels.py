@@ -721,41 +721,106 @@ def test_pair_gemm_edges(M, N, K, q4):
     assert torch.equal(y, again) and _rel(y.cpu(), yr) < 4e-3
 
 
-@pytest.mark.parametrize("M,inter,K,act", [(2048, 256, 128, "silu"), (2100, 1408, 512, "gelu_pytorch_tanh"), (4097, 640, 320, "silu")])
+@pytest.mark.parametrize("M,N,K,ldx,ldo", [(300, 520, 192, 200, 528), (1030, 1096, 416, 424, 1104)])
+@pytest.mark.parametrize("q4", [True, False])
+def test_pair_gemm_strided(M, N, K, ldx, ldo, q4):
+    """Rows of x and of the output that are parts of wider ones: what lies between them stays as it was. An output that is not 16-byte aligned is refused
+    when the pair kernel is asked for and left to the one-tile kernel otherwise; x that is not aligned is refused by both."""
+    qt, wd = _q4_weight(N, K, seed=N + K)
+    lw = (LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16)
+    wide, room = (torch.randn(M, ldx) * 0.5).to(torch.bfloat16).to(DEV), torch.full((M, ldo), 7.0, dtype=torch.bfloat16, device=DEV)
+    x = wide[:, :K]
+    yr = x.double().cpu() @ (wd if q4 else wd.to(torch.bfloat16)).double().t()
+    ops.linear(x, lw, impl=3, out=room[:, :N])
+    odd = torch.full((M, ldo), 7.0, dtype=torch.bfloat16, device=DEV)
+    with pytest.raises(RuntimeError):
+        ops.linear(x, lw, impl=3, out=odd[:, 4 : 4 + N])
+    ops.linear(x, lw, out=odd[:, 4 : 4 + N])
+    for impl in (0, 3):
+        with pytest.raises(RuntimeError):
+            ops.linear(wide[:, 4 : 4 + K], lw, impl=impl)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert _rel(room[:, :N].cpu(), yr) < 4e-3 and bool((room[:, N:] == 7.0).all())
+    assert _rel(odd[:, 4 : 4 + N].cpu(), yr) < 4e-3 and bool((odd[:, :4] == 7.0).all()) and bool((odd[:, 4 + N :] == 7.0).all())
+
+
+@pytest.mark.parametrize("M,inter,K,act", [(1, 256, 64, "silu"), (255, 264, 128, "silu"), (2048, 256, 128, "silu"), (2100, 1408, 512, "gelu_pytorch_tanh"), (4097, 640, 320, "silu")])
 @pytest.mark.parametrize("q4", [True, False])
 def test_pair_gemm_gated(M, inter, K, act, q4):
+    """One row, ragged last tiles of tokens and outputs, more tiles than pairs of SMs; halves of a JQ4 weight that do not end with a packed tile are refused."""
     qt, wd = _q4_weight(2 * inter, K, seed=inter)
     lw = (LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16)
     x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
-    h = ops.linear_gated(x, lw, act)
+    h = lw.handle().run_gated(x, ops.fused_act_kind(act), 3)
+    assert (h is None) == (q4 and inter % 128 != 0)
+    if h is None:
+        h = ops.linear_gated(x, lw, act)
     torch.cuda.synchronize()
     ops.check_status()
     f = x.double().cpu() @ (wd if q4 else wd.to(torch.bfloat16)).double().t()
     assert _rel(h.cpu(), ref.act_fn(act)(f[:, :inter]) * f[:, inter:]) < 6e-3  # (without the epilogue the projection is rounded once more)
 
 
-@pytest.mark.parametrize("heads,kv,norm,rope", [(4, 1, True, True), (6, 3, False, True), (3, 1, True, False)])
+@pytest.mark.parametrize("M", [1, 255, 257, 2310])
+@pytest.mark.parametrize("heads,kv,norm,rope,bias", [(4, 1, True, True, False), (6, 3, False, True, True), (3, 1, True, False, True)])
 @pytest.mark.parametrize("q4", [True, False])
-def test_pair_gemm_heads(heads, kv, norm, rope, q4):
-    """q | k | v epilogue: an odd number of heads (half a tile at the end), rows without a cache slot, positions behind a prefix."""
-    M, K, D = 2310, 512, 128
+def test_pair_gemm_heads(M, heads, kv, norm, rope, bias, q4):
+    """q | k | v epilogue: an odd number of heads (half a tile at the end), rows without a cache slot, positions behind a prefix, bias; and the one-tile
+    kernel on the same call."""
+    K, D = 512, 128
     qt, wd = _q4_weight((heads + 2 * kv) * D, K, seed=heads)
     lw = (LinearWeight(qt) if q4 else LinearWeight(wd.to(torch.bfloat16))).to(DEV, torch.bfloat16)
-    assert ops.require_ext() is not None
     x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
     pages = M // 32 + 2
-    slots = torch.randperm(pages * 32)[:M].to(DEV)
+    slots = torch.randperm(pages * 32)[:M]
+    slots[M // 3 :: 5] = -1
+    used = torch.zeros(pages * 32, dtype=torch.bool)
+    used[slots[slots >= 0]] = True
+    slots = slots.to(DEV)
     pos = torch.arange(M, dtype=torch.int32, device=DEV) + 37
     cos, sin = (t.to(DEV) for t in ref.rope_tables(D, 4096, 10000.0)) if rope else (None, None)
     qn, kn = ((1 + 0.1 * torch.randn(D)).to(torch.bfloat16).to(DEV) for _ in range(2)) if norm else (None, None)
-    kc, vc = (torch.zeros(pages, kv, 32, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
-    q = ops.linear_rope_kv(x, lw, pos, slots, qn, kn, cos, sin, kc, vc, heads, kv, D, 1e-6)
-    torch.cuda.synchronize()
-    ops.check_status()
-    f = x.float() @ (wd if q4 else wd.to(torch.bfloat16).float()).to(DEV).t()
+    b = torch.randn(wd.shape[0], device=DEV) if bias else None
+    f = x.float() @ (wd if q4 else wd.to(torch.bfloat16).float()).to(DEV).t() + (b if bias else 0.0)
     k2, v2 = (torch.zeros(pages, kv, 32, D, device=DEV) for _ in range(2))
-    qr = ref.qk_prepare_and_cache(f, pos.long(), slots.long(), heads, kv, D, qn, kn, 1e-6, 0.0, cos, sin, k2, v2)
-    assert _rel(q, qr.reshape(M, -1)) < 6e-3 and _rel(kc, k2) < 6e-3 and _rel(vc, v2) < 4e-3
+    scratch = torch.arange(M, device=DEV)  # (the oracle has no rows without a slot)
+    qr = ref.qk_prepare_and_cache(f, pos.long(), scratch, heads, kv, D, qn, kn, 1e-6, 0.0, cos, sin, torch.zeros_like(k2), torch.zeros_like(v2))
+    live = slots >= 0
+    if bool(live.any()):
+        ref.qk_prepare_and_cache(f[live], pos[live].long(), slots[live], heads, kv, D, qn, kn, 1e-6, 0.0, cos, sin, k2, v2)
+    for impl in (3, 0):
+        kc, vc = (torch.zeros(pages, kv, 32, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        q = lw.handle().run_qkv(x, pos, slots, qn, kn, cos, sin, kc, vc, heads, kv, 1e-6, 0.0, b, impl)
+        torch.cuda.synchronize()
+        ops.check_status()
+        assert _rel(q, qr.reshape(M, -1)) < 6e-3
+        for got, want in ((kc, k2), (vc, v2)):
+            rows = got.permute(0, 2, 1, 3).reshape(pages * 32, -1).cpu()
+            assert bool((rows[~used] == 0).all()) and (not bool(used.any()) or _rel(got, want) < 6e-3)
+
+
+@pytest.mark.parametrize("D,T", [(64, 33), (128, 70), (256, 5)])
+def test_rope_kv_unaligned_rows(D, T):
+    """Rows that start on a 2-byte boundary take the element-wise form: as the wide one does, and nothing beside them changes."""
+    H, KV, pages = 4, 2, T // 32 + 1
+    n = T * (H + 2 * KV) * D
+    base = torch.randn(n).to(torch.bfloat16).to(DEV)
+    room = torch.full((n + 2,), 7.0, dtype=torch.bfloat16, device=DEV)
+    odd = room[1 : 1 + n].view(T, -1)
+    odd.copy_(base.view(T, -1))
+    assert odd.data_ptr() % 8 == 2 and odd.is_contiguous()
+    slots, pos = torch.randperm(pages * 32)[:T].to(DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+    cos, sin = (t.to(DEV) for t in ref.rope_tables(D, 128, 10000.0))
+    w = (1 + 0.1 * torch.randn(D)).to(torch.bfloat16).to(DEV)
+    got = []
+    for t in (base.view(T, -1).clone(), odd):
+        kc, vc = (torch.zeros(pages, KV, 32, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        ops.rope_kv(t, pos, slots, w, w, cos, sin, kc, vc, H, KV, D, 1e-6)
+        got.append((t, kc, vc))
+    torch.cuda.synchronize()
+    assert all(_rel(a, b) < 1e-3 for a, b in zip(*got))  # (the sum of a head's squares is added in another order: a bf16 step here and there)
+    assert room[0].item() == 7.0 and room[-1].item() == 7.0
 
 
 @pytest.mark.parametrize("E,n,K,T,k", [(4, 512, 256, 700, 2), (3, 768, 1216, 1500, 1), (3, 512, 64, 900, 2), (40, 1280, 160, 9000, 2)])
