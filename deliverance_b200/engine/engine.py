@@ -125,7 +125,7 @@ class Engine:
         self.waiting: list[Request] = []
         self.running: list[Request] = []
         self._next_id = 0
-        self._graphs: dict[int, dict] = {}
+        self._graphs: dict[int, dict] = {}  # per batch bucket; steps whose sequences differ much in length have their own, under -bucket
         self._failed: list[Request] = []  # requests failed inside a step (reported by step())
         self._prefill_streak = 0
         self.metrics = {"steps": 0, "prefill_steps": 0, "decode_steps": 0, "prefill_tokens": 0, "decode_tokens": 0,
@@ -617,12 +617,19 @@ class Engine:
                 best, best_eff = s, eff
         return best
 
+    def _even(self, lens: list[int]) -> bool:
+        """Which of two captured steps a decode batch takes: the one for sequences of like length or the other. Batches whose attention is launched alike
+        in both cases have one only."""
+        kv, splits = self.model.n_kv, self._splits(len(lens))
+        return splits <= ops.decode_room(len(lens), getattr(self.model, "n_heads", kv), kv, getattr(self.cfg, "head_dim", 0) or 128) or ops.even_lengths(lens)
+
     def _graph_decode(self, seqs: list[dict], dev_tokens: Optional[torch.Tensor] = None) -> torch.Tensor:
         B = len(seqs)
         bucket = next(b for b in _BUCKETS if b >= B)
-        g = self._graphs.get(bucket)
+        even = self._even([s["start"] + 1 for s in seqs] + [1] * (bucket - B))
+        g = self._graphs.get(bucket if even else -bucket)
         if g is None:
-            g = self._capture(bucket)
+            g = self._capture(bucket, even)
         # stage inputs in pinned host buffers, one H2D copy per tensor
         # Two staging sets used in turn: the H2D copies below are asynchronous, and with lookahead decode the host stages step
         # N + 1 while the copies of step N may still be queued. A set is reused for step N + 2, which is staged only after the
@@ -682,7 +689,7 @@ class Engine:
         self.metrics["kernel_launches"] += g["launches"]
         return g["logits"]
 
-    def _capture(self, bucket: int) -> dict:
+    def _capture(self, bucket: int, even: bool) -> dict:
         dev = self.device
         batch = ForwardBatch(
             token_ids=torch.zeros(bucket, dtype=torch.int32, device=dev),
@@ -695,6 +702,7 @@ class Engine:
             is_decode=True,
             logits_rows=torch.arange(bucket, dtype=torch.int64, device=dev),
             decode_splits=self._splits(bucket),
+            decode_even=even,
             state_slots=torch.zeros(bucket, dtype=torch.int64, device=dev) if self.hybrid else None,
             prev_ids=torch.zeros(bucket, dtype=torch.int32, device=dev) if self.needs_prev else None,
         )
@@ -723,7 +731,7 @@ class Engine:
         } for _ in range(2)]
         g = {"graph": graph, "batch": batch, "logits": logits, "host": host, "launches": launches, "calls": 0,
              "bt_owners": [[None] * bucket, [None] * bucket]}
-        self._graphs[bucket] = g
+        self._graphs[bucket if even else -bucket] = g
         return g
 
     # ------------------------------------------------------------------------------------------------ sampling / stops

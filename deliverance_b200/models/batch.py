@@ -21,6 +21,7 @@ class ForwardBatch:
     tile_seq: Optional[torch.Tensor] = None  # prefill tiling (64 query rows per tile)
     tile_q0: Optional[torch.Tensor] = None
     decode_splits: int = 1
+    decode_even: bool = False  # decode: the sequences are known to be of like length (``ops.even_lengths``); a hint for the attention's splits
     state_slots: Optional[torch.Tensor] = None  # [S] int64 recurrent-state slot per sequence (mamba layers)
     q_len_host: list = field(default_factory=list)
     ctx_len_host: list = field(default_factory=list)
@@ -43,6 +44,19 @@ class ForwardBatch:
             self._tiles[rows] = got
         return got
 
+    def decode_plan(self, layer: int, *args):
+        """``ops.decode_plan`` for the decode attention of this layer: worked out by the first layer of a step that asks for these arguments and kept for
+        the layers behind it. A layer that is not behind the one that asked first belongs to another step, whose lengths may be others; the tensor is
+        the batch's and stays."""
+        key = ("decode",) + args[1:]
+        first, plan = self.plans.get(key, (layer, None))
+        if layer <= first:
+            from ..ops import decode_plan
+
+            plan = decode_plan(*args, out=plan)
+            self.plans[key] = (layer, plan)
+        return plan
+
     @property
     def num_tokens(self) -> int:
         return int(self.token_ids.shape[0])
@@ -58,7 +72,7 @@ def make_batch(seqs: list[dict], page_size: int, device, max_pages: Optional[int
     Each entry: ``{"tokens": [new token ids], "start": first position, "pages": [page ids], "state_slot": int}``. An entry may
     carry ``"prev"``, the token in front of its first one (-1 at the start of a sequence): ``prev_ids`` is then filled.
     """
-    from ..ops import prefill_tiles
+    from ..ops import even_lengths, prefill_tiles
 
     toks, pos, slots, qs, ql, cl = [], [], [], [], [], []  # toks / pos / slots: one tensor per sequence
     width = max_pages or max(1, max(len(s["pages"]) for s in seqs))
@@ -125,5 +139,5 @@ def make_batch(seqs: list[dict], page_size: int, device, max_pages: Optional[int
         token_ids=t(toks, torch.int32), positions=t(pos, torch.int32), slots=t(slots, torch.int64), q_start=t(qs, torch.int32),
         q_len=t(ql, torch.int32), ctx_len=t(cl, torch.int32), block_tables=bt.to(dev, non_blocking=True), is_decode=is_decode,
         logits_rows=t(last, torch.int64), tile_seq=t(ts, torch.int32) if ts else None, tile_q0=t(t0, torch.int32) if ts else None,
-        state_slots=state_slots, q_len_host=ql, ctx_len_host=cl, prev_ids=prev_ids,
+        state_slots=state_slots, q_len_host=ql, ctx_len_host=cl, prev_ids=prev_ids, decode_even=is_decode and even_lengths(cl),
     )

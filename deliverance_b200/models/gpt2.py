@@ -49,7 +49,7 @@ class Gpt2Model(DecoderModel):
                             cfg.head_dim, cfg.norm_eps, 0.0)
             if batch.is_decode:
                 a = ops.decode_attention(q, k_cache, v_cache, batch.block_tables, batch.ctx_len, self.n_heads, cfg.scale, 0.0, 0,
-                                         batch.decode_splits)
+                                         batch.decode_splits, even=batch.decode_even, plan=lambda *a: batch.decode_plan(i, *a))
             else:
                 a = ops.prefill_attention(q, k_cache, v_cache, batch.block_tables, batch.q_start, batch.q_len, batch.ctx_len,
                                           self.n_heads, cfg.scale, 0.0, 0, True, batch.tile_seq, batch.tile_q0, tiles_for=batch.tiles)

@@ -110,7 +110,7 @@ class GroupedAttention:
                         raise ValueError(f"values of {v.shape[1]} columns cannot be mixed with {first.shape[1]}")
                 gop.rope_heads_kv(s, p, batch.positions, batch.slots, self.cos, self.sin, k_cache, v_cache, self.q_norm, self.k_norm, self.eps, first, self.lam)
         with stage("groupedattention.score_value"):
-            return gop.attention(s, p, batch, k_cache, v_cache, self.scale, self.softcap, self.window, self.keep_first, self.sink, self._splits(batch), self.mult, out, self.mix)
+            return gop.attention(s, p, batch, k_cache, v_cache, self.scale, self.softcap, self.window, self.keep_first, self.sink, self._splits(batch), self.mult, out, self.mix, run)
 
     def _splits(self, batch: ForwardBatch) -> int:
         """Split-KV factor of a decode step: a captured step knows the window but not the contexts it will see."""

@@ -376,7 +376,8 @@ class DecoderModel:
         with self._stage("causalselfattention.score_value"):
             if batch.is_decode:
                 a = ops.decode_attention(q, k_cache, v_cache, batch.block_tables, batch.ctx_len, self.n_heads, cfg.scale,
-                                         cfg.attn_softcap, window, batch.decode_splits)
+                                         cfg.attn_softcap, window, batch.decode_splits, even=batch.decode_even,
+                                         plan=lambda *a: batch.decode_plan(i, *a))
             else:
                 a = ops.prefill_attention(q, k_cache, v_cache, batch.block_tables, batch.q_start, batch.q_len, batch.ctx_len,
                                           self.n_heads, cfg.scale, cfg.attn_softcap, window, True, batch.tile_seq, batch.tile_q0, tiles_for=batch.tiles)

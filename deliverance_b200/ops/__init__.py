@@ -519,13 +519,48 @@ def set_decode_merge_in_kernel(on: bool) -> None:
         ext().decode_merge_in_kernel(bool(on))
 
 
-def decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, H, scale, softcap=0.0, window=0, splits=1, impl=0):
+def even_lengths(lens) -> bool:
+    """Whether no sequence is more than 1.5 times as long as the mean of a decode batch."""
+    return not lens or 2 * max(lens) * len(lens) <= 3 * sum(lens)
+
+
+def decode_room(B: int, H: int, KV: int, D: int, sms: int = 148) -> int:
+    """Splits of decode attention that ``B`` sequences of like length have use for: 1 where (sequence, KV head) pairs make up 0.7 of the resident CTAs (us,
+    unsplit against split as the engine asks: 512 pairs x 2176 keys 88 / 100, 1024 pairs of 256-wide heads 310 / 331), otherwise two waves of CTAs (128 pairs
+    of 300 to 3000 keys: 4 splits 26.6, 9 splits 26.9, 2 splits 29.0)."""
+    pairs, room = max(1, B * KV * ((H // KV + 15) // 16)), sms * (1 if D > 128 else 2)
+    return 1 if pairs * 10 >= room * 7 else 2 * room // pairs
+
+
+def decode_plan(ctx_lens, B: int, H: int, KV: int, D: int, splits: int, window: int = 0, keep_first: int = 0, out=None):
+    """How many of ``splits`` every sequence of a decode step takes, by its length and the batch's: first column of int32 ``[B, 32]`` on the device, the same for all
+    layers with this window and these heads (``D``: the wider of keys and values)."""
+    _count()
+    return require_ext().decode_plan(ctx_lens, B, H, KV, D, splits, window, keep_first, out)
+
+
+def decode_launch(splits: int, even: bool, plan, ctx_lens, B: int, H: int, KV: int, D: int, window: int, *keep):
+    """``(splits, plan)`` that decode attention is launched with when the caller allows ``splits``. No more than :func:`decode_room` where the lengths are known
+    to be alike: CTAs that only find out that they are not used, and a merge of nothing behind them, take 3 us of 91 (64 x 2176 keys, 8 KV heads). Otherwise all of
+    them, and where that is more than the batch has use for, a plan gives them to the sequences that are long."""
+    room = decode_room(B, H, KV, D)
+    if splits <= room or B == 0:
+        return max(1, splits), None
+    return (room, None) if even else (splits, (plan or decode_plan)(ctx_lens, B, H, KV, D, splits, window, *keep))
+
+
+def decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, H, scale, softcap=0.0, window=0, splits=1, impl=0, even=False, plan=None):
     """One query row per sequence against the paged cache. q ``[B, H*D]`` -> ``[B, H*D]``. ``impl`` 0 = tensor-core kernel
-    (GQA group as MMA rows) when the shape allows, 1 = CUDA-core kernel."""
+    (GQA group as MMA rows) when the shape allows, 1 = CUDA-core kernel. ``splits``: most parts a sequence's keys are cut into; the tensor-core kernel uses as
+    many of them as the lengths have use for (:func:`decode_launch`). ``even``: the lengths are known to be alike (``even_lengths``); a wrong hint costs time only.
+    ``plan``: called with the arguments of :func:`decode_plan`, returns its result (``ForwardBatch.decode_plan`` keeps it for the layers of a step)."""
     if _cuda(q):
+        used = None
         merged = impl == 0 and _MERGE_IN_KERNEL[0] and H // k_cache.shape[1] <= 16  # the last-arriving CTA merges the splits
+        if impl == 0 and not merged:
+            splits, used = decode_launch(splits, even, plan, ctx_lens, q.shape[0], H, k_cache.shape[1], k_cache.shape[3], int(window))
         _count(1 if splits <= 1 or merged else 2)
-        return require_ext().decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, H, scale, softcap, window, splits, impl)
+        return require_ext().decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, H, scale, softcap, window, splits, impl, used=used)
     B = q.shape[0]
     D = k_cache.shape[-1]
     qs = torch.arange(B)

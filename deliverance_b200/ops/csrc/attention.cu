@@ -261,6 +261,39 @@ struct DecodeSlices {
 // Of `splits` CTAs per (sequence, KV head) as many work as have min_slices slices each: a short context is not worth a merge.
 __device__ __forceinline__ int decode_used_splits(int slices, int splits, int min_slices) { return max(1, min(splits, slices / min_slices)); }
 
+// The same for batches in which one sequence is much longer than others and more splits are allowed than all of them together have use for. Where the
+// (sequence, KV head) pairs make up 0.7 of the resident CTAs, only what is 1.5 times as long as the mean is cut, into shares of 0.75 of the mean; fewer
+// pairs make two waves together, every sequence by its part of the slices. us, unsplit (or capped by the number of pairs) / all split alike / this: one
+// sequence of 32,000 keys among 31 of 500 to 1500 371 / 95 / 81, among 15 of them 118 / 75 / 61; lengths from 100 to 4000 in 64 sequences 94 / 85 / 81.
+// One launch per step and kind of layer: worked out by every CTA of the attention kernel it took 0.9 us per layer. Every sequence has a line of its own: all CTAs
+// of a layer read it at the same time as the line of the context lengths, and the layer takes 0.5 us longer where one slice of L2 has to serve both.
+__global__ void __launch_bounds__(256) decode_plan_kernel(const int* __restrict__ ctx_lens, int* __restrict__ used, int B, int window, int keep_first, int splits,
+                                                          int groups, int room) {
+  pdl_trigger();
+  __shared__ int sums[2];
+  if (threadIdx.x < 2) sums[threadIdx.x] = 0;
+  pdl_wait();
+  __syncthreads();
+  int total = 0, active = 0;  // slices of the batch; sequences with more than one (a captured step is padded with sequences of one key)
+  for (int b = threadIdx.x; b < B; b += blockDim.x) {
+    const int n = DecodeSlices(ctx_lens[b], window, keep_first).count();
+    total += n;
+    active += n > 1 ? 1 : 0;
+  }
+  if (total > 0) {
+    atomicAdd(&sums[0], total);
+    atomicAdd(&sums[1], active);
+  }
+  __syncthreads();
+  total = max(1, sums[0]);
+  const long long pairs = static_cast<long long>(sums[1]) * groups;
+  const double share = (pairs * 10 >= static_cast<long long>(room) * 7 ? sums[1] * (4.0 / 3.0) : 2.0 * room / groups) / total;
+  for (int b = threadIdx.x; b < B; b += blockDim.x) {
+    const int n = DecodeSlices(ctx_lens[b], window, keep_first).count();
+    used[b * kDecodePlanStride] = decode_used_splits(n, min(splits, static_cast<int>(n * share * (1.0 + 1e-9))), pairs >= 64 ? 16 : 3);  // (1e-9: whole quotients)
+  }
+}
+
 // factor of one output column: out_mult, times sigmoid of the row's gate logit for the head or the column
 template <typename TIO>
 __device__ __forceinline__ float attn_gate(const AttnExtra& x, const TIO* gate, long long row, int h, int col) {
@@ -274,11 +307,20 @@ __device__ __forceinline__ float attn_gate(const AttnExtra& x, const TIO* gate, 
 // all splits twice with dependent loads: 12 us at 64 splits, more than the attention kernel it follows.)
 // EXT: with the options of AttnExtra.
 struct NoExtra {};
-// ctx_lens (nullptr: all splits were used): the attention kernel has used decode_used_splits() of them, one of which writes the output itself.
-template <bool EXT>
+// PLAN: the splits that a sequence uses come from decode_plan_kernel (a parameter that is not there costs the other form nothing: as a run-time
+// choice it was 0.2 to 0.4 us per layer)
+template <bool PLAN>
+struct DecodePlan {
+  const int* used;
+};
+template <>
+struct DecodePlan<false> {};
+// ctx_lens (nullptr: all splits were used): the attention kernel has used decode_used_splits() (PLAN: the plan's number) of them; where that is one, it
+// has written the output itself.
+template <bool EXT, bool PLAN>
 __global__ void decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                     __nv_bfloat16* __restrict__ out, int H, int D, int splits, const int* __restrict__ ctx_lens, int window, int keep_first,
-                                    int min_slices, const std::conditional_t<EXT, AttnExtra, NoExtra> x) {
+                                    int min_slices, const std::conditional_t<EXT, AttnExtra, NoExtra> x, const DecodePlan<PLAN> plan) {
   __shared__ float w_s[256];
   __shared__ float red[2][8];
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
@@ -301,7 +343,8 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
   fetch(0);
   float2 ml = d < splits ? *reinterpret_cast<const float2*>(part_ml + (base + d) * 2) : make_float2(-INFINITY, 0.f);
   if (ctx_lens != nullptr) {  // (the loads above are in flight with this one; what they bring from unused splits is not looked at)
-    splits = decode_used_splits(DecodeSlices(ctx_lens[b], window, keep_first).count(), splits, min_slices);
+    if constexpr (PLAN) splits = plan.used[b * kDecodePlanStride];
+    else splits = decode_used_splits(DecodeSlices(ctx_lens[b], window, keep_first).count(), splits, min_slices);
     if (splits == 1) return;
     if (d >= splits) ml = make_float2(-INFINITY, 0.f);
   }
@@ -373,8 +416,8 @@ static int launch_decode_t(const void* q, long long q_stride, const void* kc, co
                                                       scale, cap, window, splits);
   if (splits > 1) {
     dim3 g2(B, H);
-    launch_pdl(decode_merge_kernel<false>, dim3(g2), dim3(D), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, D, splits,
-               static_cast<const int*>(nullptr), 0, 0, 1, NoExtra{});
+    launch_pdl(decode_merge_kernel<false, false>, dim3(g2), dim3(D), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, D, splits,
+               static_cast<const int*>(nullptr), 0, 0, 1, NoExtra{}, DecodePlan<false>{});
   }
   return 0;
 }
@@ -492,12 +535,13 @@ struct DecodeOptions {
 };
 template <>
 struct DecodeOptions<0> {};
-template <int D, int EXT, int NW>
+template <int D, int EXT, int NW, bool PLAN>
 __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode_attn_mma_kernel(
     const __nv_bfloat16* __restrict__ q, long long q_stride, const __nv_bfloat16* __restrict__ k_cache,
     const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_tables, int bt_stride,
     const int* __restrict__ ctx_lens, __nv_bfloat16* __restrict__ out, float* part_o, float* part_ml, int* __restrict__ arrivals,
-    int H, int KV, int page_size, float scale, float softcap, int window, int splits, int min_slices, const DecodeOptions<EXT> opt) {
+    int H, int KV, int page_size, float scale, float softcap, int window, int splits, int min_slices, const DecodeOptions<EXT> opt,
+    const DecodePlan<PLAN> plan) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
   using L = DecodeMma<D, NW>;
@@ -519,7 +563,9 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
   const int ctx = ctx_lens[b];
   const DecodeSlices list(ctx, window, EXT == 1 ? keep_first : 0);
   const int first_key = list.first_key, kept = list.kept, sl_kept = list.n_kept, sl_skip = list.skip;
-  const int used = arrivals == nullptr ? decode_used_splits(list.count(), splits, min_slices) : splits;
+  int used;
+  if constexpr (PLAN) used = plan.used[b * kDecodePlanStride];
+  else used = arrivals == nullptr ? decode_used_splits(list.count(), splits, min_slices) : splits;
   if (sp >= used) return;
   const int per = (list.count() + used - 1) / used;
   const int s0 = sp * per, s1 = min(list.count(), s0 + per);
@@ -810,62 +856,69 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
   }
 }
 
-template <int D, int EXT>
+template <int D, int EXT, bool PLAN = false>
 static int launch_decode_mma_t(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride,
                                const int* ctx, void* out, float* po, float* pml, int* arrivals, int B, int H, int KV, int page,
-                               float scale, float cap, int window, int splits, cudaStream_t st, int dk = D, int dv = D, AttnExtra x = {}) {
+                               float scale, float cap, int window, int splits, const int* used, cudaStream_t st, int dk = D, int dv = D, AttnExtra x = {}) {
   constexpr int NW = D > 128 ? 6 : 4;
   using L = DecodeMma<D, NW>;
+  using Extra = std::conditional_t<EXT != 0, AttnExtra, NoExtra>;
+  if constexpr (!PLAN) {
+    if (used != nullptr && splits > 1)
+      return launch_decode_mma_t<D, EXT, true>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, nullptr, B, H, KV, page, scale, cap, window, splits, used, st, dk, dv, x);
+  }
   // the in-kernel merge keeps its weights in the warp-merge area of shared memory
   if (splits > 1 && (H / KV) * (splits + 1) > L::kMerge / 4) arrivals = nullptr;
-  // `splits` is an upper bound. Where (sequence, KV head) pairs alone fill 0.7 of the resident CTAs, splitting them only adds a merge (us, unsplit
-  // against what the engine asks for: 512 pairs x 2176 keys 88 / 100, 1024 pairs of 256-wide heads 310 / 331, 128 of those 42 / 63); fewer pairs
-  // are split to at most two waves (128 pairs of 300..3000 keys: 4 splits 26.6, 9 splits 26.9, 2 splits 29.0), and no CTA takes less than 16
-  // slices (128 pairs x 576 keys: 13.5 / 21.0), or 3 where a few sequences have the GPU to themselves (8 pairs x 777 keys: 16 splits 5.4, 32 splits 6.6).
-  const long long pairs = static_cast<long long>(B) * KV * ((H / KV + 15) / 16), room = static_cast<long long>(gemm_num_sms()) * (D > 128 ? 1 : 2);
-  if (arrivals == nullptr) splits = pairs * 10 >= room * 7 ? 1 : static_cast<int>(splits < 2 * room / pairs ? splits : 2 * room / pairs);
-  const int min_slices = pairs >= 64 ? 16 : 3;
+  // `splits` is an upper bound. No CTA takes less than 16 slices (128 pairs x 576 keys: 13.5 us against 21.0), or 3 where a few sequences have the GPU to
+  // themselves (8 pairs x 777 keys: 16 splits 5.4, 32 splits 6.6).
+  const int min_slices = static_cast<long long>(B) * KV * ((H / KV + 15) / 16) >= 64 ? 16 : 3;
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
-    cudaFuncSetAttribute(decode_attn_mma_kernel<D, EXT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+    cudaFuncSetAttribute(decode_attn_mma_kernel<D, EXT, NW, PLAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
   }
   dim3 grid(B, KV * ((H / KV + 15) / 16), splits);
   DecodeOptions<EXT> opt;
   if constexpr (EXT != 0) opt = {dk, dv, x};
-  launch_pdl(decode_attn_mma_kernel<D, EXT, NW>, dim3(grid), dim3(NW * 32), L::kBytes, st, static_cast<const __nv_bfloat16*>(q), q_stride,
+  DecodePlan<PLAN> plan;
+  if constexpr (PLAN) plan.used = used;
+  launch_pdl(decode_attn_mma_kernel<D, EXT, NW, PLAN>, dim3(grid), dim3(NW * 32), L::kBytes, st, static_cast<const __nv_bfloat16*>(q), q_stride,
                                                           static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(vc), bt,
                                                           bt_stride, ctx, static_cast<__nv_bfloat16*>(out), po, pml, arrivals, H, KV, page, scale,
-                                                          cap, window, splits, min_slices, opt);
+                                                          cap, window, splits, min_slices, opt, plan);
   if (splits > 1 && arrivals == nullptr) {
     dim3 g2(B, H);
     const dim3 block((dv + 31) / 32 * 32);
     const int keep = EXT == 1 ? x.keep_first : 0;
-    if constexpr (EXT != 0) launch_pdl(decode_merge_kernel<true>, g2, block, 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, ctx, window, keep,
-                                       min_slices, x);
-    else launch_pdl(decode_merge_kernel<false>, g2, block, 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, ctx, window, keep, min_slices, NoExtra{});
+    Extra extra;
+    if constexpr (EXT != 0) extra = x;
+    launch_pdl(decode_merge_kernel<EXT != 0, PLAN>, g2, block, 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits, ctx, window, keep, min_slices, extra, plan);
   }
   return 0;
 }
 
+void launch_decode_plan(const int* ctx_lens, int* used, int B, int window, int keep_first, int splits, int groups, int D, cudaStream_t st) {
+  if (B > 0) launch_pdl(decode_plan_kernel, dim3(1), dim3(256), 0, st, ctx_lens, used, B, window, keep_first, splits, groups, gemm_num_sms() * (D > 128 ? 1 : 2));
+}
+
 void launch_decode_merge(const float* po, const float* pml, void* out, int B, int H, int dv, int splits, AttnExtra x, cudaStream_t st) {
-  launch_pdl(decode_merge_kernel<true>, dim3(B, H), dim3((dv + 31) / 32 * 32), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits,
-             static_cast<const int*>(nullptr), 0, 0, 1, x);
+  launch_pdl(decode_merge_kernel<true, false>, dim3(B, H), dim3((dv + 31) / 32 * 32), 0, st, po, pml, static_cast<__nv_bfloat16*>(out), H, dv, splits,
+             static_cast<const int*>(nullptr), 0, 0, 1, x, DecodePlan<false>{});
 }
 
 // impl: 0 = tensor-core kernel when it applies (group <= 16, page_size % 16 == 0), 1 = CUDA-core kernel
 int launch_decode_attention_impl(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride,
                                  const int* ctx, void* out, float* po, float* pml, int* arrivals, int B, int H, int KV, int D, int page,
-                                 float scale, float cap, int window, int splits, int impl, cudaStream_t st) {
+                                 float scale, float cap, int window, int splits, const int* used, int impl, cudaStream_t st) {
   if (B == 0) return 0;
   const int G = H / KV;
   if (impl == 0 && G <= 16 && page % 16 == 0 && (q_stride % 2) == 0) {
     switch (D) {
       case 64: return launch_decode_mma_t<64, 0>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, arrivals, B, H, KV, page, scale, cap, window, splits,
-                                                st);
+                                                used, st);
       case 128: return launch_decode_mma_t<128, 0>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, arrivals, B, H, KV, page, scale, cap, window, splits,
-                                                st);
+                                                used, st);
       case 256: return launch_decode_mma_t<256, 0>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, arrivals, B, H, KV, page, scale, cap, window, splits,
-                                                st);
+                                                used, st);
       default: return 1;
     }
   }
@@ -874,16 +927,16 @@ int launch_decode_attention_impl(const void* q, long long q_stride, const void* 
 
 int launch_decode_attention_mma(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride, const int* ctx, void* out,
                                 float* po, float* pml, int B, int H, int KV, int dk, int dv, int page, float scale, float cap, int window, AttnExtra x,
-                                int splits, cudaStream_t st) {
+                                int splits, const int* used, cudaStream_t st) {
   if (B == 0) return 0;
   const int D = dk > dv ? dk : dv;
   if (dk % 8 != 0 || dv % 8 != 0 || D > 256 || page % 16 != 0 || q_stride % 8 != 0) return 1;
   const bool plain = dk == dv && H / KV <= 16 && x.keep_first == 0;  // only the epilogue differs from the plain kernel
 #define DLV_DEC_MMA(DD)                                                                                                                                  \
   return plain && dk == DD ? launch_decode_mma_t<DD, 2>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, nullptr, B, H, KV, page, scale, cap,      \
-                                                        window, splits, st, dk, dv, x)                                                                    \
+                                                        window, splits, used, st, dk, dv, x)                                                                    \
                            : launch_decode_mma_t<DD, 1>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, nullptr, B, H, KV, page, scale, cap,      \
-                                                        window, splits, st, dk, dv, x)
+                                                        window, splits, used, st, dk, dv, x)
   if (D <= 64) DLV_DEC_MMA(64);
   if (D <= 128) DLV_DEC_MMA(128);
   DLV_DEC_MMA(256);

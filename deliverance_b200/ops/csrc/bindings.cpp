@@ -814,7 +814,7 @@ dlv::AttnExtra attn_extra(const Tensor& q, int64_t keep_first, const c10::option
 
 Tensor decode_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& block_tables, const Tensor& ctx_lens,
                         int64_t H, double scale, double softcap, int64_t window, int64_t splits, int64_t impl, int64_t keep_first, c10::optional<Tensor> sink,
-                        c10::optional<Tensor> gate, double out_mult, c10::optional<Tensor> out_opt) {
+                        c10::optional<Tensor> gate, double out_mult, c10::optional<Tensor> out_opt, c10::optional<Tensor> used_opt) {
   TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && q.dim() == 2 && q.stride(1) == 1, "q must be bf16 [B, H*D]");
   check_bf16(k_cache, "k_cache");
   check_bf16(v_cache, "v_cache");
@@ -832,6 +832,12 @@ Tensor decode_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_
   const dlv::AttnExtra x = attn_extra(q, keep_first, sink, gate, out_mult, out_opt, B, H, DV);
   Tensor out = out_opt.has_value() ? out_opt.value() : new_out({B, H * DV}, q.options());
   if (splits < 1) splits = 1;
+  const int* used = nullptr;
+  if (used_opt.has_value()) {
+    const Tensor& u = used_opt.value();
+    TORCH_CHECK(u.is_cuda() && u.scalar_type() == at::kInt && u.is_contiguous() && u.numel() == static_cast<int64_t>(B) * dlv::kDecodePlanStride && u.device() == q.device(), "used splits must come from decode_plan");
+    used = u.data_ptr<int>();
+  }
   Tensor po, pml;
   float *pop = nullptr, *pmlp = nullptr;
   if (splits > 1) {
@@ -845,7 +851,7 @@ Tensor decode_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_
     const int rc = dlv::launch_decode_attention_mma(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr<int>(),
                                                     static_cast<int>(block_tables.stride(0)), ctx_lens.data_ptr<int>(), out.data_ptr(), pop, pmlp, B,
                                                     static_cast<int>(H), KV, D, DV, page, static_cast<float>(scale), static_cast<float>(softcap),
-                                                    static_cast<int>(window), x, static_cast<int>(splits), cur_stream());
+                                                    static_cast<int>(window), x, static_cast<int>(splits), used, cur_stream());
     TORCH_CHECK(rc == 0, "decode attention: head widths must be multiples of 8 up to 256");
     check_last_error("decode_attention");
     return out;
@@ -854,10 +860,24 @@ Tensor decode_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_
   int rc = dlv::launch_decode_attention_impl(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), block_tables.data_ptr<int>(),
                                              static_cast<int>(block_tables.stride(0)), ctx_lens.data_ptr<int>(), out.data_ptr(), pop, pmlp, arrivals, B,
                                              static_cast<int>(H), KV, D, page, static_cast<float>(scale), static_cast<float>(softcap),
-                                             static_cast<int>(window), static_cast<int>(splits), static_cast<int>(impl), cur_stream());
+                                             static_cast<int>(window), static_cast<int>(splits), used, static_cast<int>(impl), cur_stream());
   TORCH_CHECK(rc == 0, "decode attention: unsupported head_dim / group size (code ", rc, ")");
   check_last_error("decode_attention");
   return out;
+}
+
+// How many of `splits` every sequence of a decode step takes (first column of int32 [B, 32]) for decode_attention's `used`. Head width: the wider of keys and values.
+Tensor decode_plan(const Tensor& ctx_lens, int64_t B, int64_t H, int64_t KV, int64_t D, int64_t splits, int64_t window, int64_t keep_first,
+                   c10::optional<Tensor> out) {
+  check_cuda(ctx_lens, "ctx_lens");
+  TORCH_CHECK(ctx_lens.scalar_type() == at::kInt && ctx_lens.numel() >= B && B >= 0 && KV > 0 && H % KV == 0 && splits >= 1 && keep_first >= 0, "bad decode plan arguments");
+  c10::cuda::CUDAGuard guard(ctx_lens.device());
+  Tensor used = out.has_value() ? out.value() : new_out({B, dlv::kDecodePlanStride}, ctx_lens.options());
+  TORCH_CHECK(used.scalar_type() == at::kInt && used.is_contiguous() && used.numel() == B * dlv::kDecodePlanStride && used.device() == ctx_lens.device(), "bad out");
+  dlv::launch_decode_plan(ctx_lens.data_ptr<int>(), used.data_ptr<int>(), static_cast<int>(B), static_cast<int>(window), static_cast<int>(keep_first),
+                          static_cast<int>(splits), static_cast<int>(KV * ((H / KV + 15) / 16)), static_cast<int>(D), cur_stream());
+  check_last_error("decode_plan");
+  return used;
 }
 
 Tensor prefill_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& block_tables, const Tensor& q_start,
@@ -1615,7 +1635,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rope_kv", &rope_kv);
   m.def("decode_attention", &decode_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_tables"), py::arg("ctx_lens"),
         py::arg("H"), py::arg("scale"), py::arg("softcap") = 0.0, py::arg("window") = 0, py::arg("splits") = 1, py::arg("impl") = 0,
-        py::arg("keep_first") = 0, py::arg("sink") = py::none(), py::arg("gate") = py::none(), py::arg("out_mult") = 1.0, py::arg("out") = py::none());
+        py::arg("keep_first") = 0, py::arg("sink") = py::none(), py::arg("gate") = py::none(), py::arg("out_mult") = 1.0, py::arg("out") = py::none(),
+        py::arg("used") = py::none());
+  m.def("decode_plan", &decode_plan, py::arg("ctx_lens"), py::arg("B"), py::arg("H"), py::arg("KV"), py::arg("D"), py::arg("splits"), py::arg("window") = 0,
+        py::arg("keep_first") = 0, py::arg("out") = py::none());
   m.def("prefill_attention", &prefill_attention);
   m.def("prefill_attention_tc", &prefill_attention_tc, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_tables"), py::arg("q_start"),
         py::arg("q_len"), py::arg("ctx_lens"), py::arg("tile_seq"), py::arg("tile_q0"), py::arg("H"), py::arg("scale"), py::arg("softcap"), py::arg("window"),

@@ -157,11 +157,14 @@ int launch_decode_attention(const void* q, long long q_stride, const void* kc, c
                             float cap, int window, int splits, cudaStream_t st);
 int launch_decode_attention_impl(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride,
                                  const int* ctx, void* out, float* po, float* pml, int* arrivals, int B, int H, int KV, int D, int page,
-                                 float scale, float cap, int window, int splits, int impl, cudaStream_t st);
+                                 float scale, float cap, int window, int splits, const int* used, int impl, cudaStream_t st);
+constexpr int kDecodePlanStride = 32;
+// used: int32 [B] with this stride, how many of the splits every sequence takes (nullptr: as many as its own length has use for); groups: CTAs per sequence of head width D
+void launch_decode_plan(const int* ctx_lens, int* used, int B, int window, int keep_first, int splits, int groups, int D, cudaStream_t st);
 // tensor-core decode kernel with separate key and value widths (multiples of 8, at most 256) and any group size; 1: unsupported shape
 int launch_decode_attention_mma(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride, const int* ctx, void* out,
                                 float* po, float* pml, int B, int H, int KV, int dk, int dv, int page, float scale, float cap, int window, AttnExtra x,
-                                int splits, cudaStream_t st);
+                                int splits, const int* used, cudaStream_t st);
 // one CTA per (row, query head) on CUDA cores, fp32 or bf16, any width; row_seq: sequence of every row (nullptr: row number)
 // wide: queries of dk columns against whole cache rows k [pages, 1, page, dk], values v [pages, 1, page, KV * dv]
 int launch_attention_rows(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride, const int* row_seq,

@@ -158,10 +158,10 @@ def rope_heads_kv(s: GroupedShape, p, positions, slots, cos, sin, k_cache, v_cac
 
 
 def attention(s: GroupedShape, qkv, batch, k_cache, v_cache, scale: float, softcap: float, window: int, keep_first: int, sink, splits: int, mult: float = 1.0,
-              out=None, mix=None):
+              out=None, mix=None, run: int = 0):
     """Heads of every row of the batch, ``[T, H * dv]`` (``out``: a column range of wider rows to write to); the batch's keys and values are
     in the cache already. ``sink``: fp32 ``[H]`` or None. Gated shapes multiply with the sigmoid of their logits in ``qkv``, all with ``mult``.
-    ``mix``: fp32 ``[H, H]`` of shapes with mixed scores."""
+    ``mix``: fp32 ``[H, H]`` of shapes with mixed scores. ``run``: place of this mixer among the layers of the step."""
     q = qkv[:, : s.q_width]
     gate = qkv[:, s.gate_at : s.gate_at + s.gate_logits] if s.gate else None
     if not ops._cuda(qkv):
@@ -181,8 +181,10 @@ def attention(s: GroupedShape, qkv, batch, k_cache, v_cache, scale: float, softc
         ops._count()
         return e.attention_rows(q, k_cache, v_cache, batch.block_tables, None if batch.is_decode else row_sequence(batch), batch.positions, s.heads, *mask, **extra)
     if batch.is_decode:
+        splits, used = ops.decode_launch(splits, batch.decode_even, lambda *a: batch.decode_plan(run, *a), batch.ctx_len, q.shape[0], s.heads, s.kv_heads,
+                                         max(s.dk, s.dv), int(window), int(keep_first))
         ops._count(1 if splits <= 1 else 2)
-        return e.decode_attention(q, k_cache, v_cache, batch.block_tables, batch.ctx_len, s.heads, *mask, splits, 0, **extra)
+        return e.decode_attention(q, k_cache, v_cache, batch.block_tables, batch.ctx_len, s.heads, *mask, splits, 0, used=used, **extra)
     ts, t0 = batch.tiles(e.prefill_tc_tile_rows(max(s.dk, s.dv)))
     ops._count()
     return e.prefill_attention_tc(q, k_cache, v_cache, batch.block_tables, batch.q_start, batch.q_len, batch.ctx_len, ts, t0, s.heads, *mask, True, **extra)

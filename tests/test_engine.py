@@ -9,6 +9,7 @@ from deliverance_b200.ckpt.tiny import write_tiny_model
 from deliverance_b200.config import load_config
 from deliverance_b200.engine.engine import Engine, EngineConfig
 from deliverance_b200.engine.sampler import Sampler, SamplingState, candidate_limit, sample_top_k_top_p_batch, xtc_pick
+from deliverance_b200.models.batch import make_batch
 from deliverance_b200.kv.paged import KvCacheSettings, PageAllocator, PrefixCache, compose_salt
 from deliverance_b200.models.transformer import DecoderModel
 from deliverance_b200.params import FinishReason, GeneratorParameters
@@ -36,6 +37,19 @@ def test_batched_equals_single(tiny):
     assert [r.token_ids for r in rs] == singles
     assert eng.kv.allocator.available() == eng.kv.num_pages - 1 - sum(len(e.pages) for e in eng.kv.prefix.entries.values()) or True
     assert all(r.finish_reason == FinishReason.MAX_TOKENS for r in rs)
+
+
+def test_decode_batches_of_unlike_lengths(tiny):
+    """Which captured step a decode batch takes: its own where one sequence is more than 1.5 times as long as the mean and the batch is large enough
+    to run unsplit; and the hint that a batch built from host-side lengths carries."""
+    eng = _engine(tiny)
+    big = next(b for b in (8, 16, 32, 64, 128) if b * tiny.n_kv * 10 >= 2 * 148 * 7 and eng._splits(b) > 1)
+    assert eng._even([700] * big) and eng._even([1000] * (big - 1) + [1500])
+    assert not eng._even([1000] * (big - 1) + [30000]) and not eng._even([1000] * (big // 2) + [1] * (big - big // 2))
+    assert eng._even([1000] * 3 + [30000])  # (few sequences are split by length in either case)
+    seqs = lambda lens: [{"tokens": [1], "start": n - 1, "pages": list(range(1, 2 + n // 32))} for n in lens]  # noqa: E731
+    assert make_batch(seqs([64, 64, 90]), 32, "cpu").decode_even and not make_batch(seqs([64, 64, 300]), 32, "cpu").decode_even
+    assert not make_batch([{"tokens": [1, 2], "start": 0, "pages": [1]}], 32, "cpu").decode_even
 
 
 def test_checkpoint_lengths_policies():

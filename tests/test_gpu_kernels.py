@@ -903,6 +903,58 @@ def test_decode_attention_used_splits(B, H, KV, D, window, cap):
         assert d.max().item() < 6e-3, (splits, d)
 
 
+def _paged(ctx, KV, D, seed=0):
+    """Random paged cache for sequences of these lengths: k, v, block table, context lengths on the GPU (page 0 is nobody's)."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    per = [(c + 31) // 32 for c in ctx]
+    bt = torch.zeros(len(ctx), max(per), dtype=torch.int32)
+    order = torch.randperm(sum(per), generator=torch.Generator().manual_seed(seed)).to(torch.int32) + 1
+    for i, n in enumerate(per):
+        bt[i, :n] = order[sum(per[:i]):sum(per[:i]) + n]
+    kc, vc = (torch.randn(sum(per) + 1, KV, 32, D, device=DEV, generator=g, dtype=torch.bfloat16) for _ in range(2))
+    return kc, vc, bt.to(DEV), torch.tensor(ctx, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("B,H,KV,D,short,long", [(40, 32, 8, 128, 200, 6000), (10, 32, 8, 128, 40, 3000), (130, 8, 4, 64, 64, 9000), (24, 16, 8, 256, 300, 5000)])
+@pytest.mark.parametrize("window,cap", [(0, 0.0), (1000, 30.0)])
+def test_decode_attention_one_long_sequence(B, H, KV, D, short, long, window, cap):
+    """A batch whose pairs occupy the GPU unsplit, or nearly do, with one sequence many times longer than the others, padded sequences of one key among
+    them: the long one is cut, whatever the batch. bf16 probabilities and output: 2^-9 each."""
+    ctx = [short + (37 * i) % 50 for i in range(B)]
+    ctx[B // 2] = long
+    ctx[B - B // 8 :] = [1] * (B // 8)
+    kc, vc, bt, cl = _paged(ctx, KV, D)
+    q = torch.randn(B, H * D).to(torch.bfloat16).to(DEV)
+    r = ref.paged_attention(q.reshape(B, H, D).float().cpu(), kc.float().cpu(), vc.float().cpu(), bt.cpu(), torch.arange(B), torch.ones(B, dtype=torch.long), cl.cpu(),
+                            D**-0.5, cap, window)
+    for splits, even in ((1, False), (3, False), (32, False), (9, True)):
+        o = ops.decode_attention(q, kc, vc, bt, cl, H, D**-0.5, cap, window, splits, even=even)
+        torch.cuda.synchronize()
+        d = (o.cpu().float() - r.reshape(B, -1)).norm(dim=1) / r.reshape(B, -1).norm(dim=1)
+        assert d.max().item() < 6e-3, (splits, even, d)
+
+
+def test_decode_attention_long_sequence_is_cut():
+    """The splits that a caller allows are used for a sequence that is much longer than the rest: its keys do not pass through one CTA per KV head
+    (measured: 4.6 times as long at these sizes; two times are asked for)."""
+    B, H, KV, D = 32, 32, 8, 128
+    kc, vc, bt, cl = _paged([500] * (B - 1) + [24000], KV, D)
+    q = torch.randn(B, H * D).to(torch.bfloat16).to(DEV)
+
+    def best(splits):
+        times = []
+        for _ in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            ops.decode_attention(q, kc, vc, bt, cl, H, D**-0.5, 0.0, 0, splits)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    assert best(8) * 2 < best(1)
+
+
 @pytest.mark.parametrize("T", [1, 7, 1183, 1185])
 @pytest.mark.parametrize("H", [8, 1024, 2048, 2056, 2560, 3584, 4096, 4104, 8192, 8200])
 def test_rmsnorm_widths(T, H):

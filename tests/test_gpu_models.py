@@ -187,6 +187,21 @@ def test_generate_gpu_graphs_vs_eager(tmp_path, family):
     assert res[0] == res[1]
 
 
+def test_captured_steps_of_unlike_lengths(tmp_path):
+    """64 sequences, one of them much longer: their decode steps are captured apart from those of like lengths and give the same tokens as uncaptured ones."""
+    cfg, cpu, gpu = _pair(tmp_path, "qwen3")
+    g = torch.Generator().manual_seed(4)
+    prompts = [torch.randint(3, 250, (140 if i == 9 else 12,), generator=g).tolist() for i in range(64)]
+    res, keys = [], []
+    for graphs in (False, True):
+        eng = Engine(gpu, EngineConfig(num_pages=256, cuda_graphs=graphs, max_batch_tokens=1024, max_seqs=64))
+        res.append([r.token_ids for r in eng.generate_batch(prompts, GeneratorParameters(max_tokens=6))])
+        eng.generate_batch([p[:12] for p in prompts], GeneratorParameters(max_tokens=3))
+        keys = sorted(eng._graphs)
+        ops.check_status(0)
+    assert res[0] == res[1] and {-64, 64} <= set(keys)
+
+
 @pytest.mark.parametrize("family", ["qwen3", "gemma2", "mixtral", "qwen3_moe"])
 def test_fused_activation_models_gpu(tmp_path, family, monkeypatch):
     """Models loaded with the interleaved gate|up layout (activation in the GEMM epilogue) against the default layout."""
