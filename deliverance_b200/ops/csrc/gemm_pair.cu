@@ -447,7 +447,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             const float* uf = reinterpret_cast<const float*>(uv);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              const float x = gf[j];
+              // (rows behind the last one hold zeros; a division of zero leaves the straight path for a call, for all 32 rows of the warp: 300 rows
+              // of 11264 x 2048 took 69 us where 512 take 40)
+              const float x = live ? gf[j] : 1.f;
               const float a = p.act_kind == 2 ? 0.5f * x * (1.f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x))) : x / (1.f + __expf(-x));
               gf[j] = a * uf[j];
             }
