@@ -481,16 +481,16 @@ class DecoderModel:
         if lw.fused_act:
             with self._stage("mlpblock.gate_up_projection"):
                 h = ops.linear_act(x, lw.gate_up, cfg.hidden_act)
-        elif self._sp is None and not lw.lora:
-            with self._stage("mlpblock.gate_up_projection"):  # a handful of rows, or a prompt: projection and gated activation in one launch
-                h = ops.linear_gated(x, lw.gate_up, cfg.hidden_act)
         else:
             with self._stage("mlpblock.gate_up_projection"):
-                gu = self._col_parallel(x, lw.gate_up)
+                # a handful of rows, or a prompt: projection and gated activation in one launch
+                h = ops.linear_gated_fused(x, lw.gate_up, cfg.hidden_act) if self._sp is None and not lw.lora else None
+                gu = self._col_parallel(x, lw.gate_up) if h is None else None
                 if lw.lora:
                     gu = self._lora(lw, "gate_up", x, gu)
-            with self._stage("mlpblock.activation_multiply"):
-                h = ops.act_mul(gu, cfg.hidden_act)
+            if h is None:
+                with self._stage("mlpblock.activation_multiply"):
+                    h = ops.act_mul(gu, cfg.hidden_act)
         with self._stage("mlpblock.down_projection"):
             if norm_after is not None and not lw.lora:
                 x2 = self._row_parallel_norm(h, lw.down, norm_after)

@@ -272,21 +272,27 @@ def interleave_gate_up(gate, up, block: int = 64):
     return mix(gate, up.to(gate.dtype))
 
 
+def linear_gated_fused(x: torch.Tensor, w: LinearWeight, act: str) -> Optional[torch.Tensor]:
+    """:func:`linear_gated` in one kernel, or ``None`` where that takes two."""
+    if not _cuda(x) or x.dtype != torch.bfloat16 or w.bias is not None:
+        return None
+    kind = fused_act_kind(act)
+    out = None
+    if kind and x.shape[0] > GEMV_MAX_ROWS:
+        out = w.handle().run_gated(x, kind)
+    elif kind and w.q4:
+        out = w.handle().run_gemv_act(x, kind)
+    if out is not None:
+        _count()
+    return out
+
+
 def linear_gated(x: torch.Tensor, w: LinearWeight, act: str) -> torch.Tensor:
     """``act(x @ Wg^T) * (x @ Wu^T)`` for a weight that holds the gate rows followed by the up rows (plain order). One kernel for
     1..8 rows of a JQ4 weight on CUDA (the small-batch GEMV's epilogue) and for prompt-size batches (the pair kernel's), projection +
     activation kernel otherwise."""
-    if _cuda(x) and x.dtype == torch.bfloat16 and w.bias is None:
-        kind = fused_act_kind(act)
-        out = None
-        if kind and x.shape[0] > GEMV_MAX_ROWS:
-            out = w.handle().run_gated(x, kind)
-        elif kind and w.q4:
-            out = w.handle().run_gemv_act(x, kind)
-        if out is not None:
-            _count()
-            return out
-    return act_mul(linear(x, w), act)
+    out = linear_gated_fused(x, w, act)
+    return out if out is not None else act_mul(linear(x, w), act)
 
 
 def linear_act(x: torch.Tensor, w: LinearWeight, act: str, block: int = 64) -> torch.Tensor:

@@ -83,6 +83,20 @@ def test_layer_trace_hook(tmp_path):
     assert (-1, "embed", (5, 64)) in seen and (1, "out", (5, 64)) in seen
 
 
+@pytest.mark.parametrize("rows", [3, 11])
+def test_profiler_reports_the_activation_of_its_own(tmp_path, rows):
+    """The gated activation is a stage of its own wherever it is a step of its own (here always: no kernel does both on a CPU)."""
+    from deliverance_b200.utils.profiler import InferenceProfiler
+
+    d = str(tmp_path / "p")
+    write_tiny_model(d, "llama", seed=5)
+    m, eng = _ours(d)
+    m.profiler = InferenceProfiler("cpu")
+    eng.generate((PROMPT * 3)[:rows], GeneratorParameters(max_tokens=1))
+    s = m.profiler.summary()
+    assert all(f"[profile] mlpblock.{name} count={len(m.layers)} " in s for name in ("gate_up_projection", "activation_multiply", "down_projection"))
+
+
 def test_gemma3_multimodal_wrapper_config_and_prefix(tmp_path):
     """A gemma3 checkpoint in the multimodal layout (nested text_config with most fields left to defaults, wrapper tensor prefix,
     old-style rope_local_base_freq / sliding_window_pattern) loads as its text tower."""
