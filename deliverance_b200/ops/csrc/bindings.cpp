@@ -240,11 +240,17 @@ class GemmWeight {
     dlv::gemm_weight_init(&desc_);
   }
 
-  // room for the bf16 form of a JQ4 weight in front of a prompt-size product; it belongs to this call and goes back to the allocator
-  // behind it in stream order
-  Tensor expanded() const {
+  // Room for the bf16 form of a JQ4 weight (2 N K bytes) in front of a prompt-size product; it belongs to this call and goes back to the
+  // allocator behind it in stream order. false: there is no memory for it (the one-tile kernel, which needs none, takes the product).
+  bool expanded(Tensor& room) const {
     const size_t bytes = dlv::gemm_pair_expanded_bytes(&desc_);
-    return bytes > 0 ? at::empty({static_cast<int64_t>(bytes)}, w_.options().dtype(at::kByte)) : Tensor();
+    if (bytes == 0) return true;
+    try {
+      room = new_out({static_cast<int64_t>(bytes)}, w_.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {
+      return false;
+    }
+    return true;
   }
 
   // out[m, :] = x[m, :] @ W^T (+ bias). impl: 0 = auto, 1 = tcgen05, 2 = CUDA-core GEMV, 3 = tcgen05 on pairs of SMs
@@ -272,14 +278,14 @@ class GemmWeight {
     }
     if (M == 0) return out;
     const bool pair = impl == 3 || (impl == 0 && force_splits == 0 && dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0));
-    if (pair && !out_f32 && dlv::gemm_pair_supported(&desc_, desc_.N, out.data_ptr(), static_cast<int>(out.stride(0)), false, 0)) {
-      Tensor room = expanded();
+    Tensor room;
+    if (pair && !out_f32 && dlv::gemm_pair_supported(&desc_, desc_.N, out.data_ptr(), static_cast<int>(out.stride(0)), false, 0) && expanded(room)) {
       dlv::gemm_pair_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), bptr,
                          room.defined() ? room.data_ptr() : nullptr, scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
       check_last_error("pair gemm launch");
       return out;
     }
-    TORCH_CHECK(impl != 3, "shape outside the pair kernel");
+    TORCH_CHECK(impl != 3, "shape outside the pair kernel, or no memory for the weight's bf16 form");
     const bool simt = impl == 2 || (impl == 0 && M <= 1 && !desc_.is_q4);
     if (simt) {
       dlv::gemv_simt_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), out_f32,
@@ -334,8 +340,8 @@ class GemmWeight {
         (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) != 0 || !dlv::gemm_pair_act_supported(&desc_, desc_.N, nullptr, desc_.N / 2, false))
       return Tensor();
     c10::cuda::CUDAGuard guard(x.device());
-    Tensor out = new_out({M, desc_.N / 2}, x.options());
-    Tensor room = expanded();
+    Tensor out = new_out({M, desc_.N / 2}, x.options()), room;
+    if (!expanded(room)) return Tensor();
     dlv::gemm_pair_run_act(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), static_cast<int>(act),
                            room.defined() ? room.data_ptr() : nullptr, scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
     check_last_error("pair gemm (gated activation) launch");
@@ -464,14 +470,15 @@ class GemmWeight {
     Tensor q = new_out({M, H * 128}, x.options());
     if (M == 0) return q;
     DeviceScratch& s = scratch_for(x.device().index());
-    if ((impl == 3 || dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0)) && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a)) {
-      Tensor room = expanded();
+    Tensor room;
+    if ((impl == 3 || dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0)) && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a) &&
+        expanded(room)) {
       dlv::gemm_pair_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
                              room.defined() ? room.data_ptr() : nullptr, s.status.data_ptr<int>(), cur_stream());
       check_last_error("pair gemm (fused q/k/v epilogue) launch");
       return q;
     }
-    TORCH_CHECK(impl != 3, "shape outside the pair kernel");
+    TORCH_CHECK(impl != 3, "shape outside the pair kernel, or no memory for the weight's bf16 form");
     dlv::gemm_tc_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
                          s.ws.data_ptr<float>(), static_cast<size_t>(s.ws.numel()), s.counters.data_ptr<int>(),
                          static_cast<int>(s.counters.numel()), s.status.data_ptr<int>(), cur_stream());

@@ -721,6 +721,73 @@ def test_pair_gemm_edges(M, N, K, q4):
     assert torch.equal(y, again) and _rel(y.cpu(), yr) < 4e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(255, 264, 64), (257, 520, 192), (300, 1408, 2592)])
+def test_pair_gemm_room_is_guarded(M, N, K):
+    """The bf16 form of a JQ4 weight lies between guard areas like an output: the newest guarded buffer of a product with an output of the caller's. Ragged
+    rows and k of the weight write nothing beside it."""
+    ext = ops.require_ext()
+    qt, _ = _q4_weight(N, K, seed=N + K)
+    lw = LinearWeight(qt).to(DEV, torch.bfloat16)
+    x, out = torch.randn(M, K).to(torch.bfloat16).to(DEV), torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.set_bounds_check(True)
+    try:
+        ops.linear(x, lw, impl=3, out=out)
+        torch.cuda.synchronize()
+        ops.check_guards()
+        ops.linear(x, lw, impl=3, out=out)
+        ext.poke_last_guard()
+        with pytest.raises(RuntimeError, match=f"{2 * N * K}"):
+            ops.check_guards()
+        if lw.handle().run_gated(x, 1, 3) is not None:
+            ops.check_guards()
+    finally:
+        ops.set_bounds_check(False)
+
+
+def test_pair_gemm_without_room():
+    """A JQ4 weight whose bf16 form finds no memory: products run as they do without the pair kernel, which needs none. (The allocator's limit is what
+    refuses; the GPU has plenty.)"""
+    M, N, K, H, KV = 2048, 8192, 4096, 48, 8
+    qt, _ = _q4_weight(N, K, seed=3)
+    lw = LinearWeight(qt).to(DEV, torch.bfloat16)
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    pos = torch.arange(M, dtype=torch.int32, device=DEV)
+    cos, sin = (t.to(DEV) for t in ref.rope_tables(128, M, 10000.0))
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+
+    def products(kc, vc):
+        ops.linear(x, lw, out=out)
+        sums = out.cpu()
+        gated = ops.linear_gated(x, lw, "silu").cpu()
+        q = ops.linear_rope_kv(x, lw, pos, pos.long(), None, None, cos, sin, kc, vc, H, KV, 128, 1e-6)
+        return [sums, gated, q.cpu(), kc.cpu(), vc.cpu()]
+
+    caches = lambda: [torch.zeros(M // 32, KV, 32, 128, dtype=torch.bfloat16, device=DEV) for _ in range(2)]  # noqa: E731
+    ops.linear(x[:256], lw)  # (workspaces)
+    try:
+        ops.set_gemm_pairs(0)
+        want = products(*caches())
+        ops.set_gemm_pairs(-1)
+        kv = caches()
+        torch.cuda.empty_cache()
+        before = torch.cuda.memory_stats()["num_ooms"]
+        # enough for the 32 MB output of a product with its 16 MB activation, not for the 64 MB of the weight
+        total = torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (56 << 20)) / total)
+        got = products(*kv)
+        refused = torch.cuda.memory_stats()["num_ooms"] - before
+        with pytest.raises(RuntimeError):
+            ops.linear(x, lw, impl=3, out=out)
+        torch.cuda.synchronize()
+        ops.check_status()
+    finally:
+        ops.set_gemm_pairs(-1)
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert refused >= 3
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 1e-6  # (the same kernels)
+
+
 @pytest.mark.parametrize("M,N,K,ldx,ldo", [(300, 520, 192, 200, 528), (1030, 1096, 416, 424, 1104)])
 @pytest.mark.parametrize("q4", [True, False])
 def test_pair_gemm_strided(M, N, K, ldx, ldo, q4):
