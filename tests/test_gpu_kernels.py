@@ -1042,6 +1042,30 @@ def test_decode_attention_long_sequence_is_cut():
     assert best(8) * 2 < best(1)
 
 
+@pytest.mark.parametrize("lo,hi", [(4, 180), (184, 252), (256, 508)])
+def test_decode_attention_softcap_error(lo, hi):
+    """Probabilities of capped scores against 64 bits where a step of fp32 shows: a cap of 2^20, exact scores of lo / 512 to hi / 512 of it. The tensor-core
+    kernel, which has a series for small scores, is no further off than the CUDA-core kernel, which calls tanhf for all."""
+    D, n, cap = 64, 64, float(2**20)
+    first = torch.arange(lo, hi + 1, 4).float()
+    B = len(first)
+    q, k = torch.zeros(B, D), torch.zeros(B, n, D)
+    q[:, 0], q[:, 1] = 2048.0, 1.0
+    k[:, :, 0], k[:, :, 1] = first[:, None], torch.arange(n) / 16.0
+    kc, vc = (torch.cat([torch.zeros(1, 1, 32, D), t.reshape(2 * B, 1, 32, D)]).to(torch.bfloat16).to(DEV) for t in (k, torch.eye(D).repeat(B, 1)))
+    bt = torch.arange(1, 1 + 2 * B, dtype=torch.int32, device=DEV).view(B, 2)
+    cl = torch.full((B,), n, dtype=torch.int32, device=DEV)
+    s = 2048.0 * k[:, :, 0].double() + k[:, :, 1].double()
+    want = torch.log_softmax(cap * torch.tanh(s / cap), -1)
+    err = []
+    for impl in (0, 1):
+        p = ops.decode_attention(q.to(torch.bfloat16).to(DEV), kc, vc, bt, cl, 1, 1.0, cap, 0, 1, impl)
+        d = p.double().cpu().log() - want
+        err.append((d - d.mean(1, keepdim=True)).pow(2).mean().sqrt().item())
+    # (bf16 probabilities and outputs: 2^-9 each at most, about 0.0016 together, in either kernel; the kernels round them in another order)
+    assert err[0] < 1.1 * err[1] + 0.0016, err
+
+
 @pytest.mark.parametrize("T", [1, 7, 1183, 1185])
 @pytest.mark.parametrize("H", [8, 1024, 2048, 2056, 2560, 3584, 4096, 4104, 8192, 8200])
 def test_rmsnorm_widths(T, H):
