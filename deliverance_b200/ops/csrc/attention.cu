@@ -484,8 +484,8 @@ __device__ __forceinline__ uint32_t swz(int row, int chunk) {
 //   states are merged through shared memory at the end. A slice never straddles a page (page_size % 16 == 0); lanes look up the
 //   rows of the next 32 slices at once, so that no copy waits for the block table.
 // What bounds it: the K / V stream. NW 4 with three stages and two CTAs per SM for heads up to 128; 6 warps with two stages for 256-wide heads
-// (192 KB of rings; with four warps and three stages the chain of one slice set the pace: 128 x 1920 keys x 8 heads 617 us, now 333, of
-// 303 at the copy rate). (The splits as a thread-block cluster that merges through distributed shared memory, instead of a second launch:
+// (192 KB of rings; with four warps and three stages the chain of one slice set the pace: 128 x 1920 keys x 8 heads, soft-capped with
+// a tanhf per score, 734 us, now 304, of 303 at the copy rate). (The splits as a thread-block cluster that merges through distributed shared memory, instead of a second launch:
 // 106 us against 101 at 64 x 2176 keys, 10 against 6 at one sequence, because the CTAs of a cluster start and leave together. Not kept.)
 template <int D, int NW>
 struct DecodeMma {
@@ -499,7 +499,8 @@ struct DecodeMma {
 };
 
 // cap * tanh(s / cap) of a lane's eight scores: the series up to x^11 where all of the warp's arguments are below 0.35 (what it leaves out is
-// 1.2e-8 of the value there), tanhf otherwise. (tanhf's division and branch per score were a third of the slice's instructions.)
+// 1.2e-8 of the value there), tanhf otherwise. (tanhf's division and branch per score were a third of the
+// slice's instructions: 128 x 1920 keys, 256-wide heads, 304 us by the series and 380 to 450 where most warps have a score beyond it.)
 __device__ __forceinline__ void softcap_slice(float (&f)[2][4], float cap) {
   const float inv = 1.f / cap;
   float mx = 0.f;
