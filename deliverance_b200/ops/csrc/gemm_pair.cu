@@ -18,6 +18,11 @@
 // row order needs no interleaving; 2 = q | k | v heads of 128: per-head RMSNorm, rotation, paged cache write.
 // Grouped mode (experts): a work list of (expert, first row, end row) items of 256 rows takes the place of the token tiles.
 //
+// It starts in ordinary stream order, behind the whole of the kernel in front, so that no role waits for that kernel; the kernel behind it may be set
+// up early.
+//
+// 8192 x 19456 x 2560 in bf16: 516 us (590 at the power cap), the one-tile kernel 917 to 1154, cuBLAS 520 to 670 in the same runs.
+//
 // The reference multiplies prompts token by token on the CPU (native/src/main/c/simd/vector_simd.c:595).
 #include <stdexcept>
 #include <string>
@@ -213,7 +218,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == 0) {
     // ---------------- token copies ----------------
     if (lane == 0) {
-      pdl_wait();  // the tokens (and a work list) come from the kernels in front
       int g = 0;   // 64-k steps of this pair, numbered across tiles
       bool ok = true;
       for (int t = pair; t < total && ok; t += pairs) {
@@ -233,7 +237,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   } else if (warp == 3) {
     // ---------------- weight copies ----------------
     if (lane == 0) {
-      if (p.items != nullptr) pdl_wait();  // weights alone may stream under the kernel in front
       int g = 0;
       bool ok = true;
       for (int t = pair; t < total && ok; t += pairs) {
@@ -264,14 +267,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   } else if (warp == 1) {
     // ---------------- MMA issuer of the pair ----------------
     if (rank == 0) {
-      if (p.items != nullptr) pdl_wait();
       constexpr uint32_t idesc = umma_idesc_bf16(kTokens, kWRows);
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(smem));
       const bool leader = elect_one();
       int it = 0, s = 0;
       uint32_t ph = 0;
       bool ok = true, ready = false;  // ready: the next step's operands have been seen complete
-      
       for (int t = pair; t < total && ok; t += pairs) {
         const Tile tl = tile_of(t);
         if (tl.m0 < 0) continue;
@@ -280,10 +281,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (!ok) break;
         const uint32_t acc = tmem_base + b * kWRows;
         for (int k = 0; k < p.nk; ++k) {
-          
           if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[s]), ph, abort_flag, p.status));
           if (!ok) break;
-          
           tc_fence_after();
           const uint64_t da = desc0 + static_cast<uint64_t>((s * kStageBytes) >> 4), db = da + (kOpBytes >> 4);
           if (leader) {
@@ -298,13 +297,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             umma_bf16_pair(acc, da + 6, db + 6, idesc, 1u);
             umma_commit_pair(bar_done);
           }
-          
         }
         if (!ok) break;
         if (leader) umma_commit_pair(smem_u32(&bar_acc_full[b]));
         ++it;
       }
-      
       if (!ok && leader) {
         umma_commit_pair(smem_u32(bar_last));
         const unsigned long long t0 = globaltimer_ns();
@@ -316,7 +313,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   } else if (warp >= 8) {
     // ---------------- JQ4: packed stage -> bf16 operand tile ----------------
     if constexpr (Q4) {
-      if (p.items != nullptr) pdl_wait();
       const int grp = (warp - 8) >> 2, h = grp & 1, r = threadIdx.x & 127;  // group, half of the 128-k stage, weight row
       int j = 0;   // 128-k stages of this pair, numbered across tiles
       int g0 = 0;  // 64-k step of the tile's first stage
@@ -366,7 +362,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
   } else if (warp >= 4) {
     // ---------------- drain: accumulator -> global memory ----------------
-    pdl_wait();  // global memory is written only after the kernel in front has completed
     const int q = warp & 3;
     uint8_t* buf = smem + L::kOffDrain + q * 4096;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -657,8 +652,9 @@ bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ld
 // Whether the pair kernel is faster than the one-tile kernel (gemm_tc.cuh) for M rows of this weight. Both times in microseconds, by whole
 // waves of tiles: a 64-k step takes 0.29 us of a 256 x 256 tile here, 0.5 us (JQ4: 0.42) of a 128 x 256 tile there, which can split k over
 // up to eight CTAs where tiles are few (333 rows of 2560 x 9728: 31 us against 45). Expanding a JQ4 weight first writes 2 bytes per weight
-// that push others out of L2: 36 us for 19456 x 2560, so that 4-bit weights come here from about 1500 rows on. `merged`: outputs per row that
-// the epilogue saves a later kernel from reading and writing.
+// that push others out of L2: 36 us for 19456 x 2560. `merged`: outputs per row that the epilogue saves a later kernel from reading and writing.
+// So 4-bit weights come here from 769 (gated 19456 x 2560), 1537 (6144 x 2560), 1793 (2560 x 4096) or 2817 rows (2560 x 9728) on, bf16 ones from 192 (the
+// gated one), 257 or 769.
 bool gemm_pair_preferred(const GemmWeightDesc* w, int M, int n, int merged) {
   if (M < 192 || n < kWRows || g_gemm_persist || g_gemm_force_bn != 0) return false;  // (the last two: another kernel or tile was asked for)
   const double nk = (w->K + 63) / 64;
