@@ -117,6 +117,8 @@ def _experts_cuda(st, lw, x, logits, E, k, mode, renorm, act, e0, ne):
     gu_w, down_w = lw.experts_gate_up_grouped, lw.experts_down_grouped
     f32 = x.dtype == torch.float32
     bn = 64 if f32 else ops.moe_token_tile(rows if not ep else max(1, rows * ne // E), ne, gu_w.q4)
+    if bn == 256 and not lw.fused_act_experts:
+        bn = min(gu_w.prompt_rows(), down_w.prompt_rows())
     if lw.fused_act_experts:
         bn = max(bn, 16)  # interleaved expert rows exist for the tensor-core grouped GEMM's epilogue only
     max_items = min((rows + bn - 1) // bn + ne, rows) if rows >= ne else rows
@@ -174,7 +176,7 @@ def _experts_cuda(st, lw, x, logits, E, k, mode, renorm, act, e0, ne):
         if hmid is None:
             with st("moe.gate_up"):
                 xs = gathered()
-                hmid = gu_w.run_gated(xs, items, act) if bn == 256 else None
+                hmid = gu_w.run_gated(xs, items, act, bn) if bn >= 256 else None
                 gu = gu_w.run(xs, items, bn, k_splits(gu_w)) if hmid is None else None
             if hmid is None:
                 with st("moe.activation_multiply"):

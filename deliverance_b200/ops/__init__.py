@@ -723,10 +723,14 @@ class GroupedLinearWeight:
         _count()
         return out
 
-    def run_gated(self, xs: torch.Tensor, items: torch.Tensor, act: str) -> Optional[torch.Tensor]:
-        """Prompt-size work items (256 rows): gate|up projection of plain-order rows with ``act(gate) * up`` in the epilogue, or ``None``."""
+    def prompt_rows(self) -> int:
+        """Rows of a prompt-size work item, at most: 256, or the widest tile of the kernel that expands JQ4 weights once per item."""
+        return 384 if self.q4 and self.handle.wide_items(self.N) else 256
+
+    def run_gated(self, xs: torch.Tensor, items: torch.Tensor, act: str, rows: int = 256) -> Optional[torch.Tensor]:
+        """Prompt-size work items (of ``rows`` rows): gate|up projection of plain-order rows with ``act(gate) * up`` in the epilogue, or ``None``."""
         kind = fused_act_kind(act)
-        out = self.handle.run_grouped_gated(xs, items, self.N, kind) if kind and self.handle is not None else None
+        out = self.handle.run_grouped_gated(xs, items, self.N, kind, rows) if kind and self.handle is not None else None
         if out is not None:
             _count()
         return out

@@ -253,7 +253,22 @@ class GemmWeight {
     return true;
   }
 
-  // out[m, :] = x[m, :] @ W^T (+ bias). impl: 0 = auto, 1 = tcgen05, 2 = CUDA-core GEMV, 3 = tcgen05 on pairs of SMs
+  // Whether the JQ4 pair kernel takes a product of M rows, and its room for partial sums (as above). impl 4 asks for it, 0 where it is the faster one.
+  bool parts(int64_t impl, int M, const void* out, int64_t ldo, int epi, Tensor& room) const {
+    if ((impl != 4 && (impl != 0 || !dlv::gemm_parts_preferred(&desc_, M, epi))) || !dlv::gemm_parts_supported(&desc_, desc_.N, out, static_cast<int>(ldo), epi)) return false;
+    const size_t floats = dlv::gemm_parts_room(&desc_, M, epi);
+    if (floats == 0) return true;
+    try {
+      room = new_out({static_cast<int64_t>(floats)}, w_.options().dtype(at::kFloat));
+    } catch (const c10::OutOfMemoryError&) {
+      return false;
+    }
+    return true;
+  }
+  static float* floats(const Tensor& room) { return room.defined() ? room.data_ptr<float>() : nullptr; }
+
+  // out[m, :] = x[m, :] @ W^T (+ bias). impl: 0 = auto, 1 = tcgen05, 2 = CUDA-core GEMV, 3 = tcgen05 on pairs of SMs, 4 = the same with JQ4 weights
+  // expanded inside the kernel and tiles cut over k
   Tensor run(const Tensor& x, c10::optional<Tensor> out_opt, c10::optional<Tensor> bias, bool out_f32, int64_t impl,
              int64_t force_splits) {
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2, "x must be bf16 [M, K] on CUDA");
@@ -277,8 +292,15 @@ class GemmWeight {
       bptr = b.data_ptr<float>();
     }
     if (M == 0) return out;
-    const bool pair = impl == 3 || (impl == 0 && force_splits == 0 && dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0));
     Tensor room;
+    if (force_splits == 0 && parts(impl, M, out.data_ptr(), out.stride(0), 0, room)) {
+      dlv::gemm_parts_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), out_f32, bptr, floats(room),
+                           scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
+      check_last_error("JQ4 pair gemm launch");
+      return out;
+    }
+    TORCH_CHECK(impl != 4, "shape outside the JQ4 pair kernel, or no memory for its partial sums");
+    const bool pair = impl == 3 || (impl == 0 && force_splits == 0 && dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0));
     if (pair && !out_f32 && dlv::gemm_pair_supported(&desc_, desc_.N, out.data_ptr(), static_cast<int>(out.stride(0)), false, 0) && expanded(room)) {
       dlv::gemm_pair_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), bptr,
                          room.defined() ? room.data_ptr() : nullptr, scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
@@ -336,6 +358,18 @@ class GemmWeight {
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.size(1) == desc_.K && x.stride(1) == 1, "x must be bf16 [M, K]");
     TORCH_CHECK(x.device() == w_.device(), "x and weight live on different devices");
     const int M = static_cast<int>(x.size(0));
+    if ((act == 1 || act == 2) && desc_.N % 16 == 0 && M > 0 && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0) {
+      c10::cuda::CUDAGuard guard(x.device());
+      Tensor room;
+      if (parts(impl, M, nullptr, desc_.N / 2, 1, room)) {
+        Tensor out = new_out({M, desc_.N / 2}, x.options());
+        dlv::gemm_parts_run_act(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), static_cast<int>(act),
+                                 floats(room), scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
+        check_last_error("JQ4 pair gemm (gated activation) launch");
+        return out;
+      }
+    }
+    if (impl == 4) return Tensor();
     if ((act != 1 && act != 2) || desc_.N % 16 != 0 || M == 0 || (impl != 3 && !dlv::gemm_pair_preferred(&desc_, M, desc_.N, 3 * desc_.N / 2)) || x.stride(0) % 8 != 0 ||
         (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) != 0 || !dlv::gemm_pair_act_supported(&desc_, desc_.N, nullptr, desc_.N / 2, false))
       return Tensor();
@@ -347,16 +381,25 @@ class GemmWeight {
     check_last_error("pair gemm (gated activation) launch");
     return out;
   }
-  // The same for experts (items of 256 rows): [rows, n / 2], or undefined.
-  Tensor run_grouped_gated(const Tensor& xs, const Tensor& items, int64_t n_per_expert, int64_t act) {
+  // The same for experts (items of `item_rows` rows, for bf16 weights 256): [rows, n / 2], or undefined.
+  Tensor run_grouped_gated(const Tensor& xs, const Tensor& items, int64_t n_per_expert, int64_t act, int64_t item_rows) {
     TORCH_CHECK(xs.is_cuda() && xs.scalar_type() == at::kBFloat16 && xs.dim() == 2 && xs.size(1) == desc_.K && xs.stride(1) == 1, "xs must be bf16 [rows, K]");
     TORCH_CHECK(xs.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(xs.data_ptr()) & 15) == 0, "xs rows must be 16-byte aligned");
     TORCH_CHECK(items.is_cuda() && items.scalar_type() == at::kInt && items.dim() == 2 && items.size(1) == 4 && items.is_contiguous(), "items must be int32 [n, 4]");
     const int64_t per = desc_.is_q4 ? ((n_per_expert + 127) / 128) * 128 : n_per_expert;
     TORCH_CHECK(n_per_expert > 0 && desc_.N % per == 0, "stacked weight rows are not a multiple of the per-expert rows");
-    if ((act != 1 && act != 2) || n_per_expert % 16 != 0 || !dlv::gemm_pair_act_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2), true))
-      return Tensor();
+    if ((act != 1 && act != 2) || n_per_expert % 16 != 0 || item_rows < 1) return Tensor();
     c10::cuda::CUDAGuard guard(xs.device());
+    if (dlv::gemm_parts_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2), 1)) {
+      Tensor out = new_out({xs.size(0), n_per_expert / 2}, xs.options());
+      if (xs.size(0) == 0 || items.size(0) == 0) return out;
+      dlv::gemm_parts_run_grouped(&desc_, static_cast<int>(n_per_expert), xs.data_ptr(), static_cast<int>(xs.size(0)), static_cast<int>(xs.stride(0)), out.data_ptr(),
+                                  static_cast<int>(out.stride(0)), items.data_ptr<int>(), static_cast<int>(items.size(0)), static_cast<int>(item_rows),
+                                  static_cast<int>(act), scratch_for(xs.device().index()).status.data_ptr<int>(), cur_stream());
+      check_last_error("JQ4 pair gemm (grouped, gated activation) launch");
+      return out;
+    }
+    if (item_rows != 256 || !dlv::gemm_pair_act_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2), true)) return Tensor();
     Tensor out = new_out({xs.size(0), n_per_expert / 2}, xs.options());
     if (xs.size(0) == 0 || items.size(0) == 0) return out;
     dlv::gemm_pair_run_grouped(&desc_, static_cast<int>(n_per_expert), xs.data_ptr(), static_cast<int>(xs.size(0)), static_cast<int>(xs.stride(0)),
@@ -364,6 +407,11 @@ class GemmWeight {
                                static_cast<int>(act), scratch_for(xs.device().index()).status.data_ptr<int>(), cur_stream());
     check_last_error("pair gemm (grouped, gated activation) launch");
     return out;
+  }
+  // whether work items of more than 256 rows find their kernel (any number: it cuts them into equal tiles)
+  bool wide_items(int64_t n_per_expert) const {
+    c10::cuda::CUDAGuard guard(w_.device());
+    return dlv::gemm_parts_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert), 0);
   }
   bool gemv_ok(int64_t M, int64_t ldx) const { return dlv::gemv_dense_supported(&desc_, static_cast<int>(M), static_cast<int>(ldx)); }
   // Grouped (MoE) GEMM: `this` stacks the local experts' weights (n_per_expert rows each; JQ4: whole 128-row tiles per expert),
@@ -471,6 +519,13 @@ class GemmWeight {
     if (M == 0) return q;
     DeviceScratch& s = scratch_for(x.device().index());
     Tensor room;
+    if (parts(impl, M, q.data_ptr(), q.stride(0), 2, room)) {
+      dlv::gemm_parts_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a, floats(room),
+                               s.status.data_ptr<int>(), cur_stream());
+      check_last_error("JQ4 pair gemm (fused q/k/v epilogue) launch");
+      return q;
+    }
+    TORCH_CHECK(impl != 4, "shape outside the JQ4 pair kernel, or no memory for its partial sums");
     if ((impl == 3 || dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0)) && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a) &&
         expanded(room)) {
       dlv::gemm_pair_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,
@@ -1616,7 +1671,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            py::arg("sin_t"), py::arg("k_cache"), py::arg("v_cache"), py::arg("H"), py::arg("KV"), py::arg("eps"), py::arg("norm_offset"), py::arg("bias"),
            py::arg("impl") = 0)
       .def("run_gated", &GemmWeight::run_gated, py::arg("x"), py::arg("act"), py::arg("impl") = 0)
-      .def("run_grouped_gated", &GemmWeight::run_grouped_gated, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("act"))
+      .def("run_grouped_gated", &GemmWeight::run_grouped_gated, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("act"), py::arg("item_rows") = 256)
+      .def("wide_items", &GemmWeight::wide_items, py::arg("n_per_expert"))
       .def("run_grouped_act", &GemmWeight::run_grouped_act, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("bn"), py::arg("splits"),
            py::arg("act"))
       .def("run_grouped_gemv_act", &GemmWeight::run_grouped_gemv_act, py::arg("xs"), py::arg("items"), py::arg("n_per_expert"), py::arg("act"),

@@ -498,6 +498,10 @@ void gemm_tc_run_grouped(const GemmWeightDesc* w, int n_per_expert, const void* 
   if (rows <= 0 || max_items <= 0) return;
   if (ldx % 8 != 0) throw std::runtime_error("activation row pitch must be a multiple of 8 elements");
   if (max_items > 65535) throw std::runtime_error("grouped gemm: work list too long");
+  if (bn >= 256 && splits <= 1 && gemm_parts_supported(w, n_per_expert, out, ldo, 0)) {
+    gemm_parts_run_grouped(w, n_per_expert, x, rows, ldx, out, ldo, items, max_items, bn, 0, status, st);
+    return;
+  }
   if (bn == 256 && splits <= 1 && gemm_pair_supported(w, n_per_expert, out, ldo, true, 0)) {
     gemm_pair_run_grouped(w, n_per_expert, x, rows, ldx, out, ldo, items, max_items, 0, status, st);
     return;

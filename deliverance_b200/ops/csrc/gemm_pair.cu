@@ -29,6 +29,7 @@
 
 #include "gemm_api.h"
 #include "gemm_tc.cuh"
+#include "pair.cuh"
 
 namespace dlv {
 
@@ -73,44 +74,6 @@ struct PairParams {
   int act_kind;
   GemmQkvArgs qkv;
 };
-
-// ---- cluster / pair forms of the common helpers -----------------------------------------------------------------------
-__device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-// copy into this CTA's shared memory, completion on a barrier of either CTA of the pair
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// arrive on the barrier at this offset in both CTAs once the MMAs issued so far have completed
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-               "h"(static_cast<uint16_t>(3))
-               : "memory");
-}
 
 // Packed JQ4 weight -> bf16 [N, K] in global memory, in front of a product whose rows pay for it. One block per 128 x 128 stage; 16 lanes
 // write a row's 256 bytes. Bound by the 2.6 bytes per weight that it moves, most of which the product finds in L2 again.
@@ -188,7 +151,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == 2) tmem_alloc_pair(smem_u32(tmem_slot), 512);
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();  // the peer's barriers exist before anything arrives on them
+  cluster_meet();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   pdl_trigger();  // (behind the set-up: the next kernel's blocks are not to come between the two CTAs of a pair and their tensor memory)
   const uint32_t tmem_base = *tmem_slot;
@@ -563,12 +526,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();  // no CTA leaves while the pair's MMAs or arrivals may still touch its shared memory
+  cluster_meet();  // no CTA leaves while the pair's MMAs or arrivals may still touch its shared memory
   if (warp == 2) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, 512);
   }
-  cluster_sync_all();  // the release of a pair's tensor memory involves both CTAs: neither leaves before both have asked for it
+  cluster_meet();  // the release of a pair's tensor memory involves both CTAs: neither leaves before both have asked for it
 }
 
 // Pairs of SMs that can hold the kernel at one time on the current GPU, within the limit that is set; 0: none (a GPU or a share of one on
@@ -653,15 +616,18 @@ bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ld
 // waves of tiles: a 64-k step takes 0.29 us of a 256 x 256 tile here, 0.5 us (JQ4: 0.42) of a 128 x 256 tile there, which can split k over
 // up to eight CTAs where tiles are few (333 rows of 2560 x 9728: 31 us against 45). Expanding a JQ4 weight first writes 2 bytes per weight
 // that push others out of L2: 36 us for 19456 x 2560. `merged`: outputs per row that the epilogue saves a later kernel from reading and writing.
-// So 4-bit weights come here from 769 (gated 19456 x 2560), 1537 (6144 x 2560), 1793 (2560 x 4096) or 2817 rows (2560 x 9728) on, bf16 ones from 192 (the
-// gated one), 257 or 769.
+// So bf16 weights come here from 192 (the gated one), 257 or 769 rows on. For 4-bit weights gemm_parts_preferred asks first and leaves prompts of a few thousand
+// rows and more to this kernel.
+static double waves(long long tiles, long long room) { return static_cast<double>((tiles + room - 1) / room); }
+double gemm_pair_estimate(const GemmWeightDesc* w, int M, int n) {
+  const double nk = (w->K + 63) / 64;
+  return 5.0 + waves(static_cast<long long>((M + kTokens - 1) / kTokens) * ((n + 255) / 256), gemm_num_sms() / 2) * (nk * 0.29 + 1.0) +
+         (w->is_q4 ? 2.0 + static_cast<double>(w->N) * w->K * 2.6 / 3.5e6 : 0.0);
+}
 bool gemm_pair_preferred(const GemmWeightDesc* w, int M, int n, int merged) {
   if (M < 192 || n < kWRows || g_gemm_persist || g_gemm_force_bn != 0) return false;  // (the last two: another kernel or tile was asked for)
-  const double nk = (w->K + 63) / 64;
+  const double nk = (w->K + 63) / 64, pair = gemm_pair_estimate(w, M, n);
   const int m_tiles = (M + kTokens - 1) / kTokens, sms = gemm_num_sms();
-  auto waves = [](long long tiles, long long room) { return static_cast<double>((tiles + room - 1) / room); };
-  const double pair = 5.0 + waves(static_cast<long long>(m_tiles) * ((n + 255) / 256), sms / 2) * (nk * 0.29 + 1.0) +
-                      (w->is_q4 ? 2.0 + static_cast<double>(w->N) * w->K * 2.6 / 3.5e6 : 0.0);
   double one = 1e30;
   const long long tiles = static_cast<long long>((n + 127) / 128) * m_tiles;
   for (int s = 1; s <= 8 && (s == 1 || nk / s >= 4); ++s) {

@@ -451,6 +451,11 @@ __global__ void __launch_bounds__(256) moe_items_kernel(const int* __restrict__ 
   for (int e = threadIdx.x; e < ne; e += blockDim.x) {
     const int lo = offsets[e0 + e], hi = offsets[e0 + e + 1];
     int it = first[e];
+    if (bn > 256) {  // wide items: an expert's rows in equal ones, since an item costs its kernel one expansion of the weights whatever its rows
+      const int count = (hi - lo + bn - 1) / bn, per = count > 0 ? (hi - lo + count - 1) / count : 1;
+      for (int r = lo; r < hi && it < max_items; r += per, ++it) items[it] = make_int4(e, r, min(hi, r + per), 0);
+      continue;
+    }
     for (int r = lo; r < hi && it < max_items; r += bn, ++it) items[it] = make_int4(e, r, hi, 0);
   }
   for (int it = first[ne] + threadIdx.x; it < max_items; it += blockDim.x) items[it] = make_int4(-1, 0, 0, 0);

@@ -1089,3 +1089,118 @@ def test_gemv_bf16_row(N, K, f32):
     y = ops.linear(x.to(DEV), LinearWeight(w, bias).to(DEV, torch.bfloat16), out_f32=f32)
     torch.cuda.synchronize()
     assert _rel(y.cpu(), x.double() @ w.double().t() + bias.double()) < (1e-5 if f32 else 4e-3)
+
+
+# As for the pair kernel: fp32 sums rounded to bf16 once, JQ4 products rounded to bf16 twice on top.
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (31, 264, 128), (33, 136, 192), (256, 512, 1280), (257, 2560, 960), (385, 19456, 256), (700, 1000, 2624), (1537, 4104, 512)])
+def test_parts_gemm_edges(M, N, K):
+    """One row; k that ends inside a packed stage; weight tiles that end inside a tile and inside eight outputs; one and two instructions per tile, several tiles of
+    tokens; tiles in equal parts, waves with parts behind them, waves alone; bias; fp32 outputs; repeatable. Rows that are parts of wider ones, with and without 16
+    bytes at once: what lies beside them stays."""
+    qt, wd = _q4_weight(N, K, seed=N + K)
+    lw = LinearWeight(qt).to(DEV, torch.bfloat16)
+    lw.bias = torch.randn(N, device=DEV) if M % 2 else None
+    wide = (torch.randn(M, K + 8) * 0.5).to(torch.bfloat16).to(DEV)
+    x = wide[:, :K]
+    yr = x.double().cpu() @ wd.double().t() + (lw.bias.double().cpu() if lw.bias is not None else 0.0)
+    y, again, y32 = ops.linear(x, lw, impl=4), ops.linear(x, lw, impl=4), ops.linear(x, lw, impl=4, out_f32=True)
+    room = [torch.full((M, N + 24 - N % 8), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+    for at, t in zip((8, 4, 1), room):
+        ops.linear(x, lw, impl=4, out=t[:, at : at + N])
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(y, again) and _rel(y.cpu(), yr) < 4e-3 and _rel(y32.cpu(), yr) < 4e-3
+    for at, t in zip((8, 4, 1), room):
+        assert torch.equal(t[:, at : at + N], y) and bool((t[:, :at] == 7.0).all()) and bool((t[:, at + N :] == 7.0).all())
+    with pytest.raises(RuntimeError):
+        ops.linear(wide[:, 4 : 4 + K], lw, impl=4)
+
+
+def test_parts_gemm_refuses():
+    """K that ends inside 64, bf16 weights, no pair of SMs: refused when asked for, left to the other kernels otherwise."""
+    for qt, wd in (_q4_weight(512, 96),):
+        lw, dense = LinearWeight(qt).to(DEV, torch.bfloat16), LinearWeight(wd.to(torch.bfloat16)).to(DEV, torch.bfloat16)
+    ok = LinearWeight(_q4_weight(512, 128)[0]).to(DEV, torch.bfloat16)
+    x, x2 = torch.randn(300, 96).to(torch.bfloat16).to(DEV), torch.randn(300, 128).to(torch.bfloat16).to(DEV)
+    for w in (lw, dense):
+        with pytest.raises(RuntimeError):
+            ops.linear(x, w, impl=4)
+        assert w.handle().run_gated(x, 1, 4) is None and _rel(ops.linear(x, w).cpu(), x.float().cpu() @ wd.t()) < 1e-2
+    try:
+        ops.set_gemm_pairs(0)
+        with pytest.raises(RuntimeError):
+            ops.linear(x2, ok, impl=4)
+        one = ops.linear(x2, ok)
+        ops.set_gemm_pairs(3)
+        few = ops.linear(x2, ok, impl=4)
+    finally:
+        ops.set_gemm_pairs(-1)
+    assert _rel(one, few) < 6e-3
+
+
+@pytest.mark.parametrize("M,inter,K,act", [(1, 64, 64, "silu"), (65, 192, 128, "gelu_pytorch_tanh"), (333, 9728, 320, "silu"), (513, 4096, 64, "silu"), (1100, 1408, 512, "gelu_pytorch_tanh")])
+def test_parts_gemm_gated(M, inter, K, act):
+    """Halves of an odd number of 64 rows, tiles in parts, parts behind waves, guard areas around output and sums."""
+    qt, wd = _q4_weight(2 * inter, K, seed=inter)
+    lw = LinearWeight(qt).to(DEV, torch.bfloat16)
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    ops.set_bounds_check(True)
+    try:
+        h = lw.handle().run_gated(x, ops.fused_act_kind(act), 4)
+        torch.cuda.synchronize()
+        ops.check_guards()
+    finally:
+        ops.set_bounds_check(False)
+    ops.check_status()
+    f = x.double().cpu() @ wd.double().t()
+    assert _rel(h.cpu(), ref.act_fn(act)(f[:, :inter]) * f[:, inter:]) < 6e-3
+
+
+@pytest.mark.parametrize("M", [1, 129, 400, 2310])
+@pytest.mark.parametrize("heads,kv,norm,rope,bias", [(4, 1, True, True, False), (6, 3, False, True, True), (3, 1, True, False, True)])
+def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
+    """q | k | v heads against the one-tile kernel: an odd number of heads (half a tile at the end), rows without a cache slot, positions behind a prefix, bias."""
+    K, D = 512, 128
+    qt, wd = _q4_weight((heads + 2 * kv) * D, K, seed=heads)
+    lw = LinearWeight(qt).to(DEV, torch.bfloat16)
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    pages = M // 32 + 2
+    slots = torch.randperm(pages * 32)[:M]
+    slots[M // 3 :: 5] = -1
+    slots, pos = slots.to(DEV), torch.arange(M, dtype=torch.int32, device=DEV) + 37
+    cos, sin = (t.to(DEV) for t in ref.rope_tables(D, 4096, 10000.0)) if rope else (None, None)
+    qn, kn = ((1 + 0.1 * torch.randn(D)).to(torch.bfloat16).to(DEV) for _ in range(2)) if norm else (None, None)
+    b = torch.randn(wd.shape[0], device=DEV) if bias else None
+    got = []
+    for pairs, impl in ((0, 0), (-1, 4)):
+        ops.set_gemm_pairs(pairs)
+        kc, vc = (torch.zeros(pages, kv, 32, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        q = lw.handle().run_qkv(x, pos, slots, qn, kn, cos, sin, kc, vc, heads, kv, 1e-6, 0.0, b, impl)
+        got.append((q, kc, vc))
+    torch.cuda.synchronize()
+    ops.check_status()
+    for u, v in zip(*got):  # (sums in another order, rounded to bf16 up to twice: 2^-9 each)
+        assert _rel(u, v) < 4e-3 and torch.equal(u == 0, v == 0)
+
+
+@pytest.mark.parametrize("E,n,K,T,k", [(4, 512, 256, 900, 2), (3, 384, 1216, 1500, 1), (40, 1280, 128, 9000, 2)])
+def test_parts_gemm_experts(E, n, K, T, k):
+    """Equal work items of up to 384 rows (one and two instructions, more items than an expert's rows ask for at the end of the list), as the experts of a prompt have them."""
+    e = ops.require_ext()
+    made = [_q4_weight(n, K, seed=i) for i in range(E)]
+    g = ops.GroupedLinearWeight([LinearWeight(qt).to(DEV, torch.bfloat16) for qt, _ in made])
+    assert g.prompt_rows() == 384
+    x = (torch.randn(T, K) * 0.5).to(torch.bfloat16).to(DEV)
+    w, idx, counts, offsets, perm, pos = e.moe_route(torch.randn(T, E, device=DEV), k, 0, True)
+    items = e.moe_items(offsets, 0, E, 384, (T * k + 383) // 384 + E)
+    xs = e.moe_gather(x, perm, k, None, 0, 0)
+    y, h = g.run(xs, items, 384), g.run_gated(xs, items, "silu", 384)
+    torch.cuda.synchronize()
+    ops.check_status()
+    off, it = offsets.tolist(), items.tolist()
+    for i, (_, wd) in enumerate(made):
+        f = xs[off[i]:off[i + 1]].double().cpu() @ wd.double().t()
+        assert _rel(y[off[i]:off[i + 1]].cpu(), f) < 4e-3
+        assert _rel(h[off[i]:off[i + 1]].cpu(), torch.nn.functional.silu(f[:, : n // 2]) * f[:, n // 2:]) < 6e-3
+        rows = [hi - lo for a, lo, hi, _ in it if a == i]
+        assert sum(rows) == off[i + 1] - off[i] and max(rows) <= 384 and max(rows) - min(rows) < len(rows)
