@@ -12,12 +12,10 @@
 
 namespace dlv {
 
-constexpr int kMaxTopK = 16;
-
-// Top-k of one token by one warp (E <= 1024): softmax statistics, k rounds of "every lane proposes its best remaining expert"
+// Top-k of one token by one warp (E <= 1024, k <= 16): softmax statistics, k rounds of "every lane proposes its best remaining expert"
 // (ties -> lower index), weights by `mode` (0: softmax over all experts, then top-k, optional renormalisation; 1: softmax over
-// the k chosen; 2: sigmoid scores with a correction and group limits, see MoeRouting). Lane 0 stores weights and expert ids, adds to the histogram `counts` (global or shared memory) and, when
-// `idx_copy` is given, keeps a second copy of the ids there.
+// the k chosen; 2: sigmoid scores with a correction and group limits, see MoeRouting). Lanes store weights and expert ids, add to the histogram `counts` (global or shared memory) and, when
+// `idx_copy` is given, keep a second copy of the ids there.
 // best (value, index) of the warp, lower index on ties
 __device__ __forceinline__ void warp_best(float& v, int& i) {
 #pragma unroll
@@ -72,74 +70,92 @@ __device__ __forceinline__ unsigned long long moe_kept_groups(const float* __res
   return kept;
 }
 
-__device__ __forceinline__ void moe_topk_token(const float* __restrict__ row, int E, int k, const MoeRouting& rt, int lane,
-                                               float* __restrict__ w_out, int* __restrict__ idx_out, int* counts, int* idx_copy) {
-  const int mode = rt.mode;
-  float mx = -INFINITY, den = 0.f;
-  unsigned long long kept = ~0ull;
-  const int group = rt.groups > 1 ? E / rt.groups : E;
-  if (mode == 2) {
-    kept = moe_kept_groups(row, E, rt, lane);
-  } else {
-    for (int e = lane; e < E; e += 32) mx = fmaxf(mx, row[e]);
-    mx = warp_max(mx);
-    for (int e = lane; e < E; e += 32) den += __expf(row[e] - mx);
-    den = warp_sum(den);
-  }
-  float sel_v[kMaxTopK];
-  int sel_i[kMaxTopK];
-  unsigned long long taken_lo = 0ull;  // bitmask of this lane's taken slots (expert e = lane + 32 * j -> bit j)
-  for (int r = 0; r < k; ++r) {
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int e = lane, j = 0; e < E; e += 32, ++j) {
-      if ((taken_lo >> j) & 1ull) continue;
-      float v = row[e];
-      if (mode == 2) v = (kept >> (e / group)) & 1ull ? route_sigmoid(v) + (rt.correction != nullptr ? rt.correction[e] : 0.f) : -INFINITY;
-      if (v > bv || (v == bv && e < bi)) {
-        bv = v;
-        bi = e;
-      }
-    }
-    warp_best(bv, bi);
-    if (bi >= E) bi = 0;  // (not a number among the logits: stay inside the tables)
-    sel_v[r] = bv;
-    sel_i[r] = bi;
-    if ((bi & 31) == lane) taken_lo |= 1ull << (bi >> 5);
-  }
-  if (lane == 0) {
-    float wts[kMaxTopK];
-    float s = 0.f;
-    if (mode == 2) {
-      for (int r = 0; r < k; ++r) {
-        wts[r] = route_sigmoid(row[sel_i[r]]);
-        s += wts[r];
-      }
-      for (int r = 0; r < k; ++r) wts[r] = wts[r] / (s + 1e-20f) * rt.scale;
-    } else if (mode == 0) {
-      for (int r = 0; r < k; ++r) {
-        wts[r] = __expf(sel_v[r] - mx) / den;
-        s += wts[r];
-      }
-      if (rt.renorm)
-        for (int r = 0; r < k; ++r) wts[r] /= s;
-    } else {
-      for (int r = 0; r < k; ++r) {
-        wts[r] = __expf(sel_v[r] - sel_v[0]);
-        s += wts[r];
-      }
-      for (int r = 0; r < k; ++r) wts[r] /= s;
-    }
-    for (int r = 0; r < k; ++r) {
-      w_out[r] = wts[r];
-      idx_out[r] = sel_i[r];
-      if (idx_copy != nullptr) idx_copy[r] = sel_i[r];
-      atomicAdd(&counts[sel_i[r]], 1);
-    }
-  }
+// Order of floats as unsigned integers, -0 as 0; nothing (and what is not a number) below everything.
+__device__ __forceinline__ unsigned order_key(float v) {
+  const unsigned u = __float_as_uint(v + 0.f);
+  return v != v ? 0u : (u & 0x80000000u ? ~u : u | 0x80000000u);
 }
 
+// NV experts per lane (expert lane + 32 j): they stay in registers through all rounds, a round is one warp-wide maximum of their order and one minimum of the index, and
+// lane r keeps what round r chose. (With the chosen ones in arrays of a thread, which a loop of run-time length puts into local memory, and five shuffles of two
+// words per round, one block routed 32 tokens over 128 experts in 21.8 us and 64 over 8 in 15.3.)
+template <int NV>
+__device__ __forceinline__ void moe_topk_rows(const float* __restrict__ row, int E, int k, const MoeRouting& rt, int lane, float* __restrict__ w_out,
+                                              int* __restrict__ idx_out, int* counts, int* idx_copy) {
+  const int mode = rt.mode;
+  float v[NV], mx = -INFINITY, den = 0.f;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) v[j] = lane + 32 * j < E ? row[lane + 32 * j] : 0.f;
+  if (mode == 2) {
+    const unsigned long long kept = moe_kept_groups(row, E, rt, lane);
+    const int group = rt.groups > 1 ? E / rt.groups : E;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int e = lane + 32 * j;
+      if (e < E) v[j] = (kept >> (e / group)) & 1ull ? route_sigmoid(v[j]) + (rt.correction != nullptr ? rt.correction[e] : 0.f) : -INFINITY;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (lane + 32 * j < E) mx = fmaxf(mx, v[j]);
+    mx = warp_max(mx);
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (lane + 32 * j < E) den += __expf(v[j] - mx);
+    den = warp_sum(den);
+  }
+  unsigned left = 0u;  // experts that may still be chosen
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+    if (lane + 32 * j < E) left |= 1u << j;
+  float sel_v = -INFINITY;
+  int sel_i = 0;
+  for (int r = 0; r < k; ++r) {
+    unsigned bk = 0u;
+    float bv = -INFINITY;
+    int bi = 0x7fffffff;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const unsigned key = (left >> j) & 1u ? order_key(v[j]) : 0u;
+      if (key > bk) {  // (of equal ones the lower index)
+        bk = key;
+        bv = v[j];
+        bi = lane + 32 * j;
+      }
+    }
+    const unsigned best = __reduce_max_sync(0xffffffffu, bk);
+    const int i = static_cast<int>(__reduce_min_sync(0xffffffffu, bk == best && best != 0u ? static_cast<unsigned>(bi) : 0x7fffffffu));
+    const float chosen = __shfl_sync(0xffffffffu, bv, i & 31);
+    const int at = i < E ? i : 0;  // (not a number among the logits: stay inside the tables)
+    if (lane == r) {
+      sel_v = i < E ? chosen : -INFINITY;
+      sel_i = at;
+    }
+    if ((at & 31) == lane) left &= ~(1u << (at >> 5));
+  }
+  // weights: lane r those of round r, summed in order
+  float wt = 0.f;
+  if (lane < k) {
+    if (mode == 2) wt = route_sigmoid(row[sel_i]);
+    else if (mode == 0) wt = __expf(sel_v - mx) / den;
+  }
+  if (mode == 1) {
+    const float first = __shfl_sync(0xffffffffu, sel_v, 0);
+    if (lane < k) wt = __expf(sel_v - first);
+  }
+  float s = 0.f;
+  for (int r = 0; r < k; ++r) s += __shfl_sync(0xffffffffu, wt, r);
+  if (mode == 2) wt = wt / (s + 1e-20f) * rt.scale;
+  else if (mode == 1 || rt.renorm) wt /= s;
+  if (lane < k) {
+    w_out[lane] = wt;
+    idx_out[lane] = sel_i;
+    if (idx_copy != nullptr) idx_copy[lane] = sel_i;
+    if (counts != nullptr) atomicAdd(&counts[sel_i], 1);
+  }
+}
 // one warp per token
+template <int NV>
 __global__ void __launch_bounds__(256) moe_topk_kernel(const float* __restrict__ logits, int T, int E, int k, const MoeRouting rt,
                                                        float* __restrict__ w_out, int* __restrict__ idx_out, int* __restrict__ counts) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
@@ -147,11 +163,11 @@ __global__ void __launch_bounds__(256) moe_topk_kernel(const float* __restrict__
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
-  moe_topk_token(logits + static_cast<size_t>(t) * E, E, k, rt, lane, w_out + static_cast<size_t>(t) * k,
-                 idx_out + static_cast<size_t>(t) * k, counts, nullptr);
+  moe_topk_rows<NV>(logits + static_cast<size_t>(t) * E, E, k, rt, lane, w_out + static_cast<size_t>(t) * k, idx_out + static_cast<size_t>(t) * k, counts,
+                    nullptr);
 }
 
-// Routing of a decode-size batch in ONE launch of one CTA (32 warps): top-k per token, expert histogram and offsets, the stable
+// Routing of a decode-size batch in ONE launch of one CTA (32 warps; 16 above 256 experts, whose scores take the registers): top-k per token, expert histogram and offsets, the stable
 // permutation that groups (token, slot) pairs by expert, and the grouped GEMM's work list for the local experts [e0, e0 + ne)
 // with `bn` rows per item. It replaces a memset and four launches (moe_topk, moe_sort, moe_items and, where the grouped GEMV reads
 // token rows through `perm`, moe_gather), which cost more than the work at a few hundred pairs. Shared memory: T k + 2 E + ne + 3
@@ -166,7 +182,8 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
   }
   return v;
 }
-__global__ void __launch_bounds__(1024) moe_route_small_kernel(const float* __restrict__ logits, int T, int E, int k, const MoeRouting rt,
+template <int NV, int THREADS>
+__global__ void __launch_bounds__(THREADS) moe_route_small_kernel(const float* __restrict__ logits, int T, int E, int k, const MoeRouting rt,
                                                                float* __restrict__ w_out, int* __restrict__ idx_out, int* __restrict__ counts,
                                                                int* __restrict__ offsets, int* __restrict__ perm, int* __restrict__ pos, int e0,
                                                                int ne, int bn, int max_items, int4* __restrict__ items) {
@@ -179,11 +196,11 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const float* __re
   int* off_s = cnt_s + E;       // [E + 1]
   int* first_s = off_s + E + 1; // [ne + 1] first work item of every local expert
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < E; e += 1024) cnt_s[e] = 0;
+  for (int e = tid; e < E; e += THREADS) cnt_s[e] = 0;
   __syncthreads();
-  for (int t = warp; t < T; t += 32)
-    moe_topk_token(logits + static_cast<size_t>(t) * E, E, k, rt, lane, w_out + static_cast<size_t>(t) * k,
-                   idx_out + static_cast<size_t>(t) * k, cnt_s, idx_s + t * k);
+  for (int t = warp; t < T; t += THREADS / 32)
+    moe_topk_rows<NV>(logits + static_cast<size_t>(t) * E, E, k, rt, lane, w_out + static_cast<size_t>(t) * k, idx_out + static_cast<size_t>(t) * k, cnt_s,
+                      idx_s + t * k);
   __syncthreads();
   if (warp == 0) {  // exclusive scan of the histogram: lane l owns a contiguous chunk of experts
     const int chunk = (E + 31) / 32, lo = min(E, lane * chunk), hi = min(E, lo + chunk);
@@ -209,10 +226,10 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const float* __re
     if (lane == 31) first_s[ne] = incl;
   }
   __syncthreads();
-  for (int e = tid; e <= E; e += 1024) offsets[e] = off_s[e];
-  for (int e = tid; e < E; e += 1024) counts[e] = cnt_s[e];
+  for (int e = tid; e <= E; e += THREADS) offsets[e] = off_s[e];
+  for (int e = tid; e < E; e += THREADS) counts[e] = cnt_s[e];
   // stable grouping: a warp takes an expert and walks the pairs 32 at a time (ballot + prefix count keeps ascending pair order)
-  for (int e = warp; e < E; e += 32) {
+  for (int e = warp; e < E; e += THREADS / 32) {
     if (cnt_s[e] == 0) continue;
     int row = off_s[e];
     for (int p0 = 0; p0 < P; p0 += 32) {
@@ -228,12 +245,12 @@ __global__ void __launch_bounds__(1024) moe_route_small_kernel(const float* __re
     }
   }
   if (items != nullptr) {
-    for (int e = tid; e < ne; e += 1024) {
+    for (int e = tid; e < ne; e += THREADS) {
       const int lo = off_s[e0 + e], hi = off_s[e0 + e + 1];
       int it = first_s[e];
       for (int r = lo; r < hi && it < max_items; r += bn, ++it) items[it] = make_int4(e, r, hi, 0);
     }
-    for (int it = first_s[ne] + tid; it < max_items; it += 1024) items[it] = make_int4(-1, 0, 0, 0);
+    for (int it = first_s[ne] + tid; it < max_items; it += THREADS) items[it] = make_int4(-1, 0, 0, 0);
   }
 }
 
@@ -274,7 +291,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
 // histogram into offsets and the chunk counts into the first row of every (chunk, expert), (c) one warp per chunk hands out the
 // rows in pair order (__match_any_sync groups the lanes of one expert; the group's first lane advances the running row). The
 // order is the stable one: ascending pair index inside an expert.
-constexpr int kSortChunk = 1024;
+constexpr int kSortChunk = 256;
 constexpr int kSortSerialMaxPairs = 1024;  // up to here the single-CTA kernel is used
 __global__ void __launch_bounds__(256) moe_chunk_hist_kernel(const int* __restrict__ idx, int P, int E, int* __restrict__ chunk_hist) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
@@ -287,33 +304,61 @@ __global__ void __launch_bounds__(256) moe_chunk_hist_kernel(const int* __restri
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) chunk_hist[static_cast<size_t>(blockIdx.x) * E + e] = hs[e];
 }
-// chunk_hist [C, E]: counts on entry, first grouped row of the (chunk, expert) on exit
-__global__ void __launch_bounds__(1024) moe_chunk_scan_kernel(const int* __restrict__ counts, int E, int C, int* __restrict__ offsets,
-                                                              int* __restrict__ chunk_hist) {
+// chunk_hist [C, E]: counts on entry, first grouped row of the (chunk, expert) on exit. Threads of neighbouring experts read a chunk's row together, and as many
+// threads as there are take an expert's chunks in stretches, eight counts in flight. (One thread per expert, a load and a store behind one another for each of 64
+// chunks: 11 us; a warp per expert, whose lanes read a column: 70 us at 256 chunks.)
+__global__ void __launch_bounds__(1024) moe_chunk_scan_kernel(int* __restrict__ counts, int E, int C, int* __restrict__ offsets, int* __restrict__ chunk_hist) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  extern __shared__ int sh[];  // [E + 1]
-  const int lane = threadIdx.x & 31;
-  if (threadIdx.x < 32) {
-    const int chunk = (E + 31) / 32, lo = min(E, lane * chunk), hi = min(E, lo + chunk);
+  extern __shared__ int sh[];  // [E + 1] first rows, then [stretches][E] counts of an expert's stretches
+  const int S = 1024 / E > 0 ? 1024 / E : 1, per = (C + S - 1) / S;
+  int* part = sh + E + 1;
+  const int st = static_cast<int>(threadIdx.x) / E, e = static_cast<int>(threadIdx.x) - st * E, c0 = st * per, c1 = min(C, c0 + per);
+  int* col = chunk_hist + e;
+  if (st < S) {
     int sum = 0;
-    for (int e = lo; e < hi; ++e) sum += counts[e];
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) sum += col[static_cast<size_t>(c) * E];
+    part[st * E + e] = sum;
+  }
+  __syncthreads();
+  if (st == 0) {
+    int sum = 0;
+    for (int i = 0; i < S; ++i) {  // counts of the stretches -> pairs in front of them
+      const int n = part[i * E + e];
+      part[i * E + e] = sum;
+      sum += n;
+    }
+    counts[e] = sum;
+    sh[e] = sum;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, chunk = (E + 31) / 32, lo = min(E, lane * chunk), hi = min(E, lo + chunk);
+    int sum = 0;
+    for (int i = lo; i < hi; ++i) sum += sh[i];
     const int incl = warp_incl_scan(sum, lane);
     int acc = incl - sum;
-    for (int e = lo; e < hi; ++e) {
-      sh[e] = acc;
-      acc += counts[e];
+    for (int i = lo; i < hi; ++i) {
+      const int n = sh[i];
+      sh[i] = acc;
+      acc += n;
     }
     if (lane == 31) sh[E] = incl;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = sh[e];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int acc = sh[e];
-    for (int c = 0; c < C; ++c) {
-      const int h = chunk_hist[static_cast<size_t>(c) * E + e];
-      chunk_hist[static_cast<size_t>(c) * E + e] = acc;
-      acc += h;
+  for (int i = threadIdx.x; i <= E; i += blockDim.x) offsets[i] = sh[i];
+  if (st < S) {
+    int acc = sh[e] + part[st * E + e];
+    for (int c = c0; c < c1; c += 8) {
+      int n[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) n[i] = c + i < c1 ? col[static_cast<size_t>(c + i) * E] : 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (c + i < c1) col[static_cast<size_t>(c + i) * E] = acc;
+        acc += n[i];
+      }
     }
   }
 }
@@ -364,22 +409,43 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(const __nv_bfloat16* _
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
   const int t = blockIdx.x;
-  const int lo = offsets != nullptr ? offsets[e0] : 0, hi = offsets != nullptr ? offsets[e0 + ne] : 0x7fffffff;
+  // rows and weights of the token's slots first, then four slots' rows at a time (one after the other, each behind its slot's row number, made the kernel 8.5 us
+  // for 32 tokens of eight)
+  constexpr int kSlots = 64;  // (more slots look theirs up themselves)
+  __shared__ int rows[kSlots];
+  __shared__ float wts[kSlots];
+  auto row_at = [&](int j) {
+    const int r = pos[static_cast<size_t>(t) * k + j];
+    return offsets == nullptr || (r >= offsets[e0] && r < offsets[e0 + ne]) ? r : -1;  // (computed on another rank: the all-reduce adds it)
+  };
+  if (static_cast<int>(threadIdx.x) < min(k, kSlots)) {
+    rows[threadIdx.x] = row_at(threadIdx.x);
+    wts[threadIdx.x] = w[static_cast<size_t>(t) * k + threadIdx.x];
+  }
+  __syncthreads();
   for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
     float acc[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-    for (int j = 0; j < k; ++j) {
-      const float wt = w[static_cast<size_t>(t) * k + j];
-      const int prow = pos[static_cast<size_t>(t) * k + j];
-      if (prow < lo || prow >= hi) continue;  // computed on another rank; the all-reduce adds it
-      const uint4 v = reinterpret_cast<const uint4*>(ys + static_cast<size_t>(prow) * H)[i];
-      const uint32_t* vu = reinterpret_cast<const uint32_t*>(&v);
+    for (int j0 = 0; j0 < k; j0 += 4) {
+      uint4 v[4];
+      int r[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = unpack_bf162(vu[e]);
-        acc[2 * e] += wt * f.x;
-        acc[2 * e + 1] += wt * f.y;
+      for (int j = 0; j < 4; ++j) {
+        r[j] = j0 + j >= k ? -1 : (j0 + j < kSlots ? rows[j0 + j] : row_at(j0 + j));
+        if (r[j] >= 0) v[j] = __ldg(reinterpret_cast<const uint4*>(ys + static_cast<size_t>(r[j]) * H) + i);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (r[j] < 0) continue;
+        const float wt = j0 + j < kSlots ? wts[j0 + j] : w[static_cast<size_t>(t) * k + j0 + j];
+        const uint32_t vu[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = unpack_bf162(vu[e]);
+          acc[2 * e] += wt * f.x;
+          acc[2 * e + 1] += wt * f.y;
+        }
       }
     }
     uint4 o;
@@ -397,17 +463,22 @@ size_t moe_route_workspace_ints(int T, int E, int k) {
 }
 void launch_moe_route(const float* logits, int T, int E, int k, const MoeRouting& r, float* w, int* idx, int* counts, int* offsets,
                       int* perm, int* pos, int* ws, cudaStream_t st) {
-  cudaMemsetAsync(counts, 0, sizeof(int) * E, st);
+  const bool chunks = ws != nullptr && moe_route_workspace_ints(T, E, k) > 0;
+  if (!chunks) cudaMemsetAsync(counts, 0, sizeof(int) * E, st);
   if (T == 0) {
     cudaMemsetAsync(offsets, 0, sizeof(int) * (E + 1), st);
     return;
   }
-  moe_topk_kernel<<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, counts);
+  // (the chunks count their pairs themselves: 65,536 atomics on 128 counters were most of the 36 us of 8,192 tokens)
+  int* histogram = chunks ? nullptr : counts;
+  if (E <= 128) moe_topk_kernel<4><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
+  else if (E <= 256) moe_topk_kernel<8><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
+  else moe_topk_kernel<32><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   const int P = T * k;
-  if (ws != nullptr && moe_route_workspace_ints(T, E, k) > 0) {
+  if (chunks) {
     const int C = (P + kSortChunk - 1) / kSortChunk;
     moe_chunk_hist_kernel<<<C, 256, sizeof(int) * E, st>>>(idx, P, E, ws);
-    moe_chunk_scan_kernel<<<1, 1024, sizeof(int) * (E + 1), st>>>(counts, E, C, offsets, ws);
+    moe_chunk_scan_kernel<<<1, 1024, sizeof(int) * (E + 1 + 1024), st>>>(counts, E, C, offsets, ws);
     moe_chunk_rank_kernel<<<C, 32, sizeof(int) * (E + kSortChunk), st>>>(idx, P, E, ws, perm, pos);
     return;
   }
@@ -418,8 +489,13 @@ bool launch_moe_route_small(const float* logits, int T, int E, int k, const MoeR
                             int* perm, int* pos, int e0, int ne, int bn, int max_items, int* items, cudaStream_t st) {
   if (T < 1 || T > kRouteSmallMaxTokens || T * k > kRouteSmallMaxPairs || E > 1024 || ne > 1024) return false;
   const size_t smem = sizeof(int) * (static_cast<size_t>(T) * k + 2 * E + ne + 3);
-  return launch_pdl(moe_route_small_kernel, dim3(1), dim3(1024), smem, st, logits, T, E, k, r, w, idx, counts, offsets, perm, pos, e0,
-                    ne, bn, max_items, reinterpret_cast<int4*>(items)) == cudaSuccess;
+  const auto run = [&](auto kernel, int threads) {
+    return launch_pdl(kernel, dim3(1), dim3(threads), smem, st, logits, T, E, k, r, w, idx, counts, offsets, perm, pos, e0, ne, bn, max_items,
+                      reinterpret_cast<int4*>(items)) == cudaSuccess;
+  };
+  if (E <= 128) return run(moe_route_small_kernel<4, 1024>, 1024);
+  if (E <= 256) return run(moe_route_small_kernel<8, 1024>, 1024);
+  return run(moe_route_small_kernel<32, 512>, 512);
 }
 void launch_moe_gather(const void* x, const int* perm, int rows, int k, int row_bytes, void* xs, const int* offsets, int e0, int ne,
                        cudaStream_t st) {
@@ -439,13 +515,20 @@ __global__ void __launch_bounds__(256) moe_items_kernel(const int* __restrict__ 
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
   __shared__ int first[1025];
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < ne; ++e) {
+  for (int e = threadIdx.x; e < ne; e += blockDim.x) first[e] = (offsets[e0 + e + 1] - offsets[e0 + e] + bn - 1) / bn;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, chunk = (ne + 31) / 32, lo = min(ne, lane * chunk), hi = min(ne, lo + chunk);
+    int sum = 0;
+    for (int e = lo; e < hi; ++e) sum += first[e];
+    const int incl = warp_incl_scan(sum, lane);
+    int acc = incl - sum;
+    for (int e = lo; e < hi; ++e) {
+      const int n = first[e];
       first[e] = acc;
-      acc += (offsets[e0 + e + 1] - offsets[e0 + e] + bn - 1) / bn;
+      acc += n;
     }
-    first[ne] = acc;
+    if (lane == 31) first[ne] = incl;
   }
   __syncthreads();
   for (int e = threadIdx.x; e < ne; e += blockDim.x) {

@@ -1204,3 +1204,40 @@ def test_parts_gemm_experts(E, n, K, T, k):
         assert _rel(h[off[i]:off[i + 1]].cpu(), torch.nn.functional.silu(f[:, : n // 2]) * f[:, n // 2:]) < 6e-3
         rows = [hi - lo for a, lo, hi, _ in it if a == i]
         assert sum(rows) == off[i + 1] - off[i] and max(rows) <= 384 and max(rows) - min(rows) < len(rows)
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 3, 3), (33, 8, 2), (70, 128, 8), (128, 129, 16), (50, 256, 8), (40, 257, 9), (20, 1000, 16), (700, 128, 8), (3000, 40, 6), (130, 1024, 16)])
+def test_moe_route_choices(T, E, k):
+    """Experts and groups of the routing kernels against a sort: equal logits (the lower expert first), both zeros equal, minus infinity chosen last; one launch and
+    several, 32 experts per register and their remainders, the pairs grouped chunk by chunk and by one block."""
+    e = ops.require_ext()
+    z = torch.randint(-4, 5, (T, E)).float() * torch.where(torch.rand(T, E) < 0.5, 1.0, -1.0)  # (minus zeros among them)
+    z[::3, : E // 2] = -math.inf
+    z[1::4] = torch.randn(z[1::4].shape)
+    idx = torch.sort(z + 0.0, dim=-1, descending=True, stable=True).indices[:, :k]
+    order = torch.sort(idx.flatten(), stable=True).indices
+    for mode in (0, 1):
+        routed = [e.moe_route(z.to(DEV), k, mode, True)]
+        if T <= 128:
+            routed.append(e.moe_route_items(z.to(DEV), k, mode, True, 0, E, 8, T * k))
+        for r in routed:
+            w, got, counts, offsets, perm, pos = (t.cpu() for t in r[:6])
+            wr = torch.softmax(z.gather(1, idx), -1)
+            assert torch.equal(got.long(), idx) and torch.allclose(w, wr, rtol=1e-5, atol=1e-7)  # (ratios of __expf, 2 ulp and the rounding of its argument)
+            assert torch.equal(counts.long(), torch.bincount(idx.flatten(), minlength=E)) and torch.equal(offsets[1:].long(), counts.long().cumsum(0))
+            assert torch.equal(perm.long(), order) and torch.equal(perm[pos.flatten().long()].long(), torch.arange(T * k))
+
+
+@pytest.mark.parametrize("T,k,H", [(1, 1, 8), (3, 5, 1032), (9, 8, 2048), (2, 70, 128)])
+def test_moe_combine_slots(T, k, H):
+    """Slots that do not fill a group of four, more of them than are looked up ahead, rows of another rank's experts."""
+    e = ops.require_ext()
+    ys, w = torch.randn(T * k, H).to(torch.bfloat16), torch.rand(T, k)
+    pos = torch.randperm(T * k).view(T, k)
+    lo, hi = T * k // 4, T * k - T * k // 3
+    for rng in (False, True):
+        offsets = torch.tensor([0, lo, hi, T * k], dtype=torch.int32, device=DEV)
+        out = e.moe_combine(ys.to(DEV), pos.int().to(DEV), w.to(DEV), T, k, *((offsets, 1, 1) if rng else (None, 0, 0)))
+        own = ((pos >= lo) & (pos < hi)).double() if rng else torch.ones(T, k).double()
+        r = (ys.double()[pos] * (w.double() * own).unsqueeze(-1)).sum(1)
+        assert (out.cpu().double() - r).abs().max() <= 2.0**-8 * max(1e-6, r.abs().max().item())
