@@ -753,7 +753,8 @@ def moe_token_tile(rows: int, local_experts: int, q4: bool = True) -> int:
     # that many local experts (comparisons).
     # (bf16 experts still have the CUDA-core GEMV only: worth it just for very many experts, as measured with that kernel)
     need = _GEMV_MIN_EXPERTS if q4 else max(96, _GEMV_MIN_EXPERTS)
-    if local_experts >= need and avg <= 3:
+    # (the mma.sync GEMV takes up to eight rows at the price of one: items of four only double the experts that have more)
+    if local_experts >= need and avg <= 3 and not q4:
         return 4
     if local_experts >= need and avg <= 6:
         return 8
