@@ -390,7 +390,7 @@ class GemmWeight {
     TORCH_CHECK(n_per_expert > 0 && desc_.N % per == 0, "stacked weight rows are not a multiple of the per-expert rows");
     if ((act != 1 && act != 2) || n_per_expert % 16 != 0 || item_rows < 1) return Tensor();
     c10::cuda::CUDAGuard guard(xs.device());
-    if (dlv::gemm_parts_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2), 1)) {
+    if (desc_.is_q4 && dlv::gemm_parts_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2), 1)) {
       Tensor out = new_out({xs.size(0), n_per_expert / 2}, xs.options());
       if (xs.size(0) == 0 || items.size(0) == 0) return out;
       dlv::gemm_parts_run_grouped(&desc_, static_cast<int>(n_per_expert), xs.data_ptr(), static_cast<int>(xs.size(0)), static_cast<int>(xs.stride(0)), out.data_ptr(),
@@ -411,7 +411,7 @@ class GemmWeight {
   // whether work items of more than 256 rows find their kernel (any number: it cuts them into equal tiles)
   bool wide_items(int64_t n_per_expert) const {
     c10::cuda::CUDAGuard guard(w_.device());
-    return dlv::gemm_parts_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert), 0);
+    return desc_.is_q4 && dlv::gemm_parts_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert), 0);
   }
   bool gemv_ok(int64_t M, int64_t ldx) const { return dlv::gemv_dense_supported(&desc_, static_cast<int>(M), static_cast<int>(ldx)); }
   // Grouped (MoE) GEMM: `this` stacks the local experts' weights (n_per_expert rows each; JQ4: whole 128-row tiles per expert),

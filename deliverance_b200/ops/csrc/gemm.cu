@@ -67,6 +67,19 @@ void encode_map_kchunks(CUtensorMap* map, const void* base, uint64_t rows, uint6
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled (3-D) failed with code " + std::to_string(static_cast<int>(r)));
 }
 
+// Gate rows [0, half) and up rows [half, 2 half) of a bf16 weight (K % 64 == 0, half % 8 == 0) in turn: one box = 64 k of eight gate rows, the up rows of the same
+// outputs, the next eight gate rows, ..., 128 rows in all. Dimensions: k in a chunk, row in eight, gate / up, eights, chunks.
+void encode_map_gate_up(CUtensorMap* map, const void* base, uint64_t half, uint64_t K) {
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || K % 64 != 0 || half % 8 != 0) throw std::runtime_error("gate | up TMA map needs whole chunks of 64 k and eights of rows");
+  cuuint64_t dims[5] = {64, 8, 2, half / 8, K / 64};
+  cuuint64_t strides[4] = {K * 2, half * K * 2, 8 * K * 2, 128};
+  cuuint32_t box[5] = {64, 8, 2, 8, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = get_encode()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled (gate | up) failed with code " + std::to_string(static_cast<int>(r)));
+}
+
 // ------------------------------------------------------------------------------------------------ weight handle
 void gemm_weight_init(GemmWeightDesc* w) {
   if (w->is_q4) {
@@ -498,7 +511,7 @@ void gemm_tc_run_grouped(const GemmWeightDesc* w, int n_per_expert, const void* 
   if (rows <= 0 || max_items <= 0) return;
   if (ldx % 8 != 0) throw std::runtime_error("activation row pitch must be a multiple of 8 elements");
   if (max_items > 65535) throw std::runtime_error("grouped gemm: work list too long");
-  if (bn >= 256 && splits <= 1 && gemm_parts_supported(w, n_per_expert, out, ldo, 0)) {
+  if (w->is_q4 && bn >= 256 && splits <= 1 && gemm_parts_supported(w, n_per_expert, out, ldo, 0)) {
     gemm_parts_run_grouped(w, n_per_expert, x, rows, ldx, out, ldo, items, max_items, bn, 0, status, st);
     return;
   }

@@ -38,6 +38,7 @@
 namespace dlv {
 
 void encode_map_kchunks(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint64_t pitch_bytes, uint32_t box_rows, uint32_t chunks = 2);
+void encode_map_gate_up(CUtensorMap* map, const void* base, uint64_t half, uint64_t K);
 
 namespace {
 
@@ -51,6 +52,8 @@ constexpr int kOffRaw = kXRoom;
 constexpr int kOffDrain = kOffRaw + kRawStages * kQ4StageBytes;
 constexpr int kOffCtrl = kOffDrain + 4 * 2 * kDrainBytes;
 constexpr int kSmemBytes = kOffCtrl + 1024 + 1024;  // barriers + alignment slack
+constexpr int kWStage = 128 * 128;            // bf16 weights: a CTA's 128 rows of a 64-k stage, in front of its tokens
+constexpr int kStageRoom = kOffDrain;         // (they have the room of the packed stages too)
 constexpr int kThreads = 672;
 static_assert(kThreads == 640 + 32, "named barrier of the set-up");
 static_assert(kSmemBytes <= 232448, "shared memory of an SM");
@@ -66,10 +69,10 @@ struct Divisor {
 };
 struct PartParams {
   int M, N;
-  int kq;                 // 128-k stages of a tile
+  int kq;                 // stages of a tile: 128 k, bf16 weights 64 k
   int bn, box;            // tokens of a tile (a multiple of 32) and of a CTA's half of one instruction
-  int x_stages;           // 128-k stages of tokens
-  int slots;              // 128-k stages of expanded weights in tensor memory (2 or 4)
+  int x_stages;           // stages of tokens (bf16: and weights) in shared memory
+  int slots;              // JQ4: stages of expanded weights in tensor memory (2 or 4); bf16: accumulators (2 where they fit)
   int n_tiles, m_tiles;   // grouped: m_tiles counts work items
   int pairs, waves;       // whole tiles: waves * pairs of them
   int parts;              // parts of each of the other tiles (0: there are none)
@@ -90,7 +93,7 @@ struct PartParams {
 
 struct Piece {
   int m0, m_lim, n_tile, expert;
-  int k0, k1;   // 128-k stages
+  int k0, k1;   // stages
   int n1, n2;   // tokens of the first and the second instruction (multiples of 32; 0: there is no second one)
   int slot;     // where the sums go that the second kernel finishes, < 0: the drain does
 };
@@ -299,8 +302,8 @@ __device__ __forceinline__ void row_sums(const float* row, int lane, float (&s)[
   }
 }
 
-template <int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_parts_kernel(const __grid_constant__ CUtensorMap map_x, const PartParams p) {
+template <bool Q4, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_parts_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const PartParams p) {
   constexpr int NR = kRawStages;
   extern __shared__ uint8_t gr_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gr_raw) + 1023) & ~uintptr_t(1023));
@@ -310,8 +313,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
   uint64_t* bar_raw_full = bar_a_full + kMaxA;
   uint64_t* bar_raw_empty = bar_raw_full + NR;
   uint64_t* bar_acc_full = bar_raw_empty + NR;
-  uint64_t* bar_acc_empty = bar_acc_full + 1;
-  uint64_t* bar_turn = bar_acc_empty + 1;  // [4][2] sixteen tokens of a group's drain are complete in shared memory
+  uint64_t* bar_acc_empty = bar_acc_full + 2;
+  uint64_t* bar_turn = bar_acc_empty + 2;  // [4][2] sixteen tokens of a group's drain are complete in shared memory
   uint64_t* bar_last = bar_turn + 8;       // abort path: MMAs in flight have retired
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_last + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -321,7 +324,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
   const int pair = static_cast<int>(blockIdx.x) >> 1;
   const int NA = p.slots, NX = p.x_stages;
   const bool two = p.bn > kOneMma;  // tiles may take a second instruction, whose tokens have a region of their own
-  const int region = p.box * 256, x_bytes = two ? 2 * region : region;  // one CTA's half of a stage of tokens
+  const int region = p.box * (Q4 ? 256 : 128), x_bytes = (two ? 2 * region : region) + (Q4 ? 0 : kWStage);  // one CTA's half of a stage
+  const uint32_t NACC = Q4 ? 1 : NA;  // accumulators
 
   Piece pc;
   Walk<EPI> walk(p, pair);
@@ -351,16 +355,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
       mbar_init(smem_u32(&bar_done[s]), 1);
     }
     for (int s = 0; s < kMaxA; ++s) mbar_init(smem_u32(&bar_a_full[s]), 2 * 8);
-    mbar_init(smem_u32(bar_acc_full), 1);
-    mbar_init(smem_u32(bar_acc_empty), 2 * 16);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&bar_acc_full[b]), 1);
+      mbar_init(smem_u32(&bar_acc_empty[b]), 2 * 16);
+    }
     for (int s = 0; s < 8; ++s) mbar_init(smem_u32(&bar_turn[s]), 4);
     mbar_init(smem_u32(bar_last), 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_x);
+    if (!Q4) tma_prefetch_desc(&map_w);
   }
   __syncwarp();
-  if (warp == 3) {
+  if (Q4 && warp == 3) {
     // The first packed stages are on their way while the rest is set up: this warp only announces their barriers to the others (who find them behind the
     // cluster barrier) and copies before it waits for anyone.
     if (lane == 0) {
@@ -379,7 +386,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
     if (warp == 2) tmem_alloc_pair(smem_u32(tmem_slot), 512);
     tc_fence_before();
     __syncwarp();
-    asm volatile("bar.sync 1, 640;" ::: "memory");  // (the other twenty warps: the address of tensor memory)
+    if (Q4) asm volatile("bar.sync 1, 640;" ::: "memory");  // (the other twenty warps: the address of tensor memory)
+    else __syncthreads();
     cluster_meet();  // the peer's barriers exist before anything arrives on them
     tc_fence_after();
   }
@@ -387,28 +395,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_a = tmem_base + (NA == 2 ? kMaxTokens : 256);
 
-  if (warp == 0 || warp == 2) {
-    // ---------------- token copies: one per stage and instruction ----------------
-    const int mine = warp >> 1;
-    if (lane == 0 && (mine == 0 || two)) {
-      int g = 0, s = 0;  // 128-k stages of this pair, numbered across pieces; ring position
+  if (warp == 0 || warp == 2 || (!Q4 && warp == 3)) {
+    // ---------------- token copies: one per stage and instruction; bf16 weight copies ----------------
+    const int mine = warp == 3 ? 2 : warp >> 1;
+    if (lane == 0 && (mine != 1 || two)) {
+      int g = 0, s = 0;  // stages of this pair, numbered across pieces; ring position
       uint32_t ph = 0;
       bool ok = true;
       for (bool more = any; ok && more; more = walk.next(pc)) {
         const int row = mine == 0 ? pc.m0 + rank * (pc.n1 >> 1) : pc.m0 + pc.n1 + rank * (pc.n2 >> 1);
-        const uint32_t bytes = static_cast<uint32_t>(pc.n2 > 0 ? 4 * region : 2 * region);  // of both CTAs
+        const int half_tile = pc.n_tile * 2 + rank;
+        const uint32_t bytes = static_cast<uint32_t>((pc.n2 > 0 ? 4 * region : 2 * region) + (Q4 ? 0 : 2 * kWStage));  // of both CTAs
         for (int q = pc.k0; q < pc.k1; ++q, ++g) {
           ok = g < NX || mbar_wait(smem_u32(&bar_done[s]), ph ^ 1, abort_flag, p.status);
           if (!ok) break;
           if (rank == 0 && mine == 0) mbar_expect_tx(smem_u32(&bar_x_full[s]), bytes);  // (for all copies; the barrier waits for this arrival)
-          if (mine == 0 || pc.n2 > 0) tma_load_3d_pair(smem_u32(smem + s * x_bytes + mine * region), &map_x, mapa_u32(smem_u32(&bar_x_full[s]), 0), 0, row, 2 * q);
+          const uint32_t at = smem_u32(smem + s * x_bytes), full = mapa_u32(smem_u32(&bar_x_full[s]), 0);
+          if (mine == 2) {
+            if (EPI == 1) tma_load_5d_pair(at, &map_w, full, 0, 0, 0, half_tile * 8, q);
+            else tma_load_2d_pair(at, &map_w, full, q * 64, half_tile * 128);
+          } else if (mine == 0 || pc.n2 > 0) {
+            tma_load_3d_pair(at + (Q4 ? 0 : kWStage) + mine * region, &map_x, full, 0, row, Q4 ? 2 * q : q);
+          }
           if (++s == NX) { s = 0; ph ^= 1; }
         }
       }
       // the pair's last commits have arrived here before this CTA may leave
       for (int j = g < NX ? g : NX; ok && j > 0; --j) ok = mbar_wait(smem_u32(&bar_done[(g - j) % NX]), ((g - j) / NX) & 1, abort_flag, p.status);
     }
-  } else if (warp == 3 || warp == 20) {
+  } else if (Q4 && (warp == 3 || warp == 20)) {
     // ---------------- packed weight copies: alternate stages, or (EPI 1) the gate and the up rows of every stage ----------------
     const int mine = warp == 3 ? 0 : 1, ahead = any ? min(pc.k1 - pc.k0, NR) : 0;
     int g = 0;
@@ -425,48 +440,55 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
   } else if (warp == 1) {
     // ---------------- MMA issuer of the pair ----------------
     if (rank == 0) {
-      const uint64_t desc0 = umma_desc_k_sw128(smem_u32(smem));
-      const uint64_t half_stage = static_cast<uint64_t>(region >> 5), second = static_cast<uint64_t>(region >> 4);  // 64 k; the second instruction's tokens
+      constexpr int KS = Q4 ? 8 : 4;  // instructions of 16 k per stage
+      const uint64_t desc_w = umma_desc_k_sw128(smem_u32(smem)), desc0 = umma_desc_k_sw128(smem_u32(smem + (Q4 ? 0 : kWStage)));
+      const uint64_t half_stage = static_cast<uint64_t>(region >> 5), second = static_cast<uint64_t>(region >> 4);  // JQ4: 64 k; the second instruction's tokens
       const bool leader = elect_one();
       int it = 0, sx = 0, sa = 0;
       uint32_t phx = 0, pha = 0;
       bool ok = true, ready = false;  // ready: the next stage's operands have been seen complete
       for (bool more = any; ok && more; more = walk.next(pc), ++it) {
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar_acc_empty), (it & 1) ^ 1, abort_flag, p.status));
+        const int b = NACC == 2 ? it & 1 : 0;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc_empty[b]), ((NACC == 2 ? it >> 1 : it) & 1) ^ 1, abort_flag, p.status));
         if (!ok) break;
-        const uint32_t idesc1 = umma_idesc_bf16(256, pc.n1), idesc2 = umma_idesc_bf16(256, pc.n2), acc2 = tmem_base + pc.n1;
+        const uint32_t idesc1 = umma_idesc_bf16(256, pc.n1), idesc2 = umma_idesc_bf16(256, pc.n2), acc1 = tmem_base + b * kOneMma, acc2 = acc1 + pc.n1;
         const bool both = pc.n2 > 0;
         const int steps = pc.k1 - pc.k0;
         for (int k = 0; k < steps; ++k) {
           if (!ready) {
             ok = mbar_wait(smem_u32(&bar_x_full[sx]), phx, abort_flag, p.status);
-            ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bar_a_full[sa]), pha, abort_flag, p.status));
+            ok = __all_sync(0xffffffffu, ok && (!Q4 || mbar_wait(smem_u32(&bar_a_full[sa]), pha, abort_flag, p.status)));
           }
           if (!ok) break;
           tc_fence_after();
-          const uint64_t db = desc0 + static_cast<uint64_t>((sx * x_bytes) >> 4);
+          const uint64_t at = static_cast<uint64_t>((sx * x_bytes) >> 4), db = desc0 + at, dw = desc_w + at;
           const uint32_t ta = tmem_a + sa * 64;
+          auto product = [&](int j, uint32_t add) {
+            const uint64_t d = db + (j < 4 ? 0 : half_stage) + (j & 3) * 2;
+            if (Q4) {
+              umma_bf16_pair_ts(acc1, ta + j * 8, d, idesc1, add);
+              if (both) umma_bf16_pair_ts(acc2, ta + j * 8, d + second, idesc2, add);
+            } else {
+              umma_bf16_pair(acc1, dw + j * 2, d, idesc1, add);
+              if (both) umma_bf16_pair(acc2, dw + j * 2, d + second, idesc2, add);
+            }
+          };
           if (leader) {
 #pragma unroll
-            for (int j = 0; j < 7; ++j) {
-              const uint64_t d = db + (j < 4 ? 0 : half_stage) + (j & 3) * 2;
-              umma_bf16_pair_ts(tmem_base, ta + j * 8, d, idesc1, (k > 0 || j > 0) ? 1u : 0u);
-              if (both) umma_bf16_pair_ts(acc2, ta + j * 8, d + second, idesc2, (k > 0 || j > 0) ? 1u : 0u);
-            }
+            for (int j = 0; j < KS - 1; ++j) product(j, (k > 0 || j > 0) ? 1u : 0u);
           }
           const uint32_t done = smem_u32(&bar_done[sx]);
           if (++sx == NX) { sx = 0; phx ^= 1; }
-          if (++sa == NA) { sa = 0; pha ^= 1; }
+          if (Q4 && ++sa == NA) { sa = 0; pha ^= 1; }
           // look at the next stage's operands while the pipe works on these
-          ready = k + 1 < steps && __all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bar_x_full[sx]), phx) && mbar_try_wait(smem_u32(&bar_a_full[sa]), pha));
+          ready = k + 1 < steps && __all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bar_x_full[sx]), phx) && (!Q4 || mbar_try_wait(smem_u32(&bar_a_full[sa]), pha)));
           if (leader) {
-            umma_bf16_pair_ts(tmem_base, ta + 56, db + half_stage + 6, idesc1, 1u);
-            if (both) umma_bf16_pair_ts(acc2, ta + 56, db + half_stage + 6 + second, idesc2, 1u);
+            product(KS - 1, 1u);
             umma_commit_pair(done);
           }
         }
         if (!ok) break;
-        if (leader) umma_commit_pair(smem_u32(bar_acc_full));
+        if (leader) umma_commit_pair(smem_u32(&bar_acc_full[b]));
       }
       if (!ok && leader) {
         umma_commit_pair(smem_u32(bar_last));
@@ -483,7 +505,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
     // packed row of this lane: its own, or (EPI 1) eight gate rows and the up rows of the same outputs in turn
     const int r = EPI == 1 ? ((lane >> 3) & 1) * 64 + q4 * 16 + (lane >> 4) * 8 + (lane & 7) : q4 * 32 + lane;
     const uint32_t lanes = static_cast<uint32_t>(q4 * 32) << 16;
-    const uint32_t lane_a = tmem_a + lanes + h * 32;
+    const uint32_t lane_a = tmem_a + lanes + h * 32;  // (JQ4)
     const uint32_t remote_full = mapa_u32(smem_u32(bar_a_full), 0);
     const uint8_t* raw0 = smem + kOffRaw + r * 64 + (((2 * h) ^ ((r >> 1) & 3)) << 4);
     const uint8_t* raw1 = smem + kOffRaw + r * 64 + (((2 * h + 1) ^ ((r >> 1) & 3)) << 4);
@@ -492,7 +514,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
     const bool turned = !p.out_f32 && p.vec == 8;
     bool ok = true;
     for (bool more = any; ok && more; more = walk.next(pc), ++it) {
-      for (int q = pc.k0; q < pc.k1; ++q, ++j) {
+      for (int q = pc.k0; Q4 && q < pc.k1; ++q, ++j) {
         if ((j & 1) != (grp >> 1)) continue;
         const int sr = j % NR, sa = j & (NA - 1);
         ok = mbar_wait(smem_u32(&bar_raw_full[sr]), (j / NR) & 1, abort_flag, p.status);
@@ -530,15 +552,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
         if (lane == 0) mbar_arrive_remote(remote_full + sa * 8);
       }
       // ---- drain: the warps of a quarter take every fourth sixteen columns ----
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(bar_acc_full), it & 1, abort_flag, p.status));
+      const int b = NACC == 2 ? it & 1 : 0;
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&bar_acc_full[b]), (NACC == 2 ? it >> 1 : it) & 1, abort_flag, p.status));
       if (!ok) break;
       tc_fence_after();
       const int tokens = pc.m_lim - pc.m0, cols = pc.n1 + pc.n2;
+      const uint32_t acc = tmem_base + b * kOneMma + lanes;
       if (EPI == 2 || pc.slot >= 0) {
         float* dst = p.sums + static_cast<size_t>(2 * pc.slot + rank) * p.bn * 128 + q4 * 32 + lane;
         for (int c0 = grp * 16; c0 < cols; c0 += 64) {
           uint32_t v[16];
-          tmem_ld_x16(tmem_base + lanes + c0, v);
+          tmem_ld_x16(acc + c0, v);
           tmem_ld_wait();
 #pragma unroll
           for (int c = 0; c < 16; ++c) dst[static_cast<size_t>(c0 + c) * 128] = __uint_as_float(v[c]);
@@ -551,7 +575,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
         const size_t at = static_cast<size_t>(pc.m0) * p.ldo + n;
         for (int c0 = grp * kDrain; c0 < cols; c0 += 4 * kDrain) {
           uint32_t v[16];
-          tmem_ld_x16(tmem_base + lanes + c0, v);
+          tmem_ld_x16(acc + c0, v);
           tmem_ld_wait();
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
@@ -580,8 +604,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
         for (int c0 = grp * kDrain; c0 < cols; c0 += 4 * kDrain, ++turn) {
           uint8_t* buf = smem + kOffDrain + (grp * 2 + (turn & 1)) * kDrainBytes;
           float v[2][8];  // [sixteen rows][token c, c + 1 of rows r and r + 8; the same of tokens + 8]
-          tmem_ld_16x256_x2(tmem_base + lanes + c0, reinterpret_cast<uint32_t*>(v[0]));
-          tmem_ld_16x256_x2(tmem_base + lanes + (16u << 16) + c0, reinterpret_cast<uint32_t*>(v[1]));
+          tmem_ld_16x256_x2(acc + c0, reinterpret_cast<uint32_t*>(v[0]));
+          tmem_ld_16x256_x2(acc + (16u << 16) + c0, reinterpret_cast<uint32_t*>(v[1]));
           tmem_ld_wait();
           if constexpr (EPI == 0) {
 #pragma unroll
@@ -625,7 +649,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(bar_acc_empty), 0));  // the accumulator has been read
+      if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(&bar_acc_empty[b]), 0));  // the accumulator has been read
     }
   }
 
@@ -692,13 +716,13 @@ __global__ void __launch_bounds__(128) gemm_parts_sum_kernel(const PartParams p)
 }
 
 // Pairs of SMs that can hold the kernel at one time on the current GPU, within the limit that is set (as in gemm_pair.cu); 0: none.
-template <int EPI>
+template <bool Q4, int EPI>
 int part_pairs() {
   static int caps[64];  // per GPU; 0: not asked yet, -1: none
   int dev = 0;
   if (g_gemm_pairs == 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   if (caps[dev] == 0) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_parts_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(gemm_parts_kernel<Q4, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     int n = 0;
     if (e == cudaSuccess) {
       cudaLaunchConfig_t cfg = {};
@@ -712,7 +736,7 @@ int part_pairs() {
       attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      e = cudaOccupancyMaxActiveClusters(&n, gemm_parts_kernel<EPI>, &cfg);
+      e = cudaOccupancyMaxActiveClusters(&n, gemm_parts_kernel<Q4, EPI>, &cfg);
     }
     if (e != cudaSuccess) (void)cudaGetLastError();  // (this query's own error; nothing was launched)
     caps[dev] = e == cudaSuccess && n > 0 ? n : -1;
@@ -720,7 +744,11 @@ int part_pairs() {
   const int cap = caps[dev] < 0 ? 0 : caps[dev];
   return g_gemm_pairs > 0 && g_gemm_pairs < cap ? g_gemm_pairs : cap;
 }
-int part_pairs_of(int epi) { return epi == 1 ? part_pairs<1>() : (epi == 2 ? part_pairs<2>() : part_pairs<0>()); }
+int part_pairs_of(bool q4, int epi) {
+  if (q4) return epi == 1 ? part_pairs<true, 1>() : (epi == 2 ? part_pairs<true, 2>() : part_pairs<true, 0>());
+  return epi == 1 ? part_pairs<false, 1>() : (epi == 2 ? part_pairs<false, 2>() : part_pairs<false, 0>());
+}
+int stages_of(const GemmWeightDesc* w) { return w->is_q4 ? (w->K + 127) / 128 : w->K / 64; }
 
 int width_of(const void* out, int ldo, bool f32) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(out) * (f32 ? 1 : 2);
@@ -734,14 +762,15 @@ struct PartPlan {
 };
 // Token tiles, whole waves and parts; in thousands of cycles. A 128-k stage takes 8 instructions of cols / 2 cycles and no less than its expansion, a piece its
 // drain and the first stage that the pipe waits for (an SM stores some 30 bytes per cycle); cut tiles cost the second kernel (four parts at a time) and their sums' way back from L2.
-PartPlan plan_parts(int M, int epi, int n_tiles, int kq, int cap) {
+PartPlan plan_parts(const GemmWeightDesc* w, int M, int epi) {
   PartPlan best;
   const auto up = [](int a, int b) { return (a + b - 1) / b; };
+  const int n_tiles = tiles_of(w->N, epi), kq = stages_of(w), cap = part_pairs_of(w->is_q4, epi);
   if (cap <= 0) return best;
   const int few = up(M, kMaxTokens);
   for (int want = few; want <= few + 1; ++want) {
     const int bn = (up(M, want) + 31) & ~31, m_tiles = up(M, bn), tiles = n_tiles * m_tiles;
-    const double stage = std::max(0.95, bn * 4e-3), part = 0.8 + bn * 17e-3, turn = epi == 0 ? 1.0 + bn * 11.5e-3 : part;
+    const double stage = w->is_q4 ? std::max(0.95, bn * 4e-3) : std::max(0.6, bn * 2.1e-3), part = 0.8 + bn * 17e-3, turn = epi == 0 ? 1.0 + bn * 11.5e-3 : part;
     const int waves = tiles / cap, cut = tiles - waves * cap;
     for (int f = cut > 0 ? 1 : 0; f <= (cut > 0 ? std::min(kq, cap / cut) : 0); ++f) {
       double cost = waves * (kq * stage + turn);
@@ -763,36 +792,37 @@ PartPlan plan_parts(int M, int epi, int n_tiles, int kq, int cap) {
 }
 int cut_tiles(const PartPlan& q) { return q.n_tiles * q.m_tiles - q.waves * q.pairs * (q.waves > 0); }
 
-template <int EPI>
+template <bool Q4, int EPI>
 void launch_parts(const GemmWeightDesc* w, const void* x, int rows, int ldx, PartParams p, cudaStream_t st) {
   CUtensorMap map_x;
   p.box = (p.bn <= kOneMma ? p.bn : (((p.bn >> 1) + 31) & ~31)) / 2;
-  encode_map_kchunks(&map_x, x, static_cast<uint64_t>(rows), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, p.box);
+  encode_map_kchunks(&map_x, x, static_cast<uint64_t>(rows), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, p.box, Q4 ? 2 : 1);
+  CUtensorMap map_w = Q4 ? map_x : w->map_w64;
+  if (!Q4 && EPI == 1) encode_map_gate_up(&map_w, w->data, static_cast<uint64_t>(w->N / 2), static_cast<uint64_t>(w->K));
   p.wq = static_cast<const uint8_t*>(w->data);
-  p.slots = p.bn <= 256 ? 4 : 2;
+  p.slots = Q4 ? (p.bn <= 256 ? 4 : 2) : (p.bn <= 256 ? 2 : 1);
   p.by_m.set(p.m_tiles);
   p.by_parts.set(p.parts);
   p.by_group.set(8 * p.n_tiles);
-  p.x_stages = std::min(kMaxX, kXRoom / (p.box * 256 * (p.bn > kOneMma ? 2 : 1)));
-  if (part_pairs<EPI>() < p.pairs || p.pairs < 1) throw std::runtime_error("JQ4 pair gemm: no pair of SMs can hold the kernel");
+  p.x_stages = Q4 ? std::min(kMaxX, kXRoom / (p.box * 256 * (p.bn > kOneMma ? 2 : 1))) : std::min(kMaxX, kStageRoom / (kWStage + p.box * 128 * (p.bn > kOneMma ? 2 : 1)));
+  if (part_pairs<Q4, EPI>() < p.pairs || p.pairs < 1) throw std::runtime_error("JQ4 pair gemm: no pair of SMs can hold the kernel");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * p.pairs);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = st;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_parts_kernel<EPI>, map_x, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_parts_kernel<Q4, EPI>, map_x, map_w, p);
   const int tiles = p.n_tiles * p.m_tiles, second = EPI == 2 ? tiles : (p.parts > 1 ? tiles - p.waves * p.pairs : 0);
   if (e == cudaSuccess && p.items == nullptr && second > 0) e = launch_pdl(gemm_parts_sum_kernel<EPI>, dim3(2 * second, (p.bn + 7) / 8), dim3(128), 0, st, p);
   if (e != cudaSuccess) throw std::runtime_error(std::string("JQ4 pair gemm launch: ") + cudaGetErrorString(e));
 }
 
 PartParams dense_params(const GemmWeightDesc* w, int M, int epi, float* sums, int* status) {
-  const int kq = (w->K + 127) / 128;
-  const PartPlan plan = plan_parts(M, epi, tiles_of(w->N, epi), kq, part_pairs_of(epi));
+  const PartPlan plan = plan_parts(w, M, epi);
   PartParams p = {};
   p.M = M;
   p.N = w->N;
-  p.kq = kq;
+  p.kq = stages_of(w);
   p.bn = plan.bn;
   p.n_tiles = plan.n_tiles;
   p.m_tiles = plan.m_tiles;
@@ -811,30 +841,46 @@ PartParams dense_params(const GemmWeightDesc* w, int M, int epi, float* sums, in
 // Weights and outputs the kernel takes: k in whole chunks of 64, as the token copies fetch them. `n`: rows of the weight (of one expert). EPI 1: whole
 // halves of 64 rows, so that gate and up rows begin on a half tile.
 bool gemm_parts_supported(const GemmWeightDesc* w, int n, const void* out, int ldo, int epi) {
-  if (!w->is_q4 || w->K % 64 != 0 || w->K < 64 || n < 64 || part_pairs_of(epi) <= 0) return false;
-  if (epi == 1) return n % 128 == 0 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  if (w->K % 64 != 0 || w->K < 64 || n < 64 || part_pairs_of(w->is_q4, epi) <= 0) return false;
+  if (epi == 1) return n % (w->is_q4 ? 128 : 16) == 0 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   if (epi == 2) return ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
   return true;
 }
 
-// Whether this kernel is the faster one for M rows of a dense JQ4 weight.
-// Below: the one-tile kernel, which may start under the kernel in front and so saves some two microseconds, up to 128 rows, and the gated form (whose
+// Whether this kernel is the faster one for M rows of a dense weight; all times in microseconds, 1.62 thousand cycles of the plan are one.
+// JQ4, below: the one-tile kernel, which may start under the kernel in front and so saves some two microseconds, up to 128 rows, and the gated form (whose
 // activation would be a launch of its own) up to 32: 19456 x 2560, 64 rows 22.4 us against 22.3 and two launches, 128 rows 24.3 against 29.5, 333 rows 38
 // against 51; 6144 x 2560 with heads 333 rows 22 against 38; 2560 x 9728 128 rows 15.4 against 13.0, 333 rows 23 against 27.
-// Above: the pair kernel behind an expansion to bf16, whose drain runs under the next tile; by both kernels' estimated times (here 1.62 thousand cycles are a
-// microsecond). The pair kernel's estimate must be a seventh longer: where they are closer than that, prompts of several thousand rows that pull the clock
+// Above: the pair kernel behind an expansion to bf16, whose drain runs under the next tile; by both kernels' estimated times. The pair kernel's
+// estimate must be a seventh longer: where they are closer than that, prompts of several thousand rows that pull the clock
 // down by their power ran up to a tenth longer here (19456 x 2560, 1536 rows 119 us against 143, 2048 rows 154 against 174, 4096 rows 332 against
 // 322; 2560 x 9728, 2048 rows 68 against 112).
+// bf16, gated: from 33 rows on, against the pair kernel's 1.2 estimates and 8 us (its drain takes longer than the plain one): 28672 x 3584, 48 rows 42.7 against
+// 44.5 in two launches, 128 rows 44.8 against 56.4, 384 rows 69 against 86, 896 rows 137 against 149, but 1280 rows 187 against 179 and 2048 rows 298 against 281; 11264 x 2048, 128 rows 15.1
+// against 20.1, 384 rows 22.9 against 35.5, 1536 rows 54 against 65. Heads: one token tile (64 to 384 rows: every sum goes through the second kernel),
+// 6144 x 4096, 128 rows 18.0 against 22.4, 320 rows 25.2 against 31.6, 512 rows 35.5 against 31.9. Plain: from 193 rows on, against the better of the others (one-tile
+// while gemm_pair_preferred says so): 3584 x 14336, 384 rows 40 against 58, 700 rows 64 against 70, 1024 rows 91 against 79; 2560 x 2048, 256 rows 11.5 against
+// 12.9, 2048 rows 18.1 against 24.9; 2048 x 2048, 256 rows 11.1 against 12.4, 512 rows 13.3 against 12.8.
+// Plain, fewer rows: the one-tile kernel reads weights at some 4.3 TB/s with 65 to 128 rows and 5.8 with 33 to 64, this one at 5.7 and 6.2 and starts some 4 us later:
+// 36 M and some 170 M weights (256000 x 3584, 128 rows 323 us against 429, 64 rows 295 against 317; 3584 x 14336, 128 rows 28.4 against 29.9).
 bool gemm_parts_preferred(const GemmWeightDesc* w, int M, int epi) {
-  if (!w->is_q4 || M <= (epi == 1 ? 32 : 128) || g_gemm_persist || g_gemm_force_bn != 0) return false;  // (the last two: another kernel or tile was asked for)
-  const PartPlan plan = plan_parts(M, epi, tiles_of(w->N, epi), (w->K + 127) / 128, part_pairs_of(epi));
+  if (M <= 32 || g_gemm_persist || g_gemm_force_bn != 0) return false;  // (the last two: another kernel or tile was asked for)
+  const double weights = static_cast<double>(w->N) * w->K;
+  if (w->is_q4 ? (epi != 1 && M <= 128) : (epi == 0 && M <= 192 && weights < (M > 64 ? 36e6 : 170e6))) return false;
+  if (epi == 2 && M <= 64) return false;
+  const PartPlan plan = plan_parts(w, M, epi);
   if (plan.pairs == 0) return false;
-  return M < 768 || 2.5 + plan.cost / 1.62 < 0.86 * gemm_pair_estimate(w, M, w->N);
+  const double pair = gemm_pair_estimate(w, M, w->N);
+  if (w->is_q4) return M < 768 || 2.5 + plan.cost / 1.62 < 0.86 * pair;
+  const double here = 3.0 + plan.cost / 1.62;
+  if (epi == 1) return M < 2048 && here < 0.95 * (1.2 * pair + 8.0);
+  if (epi == 2) return M <= kMaxTokens || here < 0.86 * pair;
+  return M <= 192 || here < (gemm_pair_preferred(w, M, w->N, 0) ? 0.95 : 1.08) * pair;
 }
 
 // fp32 room for the sums that the second kernel finishes (0: none)
 size_t gemm_parts_room(const GemmWeightDesc* w, int M, int epi) {
-  const PartPlan plan = plan_parts(M, epi, tiles_of(w->N, epi), (w->K + 127) / 128, part_pairs_of(epi));
+  const PartPlan plan = plan_parts(w, M, epi);
   const size_t cut = static_cast<size_t>(cut_tiles(plan)), slots = cut * plan.parts + (epi == 2 ? static_cast<size_t>(plan.waves) * plan.pairs : 0);
   return epi == 2 || plan.parts > 1 ? slots * 2 * plan.bn * 128 : 0;
 }
@@ -847,7 +893,8 @@ void gemm_parts_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void
   p.out_f32 = out_f32 ? 1 : 0;
   p.vec = width_of(out, ldo, out_f32);
   p.bias = bias;
-  launch_parts<0>(w, x, M, ldx, p, st);
+  if (w->is_q4) launch_parts<true, 0>(w, x, M, ldx, p, st);
+  else launch_parts<false, 0>(w, x, M, ldx, p, st);
 }
 
 void gemm_parts_run_act(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, int act, float* sums, int* status, cudaStream_t st) {
@@ -855,7 +902,8 @@ void gemm_parts_run_act(const GemmWeightDesc* w, const void* x, int M, int ldx, 
   p.out = out;
   p.ldo = ldo;
   p.act_kind = act;
-  launch_parts<1>(w, x, M, ldx, p, st);
+  if (w->is_q4) launch_parts<true, 1>(w, x, M, ldx, p, st);
+  else launch_parts<false, 1>(w, x, M, ldx, p, st);
 }
 
 void gemm_parts_run_qkv(const GemmWeightDesc* w, const void* x, int M, int ldx, void* q_out, int ldo, const float* bias, const GemmQkvArgs* a, float* sums,
@@ -865,7 +913,8 @@ void gemm_parts_run_qkv(const GemmWeightDesc* w, const void* x, int M, int ldx, 
   p.ldo = ldo;
   p.bias = bias;
   p.qkv = *a;
-  launch_parts<2>(w, x, M, ldx, p, st);
+  if (w->is_q4) launch_parts<true, 2>(w, x, M, ldx, p, st);
+  else launch_parts<false, 2>(w, x, M, ldx, p, st);
 }
 
 // Experts: work items of up to `item_rows` rows (384 at most); act 0: out [rows, n], otherwise act(gate) * up: out [rows, n / 2].
@@ -879,7 +928,7 @@ void gemm_parts_run_grouped(const GemmWeightDesc* w, int n_per_expert, const voi
   p.bn = (item_rows + 31) & ~31;
   p.n_tiles = tiles_of(n_per_expert, act ? 1 : 0);
   p.m_tiles = max_items;
-  p.pairs = std::min(p.n_tiles * p.m_tiles, part_pairs_of(act ? 1 : 0));
+  p.pairs = std::min(p.n_tiles * p.m_tiles, part_pairs_of(true, act ? 1 : 0));
   p.w_tiles = (n_per_expert + 127) / 128;
   p.half = n_per_expert / 2;
   p.out = out;
@@ -888,8 +937,8 @@ void gemm_parts_run_grouped(const GemmWeightDesc* w, int n_per_expert, const voi
   p.items = reinterpret_cast<const int4*>(items);
   p.act_kind = act;
   p.status = status;
-  if (act == 0) launch_parts<0>(w, x, rows, ldx, p, st);
-  else launch_parts<1>(w, x, rows, ldx, p, st);
+  if (act == 0) launch_parts<true, 0>(w, x, rows, ldx, p, st);
+  else launch_parts<true, 1>(w, x, rows, ldx, p, st);
 }
 
 }  // namespace dlv

@@ -1183,6 +1183,53 @@ def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
         assert _rel(u, v) < 4e-3 and torch.equal(u == 0, v == 0)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 256, 64), (70, 272, 192), (200, 136, 64), (257, 1040, 2624), (385, 528, 192), (800, 11264, 192), (2600, 3072, 320), (900, 19200, 128)])
+def test_parts_gemm_bf16(M, N, K):
+    """bf16 weights: 64-k stages of their own, one and two accumulators, halves of an odd number of eights (gated), rows that end inside a half tile, several waves with
+    two accumulators in turn, rows without 16 bytes at once, fp32 outputs; guard areas around output and sums. fp32 sums, rounded once: 2^-9, gated products once more."""
+    wd = (torch.randn(N, K) * 0.05).to(torch.bfloat16)
+    lw = LinearWeight(wd).to(DEV, torch.bfloat16)
+    x = (torch.randn(M, K + 8) * 0.5).to(torch.bfloat16).to(DEV)[:, :K]
+    f = x.double().cpu() @ wd.double().t()
+    odd = torch.full((M, N + 1), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.set_bounds_check(True)
+    try:
+        y, y32 = ops.linear(x, lw, impl=4), ops.linear(x, lw, impl=4, out_f32=True)
+        ops.linear(x, lw, impl=4, out=odd[:, :N])
+        h = lw.handle().run_gated(x, 1, 4)
+        torch.cuda.synchronize()
+        ops.check_guards()
+    finally:
+        ops.set_bounds_check(False)
+    ops.check_status()
+    assert _rel(y.cpu(), f) < 3e-3 and _rel(y32.cpu(), f) < 2e-5 and torch.equal(odd[:, :N], y) and bool((odd[:, N] == 7.0).all())
+    if N % 16 == 0:
+        assert _rel(h.cpu(), torch.nn.functional.silu(f[:, : N // 2]) * f[:, N // 2 :]) < 3e-3
+    else:
+        assert h is None
+
+
+@pytest.mark.parametrize("M", [1, 129, 900])
+def test_parts_gemm_bf16_heads(M):
+    """q | k | v heads of bf16 weights against the one-tile kernel, an odd number of heads."""
+    heads, kv, K, D = 5, 2, 320, 128
+    lw = LinearWeight((torch.randn((heads + 2 * kv) * D, K) * 0.05).to(torch.bfloat16)).to(DEV, torch.bfloat16)
+    x = (torch.randn(M, K) * 0.5).to(torch.bfloat16).to(DEV)
+    slots, pos = torch.randperm((M // 32 + 2) * 32, device=DEV)[:M], torch.arange(M, dtype=torch.int32, device=DEV) + 37
+    cos, sin = (t.to(DEV) for t in ref.rope_tables(D, 4096, 10000.0))
+    qn, kn = ((1 + 0.1 * torch.randn(D)).to(torch.bfloat16).to(DEV) for _ in range(2))
+    got = []
+    for pairs, impl in ((0, 0), (-1, 4)):
+        ops.set_gemm_pairs(pairs)
+        kc, vc = (torch.zeros(M // 32 + 2, kv, 32, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        q = lw.handle().run_qkv(x, pos, slots, qn, kn, cos, sin, kc, vc, heads, kv, 1e-6, 0.0, None, impl)
+        got.append((q, kc, vc))
+    torch.cuda.synchronize()
+    ops.check_status()
+    for u, v in zip(*got):  # (sums in another order, rounded to bf16 up to twice: 2^-9 each)
+        assert _rel(u, v) < 4e-3 and torch.equal(u == 0, v == 0)
+
+
 @pytest.mark.parametrize("E,n,K,T,k", [(4, 512, 256, 900, 2), (3, 384, 1216, 1500, 1), (40, 1280, 128, 9000, 2)])
 def test_parts_gemm_experts(E, n, K, T, k):
     """Equal work items of up to 384 rows (one and two instructions, more items than an expert's rows ask for at the end of the list), as the experts of a prompt have them."""
