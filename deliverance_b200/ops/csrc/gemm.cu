@@ -631,52 +631,96 @@ void gemm_tc_run_grouped_act(const GemmWeightDesc* w, int n_per_expert, const vo
 __device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ------------------------------------------------------------------------------------------------ one row of bf16 weights
-// One token row against a dense weight: a warp per weight row, 16 bytes per lane and chunk of 256 elements. Bound by the weight stream, and at
-// a few megabytes by how early and how widely it starts: the row is on its way to L2 while the kernel in front finishes, and eight chunks per
-// lane are in flight behind the wait. gemv_simt_kernel, which it replaces here, had one or two chunks in flight behind an
-// ordinary launch (tinyllama's 22 layers at one token: 638 us of GEMVs for 2.07 GB).
-constexpr int kGemvChunks = 8;
-template <bool OUTF>
-__global__ void __launch_bounds__(128) gemv_bf16_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x, void* __restrict__ out,
-                                                        const float* __restrict__ bias, int N, int K) {
+// One token row against a dense weight: a warp per weight row, in pieces of up to 2048 elements. Bound by the weight stream, and at a few megabytes by how early and
+// how widely it starts. So all CTAs are resident at one time, and every warp has its first pieces copied into shared memory (28 MB on the whole GPU, all of most
+// projections of a small model) while the kernel in front finishes: behind the wait only the row and the products are left. A lane copies what it reads itself, so
+// no barrier is needed. Measured against rows that were on their way to L2 only, eight loads per lane behind the wait (in a chain of such products): 2048 x 2048 4.1 -> 2.5 us,
+// 2048 x 5632 9.2 -> 6.1, 11264 x 2048 10.5 -> 9.9, 3584 x 14336 37.5 -> 21.0, 28672 x 3584 36.8 -> 34.0; tinyllama's step at one token 937 -> 795.
+// From 24 rows per warp on (an output head), CTAs of four rows per warp as room comes up, because SMs do not get equal shares of the memory: 256000 x 3584
+// 283 -> 251 us.
+constexpr int kRowPiece = 2048, kRowRing = 6144, kRowWarps = 4, kRowCtas = 4;  // elements of a piece and of a warp's ring (48 KB per CTA), warps per CTA, CTAs per SM
+// CH: chunks of 256 elements per piece (a constant: 151936 x 2560 took 125 us with eight of which five were predicated on, and takes 114)
+template <bool OUTF, int CH>
+__global__ void __launch_bounds__(kRowWarps * 32, kRowCtas) gemv_bf16_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x,
+                                                                            void* __restrict__ out, const float* __restrict__ bias, int N, int K) {
+  constexpr int piece = CH * 256, PIECES = kRowRing / piece;
   pdl_trigger();
-  const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const __nv_bfloat16* row = w + static_cast<size_t>(min(n, N - 1)) * K;
-  uint4 wv[kGemvChunks];
-  auto fetch = [&](int k0) {
+  extern __shared__ uint4 row_pieces[];  // [warp][piece][chunk of 256 elements][lane]
+  const int lane = threadIdx.x & 31, first = blockIdx.x * kRowWarps + (threadIdx.x >> 5), step = gridDim.x * kRowWarps;
+  uint4* ring = row_pieces + (threadIdx.x >> 5) * (kRowRing / 8) + lane;
+  int fn = first, fk = 0, fs = 0;  // next piece to copy: row, element, place in the ring
+  auto copy = [&] {
+    if (fn < N) {
+      const __nv_bfloat16* src = w + static_cast<size_t>(fn) * K + fk + lane * 8;
+      const uint32_t dst = smem_u32(ring + fs * (piece / 8));
+      const int len = min(piece, K - fk);
 #pragma unroll
-    for (int i = 0; i < kGemvChunks; ++i) {
-      const int k = k0 + i * 256 + lane * 8;
-      wv[i] = k < K ? __ldg(reinterpret_cast<const uint4*>(row + k)) : make_uint4(0u, 0u, 0u, 0u);
+      for (int i = 0; i < CH; ++i) {
+        if (i * 256 + lane * 8 < len) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 512), "l"(src + i * 256) : "memory");
+      }
+      fk += piece;
+      if (fk >= K) {
+        fk = 0;
+        fn += step;
+      }
+      fs = fs + 1 == PIECES ? 0 : fs + 1;
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int k = lane * 8; k < K; k += 256) l2_prefetch(row + k);
+  for (int i = 0; i < PIECES; ++i) copy();
   pdl_wait();
-  if (n >= N) return;
-  fetch(0);
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < K; k0 += kGemvChunks * 256) {
-    if (k0 > 0) fetch(k0);
+  int s = 0;
+  uint4 xv[CH];
+  for (int n = first; n < N; n += step) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int k0 = 0; k0 < K; k0 += piece) {
+      const int len = min(piece, K - k0);
+      if (K > piece || n == first) {  // (a row of one piece stays in registers)
 #pragma unroll
-    for (int i = 0; i < kGemvChunks; ++i) {
-      const int k = k0 + i * 256 + lane * 8;
-      if (k < K) {
-        const uint4 xv = *reinterpret_cast<const uint4*>(x + k);
-        const uint32_t wu[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w}, xu[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 a = unpack_bf162(wu[e]), b = unpack_bf162(xu[e]);
-          acc[e] += a.x * b.x + a.y * b.y;
+        for (int i = 0; i < CH; ++i) {
+          const int k = i * 256 + lane * 8;
+          xv[i] = k < len ? *reinterpret_cast<const uint4*>(x + k0 + k) : make_uint4(0u, 0u, 0u, 0u);
         }
       }
+      asm volatile("cp.async.wait_group %0;" ::"n"(PIECES - 1) : "memory");
+      const uint4* at = ring + s * (piece / 8);
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        if (i * 256 + lane * 8 < len) {
+          const uint4 wv = at[i * 32];
+          const uint32_t wu[4] = {wv.x, wv.y, wv.z, wv.w}, xu[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 a = unpack_bf162(wu[e]), b = unpack_bf162(xu[e]);
+            acc[e] += a.x * b.x + a.y * b.y;
+          }
+        }
+      }
+      copy();  // into the place that this lane has just read
+      s = s + 1 == PIECES ? 0 : s + 1;
+    }
+    const float sum = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+    if (lane == 0) {
+      const float v = sum + (bias != nullptr ? bias[n] : 0.f);
+      if (OUTF) static_cast<float*>(out)[n] = v;
+      else static_cast<__nv_bfloat16*>(out)[n] = f2bf(v);
     }
   }
-  const float sum = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
-  if (lane == 0) {
-    const float v = sum + (bias != nullptr ? bias[n] : 0.f);
-    if (OUTF) static_cast<float*>(out)[n] = v;
-    else static_cast<__nv_bfloat16*>(out)[n] = f2bf(v);
-  }
+}
+template <bool OUTF>
+static void gemv_bf16_launch(const __nv_bfloat16* w, const __nv_bfloat16* x, void* out, const float* bias, int N, int K, cudaStream_t st) {
+  const int all = gemm_num_sms() * kRowCtas, few = (N + kRowWarps - 1) / kRowWarps;
+  const dim3 ctas(N > all * kRowWarps * 24 ? (few + 3) / 4 : std::min(few, all));
+  // pieces of like length, as many as the ring takes (2560 elements: four halves of a row, not three pieces of 2048 and 512)
+  const int cuts = (K + kRowPiece - 1) / kRowPiece, ch = ((K + cuts - 1) / cuts + 255) / 256;
+  constexpr int kBytes = kRowWarps * kRowRing * 2;  // (48 KB: what a kernel may have without asking)
+  auto run = [&](auto kernel) { return launch_pdl(kernel, ctas, dim3(kRowWarps * 32), kBytes, st, w, x, out, bias, N, K); };
+  const cudaError_t e = ch <= 4   ? run(gemv_bf16_kernel<OUTF, 4>)
+                        : ch == 5 ? run(gemv_bf16_kernel<OUTF, 5>)
+                        : ch == 6 ? run(gemv_bf16_kernel<OUTF, 6>)
+                        : ch == 7 ? run(gemv_bf16_kernel<OUTF, 7>)
+                                  : run(gemv_bf16_kernel<OUTF, 8>);
+  if (e != cudaSuccess) throw std::runtime_error(std::string("one-row gemv launch: ") + cudaGetErrorString(e));
 }
 
 // ------------------------------------------------------------------------------------------------ CUDA-core GEMV
@@ -1199,8 +1243,8 @@ void gemv_simt_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void*
   const unsigned grid = (w->N + 3) / 4;
   if (M == 1 && !w->is_q4 && (reinterpret_cast<uintptr_t>(w->data) & 15) == 0) {  // (K % 8 == 0 and aligned x rows: checked at the entry points)
     const __nv_bfloat16 *wp = static_cast<const __nv_bfloat16*>(w->data), *xp = static_cast<const __nv_bfloat16*>(x);
-    if (out_f32) launch_pdl(gemv_bf16_kernel<true>, dim3(grid), dim3(128), 0, st, wp, xp, out, bias, w->N, w->K);
-    else launch_pdl(gemv_bf16_kernel<false>, dim3(grid), dim3(128), 0, st, wp, xp, out, bias, w->N, w->K);
+    if (out_f32) gemv_bf16_launch<true>(wp, xp, out, bias, w->N, w->K, st);
+    else gemv_bf16_launch<false>(wp, xp, out, bias, w->N, w->K, st);
     return;
   }
   for (int m0 = 0; m0 < M; m0 += 4) {

@@ -1092,6 +1092,19 @@ def test_gemv_bf16_row(N, K, f32):
 
 
 # As for the pair kernel: fp32 sums rounded to bf16 once, JQ4 products rounded to bf16 twice on top.
+@pytest.mark.parametrize("N,K", [(1, 8), (7, 1024), (2500, 1032), (5000, 256), (9, 2056), (2400, 2560), (300, 3080), (33, 14336), (57001, 64), (60000, 1544)])
+def test_gemv_bf16_pieces(N, K):
+    """Rows of one and several pieces, three to six of them in a warp's ring, fewer rows than warps, several rows per warp, more rows than resident CTAs take, and rows
+    wider than a ring. fp32 sums, rounded once for bf16 outputs (2^-9)."""
+    w = LinearWeight((torch.randn(N, K) * 0.05).to(torch.bfloat16)).to(DEV, torch.bfloat16)
+    w.bias = torch.randn(N, device=DEV)
+    x = torch.randn(1, K).to(torch.bfloat16).to(DEV)
+    y, y32, again = ops.linear(x, w), ops.linear(x, w, out_f32=True), ops.linear(x, w)
+    f = x.double() @ w.w.double().t() + w.bias.double()
+    torch.cuda.synchronize()
+    assert _rel(y32, f) < 1e-5 and torch.equal(y, y32.to(torch.bfloat16)) and torch.equal(y, again)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (31, 264, 128), (33, 136, 192), (256, 512, 1280), (257, 2560, 960), (385, 19456, 256), (700, 1000, 2624), (1537, 4104, 512)])
 def test_parts_gemm_edges(M, N, K):
     """One row; k that ends inside a packed stage; weight tiles that end inside a tile and inside eight outputs; one and two instructions per tile, several tiles of
