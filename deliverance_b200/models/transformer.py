@@ -358,7 +358,13 @@ class DecoderModel:
         k_cache, v_cache = kv.layer(i)
         local_rope = lw.kind == "sliding" and self.cos_local is not None
         cos, sin = (self.cos_local, self.sin_local) if local_rope else (self.cos, self.sin)
-        if self.fused_rope and "qkv" not in lw.lora and self._sp is None:
+        inside = batch.is_decode and self._sp is None and ops.rope_in_attention(x.device, self.n_heads, self.n_kv, cfg.head_dim)
+        if inside:  # norm + rotary + cache write in the attention kernel
+            with self._stage("causalselfattention.qkv_projection"):
+                q = self._col_parallel(x, lw.qkv)
+                if lw.lora:
+                    q = self._lora(lw, "qkv", x, q)
+        elif self.fused_rope and "qkv" not in lw.lora and self._sp is None:
             # norm + rotary + cache write in the projection's epilogue (one launch instead of two, q is written once); a
             # sequence-parallel forward gathers its input inside the projection and keeps the two-kernel form
             with self._stage("causalselfattention.qkv_projection"):
@@ -374,7 +380,11 @@ class DecoderModel:
                                 self.n_heads, self.n_kv, cfg.head_dim, cfg.norm_eps, cfg.norm_weight_offset)
         window = cfg.window(i)
         with self._stage("causalselfattention.score_value"):
-            if batch.is_decode:
+            if inside:
+                a = ops.decode_attention_rope(q, batch.positions, batch.slots, lw.q_norm, lw.k_norm, cos, sin, k_cache, v_cache, batch.block_tables, batch.ctx_len,
+                                              self.n_heads, cfg.scale, cfg.attn_softcap, window, batch.decode_splits, cfg.norm_eps, cfg.norm_weight_offset,
+                                              batch.decode_even, lambda *a: batch.decode_plan(i, *a))
+            elif batch.is_decode:
                 a = ops.decode_attention(q, k_cache, v_cache, batch.block_tables, batch.ctx_len, self.n_heads, cfg.scale,
                                          cfg.attn_softcap, window, batch.decode_splits, even=batch.decode_even,
                                          plan=lambda *a: batch.decode_plan(i, *a))

@@ -575,6 +575,23 @@ def decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, H, scale, soft
     return o.reshape(B, H * D)
 
 
+def rope_in_attention(device: torch.device, H: int, KV: int, D: int) -> bool:
+    """Whether a decode step's norm, rotation and cache write go into the attention kernel (:func:`decode_attention_rope`): heads of 64, whose projection does not do them in
+    its epilogue."""
+    return device.type == "cuda" and D == 64 and H // KV <= 16 and not _MERGE_IN_KERNEL[0]
+
+
+def decode_attention_rope(qkv, positions, slots, q_norm_w, k_norm_w, cos, sin, k_cache, v_cache, block_tables, ctx_lens, H, scale, softcap=0.0, window=0, splits=1,
+                          eps=1e-6, norm_offset=0.0, even=False, plan=None):
+    """:func:`rope_kv` and :func:`decode_attention` in one kernel: qkv ``[B, (H + 2 KV) * D]``, one new row per sequence, the last of its ``ctx_lens`` keys."""
+    D = k_cache.shape[3]
+    _check_full_rotary(cos, D)
+    splits, used = decode_launch(splits, even, plan, ctx_lens, qkv.shape[0], H, k_cache.shape[1], D, int(window))
+    _count(1 if splits <= 1 else 2)
+    return require_ext().decode_attention_rope(qkv, positions.to(torch.int32), slots, q_norm_w, k_norm_w, cos, sin, k_cache, v_cache, block_tables, ctx_lens, H, scale,
+                                               softcap, window, splits, eps, norm_offset, used)
+
+
 def prefill_tiles(q_lens: list[int], tile: int = 64) -> tuple[list[int], list[int]]:
     seqs, q0s = [], []
     for i, n in enumerate(q_lens):

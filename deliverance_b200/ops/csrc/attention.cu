@@ -533,13 +533,20 @@ struct DecodeOptions {
 };
 template <>
 struct DecodeOptions<0> {};
-template <int D, int EXT, int NW, bool PLAN>
+// ROPE: q holds the projection's rows, q | k | v heads, before norm, rotation and cache write. Every warp prepares the query rows for itself while its first slices are
+// on their way; the warp that has the last slice prepares the new key and value, keeps them in the cache and puts them into its slice in shared
+// memory (the copy leaves that row out). A kernel of its own for this stood between the projection and the attention with nothing to stream meanwhile.
+template <bool ROPE>
+struct DecodeRope {};
+template <>
+struct DecodeRope<true> : DecodeRopeArgs {};
+template <int D, int EXT, int NW, bool PLAN, bool ROPE>
 __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode_attn_mma_kernel(
     const __nv_bfloat16* __restrict__ q, long long q_stride, const __nv_bfloat16* __restrict__ k_cache,
     const __nv_bfloat16* __restrict__ v_cache, const int* __restrict__ block_tables, int bt_stride,
     const int* __restrict__ ctx_lens, __nv_bfloat16* __restrict__ out, float* part_o, float* part_ml, int* __restrict__ arrivals,
     int H, int KV, int page_size, float scale, float softcap, int window, int splits, int min_slices, const DecodeOptions<EXT> opt,
-    const DecodePlan<PLAN> plan) {
+    const DecodePlan<PLAN> plan, const DecodeRope<ROPE> rope) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
   using L = DecodeMma<D, NW>;
@@ -612,7 +619,7 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
     for (int i = 0; i < 16 * CPR / 32; ++i) {
       const int c = i * 32 + lane;
       const int r = c / CPR, cc = c % CPR;
-      const bool valid = key0 + r < ctx;
+      const bool valid = key0 + r < (ROPE ? ctx - 1 : ctx);  // (ROPE: the new row comes from registers)
       if constexpr (EXT == 1) {
         const bool vk = valid && cc * 8 < dk, vv = valid && cc * 8 < dv;
         cp_async16(kdst + swz<D>(r, cc), kb + (vk ? r * dk + cc * 8 : 0), vk);
@@ -634,6 +641,113 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
     if (j < n_mine) load_slice(j, j);
     cp_async_commit();
   }
+  [[maybe_unused]] uint32_t new_k[2] = {}, new_v[2] = {};  // ROPE: this lane's part of the new row: elements PER * lane .. and the same of the upper half
+  [[maybe_unused]] bool has_new = false;
+  if constexpr (ROPE) {
+    static_assert(D <= 128 && EXT == 0, "query rows in registers, one CTA per KV head");
+    constexpr int HALF = D / 2, PER = HALF / 32;
+    int pos = 0;
+    if (rope.cos_t != nullptr) {
+      pos = rope.positions[b];
+      pos = pos < 0 ? 0 : (pos >= rope.max_pos ? rope.max_pos - 1 : pos);
+    }
+    const float *cs = rope.cos_t + static_cast<size_t>(pos) * HALF, *sn = rope.sin_t + static_cast<size_t>(pos) * HALF;
+    const __nv_bfloat16 *qn = static_cast<const __nv_bfloat16*>(rope.q_norm_w), *kn = static_cast<const __nv_bfloat16*>(rope.k_norm_w);
+#pragma unroll
+    for (int hr = 0; hr < 2; ++hr) {  // rows g and g + 8; words hr and hr + 2 of a fragment hold elements d0, d0 + 1 and d0 + 8, d0 + 9
+      if (hr * 8 >= G) continue;      // (the whole warp; rows past G hold zeros and stay zeros)
+      float inv = 1.f;
+      if (qn != nullptr) {
+        float ss = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float2 f = unpack_bf162(qa[ks][hr + 2 * e]);
+            ss += f.x * f.x + f.y * f.y;
+          }
+        }
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        inv = rsqrtf(ss / D + rope.eps);
+      }
+#pragma unroll
+      for (int ks = 0; ks < D / 32; ++ks) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int d0 = ks * 16 + 2 * t4 + 8 * e;
+          float2 lo = unpack_bf162(qa[ks][hr + 2 * e]), hi = unpack_bf162(qa[ks + D / 32][hr + 2 * e]);
+          if (qn != nullptr) {  // round through bf16 like a separate norm kernel would
+            const float2 wl = unpack_bf162(*reinterpret_cast<const uint32_t*>(qn + d0)), wh = unpack_bf162(*reinterpret_cast<const uint32_t*>(qn + HALF + d0));
+            lo.x = bf2f(f2bf(lo.x * inv * (wl.x + rope.norm_offset)));
+            lo.y = bf2f(f2bf(lo.y * inv * (wl.y + rope.norm_offset)));
+            hi.x = bf2f(f2bf(hi.x * inv * (wh.x + rope.norm_offset)));
+            hi.y = bf2f(f2bf(hi.y * inv * (wh.y + rope.norm_offset)));
+          }
+          if (rope.cos_t != nullptr) {
+            const float2 c = *reinterpret_cast<const float2*>(cs + d0), n = *reinterpret_cast<const float2*>(sn + d0);
+            const float2 x0 = lo, x1 = hi;
+            lo.x = x0.x * c.x - x1.x * n.x;
+            hi.x = x1.x * c.x + x0.x * n.x;
+            lo.y = x0.y * c.y - x1.y * n.y;
+            hi.y = x1.y * c.y + x0.y * n.y;
+          }
+          qa[ks][hr + 2 * e] = pack_bf162(lo.x, lo.y);
+          qa[ks + D / 32][hr + 2 * e] = pack_bf162(hi.x, hi.y);
+        }
+      }
+    }
+    const int last = list.count() - 1;
+    has_new = last < 0 ? sp == 0 && warp == 0 : last >= s0 && last < s1 && (last - s0) % NW == warp;
+    if (has_new) {
+      const __nv_bfloat16 *kr = q + static_cast<long long>(b) * q_stride + static_cast<long long>(H + kvh) * D, *vr = kr + static_cast<long long>(KV) * D;
+      float a[PER], c[PER];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        a[i] = bf2f(kr[lane * PER + i]);
+        c[i] = bf2f(kr[HALF + lane * PER + i]);
+        const unsigned short *v = reinterpret_cast<const unsigned short*>(vr) + lane * PER + i;
+        new_v[0] |= static_cast<uint32_t>(v[0]) << (16 * i);
+        new_v[1] |= static_cast<uint32_t>(v[HALF]) << (16 * i);
+      }
+      if (kn != nullptr) {
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) ss += a[i] * a[i] + c[i] * c[i];
+        const float inv = rsqrtf(warp_sum(ss) / D + rope.eps);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          a[i] = bf2f(f2bf(a[i] * inv * (bf2f(kn[lane * PER + i]) + rope.norm_offset)));
+          c[i] = bf2f(f2bf(c[i] * inv * (bf2f(kn[HALF + lane * PER + i]) + rope.norm_offset)));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        if (rope.cos_t != nullptr) {
+          const float co = cs[lane * PER + i], si = sn[lane * PER + i], x0 = a[i], x1 = c[i];
+          a[i] = x0 * co - x1 * si;
+          c[i] = x1 * co + x0 * si;
+        }
+        new_k[0] |= static_cast<uint32_t>(__bfloat16_as_ushort(f2bf(a[i]))) << (16 * i);
+        new_k[1] |= static_cast<uint32_t>(__bfloat16_as_ushort(f2bf(c[i]))) << (16 * i);
+      }
+      const long long slot = rope.slots[b];
+      if (slot >= 0) {
+        const long long at = ((slot / page_size * KV + kvh) * page_size + slot % page_size) * D + lane * PER;
+        __nv_bfloat16 *kd = static_cast<__nv_bfloat16*>(rope.k_cache) + at, *vd = static_cast<__nv_bfloat16*>(rope.v_cache) + at;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if constexpr (PER == 2) {
+            *reinterpret_cast<uint32_t*>(kd + h * HALF) = new_k[h];
+            *reinterpret_cast<uint32_t*>(vd + h * HALF) = new_v[h];
+          } else {
+            *reinterpret_cast<unsigned short*>(kd + h * HALF) = static_cast<unsigned short>(new_k[h]);
+            *reinterpret_cast<unsigned short*>(vd + h * HALF) = static_cast<unsigned short>(new_v[h]);
+          }
+        }
+      }
+    }
+  }
   for (int j = 0; j < n_mine; ++j) {
     const int stage = j % L::kStages;
     if (j + L::kStages - 1 < n_mine) load_slice(j + L::kStages - 1, (j + L::kStages - 1) % L::kStages);
@@ -642,6 +756,25 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
     __syncwarp();
     const int key0 = slice_at(first + NW * j) * 16;
     const uint32_t kbase = ring_u + stage * 2 * L::kSliceBytes, vbase = kbase + L::kSliceBytes;
+    if constexpr (ROPE) {
+      if (has_new && j == n_mine - 1) {
+        constexpr int PER = D / 64;
+        const int row = (ctx - 1) & 15;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int d = h * (D / 2) + lane * PER;
+          uint8_t* at = ring + stage * 2 * L::kSliceBytes + swz<D>(row, d >> 3) + (d & 7) * 2;
+          if constexpr (PER == 2) {
+            *reinterpret_cast<uint32_t*>(at) = new_k[h];
+            *reinterpret_cast<uint32_t*>(at + L::kSliceBytes) = new_v[h];
+          } else {
+            *reinterpret_cast<unsigned short*>(at) = static_cast<unsigned short>(new_k[h]);
+            *reinterpret_cast<unsigned short*>(at + L::kSliceBytes) = static_cast<unsigned short>(new_v[h]);
+          }
+        }
+        __syncwarp();
+      }
+    }
     // S (16 heads x 16 keys) = Q K^T
     float sc[2][4], sd[2][4];  // (two chains of products: one of D / 16 dependent MMAs is what a warp would wait for)
 #pragma unroll
@@ -854,16 +987,16 @@ __global__ void __launch_bounds__(NW * 32, (D <= 128 && NW == 4 ? 2 : 1)) decode
   }
 }
 
-template <int D, int EXT, bool PLAN = false>
+template <int D, int EXT, bool PLAN = false, bool ROPE = false>
 static int launch_decode_mma_t(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride,
                                const int* ctx, void* out, float* po, float* pml, int* arrivals, int B, int H, int KV, int page,
-                               float scale, float cap, int window, int splits, const int* used, cudaStream_t st, int dk = D, int dv = D, AttnExtra x = {}) {
+                               float scale, float cap, int window, int splits, const int* used, cudaStream_t st, int dk = D, int dv = D, AttnExtra x = {}, const DecodeRope<ROPE>& rope = {}) {
   constexpr int NW = D > 128 ? 6 : 4;
   using L = DecodeMma<D, NW>;
   using Extra = std::conditional_t<EXT != 0, AttnExtra, NoExtra>;
   if constexpr (!PLAN) {
     if (used != nullptr && splits > 1)
-      return launch_decode_mma_t<D, EXT, true>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, nullptr, B, H, KV, page, scale, cap, window, splits, used, st, dk, dv, x);
+      return launch_decode_mma_t<D, EXT, true, ROPE>(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, nullptr, B, H, KV, page, scale, cap, window, splits, used, st, dk, dv, x, rope);
   }
   // the in-kernel merge keeps its weights in the warp-merge area of shared memory
   if (splits > 1 && (H / KV) * (splits + 1) > L::kMerge / 4) arrivals = nullptr;
@@ -872,17 +1005,17 @@ static int launch_decode_mma_t(const void* q, long long q_stride, const void* kc
   const int min_slices = static_cast<long long>(B) * KV * ((H / KV + 15) / 16) >= 64 ? 16 : 3;
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
-    cudaFuncSetAttribute(decode_attn_mma_kernel<D, EXT, NW, PLAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+    cudaFuncSetAttribute(decode_attn_mma_kernel<D, EXT, NW, PLAN, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
   }
   dim3 grid(B, KV * ((H / KV + 15) / 16), splits);
   DecodeOptions<EXT> opt;
   if constexpr (EXT != 0) opt = {dk, dv, x};
   DecodePlan<PLAN> plan;
   if constexpr (PLAN) plan.used = used;
-  launch_pdl(decode_attn_mma_kernel<D, EXT, NW, PLAN>, dim3(grid), dim3(NW * 32), L::kBytes, st, static_cast<const __nv_bfloat16*>(q), q_stride,
+  launch_pdl(decode_attn_mma_kernel<D, EXT, NW, PLAN, ROPE>, dim3(grid), dim3(NW * 32), L::kBytes, st, static_cast<const __nv_bfloat16*>(q), q_stride,
                                                           static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(vc), bt,
                                                           bt_stride, ctx, static_cast<__nv_bfloat16*>(out), po, pml, arrivals, H, KV, page, scale,
-                                                          cap, window, splits, min_slices, opt, plan);
+                                                          cap, window, splits, min_slices, opt, plan, rope);
   if (splits > 1 && arrivals == nullptr) {
     dim3 g2(B, H);
     const dim3 block((dv + 31) / 32 * 32);
@@ -921,6 +1054,17 @@ int launch_decode_attention_impl(const void* q, long long q_stride, const void* 
     }
   }
   return launch_decode_attention(q, q_stride, kc, vc, bt, bt_stride, ctx, out, po, pml, B, H, KV, D, page, scale, cap, window, splits, st);
+}
+
+int launch_decode_attention_rope(const void* qkv, long long pitch, const DecodeRopeArgs* a, const int* bt, int bt_stride, const int* ctx, void* out, float* po,
+                                 float* pml, int B, int H, int KV, int D, int page, float scale, float cap, int window, int splits, const int* used, cudaStream_t st) {
+  if (B == 0) return 0;
+  if (H / KV > 16 || page % 16 != 0 || pitch % 2 != 0) return 1;
+  DecodeRope<true> rope;
+  static_cast<DecodeRopeArgs&>(rope) = *a;
+  if (D != 64) return 1;
+  return launch_decode_mma_t<64, 0, false, true>(qkv, pitch, a->k_cache, a->v_cache, bt, bt_stride, ctx, out, po, pml, nullptr, B, H, KV, page, scale, cap, window, splits,
+                                                 used, st, 64, 64, {}, rope);
 }
 
 int launch_decode_attention_mma(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride, const int* ctx, void* out,

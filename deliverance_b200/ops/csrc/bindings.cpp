@@ -928,6 +928,69 @@ Tensor decode_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_
   return out;
 }
 
+// rope_kv and decode_attention in one: qkv is the projection's output, which stays as it is. Heads of 64.
+Tensor decode_attention_rope(const Tensor& qkv, const Tensor& positions, const Tensor& slots, c10::optional<Tensor> q_norm_w, c10::optional<Tensor> k_norm_w,
+                             c10::optional<Tensor> cos_t, c10::optional<Tensor> sin_t, Tensor& k_cache, Tensor& v_cache, const Tensor& block_tables, const Tensor& ctx_lens,
+                             int64_t H, double scale, double softcap, int64_t window, int64_t splits, double eps, double norm_offset, c10::optional<Tensor> used_opt) {
+  check_bf16(qkv, "qkv");
+  check_bf16(k_cache, "k_cache");
+  check_bf16(v_cache, "v_cache");
+  for (const Tensor* t : {&positions, &block_tables, &ctx_lens}) {
+    check_cuda(*t, "index tensor");
+    TORCH_CHECK(t->scalar_type() == at::kInt, "positions, block tables and context lengths must be int32");
+  }
+  check_cuda(slots, "slots");
+  const int B = static_cast<int>(qkv.size(0)), KV = static_cast<int>(k_cache.size(1)), page = static_cast<int>(k_cache.size(2)), D = static_cast<int>(k_cache.size(3));
+  TORCH_CHECK(k_cache.dim() == 4 && v_cache.sizes() == k_cache.sizes() && page % 32 == 0 && H % KV == 0, "bad cache shape");
+  TORCH_CHECK(qkv.dim() == 2 && qkv.size(1) == (H + 2 * KV) * D && positions.numel() == B && slots.scalar_type() == at::kLong && slots.numel() == B, "bad qkv shape");
+  TORCH_CHECK(block_tables.dim() == 2 && block_tables.size(0) >= B && ctx_lens.numel() >= B, "bad table shapes");
+  dlv::DecodeRopeArgs a = {};
+  a.positions = positions.data_ptr<int>();
+  a.slots = reinterpret_cast<const long long*>(slots.data_ptr<int64_t>());
+  if (q_norm_w.has_value()) {
+    check_bf16(q_norm_w.value(), "q_norm");
+    check_bf16(k_norm_w.value(), "k_norm");
+    TORCH_CHECK(q_norm_w.value().numel() == D && k_norm_w.value().numel() == D && (reinterpret_cast<uintptr_t>(q_norm_w.value().data_ptr()) & 3) == 0, "bad q/k norm weights");
+    a.q_norm_w = q_norm_w.value().data_ptr();
+    a.k_norm_w = k_norm_w.value().data_ptr();
+  }
+  if (cos_t.has_value()) {
+    for (const Tensor* t : {&cos_t.value(), &sin_t.value()}) {
+      check_cuda(*t, "cos / sin");
+      TORCH_CHECK(t->scalar_type() == at::kFloat && t->dim() == 2 && t->is_contiguous() && t->size(1) * 2 == D && t->size(0) == cos_t.value().size(0) &&
+                  (reinterpret_cast<uintptr_t>(t->data_ptr()) & 7) == 0, "cos / sin must be contiguous fp32 [max_pos, D / 2]");
+    }
+    a.cos_t = cos_t.value().data_ptr<float>();
+    a.sin_t = sin_t.value().data_ptr<float>();
+    a.max_pos = static_cast<int>(cos_t.value().size(0));
+  }
+  a.k_cache = k_cache.data_ptr();
+  a.v_cache = v_cache.data_ptr();
+  a.eps = static_cast<float>(eps);
+  a.norm_offset = static_cast<float>(norm_offset);
+  c10::cuda::CUDAGuard guard(qkv.device());
+  Tensor out = new_out({B, H * D}, qkv.options());
+  if (splits < 1) splits = 1;
+  const int* used = nullptr;
+  if (used_opt.has_value()) {
+    const Tensor& u = used_opt.value();
+    TORCH_CHECK(u.is_cuda() && u.scalar_type() == at::kInt && u.is_contiguous() && u.numel() == static_cast<int64_t>(B) * dlv::kDecodePlanStride && u.device() == qkv.device(), "used splits must come from decode_plan");
+    used = u.data_ptr<int>();
+  }
+  Tensor po, pml;
+  if (splits > 1) {
+    po = new_out({B, H, splits, D}, qkv.options().dtype(at::kFloat));
+    pml = new_out({B, H, splits, 2}, qkv.options().dtype(at::kFloat));
+  }
+  const int rc = dlv::launch_decode_attention_rope(qkv.data_ptr(), qkv.stride(0), &a, block_tables.data_ptr<int>(), static_cast<int>(block_tables.stride(0)),
+                                                   ctx_lens.data_ptr<int>(), out.data_ptr(), splits > 1 ? po.data_ptr<float>() : nullptr,
+                                                   splits > 1 ? pml.data_ptr<float>() : nullptr, B, static_cast<int>(H), KV, D, page, static_cast<float>(scale),
+                                                   static_cast<float>(softcap), static_cast<int>(window), static_cast<int>(splits), used, cur_stream());
+  TORCH_CHECK(rc == 0, "decode attention with rotary embedding: heads of 64, groups of up to 16 heads");
+  check_last_error("decode_attention_rope");
+  return out;
+}
+
 // How many of `splits` every sequence of a decode step takes (first column of int32 [B, 32]) for decode_attention's `used`. Head width: the wider of keys and values.
 Tensor decode_plan(const Tensor& ctx_lens, int64_t B, int64_t H, int64_t KV, int64_t D, int64_t splits, int64_t window, int64_t keep_first,
                    c10::optional<Tensor> out) {
@@ -1695,6 +1758,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("activation", &activation);
   m.def("embedding", &embedding, py::arg("table"), py::arg("ids"), py::arg("scale") = 1.0, py::arg("pos_table") = py::none(),
         py::arg("pos") = py::none(), py::arg("type_table") = py::none(), py::arg("types") = py::none());
+  m.def("decode_attention_rope", &decode_attention_rope);
   m.def("rope_kv", &rope_kv);
   m.def("decode_attention", &decode_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_tables"), py::arg("ctx_lens"),
         py::arg("H"), py::arg("scale"), py::arg("softcap") = 0.0, py::arg("window") = 0, py::arg("splits") = 1, py::arg("impl") = 0,

@@ -168,6 +168,19 @@ struct AttnExtra {
 int launch_decode_attention(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride,
                             const int* ctx, void* out, float* po, float* pml, int B, int H, int KV, int D, int page, float scale,
                             float cap, int window, int splits, cudaStream_t st);
+// Decode attention that takes the projection's rows as they are (q | k | v heads): per-head q / k RMSNorm, rotation over the whole head and the new row's way into the
+// cache happen in it. cos_t: [max_pos, D / 2] fp32 or null; norm weights may be null; slots < 0: the row is not kept.
+struct DecodeRopeArgs {
+  const int* positions;
+  const long long* slots;
+  const void *q_norm_w, *k_norm_w;
+  const float *cos_t, *sin_t;
+  void *k_cache, *v_cache;
+  float eps, norm_offset;
+  int max_pos;
+};
+int launch_decode_attention_rope(const void* qkv, long long pitch, const DecodeRopeArgs* a, const int* bt, int bt_stride, const int* ctx, void* out, float* po,
+                                 float* pml, int B, int H, int KV, int D, int page, float scale, float cap, int window, int splits, const int* used, cudaStream_t st);
 int launch_decode_attention_impl(const void* q, long long q_stride, const void* kc, const void* vc, const int* bt, int bt_stride,
                                  const int* ctx, void* out, float* po, float* pml, int* arrivals, int B, int H, int KV, int D, int page,
                                  float scale, float cap, int window, int splits, const int* used, int impl, cudaStream_t st);

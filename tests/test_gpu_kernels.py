@@ -1301,3 +1301,33 @@ def test_moe_combine_slots(T, k, H):
         own = ((pos >= lo) & (pos < hi)).double() if rng else torch.ones(T, k).double()
         r = (ys.double()[pos] * (w.double() * own).unsqueeze(-1)).sum(1)
         assert (out.cpu().double() - r).abs().max() <= 2.0**-8 * max(1e-6, r.abs().max().item())
+
+
+@pytest.mark.parametrize("D,H,KV", [(64, 32, 8), (64, 16, 1), (64, 32, 4), (64, 12, 12), (64, 9, 1)])
+@pytest.mark.parametrize("norm,rope,window,cap,splits", [(True, True, 0, 0.0, 1), (False, True, 0, 0.0, 8), (True, False, 40, 0.0, 3), (False, True, 33, 20.0, 32), (True, True, 0, 0.0, 64)])
+def test_decode_attention_rope(D, H, KV, norm, rope, window, cap, splits):
+    """Norm, rotation and cache write inside decode attention against the two kernels: one key, the edges of a slice and of a page, contexts cut into several parts (by
+    themselves and by a plan), a row that is not kept, positions past the table. The caches bit for bit; the output within one rounding (2^-9: the rotation's
+    products may be contracted otherwise)."""
+    ctx = [1, 15, 16, 17, 32, 33, 200, 777, 1500]
+    B, per = len(ctx), 48
+    pages = B * per
+    bt = torch.randperm(pages).reshape(B, per).int().to(DEV)
+    pos = torch.tensor([c - 1 for c in ctx], dtype=torch.int32)
+    slots = torch.tensor([int(bt[i, (c - 1) // 32]) * 32 + (c - 1) % 32 for i, c in enumerate(ctx)])
+    slots[4] = -1
+    pos[5] = 5000
+    qkv = torch.randn(B, (H + 2 * KV) * D).to(torch.bfloat16).to(DEV)
+    kc, vc = (torch.randn(pages, KV, 32, D).to(torch.bfloat16).to(DEV) for _ in range(2))
+    qn, kn = ((1 + 0.1 * torch.randn(D)).to(torch.bfloat16).to(DEV) for _ in range(2)) if norm else (None, None)
+    cos, sin = (t.to(DEV) for t in ref.rope_tables(D, 4096, 10000.0)) if rope else (None, None)
+    cl, pos, slots = torch.tensor(ctx, dtype=torch.int32, device=DEV), pos.to(DEV), slots.to(DEV)
+    kc2, vc2, raw = kc.clone(), vc.clone(), qkv.clone()
+    for even in (True, False):
+        q = ops.rope_kv(qkv.clone(), pos, slots, qn, kn, cos, sin, kc2, vc2, H, KV, D, 1e-6, 0.5)
+        want = ops.decode_attention(q, kc2, vc2, bt, cl, H, 0.1, cap, window, splits, even=even)
+        got = ops.decode_attention_rope(qkv, pos, slots, qn, kn, cos, sin, kc, vc, bt, cl, H, 0.1, cap, window, splits, 1e-6, 0.5, even=even)
+        torch.cuda.synchronize()
+        keep = [i for i in range(B) if i != 4]  # (what is not kept there is not seen either)
+        assert torch.equal(qkv, raw) and torch.equal(kc, kc2) and torch.equal(vc, vc2)
+        assert _rel(got[keep], want[keep]) < 2e-3 and bool(torch.isfinite(got).all())
