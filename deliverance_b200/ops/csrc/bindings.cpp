@@ -253,7 +253,7 @@ class GemmWeight {
     return true;
   }
 
-  // Whether the JQ4 pair kernel takes a product of M rows, and its room for partial sums (as above). impl 4 asks for it, 0 where it is the faster one.
+  // Whether the pair kernel with tiles cut over k (gemm_parts.cu) takes a product of M rows, and its room for partial sums (as above). impl 4 asks for it, 0 where it is the faster one.
   bool parts(int64_t impl, int M, const void* out, int64_t ldo, int epi, Tensor& room) const {
     if ((impl != 4 && (impl != 0 || !dlv::gemm_parts_preferred(&desc_, M, epi))) || !dlv::gemm_parts_supported(&desc_, desc_.N, out, static_cast<int>(ldo), epi)) return false;
     const size_t floats = dlv::gemm_parts_room(&desc_, M, epi);
@@ -267,8 +267,8 @@ class GemmWeight {
   }
   static float* floats(const Tensor& room) { return room.defined() ? room.data_ptr<float>() : nullptr; }
 
-  // out[m, :] = x[m, :] @ W^T (+ bias). impl: 0 = auto, 1 = tcgen05, 2 = CUDA-core GEMV, 3 = tcgen05 on pairs of SMs, 4 = the same with JQ4 weights
-  // expanded inside the kernel and tiles cut over k
+  // out[m, :] = x[m, :] @ W^T (+ bias). impl: 0 = auto, 1 = tcgen05, 2 = CUDA-core GEMV, 3 = tcgen05 on pairs of SMs, 4 = pairs with tiles
+  // cut over k, JQ4 weights expanded inside the kernel
   Tensor run(const Tensor& x, c10::optional<Tensor> out_opt, c10::optional<Tensor> bias, bool out_f32, int64_t impl,
              int64_t force_splits) {
     TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2, "x must be bf16 [M, K] on CUDA");
@@ -299,7 +299,7 @@ class GemmWeight {
       check_last_error("JQ4 pair gemm launch");
       return out;
     }
-    TORCH_CHECK(impl != 4, "shape outside the JQ4 pair kernel, or no memory for its partial sums");
+    TORCH_CHECK(impl != 4, "shape outside the pair kernel with cut tiles, or no memory for its partial sums");
     const bool pair = impl == 3 || (impl == 0 && force_splits == 0 && dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0));
     if (pair && !out_f32 && dlv::gemm_pair_supported(&desc_, desc_.N, out.data_ptr(), static_cast<int>(out.stride(0)), false, 0) && expanded(room)) {
       dlv::gemm_pair_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), bptr,
@@ -525,7 +525,7 @@ class GemmWeight {
       check_last_error("JQ4 pair gemm (fused q/k/v epilogue) launch");
       return q;
     }
-    TORCH_CHECK(impl != 4, "shape outside the JQ4 pair kernel, or no memory for its partial sums");
+    TORCH_CHECK(impl != 4, "shape outside the pair kernel with cut tiles, or no memory for its partial sums");
     if ((impl == 3 || dlv::gemm_pair_preferred(&desc_, M, desc_.N, 0)) && dlv::gemm_pair_qkv_supported(&desc_, q.data_ptr(), static_cast<int>(q.stride(0)), &a) &&
         expanded(room)) {
       dlv::gemm_pair_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a,

@@ -1,5 +1,5 @@
-// JQ4 GEMM  out[m, n] = sum_k X[m, k] * W[n, k]  for some dozens to some hundreds of rows, and for experts, on pairs of SMs (tcgen05
-// cta_group::2), weights as the M operand out of tensor memory.
+// GEMM  out[m, n] = sum_k X[m, k] * W[n, k]  for some dozens to some hundreds of rows, and for JQ4 experts, on pairs of SMs (tcgen05 cta_group::2),
+// weights as the M operand: JQ4 out of tensor memory, bf16 out of shared memory.
 //
 // What bounds it: the tensor pipe for tiles of 256 tokens and more, the expansion of the weights (about 900 cycles per 128-k stage) for narrower
 // ones. With 128 weight rows per CTA (gemm_tc.cuh) the activations alone ask for 64 bytes per cycle and SM, all that L2 gives, and expanding into
@@ -9,12 +9,14 @@
 // expanded once for all of them; its accumulators and two to four stages of weights fill tensor memory. Expanding is half of what the SM
 // issues, so nothing else may be expensive: one commit per 128 k (each costs its thread more than a hundred cycles), and the expanding warps
 // drain the accumulators themselves.
+// bf16 weights come as TMA boxes in stages of 64 k beside their tokens (bound by HBM up to some 200 tokens, then by L2 and the pipe); sixteen warps only drain, and
+// where a tile's accumulators fit twice the next tile runs meanwhile. Gate and up rows are fetched in turn by a five-dimensional box. Measured at gemm_parts_preferred.
 //
 // The tiles go to the pairs in whole waves. What is left over, or all of them where tiles are few, is cut over k into equal parts, whose fp32 sums a
 // second small kernel adds up in order of k and finishes (plan_parts weighs it): 19456 x 2560 are 76 tiles on 74 pairs, 20 stages for everyone
 // and 2 stages for twenty of them, not two waves of 20. No CTA waits for another pair.
 //
-// Roles per CTA: warps 0 and 2 copy tokens (of the first and the second instruction), warps 3 and 20 packed stages, warp 1 of the even CTA issues all
+// Roles per CTA: warps 0 and 2 copy tokens (of the first and the second instruction), warps 3 and 20 packed stages (bf16: warp 3 weights), warp 1 of the even CTA issues all
 // MMAs of the pair, warp 2 owns tensor memory, warps 4-19 expand (two groups of four per 128-k stage, one per half, alternating) and drain.
 // Barriers: x_full, a_full (even CTA) count both CTAs' copies and expanding warps; done (per stage: tokens and expanded weights may be overwritten)
 // and acc_full are multicast commits; acc_empty (even CTA) counts both CTAs' draining warps. All waits are bounded as everywhere.
@@ -760,7 +762,8 @@ struct PartPlan {
   int bn = 0, m_tiles = 0, n_tiles = 0, pairs = 0, waves = 0, parts = 0;
   double cost = 1e30;
 };
-// Token tiles, whole waves and parts; in thousands of cycles. A 128-k stage takes 8 instructions of cols / 2 cycles and no less than its expansion, a piece its
+// Token tiles, whole waves and parts; in thousands of cycles. A 128-k stage takes 8 instructions of cols / 2 cycles and no less than its expansion (bf16: a 64-k stage 4,
+// and no less than HBM needs for 32 KB per pair; with these constants the estimate is within a tenth of what 130 products of 64 to 2048 rows took), a piece its
 // drain and the first stage that the pipe waits for (an SM stores some 30 bytes per cycle); cut tiles cost the second kernel (four parts at a time) and their sums' way back from L2.
 PartPlan plan_parts(const GemmWeightDesc* w, int M, int epi) {
   PartPlan best;
@@ -805,7 +808,7 @@ void launch_parts(const GemmWeightDesc* w, const void* x, int rows, int ldx, Par
   p.by_parts.set(p.parts);
   p.by_group.set(8 * p.n_tiles);
   p.x_stages = Q4 ? std::min(kMaxX, kXRoom / (p.box * 256 * (p.bn > kOneMma ? 2 : 1))) : std::min(kMaxX, kStageRoom / (kWStage + p.box * 128 * (p.bn > kOneMma ? 2 : 1)));
-  if (part_pairs<Q4, EPI>() < p.pairs || p.pairs < 1) throw std::runtime_error("JQ4 pair gemm: no pair of SMs can hold the kernel");
+  if (part_pairs<Q4, EPI>() < p.pairs || p.pairs < 1) throw std::runtime_error("pair gemm (parts): no pair of SMs can hold the kernel");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * p.pairs);
   cfg.blockDim = dim3(kThreads);
@@ -814,7 +817,7 @@ void launch_parts(const GemmWeightDesc* w, const void* x, int rows, int ldx, Par
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_parts_kernel<Q4, EPI>, map_x, map_w, p);
   const int tiles = p.n_tiles * p.m_tiles, second = EPI == 2 ? tiles : (p.parts > 1 ? tiles - p.waves * p.pairs : 0);
   if (e == cudaSuccess && p.items == nullptr && second > 0) e = launch_pdl(gemm_parts_sum_kernel<EPI>, dim3(2 * second, (p.bn + 7) / 8), dim3(128), 0, st, p);
-  if (e != cudaSuccess) throw std::runtime_error(std::string("JQ4 pair gemm launch: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) throw std::runtime_error(std::string("pair gemm (parts) launch: ") + cudaGetErrorString(e));
 }
 
 PartParams dense_params(const GemmWeightDesc* w, int M, int epi, float* sums, int* status) {
