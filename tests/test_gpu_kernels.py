@@ -1266,7 +1266,7 @@ def test_parts_gemm_experts(E, n, K, T, k):
         assert sum(rows) == off[i + 1] - off[i] and max(rows) <= 384 and max(rows) - min(rows) < len(rows)
 
 
-@pytest.mark.parametrize("T,E,k", [(1, 3, 3), (33, 8, 2), (70, 128, 8), (128, 129, 16), (50, 256, 8), (40, 257, 9), (20, 1000, 16), (700, 128, 8), (3000, 40, 6), (130, 1024, 16)])
+@pytest.mark.parametrize("T,E,k", [(1, 3, 3), (33, 8, 2), (70, 128, 8), (128, 129, 16), (50, 256, 8), (40, 257, 9), (20, 1000, 16), (700, 128, 8), (3000, 40, 6), (130, 1024, 16), (129, 8, 2), (442, 8, 2)])
 def test_moe_route_choices(T, E, k):
     """Experts and groups of the routing kernels against a sort: equal logits (the lower expert first), both zeros equal, minus infinity chosen last; one launch and
     several, 32 experts per register and their remainders, the pairs grouped chunk by chunk and by one block."""
