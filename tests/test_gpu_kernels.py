@@ -1192,8 +1192,9 @@ def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
         got.append((q, kc, vc))
     torch.cuda.synchronize()
     ops.check_status()
-    for u, v in zip(*got):  # (sums in another order, rounded to bf16 up to twice: 2^-9 each)
-        assert _rel(u, v) < 4e-3 and torch.equal(u == 0, v == 0)
+    # (sums in another order, rounded to bf16 up to twice: 2^-9 each; rows that are not kept stay zeros, whole: a single sum may cancel in one order and not in the other)
+    for u, v in zip(*got):
+        assert _rel(u, v) < 4e-3 and torch.equal((u == 0).all(-1), (v == 0).all(-1))
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 256, 64), (70, 272, 192), (200, 136, 64), (257, 1040, 2624), (385, 528, 192), (800, 11264, 192), (2600, 3072, 320), (900, 19200, 128)])
@@ -1239,8 +1240,9 @@ def test_parts_gemm_bf16_heads(M):
         got.append((q, kc, vc))
     torch.cuda.synchronize()
     ops.check_status()
-    for u, v in zip(*got):  # (sums in another order, rounded to bf16 up to twice: 2^-9 each)
-        assert _rel(u, v) < 4e-3 and torch.equal(u == 0, v == 0)
+    # (sums in another order, rounded to bf16 up to twice: 2^-9 each; rows that are not kept stay zeros, whole: a single sum may cancel in one order and not in the other)
+    for u, v in zip(*got):
+        assert _rel(u, v) < 4e-3 and torch.equal((u == 0).all(-1), (v == 0).all(-1))
 
 
 @pytest.mark.parametrize("E,n,K,T,k", [(4, 512, 256, 900, 2), (3, 384, 1216, 1500, 1), (40, 1280, 128, 9000, 2)])
