@@ -18,6 +18,12 @@ def _rel(a, b):
     return ((a.float() - b.float()).norm() / (b.float().norm() + 1e-12)).item()
 
 
+def _rounded_once(y, want, slack):
+    """Whether every bf16 value of ``y`` is ``want`` rounded once: 2^-8 of the value at most (half a step at the low end of its power of two), and on top of it the error
+    ``slack`` of what stands in front of the rounding."""
+    return bool(((y.double() - want).abs() <= (want.abs() + slack) * 2.0**-8 + slack).all())
+
+
 def _q4_weight(N, K, seed=0):
     g = torch.Generator().manual_seed(seed)
     w = torch.randn(N, K, generator=g) * 0.05
@@ -704,7 +710,7 @@ def test_persistent_prefill_gemm(N, K, M):
     assert _rel(y.cpu().float(), y0.cpu().float()) < 1e-2
 
 
-# The pair kernel rounds its fp32 sums to bf16 once: 2^-9 per value at most, about 1.7e-3 in the 2-norm; JQ4 weights are products rounded to
+# The pair kernel rounds its fp32 sums to bf16 once: 2^-8 of a value at most, about 1.7e-3 in the 2-norm; JQ4 weights are products rounded to
 # bf16 twice on top (scale, then nibble times scale): another 1.4e-3. 4e-3 holds both.
 @pytest.mark.parametrize("M,N,K", [(1, 256, 64), (255, 264, 64), (257, 520, 192), (300, 512, 2592), (1030, 1096, 416), (2049, 512, 1280)])
 @pytest.mark.parametrize("q4", [True, False])
@@ -964,7 +970,7 @@ def test_pair_gemm_limits(q4):
         ops.set_gemm_pairs(-1)
     for u, v in zip(got[3], got[-1]):
         assert torch.equal(u, v)
-    for u, v in zip(got[0], got[-1]):  # (sums in another order, rounded to bf16 once or twice: 2^-9 each)
+    for u, v in zip(got[0], got[-1]):  # (sums in another order, rounded to bf16 once or twice: about 1.7e-3 each in the 2-norm)
         assert _rel(u, v) < 6e-3
 
 
@@ -972,7 +978,7 @@ def test_pair_gemm_limits(q4):
 @pytest.mark.parametrize("window,cap", [(0, 0.0), (100, 30.0)])
 def test_decode_attention_used_splits(B, H, KV, D, window, cap):
     """Contexts around the lengths at which one more split is used (3 and 16 slices of 16 keys), for few and many (sequence, KV head) pairs; a batch
-    mixes sequences that write their output alone with ones that are merged. bf16 probabilities and output: 2^-9 each."""
+    mixes sequences that write their output alone with ones that are merged. bf16 probabilities and output: about 1.7e-3 each in the 2-norm."""
     lens = [1, 15, 16, 17, 47, 48, 49, 95, 97, 255, 257, 511, 513, 700, 1500]
     ctx = torch.tensor([lens[(7 * i) % len(lens)] for i in range(B)], dtype=torch.int32)
     per = [(int(c) + 31) // 32 for c in ctx]
@@ -1006,7 +1012,7 @@ def _paged(ctx, KV, D, seed=0):
 @pytest.mark.parametrize("window,cap", [(0, 0.0), (1000, 30.0)])
 def test_decode_attention_one_long_sequence(B, H, KV, D, short, long, window, cap):
     """A batch whose pairs occupy the GPU unsplit, or nearly do, with one sequence many times longer than the others, padded sequences of one key among
-    them: the long one is cut, whatever the batch. bf16 probabilities and output: 2^-9 each."""
+    them: the long one is cut, whatever the batch. bf16 probabilities and output: about 1.7e-3 each in the 2-norm."""
     ctx = [short + (37 * i) % 50 for i in range(B)]
     ctx[B // 2] = long
     ctx[B - B // 8 :] = [1] * (B // 8)
@@ -1062,7 +1068,7 @@ def test_decode_attention_softcap_error(lo, hi):
         p = ops.decode_attention(q.to(torch.bfloat16).to(DEV), kc, vc, bt, cl, 1, 1.0, cap, 0, 1, impl)
         d = p.double().cpu().log() - want
         err.append((d - d.mean(1, keepdim=True)).pow(2).mean().sqrt().item())
-    # (bf16 probabilities and outputs: 2^-9 each at most, about 0.0016 together, in either kernel; the kernels round them in another order)
+    # (bf16 probabilities and outputs: about 0.0016 together in the 2-norm, in either kernel; the kernels round them in another order)
     assert err[0] < 1.1 * err[1] + 0.0016, err
 
 
@@ -1078,7 +1084,17 @@ def test_rmsnorm_widths(T, H):
     torch.cuda.synchronize()
     want_res = (res.float() + 0.5 * x.float()).to(torch.bfloat16)
     assert torch.equal(got_res.cpu(), want_res)
-    assert _rel(y.cpu(), ref.rmsnorm(x.double(), w.double(), 1e-6, 1.0)) < 3e-3 and _rel(z.cpu(), ref.rmsnorm(want_res.double(), w.double(), 1e-6)) < 3e-3
+    # in front of the rounding, in fp32: at most H / 32 squares added up by a thread and ten sums across threads (the root halves their error), then a division, a
+    # reciprocal root, the weight's offset and two products
+    slack = (H / 64 + 16) * 2.0**-24
+    for got, want in ((y.cpu(), ref.rmsnorm(x.double(), w.double(), 1e-6, 1.0)), (z.cpu(), ref.rmsnorm(want_res.double(), w.double(), 1e-6))):
+        assert _rounded_once(got, want, slack * want.abs())
+
+
+def _row_slack(x, w, bias):
+    """Error of the one-row GEMV's fp32 sums: products of bf16 are exact; a lane adds two in a row per 256 elements, two sums of its own follow, five across the warp and the
+    bias. Relative to the sum of magnitudes, because a sum may cancel."""
+    return (2 * -(-w.shape[1] // 256) + 9) * 2.0**-24 * (x.double().abs() @ w.double().abs().t() + bias.double().abs())
 
 
 @pytest.mark.parametrize("N,K", [(5, 8), (130, 2040), (64, 2048), (33, 2056), (3, 5632)])
@@ -1086,23 +1102,23 @@ def test_rmsnorm_widths(T, H):
 def test_gemv_bf16_row(N, K, f32):
     w, x = (torch.randn(N, K) * 0.05).to(torch.bfloat16), torch.randn(1, K).to(torch.bfloat16)
     bias = torch.randn(N)
-    y = ops.linear(x.to(DEV), LinearWeight(w, bias).to(DEV, torch.bfloat16), out_f32=f32)
-    torch.cuda.synchronize()
-    assert _rel(y.cpu(), x.double() @ w.double().t() + bias.double()) < (1e-5 if f32 else 4e-3)
+    y = ops.linear(x.to(DEV), LinearWeight(w, bias).to(DEV, torch.bfloat16), out_f32=f32).cpu()
+    want, slack = x.double() @ w.double().t() + bias.double(), _row_slack(x, w, bias)
+    assert bool(((y.double() - want).abs() <= slack).all()) if f32 else _rounded_once(y, want, slack)
 
 
 # As for the pair kernel: fp32 sums rounded to bf16 once, JQ4 products rounded to bf16 twice on top.
 @pytest.mark.parametrize("N,K", [(1, 8), (7, 1024), (2500, 1032), (5000, 256), (9, 2056), (2400, 2560), (300, 3080), (33, 14336), (57001, 64), (60000, 1544)])
 def test_gemv_bf16_pieces(N, K):
     """Rows of one and several pieces, three to six of them in a warp's ring, fewer rows than warps, several rows per warp, more rows than resident CTAs take, and rows
-    wider than a ring. fp32 sums, rounded once for bf16 outputs (2^-9)."""
+    wider than a ring. fp32 sums, which bf16 outputs round once."""
     w = LinearWeight((torch.randn(N, K) * 0.05).to(torch.bfloat16)).to(DEV, torch.bfloat16)
     w.bias = torch.randn(N, device=DEV)
     x = torch.randn(1, K).to(torch.bfloat16).to(DEV)
     y, y32, again = ops.linear(x, w), ops.linear(x, w, out_f32=True), ops.linear(x, w)
     f = x.double() @ w.w.double().t() + w.bias.double()
     torch.cuda.synchronize()
-    assert _rel(y32, f) < 1e-5 and torch.equal(y, y32.to(torch.bfloat16)) and torch.equal(y, again)
+    assert bool(((y32.double() - f).abs() <= _row_slack(x, w.w, w.bias)).all()) and torch.equal(y, y32.to(torch.bfloat16)) and torch.equal(y, again)
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (31, 264, 128), (33, 136, 192), (256, 512, 1280), (257, 2560, 960), (385, 19456, 256), (700, 1000, 2624), (1537, 4104, 512)])
@@ -1192,7 +1208,7 @@ def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
         got.append((q, kc, vc))
     torch.cuda.synchronize()
     ops.check_status()
-    # (sums in another order, rounded to bf16 up to twice: 2^-9 each; rows that are not kept stay zeros, whole: a single sum may cancel in one order and not in the other)
+    # (sums in another order, rounded to bf16 up to twice: about 1.7e-3 each in the 2-norm; rows that are not kept stay zeros, whole: a single sum may cancel in one order and not in the other)
     for u, v in zip(*got):
         assert _rel(u, v) < 4e-3 and torch.equal((u == 0).all(-1), (v == 0).all(-1))
 
@@ -1200,7 +1216,8 @@ def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
 @pytest.mark.parametrize("M,N,K", [(1, 256, 64), (70, 272, 192), (200, 136, 64), (257, 1040, 2624), (385, 528, 192), (800, 11264, 192), (2600, 3072, 320), (900, 19200, 128)])
 def test_parts_gemm_bf16(M, N, K):
     """bf16 weights: 64-k stages of their own, one and two accumulators, halves of an odd number of eights (gated), rows that end inside a half tile, several waves with
-    two accumulators in turn, rows without 16 bytes at once, fp32 outputs; guard areas around output and sums. fp32 sums, rounded once: 2^-9, gated products once more."""
+    two accumulators in turn, rows without 16 bytes at once, fp32 outputs; guard areas around output and sums. fp32 sums, rounded once (gated
+    products behind the activation): 2^-8 of a value at most, so no more in the 2-norm."""
     wd = (torch.randn(N, K) * 0.05).to(torch.bfloat16)
     lw = LinearWeight(wd).to(DEV, torch.bfloat16)
     x = (torch.randn(M, K + 8) * 0.5).to(torch.bfloat16).to(DEV)[:, :K]
@@ -1216,9 +1233,9 @@ def test_parts_gemm_bf16(M, N, K):
     finally:
         ops.set_bounds_check(False)
     ops.check_status()
-    assert _rel(y.cpu(), f) < 3e-3 and _rel(y32.cpu(), f) < 2e-5 and torch.equal(odd[:, :N], y) and bool((odd[:, N] == 7.0).all())
+    assert _rel(y.cpu(), f) < 4e-3 and _rel(y32.cpu(), f) < 2e-5 and torch.equal(odd[:, :N], y) and bool((odd[:, N] == 7.0).all())
     if N % 16 == 0:
-        assert _rel(h.cpu(), torch.nn.functional.silu(f[:, : N // 2]) * f[:, N // 2 :]) < 3e-3
+        assert _rel(h.cpu(), torch.nn.functional.silu(f[:, : N // 2]) * f[:, N // 2 :]) < 4e-3
     else:
         assert h is None
 
@@ -1240,7 +1257,7 @@ def test_parts_gemm_bf16_heads(M):
         got.append((q, kc, vc))
     torch.cuda.synchronize()
     ops.check_status()
-    # (sums in another order, rounded to bf16 up to twice: 2^-9 each; rows that are not kept stay zeros, whole: a single sum may cancel in one order and not in the other)
+    # (sums in another order, rounded to bf16 up to twice: about 1.7e-3 each in the 2-norm; rows that are not kept stay zeros, whole: a single sum may cancel in one order and not in the other)
     for u, v in zip(*got):
         assert _rel(u, v) < 4e-3 and torch.equal((u == 0).all(-1), (v == 0).all(-1))
 
@@ -1309,8 +1326,8 @@ def test_moe_combine_slots(T, k, H):
 @pytest.mark.parametrize("norm,rope,window,cap,splits", [(True, True, 0, 0.0, 1), (False, True, 0, 0.0, 8), (True, False, 40, 0.0, 3), (False, True, 33, 20.0, 32), (True, True, 0, 0.0, 64)])
 def test_decode_attention_rope(D, H, KV, norm, rope, window, cap, splits):
     """Norm, rotation and cache write inside decode attention against the two kernels: one key, the edges of a slice and of a page, contexts cut into several parts (by
-    themselves and by a plan), a row that is not kept, positions past the table. The caches bit for bit; the output within one rounding (2^-9: the rotation's
-    products may be contracted otherwise)."""
+    themselves and by a plan), a row that is not kept, positions past the table. The caches bit for bit; the output but for the
+    few values whose rounding falls the other way (the rotation's products may be contracted otherwise): less than one rounding of all, 2e-3 in the 2-norm."""
     ctx = [1, 15, 16, 17, 32, 33, 200, 777, 1500]
     B, per = len(ctx), 48
     pages = B * per
