@@ -943,6 +943,7 @@ Tensor decode_attention_rope(const Tensor& qkv, const Tensor& positions, const T
   const int B = static_cast<int>(qkv.size(0)), KV = static_cast<int>(k_cache.size(1)), page = static_cast<int>(k_cache.size(2)), D = static_cast<int>(k_cache.size(3));
   TORCH_CHECK(k_cache.dim() == 4 && v_cache.sizes() == k_cache.sizes() && page % 32 == 0 && H % KV == 0, "bad cache shape");
   TORCH_CHECK(qkv.dim() == 2 && qkv.size(1) == (H + 2 * KV) * D && positions.numel() == B && slots.scalar_type() == at::kLong && slots.numel() == B, "bad qkv shape");
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 3) == 0, "qkv misaligned");  // (rows are an even number of elements apart)
   TORCH_CHECK(block_tables.dim() == 2 && block_tables.size(0) >= B && ctx_lens.numel() >= B, "bad table shapes");
   dlv::DecodeRopeArgs a = {};
   a.positions = positions.data_ptr<int>();

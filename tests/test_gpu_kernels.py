@@ -1350,3 +1350,24 @@ def test_decode_attention_rope(D, H, KV, norm, rope, window, cap, splits):
         keep = [i for i in range(B) if i != 4]  # (what is not kept there is not seen either)
         assert torch.equal(qkv, raw) and torch.equal(kc, kc2) and torch.equal(vc, vc2)
         assert _rel(got[keep], want[keep]) < 2e-3 and bool(torch.isfinite(got).all())
+
+
+def test_decode_attention_rope_alignment():
+    """Rows that start on an odd element are refused; norm weights and tables that start between the kernel's words give what the two kernels give."""
+    B, H, KV, D, ctx = 2, 4, 2, 64, 40
+    qkv = torch.randn(B, (H + 2 * KV) * D).to(torch.bfloat16).to(DEV)
+    kc, vc = (torch.randn(4, KV, 32, D).to(torch.bfloat16).to(DEV) for _ in range(2))
+    bt, cl = torch.arange(4, dtype=torch.int32, device=DEV).view(B, 2), torch.full((B,), ctx, dtype=torch.int32, device=DEV)
+    pos, slots = cl - 1, torch.tensor([39, 103], device=DEV)
+    wide = torch.randn(2 * D + 1, device=DEV).to(torch.bfloat16)
+    tables = [torch.cat([torch.zeros(1), t.flatten()]).to(DEV)[1:].view(t.shape) for t in ref.rope_tables(D, 64, 10000.0)]
+    odd = torch.empty(qkv.numel() + 1, dtype=torch.bfloat16, device=DEV)[1:].view(qkv.shape).copy_(qkv)
+    even = [t.clone() for t in tables]
+    with pytest.raises(RuntimeError, match="misaligned"):
+        ops.decode_attention_rope(odd, pos, slots, None, None, *even, kc, vc, bt, cl, H, 0.1)
+    for qn, kn, cs in ((wide[1 : D + 1], wide[D + 1 :], even), (None, None, tables)):
+        c = [t.clone() for t in (kc, vc, kc, vc)]
+        q = ops.rope_kv(qkv.clone(), pos, slots, qn, kn, *cs, c[0], c[1], H, KV, D, 1e-6)
+        want = ops.decode_attention(q, c[0], c[1], bt, cl, H, 0.1)
+        got = ops.decode_attention_rope(qkv.clone(), pos, slots, qn, kn, *cs, c[2], c[3], bt, cl, H, 0.1)
+        assert torch.equal(got, want) and torch.equal(c[0], c[2]) and torch.equal(c[1], c[3])
