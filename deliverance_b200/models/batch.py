@@ -29,6 +29,22 @@ class ForwardBatch:
     prev_ids: Optional[torch.Tensor] = None  # [T] int32 token before each token of its sequence (-1: none), for models that read it
     plans: dict = field(default_factory=dict)  # per-batch work plans of model mechanisms, built once and shared by the layers
     _tiles: dict = field(default_factory=dict)  # tile height -> (tile_seq, tile_q0) device tensors
+    host_tables: Optional[tuple] = None  # decode: block tables on the host and the page size, what ``rows_apart`` looks at
+
+    def rows_apart(self) -> bool:
+        """Decode: whether no row's keys hold another row's new one, as with one row per sequence. Several entries of one sequence, or a page that is still being
+        filled and shared, need the new keys of all rows in the cache before any row reads them. Without host tables the batch states that itself."""
+        if "rows_apart" not in self.plans:
+            apart = True
+            if self.host_tables is not None and len(self.ctx_len_host) > 1:
+                tables, page = self.host_tables
+                last = (torch.tensor(self.ctx_len_host) - 1) // page
+                written = tables.gather(1, last.view(-1, 1))
+                mine = torch.arange(tables.shape[1]) <= last.view(-1, 1)
+                # (all written pages are different ones, and none is found but in its own row)
+                apart = written.unique().numel() == tables.shape[0] == int((torch.isin(tables, written) & mine).sum())
+            self.plans["rows_apart"] = apart
+        return self.plans["rows_apart"]
 
     def tiles(self, rows: int):
         """Device tile arrays ``(tile_seq, tile_q0)`` for query tiles of ``rows`` rows (built once per height from ``q_len_host``)."""
@@ -140,4 +156,5 @@ def make_batch(seqs: list[dict], page_size: int, device, max_pages: Optional[int
         q_len=t(ql, torch.int32), ctx_len=t(cl, torch.int32), block_tables=bt.to(dev, non_blocking=True), is_decode=is_decode,
         logits_rows=t(last, torch.int64), tile_seq=t(ts, torch.int32) if ts else None, tile_q0=t(t0, torch.int32) if ts else None,
         state_slots=state_slots, q_len_host=ql, ctx_len_host=cl, prev_ids=prev_ids, decode_even=is_decode and even_lengths(cl),
+        host_tables=(bt, page_size) if is_decode else None,
     )

@@ -583,8 +583,9 @@ def rope_in_attention(device: torch.device, H: int, KV: int, D: int) -> bool:
 
 def decode_attention_rope(qkv, positions, slots, q_norm_w, k_norm_w, cos, sin, k_cache, v_cache, block_tables, ctx_lens, H, scale, softcap=0.0, window=0, splits=1,
                           eps=1e-6, norm_offset=0.0, even=False, plan=None):
-    """:func:`rope_kv` and :func:`decode_attention` in one kernel: qkv ``[B, (H + 2 KV) * D]``, one new row per sequence, the last of its ``ctx_lens`` keys. Norm weights
-    and rotary tables that do not start on 4 and 8 bytes take the two kernels (which leave the rotated heads in ``qkv``)."""
+    """:func:`rope_kv` and :func:`decode_attention` in one kernel: qkv ``[B, (H + 2 KV) * D]``, one new row per sequence, the last of its ``ctx_lens`` keys. No row's keys
+    may hold another row's new one (``ForwardBatch.rows_apart``): it is written while others read. Norm weights and rotary
+    tables that do not start on 4 and 8 bytes take the two kernels (which leave the rotated heads in ``qkv``)."""
     D = k_cache.shape[3]
     if any(t is not None and t.data_ptr() % n for t, n in ((q_norm_w, 4), (k_norm_w, 4), (cos, 8), (sin, 8))):
         q = rope_kv(qkv, positions, slots, q_norm_w, k_norm_w, cos, sin, k_cache, v_cache, H, k_cache.shape[1], D, eps, norm_offset)

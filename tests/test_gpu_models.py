@@ -236,6 +236,25 @@ def test_fused_activation_models_gpu(tmp_path, family, monkeypatch):
     assert all(r.generated_tokens == 8 for r in rs)
 
 
+def test_decode_rows_of_one_sequence_gpu(tmp_path):
+    """Heads of 64: a decode batch with three positions of one sequence, and a page's end between them, against one position after the other."""
+    d = str(tmp_path / "m")
+    write_tiny_model(d, "llama", seed=13, std=0.05, quantize=True, max_position_embeddings=1024, hidden_size=256, num_attention_heads=4, num_key_value_heads=2, head_dim=64)
+    m = DecoderModel(load_config(d), "cuda:0").load(WeightLoader(d))
+    toks = torch.randint(3, 250, (98,), generator=torch.Generator().manual_seed(4)).tolist()
+    pages, got = [1, 2, 3, 4], []
+    for together in (False, True):
+        eng = Engine(m, EngineConfig(num_pages=16, cuda_graphs=False))
+        m.forward(make_batch([{"tokens": toks[:95], "start": 0, "pages": pages, "state_slot": 0}], 32, m.device), eng.kv)
+        rows = [{"tokens": [toks[p]], "start": p, "pages": pages, "state_slot": 0} for p in (95, 96, 97)]
+        batches = [rows] if together else [[r] for r in rows]
+        out = torch.cat([m.forward(make_batch(b, 32, m.device), eng.kv) for b in batches])
+        got.append((out.float().cpu(), eng.kv.k[-1].float().cpu(), eng.kv.v[-1].float().cpu()))
+    ops.check_status(0)
+    for a, b in zip(*got):  # (other kernels by the number of rows: roundings of two layers)
+        assert ((a - b).norm() / a.norm()).item() < 2e-2
+
+
 @pytest.mark.parametrize("family,over", [("qwen3", dict(hidden_size=256, num_attention_heads=4, num_key_value_heads=2, head_dim=128)),
                                          ("llama", dict(hidden_size=512, num_attention_heads=4, num_key_value_heads=2))])
 def test_fused_rope_models_gpu(tmp_path, family, over, monkeypatch):

@@ -251,3 +251,23 @@ def test_make_batch_long_and_short_sequences():
     assert b.block_tables[0, :20].tolist() == list(range(40, 60)) and b.block_tables[2, 0].item() == 400
     d = make_batch([{"tokens": [7], "start": 100, "pages": list(range(5))} for _ in range(3)], page, "cpu")
     assert d.is_decode and d.slots.tolist() == [3 * page + 4] * 3
+
+
+def test_decode_rows_apart():
+    """Which decode batches have a row that reads another row's new key: two positions of one sequence, in one page and on either side of a page's end; the same entry twice; a shared
+    page that is being filled. Shared full pages, unused entries behind a sequence's last page and prompts of one token are none."""
+    from deliverance_b200.models.batch import make_batch
+
+    def rows(*seqs):
+        b = make_batch([{"tokens": [7], "start": start, "pages": pages} for start, pages in seqs], 32, "cpu")
+        assert b.is_decode
+        return b.rows_apart()
+
+    assert rows((100, [1, 2, 3, 4])) and rows((100, [1, 2, 3, 4]), (100, [5, 6, 7, 8]), (0, [9]), (31, [10]), (32, [11, 12]))
+    assert rows((100, [1, 2, 3, 4]), (70, [1, 2, 5]), (64, [1, 2, 6]))  # a prefix of whole pages
+    assert rows((40, [1, 2, 3]), (40, [4, 5, 2]))  # (page 2 lies behind what the second row reads)
+    assert rows((100, [1, 2, 3, 4]), (40, [0, 5])) and rows((40, [0, 5]), (0, [6]))
+    assert not rows((40, [1, 2]), (41, [1, 2])) and not rows((63, [1, 2, 3]), (64, [1, 2, 3])) and not rows((64, [1, 2, 3]), (63, [1, 2, 3]))
+    assert not rows((40, [1, 2]), (40, [1, 2])) and not rows((40, [1, 2]), (100, [1, 2, 3, 4]), (5, [9]))
+    b = make_batch([{"tokens": [7, 8], "start": 0, "pages": [1]}], 32, "cpu")
+    assert not b.is_decode and b.host_tables is None
