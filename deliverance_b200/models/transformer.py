@@ -108,6 +108,7 @@ class DecoderModel:
         # DLV_FUSED_ROPE=1 forces it on the CPU oracle path (tests of the composition).
         want = os.environ.get("DLV_FUSED_ROPE", "auto")
         self.fused_rope = (want == "1" or (want != "0" and torch.device(device).type == "cuda")) and cfg.head_dim == 128 and cfg.use_rope
+        self.rope_in_attention = want != "0"  # heads of 64, decode steps: the same inside the attention kernel (``ops.rope_in_attention`` says where)
         self.vocab_shard: Optional[tuple] = None
         self._moe_impl = None
         # opt-in (DLV_TP_SEQ_PARALLEL=1): sequence-parallel prefill under tensor parallelism for batches of at least this many rows
@@ -358,7 +359,7 @@ class DecoderModel:
         k_cache, v_cache = kv.layer(i)
         local_rope = lw.kind == "sliding" and self.cos_local is not None
         cos, sin = (self.cos_local, self.sin_local) if local_rope else (self.cos, self.sin)
-        inside = (batch.is_decode and self._sp is None and ops.rope_in_attention(x.device, self.n_heads, self.n_kv, cfg.head_dim) and
+        inside = (self.rope_in_attention and batch.is_decode and self._sp is None and ops.rope_in_attention(x.device, self.n_heads, self.n_kv, cfg.head_dim) and
                   batch.rows_apart())  # (else every new key is in the cache before any row reads it)
         if inside:  # norm + rotary + cache write in the attention kernel
             with self._stage("causalselfattention.qkv_projection"):

@@ -219,7 +219,7 @@ def main() -> int:
             model = DecoderModel(cfg, dev, torch.bfloat16, ctx).load(SyntheticLoader(shape, 3, True, dev, std=0.05), head_quant="Q4")
             # a sequence-parallel forward keeps projection and rotary embedding as two kernels; the reference run does the same, so that
             # the comparison of greedy tokens of a random-weight model (near-ties between logits) is between equal roundings
-            model.fused_rope = False
+            model.fused_rope = model.rope_in_attention = False
             used = []
             plan = model._sp_plan
             model._sp_plan = lambda b, plan=plan, used=used: (used.append(plan(b)), used[-1])[1]
@@ -300,7 +300,7 @@ def main() -> int:
         toks = {}
         for name, ctx in (("single", TensorParallelContext()), ("ep_sp", tp)):
             m2 = DecoderModel(mcfg, dev, torch.bfloat16, ctx).load(SyntheticLoader(mshape, 5, True, dev, std=0.05))
-            m2.fused_rope = False  # as above: equal roundings on both sides
+            m2.fused_rope = m2.rope_in_attention = False  # as above: equal roundings on both sides
             used = []
             plan = m2._sp_plan
             m2._sp_plan = lambda b, plan=plan, used=used: (used.append(plan(b)), used[-1])[1]

@@ -236,6 +236,38 @@ def test_fused_activation_models_gpu(tmp_path, family, monkeypatch):
     assert all(r.generated_tokens == 8 for r in rs)
 
 
+def test_rope_in_attention_models_gpu(tmp_path, monkeypatch):
+    """Heads of 64: norm, rotation and cache write of decode steps inside the attention kernel (the default) against a kernel of their own (``DLV_FUSED_ROPE=0``): logits and caches of
+    a step with a row that has no slot, and tokens through the engine, whose captured step of three sequences has a padded row."""
+    d = str(tmp_path / "m")
+    write_tiny_model(d, "qwen3", seed=13, std=0.05, quantize=True, max_position_embeddings=1024, hidden_size=256, num_attention_heads=4, num_key_value_heads=2, head_dim=64)
+    monkeypatch.setenv("DLV_FUSED_ROPE", "0")
+    plain = DecoderModel(load_config(d), "cuda:0").load(WeightLoader(d))
+    monkeypatch.setenv("DLV_FUSED_ROPE", "auto")
+    inside = DecoderModel(load_config(d), "cuda:0").load(WeightLoader(d))
+    g = torch.Generator().manual_seed(4)
+    seqs = [torch.randint(3, 250, (n,), generator=g).tolist() for n in (200, 33, 64)]
+    pages = [list(range(1, 9)), [9, 10], [11, 12, 13]]
+    got, launches, tokens = [], [], []
+    for m in (plain, inside):
+        eng = Engine(m, EngineConfig(num_pages=128, cuda_graphs=False))
+        m.forward(make_batch([{"tokens": t[:-1], "start": 0, "pages": p, "state_slot": i} for i, (t, p) in enumerate(zip(seqs, pages))], 32, m.device), eng.kv)
+        b = make_batch([{"tokens": t[-1:], "start": len(t) - 1, "pages": p, "state_slot": i} for i, (t, p) in enumerate(zip(seqs, pages))], 32, m.device)
+        b.slots[1] = -1
+        n = ops.LAUNCHES[0]
+        out = m.forward(b, eng.kv).float().cpu()
+        launches.append(ops.LAUNCHES[0] - n)
+        got.append((out[::2], *(t[1:].float().cpu() for t in (eng.kv.k[0], eng.kv.v[0], eng.kv.k[-1], eng.kv.v[-1]))))
+        ops.check_status(0)
+        eng = Engine(m, EngineConfig(num_pages=128, max_batch_tokens=2048))
+        tokens.append([r.token_ids for r in eng.generate_batch(seqs, GeneratorParameters(max_tokens=6))])
+    assert launches[0] - launches[1] == plain.cfg.num_layers
+    assert torch.equal(got[0][1], got[1][1]) and torch.equal(got[0][2], got[1][2])  # (the first layer's caches: nothing that is rounded otherwise stands in front)
+    for a, b in zip(*got):
+        assert ((a - b).norm() / a.norm()).item() < 2e-2
+    assert [r[0] for r in tokens[0]] == [r[0] for r in tokens[1]]
+
+
 def test_decode_rows_of_one_sequence_gpu(tmp_path):
     """Heads of 64: a decode batch with three positions of one sequence, and a page's end between them, against one position after the other."""
     d = str(tmp_path / "m")
