@@ -9,6 +9,7 @@
 #include <unordered_map>
 
 #include "chain_api.h"
+#include "divisor.h"
 #include "gemm_api.h"
 
 namespace {
@@ -1760,6 +1761,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding", &embedding, py::arg("table"), py::arg("ids"), py::arg("scale") = 1.0, py::arg("pos_table") = py::none(),
         py::arg("pos") = py::none(), py::arg("type_table") = py::none(), py::arg("types") = py::none());
   m.def("decode_attention_rope", &decode_attention_rope);
+  m.def("divide", [](int64_t n, int64_t d) {
+    TORCH_CHECK(n >= 0 && n < (1ll << 31) && d >= 1 && d < (1ll << 31), "n and d must lie in [0, 2^31) and [1, 2^31)");
+    dlv::Divisor by;
+    by.set(static_cast<int>(d));
+    return static_cast<int64_t>(by.of(static_cast<int>(n)));
+  });  // the division of the kernels' tile walks
   m.def("rope_kv", &rope_kv);
   m.def("decode_attention", &decode_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_tables"), py::arg("ctx_lens"),
         py::arg("H"), py::arg("scale"), py::arg("softcap") = 0.0, py::arg("window") = 0, py::arg("splits") = 1, py::arg("impl") = 0,

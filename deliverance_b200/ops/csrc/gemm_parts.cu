@@ -33,6 +33,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "divisor.h"
 #include "gemm_api.h"
 #include "gemm_tc.cuh"
 #include "pair.cuh"
@@ -60,15 +61,6 @@ constexpr int kThreads = 672;
 static_assert(kThreads == 640 + 32, "named barrier of the set-up");
 static_assert(kSmemBytes <= 232448, "shared memory of an SM");
 
-// n / d for n * d < 2^32 without a division (the walk's divisions kept the first copies back by some 2,000 cycles): high word of n * ceil(2^32 / d)
-struct Divisor {
-  unsigned d, m;  // m = 0: d is 1
-  __host__ void set(int n) {
-    d = static_cast<unsigned>(n < 1 ? 1 : n);
-    m = d > 1 ? static_cast<unsigned>(((1ull << 32) + d - 1) / d) : 0u;
-  }
-  __device__ __forceinline__ int of(int n) const { return m == 0u ? n : static_cast<int>(__umulhi(static_cast<unsigned>(n), m)); }
-};
 struct PartParams {
   int M, N;
   int kq;                 // stages of a tile: 128 k, bf16 weights 64 k
@@ -80,7 +72,7 @@ struct PartParams {
   int parts;              // parts of each of the other tiles (0: there are none)
   int w_tiles;            // packed 128-row tiles of the weight (of one expert)
   int half;               // EPI 1: outputs per row (gate rows); the up rows follow them
-  Divisor by_m, by_parts, by_group;  // m_tiles, parts, eight rows of weight tiles (grouped)
+  Divisor by_m, by_parts, by_group;  // m_tiles, parts, eight rows of weight tiles (grouped); the walk's divisions kept the first copies back by some 2,000 cycles
   const uint8_t* wq;
   void* out;
   int ldo, out_f32;
@@ -797,6 +789,7 @@ int cut_tiles(const PartPlan& q) { return q.n_tiles * q.m_tiles - q.waves * q.pa
 
 template <bool Q4, int EPI>
 void launch_parts(const GemmWeightDesc* w, const void* x, int rows, int ldx, PartParams p, cudaStream_t st) {
+  if ((static_cast<long long>(p.m_tiles) + 16) * p.n_tiles + p.pairs > 0x7fffffffll) throw std::runtime_error("pair gemm (parts): more tiles than the walk can number");
   CUtensorMap map_x;
   p.box = (p.bn <= kOneMma ? p.bn : (((p.bn >> 1) + 31) & ~31)) / 2;
   encode_map_kchunks(&map_x, x, static_cast<uint64_t>(rows), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, p.box, Q4 ? 2 : 1);

@@ -886,6 +886,25 @@ def test_lz4_block_format_golden_and_roundtrip():
     assert len(e.lz4_compress(bytes(70000))) < 400
 
 
+def test_tile_walk_division():
+    """Division by multiplication of the kernels' tile walks: exact for all 31-bit numbers, also where n * d passes 2^32 (the high word alone is one too large at 6,711,039 / 896,
+    60,000 work items of 112 weight tiles)."""
+    from deliverance_b200 import ops
+
+    e = ops.ext()
+    if e is None:
+        pytest.skip("extension not built")
+    assert (6711039 * -(-(2**32) // 896)) >> 32 == 6711039 // 896 + 1  # (what the correction is for)
+    rnd = random.Random(5)
+    top = 2**31 - 1
+    cases = [(6711039, 896), (0, 1), (top, 1), (top, 2), (top, top), (top - 1, top), (0, top)]
+    for _ in range(20000):
+        d = max(1, int(2 ** rnd.uniform(0, 31)) - 1)
+        q = rnd.randrange(0, top // d + 1)
+        cases += [(n, d) for n in (q * d - 1, q * d, q * d + d - 1, rnd.randrange(0, top + 1)) if 0 <= n <= top]
+    assert all(e.divide(n, d) == n // d for n, d in cases)
+
+
 def test_guard_area_checker_on_host_memory():
     """The bounds-checking allocator of the extension: an output cut out between two guard areas, the checker passes while they are
     intact and names the output once a guard byte has changed (the change is made from the host)."""
