@@ -889,6 +889,8 @@ def test_lz4_block_format_golden_and_roundtrip():
 def test_tile_walk_division():
     """Division by multiplication of the kernels' tile walks: exact for all 31-bit numbers, also where n * d passes 2^32 (the high word alone is one too large at 6,711,039 / 896,
     60,000 work items of 112 weight tiles)."""
+    import random
+
     from deliverance_b200 import ops
 
     e = ops.ext()
