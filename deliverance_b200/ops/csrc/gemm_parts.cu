@@ -372,11 +372,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) gemm_pa
       mbar_fence_init();
     }
     __syncwarp();
-    cluster_arrive_relaxed();
+    cluster_arrive_relaxed();  // (orders nothing that thread 0 has stored: barrier 2 below does, for the abort flag)
     for (int i = 0; any && i < min(pc.k1 - pc.k0, NR); ++i) copy_stage(pc, pc.k0 + i, i, 0, 1);
+    asm volatile("bar.sync 2, 64;" ::: "memory");
     cluster_wait();
     __syncwarp();
   } else {
+    if (Q4 && warp == 0) asm volatile("bar.arrive 2, 64;" ::: "memory");  // the abort flag is clear, before warp 3 first looks at it
     if (warp == 2) tmem_alloc_pair(smem_u32(tmem_slot), 512);
     tc_fence_before();
     __syncwarp();
