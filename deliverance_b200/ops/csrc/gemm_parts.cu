@@ -169,7 +169,7 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uin
 
 __device__ __forceinline__ float apply_act(int kind, float g) {
   if (kind == 2) return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
-  return __fdividef(g, 1.f + __expf(-g));
+  return g / (1.f + __expf(-g));  // (as in the other kernels: __fdividef is 0 where the divisor passes 2^126)
 }
 
 // What becomes of the sums of one token: a warp holds the token's 128 rows of a CTA's half tile, lane l rows 4 l .. + 3 (EPI 1: gate rows 2 l, 2 l + 1

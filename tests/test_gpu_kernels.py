@@ -1185,6 +1185,30 @@ def test_parts_gemm_gated(M, inter, K, act):
     assert _rel(h.cpu(), ref.act_fn(act)(f[:, :inter]) * f[:, inter:]) < 6e-3
 
 
+@pytest.mark.parametrize("q4", [True, False])
+def test_parts_gemm_gated_far_below_zero(q4):
+    """SiLU of gates around -88, where 1 + exp(-g) passes 2^126 but is a number still: the activation is small, its product with a large up row is not. As the activation kernel
+    has it, one rounding apart."""
+    inter, K, M = 128, 64, 4
+    w = torch.zeros(2 * inter, K)
+    w[:inter, 0], w[inter:, 1] = torch.linspace(-88.5, -86.0, inter).to(torch.bfloat16).float(), 1.0
+    x = torch.zeros(M, K)
+    x[:, 0], x[:, 1] = 1.0, torch.tensor([2.0**100, -(2.0**115), 2.0**120, 1.0])
+    if q4:
+        w[:inter, 0] = -88.0  # (one scale per 32: 11 for the gate rows' block)
+        p, s = q4_quantize(w)
+        lw = LinearWeight(Q4Tensor(p, s, tuple(w.shape))).to(DEV, torch.bfloat16)
+    else:
+        lw = LinearWeight(w.to(torch.bfloat16)).to(DEV, torch.bfloat16)
+    x = x.to(torch.bfloat16).to(DEV)
+    h, f = lw.handle().run_gated(x, 1, 4), ops.linear(x, lw, out_f32=True).double().cpu()
+    torch.cuda.synchronize()
+    ops.check_status()
+    want = f[:, :inter] / (1 + torch.exp(-f[:, :inter])) * f[:, inter:]
+    # (__expf is 2 ulp and the rounding of its argument, some 2^-17 of the value here)
+    assert bool((want[1] != 0).all()) and _rounded_once(h.cpu(), want, 2.0**-16 * want.abs() + 2.0**-130)
+
+
 @pytest.mark.parametrize("M", [1, 129, 400, 2310])
 @pytest.mark.parametrize("heads,kv,norm,rope,bias", [(4, 1, True, True, False), (6, 3, False, True, True), (3, 1, True, False, True)])
 def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
