@@ -239,6 +239,8 @@ class GemmWeight {
     desc_.data = w.data_ptr();
     c10::cuda::CUDAGuard guard(w.device());
     dlv::gemm_weight_init(&desc_);
+    dlv::gemm_weight_settle(cur_stream());  // (a cast or a repack may be the last kernel in this stream)
+    check_last_error("weight handle");
   }
 
   // Room for the bf16 form of a JQ4 weight (2 N K bytes) in front of a prompt-size product; it belongs to this call and goes back to the

@@ -97,6 +97,9 @@ void gemm_weight_init(GemmWeightDesc* w) {
   }
 }
 
+__global__ void settle_kernel() {}
+void gemm_weight_settle(cudaStream_t st) { settle_kernel<<<1, 1, 0, st>>>(); }
+
 bool g_pdl_enabled = true;
 bool& g_gemm_pdl = g_pdl_enabled;  // programmatic dependent launch of the GEMM kernels (ops.set_gemm_pdl / DLV_GEMM_PDL=0 turn it off)
 void gemm_set_pdl(bool on) { g_gemm_pdl = on; }

@@ -63,6 +63,9 @@ GemmScatterPlan gemm_scatter_plan(int M, int N, int size);
 bool gemm_scatter_supported(const GemmWeightDesc* w, int M, const GemmScatterArgs* a);
 
 void gemm_weight_init(GemmWeightDesc* w);
+// An empty launch in ordinary stream order. The products read their weights ahead of the wait for the kernel in front of them, so a weight must be complete when that kernel
+// begins: whoever writes one in stream order puts this behind (ops' GemmWeight does when it is made; the same goes for a weight that is changed in place later).
+void gemm_weight_settle(cudaStream_t st);
 int gemm_num_sms();
 void gemm_set_pdl(bool on);  // programmatic dependent launch of the GEMM kernels (on by default)
 void gemm_tc_run(const GemmWeightDesc* w, const void* x, int M, int ldx, void* out, int ldo, bool out_f32, const float* bias,

@@ -1121,6 +1121,18 @@ def test_gemv_bf16_pieces(N, K):
     assert bool(((y32.double() - f).abs() <= _row_slack(x, w.w, w.bias)).all()) and torch.equal(y, y32.to(torch.bfloat16)) and torch.equal(y, again)
 
 
+def test_first_product_of_a_fresh_weight():
+    """Products directly behind the kernels that make the weight (a cast, a repack, a stack of experts), whose bytes they read ahead of their wait: the same as later."""
+    x = torch.randn(1, 2048, device=DEV).to(torch.bfloat16)
+    torch.cuda.synchronize()
+    for i in range(20):
+        w = LinearWeight(torch.randn(11264, 2048, device=DEV))
+        q = LinearWeight(Q4Tensor(*q4_quantize(torch.randn(64, 2048)), (64, 2048)))
+        first = [ops.linear(x, w), ops.linear(x, q.to(DEV, torch.bfloat16))]
+        torch.cuda.synchronize()
+        assert torch.equal(first[0], ops.linear(x, w)) and torch.equal(first[1], ops.linear(x, q.to(DEV, torch.bfloat16)))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (31, 264, 128), (33, 136, 192), (256, 512, 1280), (257, 2560, 960), (385, 19456, 256), (700, 1000, 2624), (1537, 4104, 512)])
 def test_parts_gemm_edges(M, N, K):
     """One row; k that ends inside a packed stage; weight tiles that end inside a tile and inside eight outputs; one and two instructions per tile, several tiles of
