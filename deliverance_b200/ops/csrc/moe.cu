@@ -76,7 +76,8 @@ __device__ __forceinline__ unsigned order_key(float v) {
   return v != v ? 0u : (u & 0x80000000u ? ~u : u | 0x80000000u);
 }
 
-// NV experts per lane (expert lane + 32 j): they stay in registers through all rounds, a round is one warp-wide maximum of their order and one minimum of the index, and
+// NV experts per lane (expert lane + 32 j; 4, 8, 16 or 32: with 32 for all beyond 256, and the half of the warps that its registers leave, one launch took 122 us for 128 tokens x 300
+// experts, and 76 with 16): they stay in registers through all rounds, a round is one warp-wide maximum of their order and one minimum of the index, and
 // lane r keeps what round r chose. (With the chosen ones in arrays of a thread, which a loop of run-time length puts into local memory, and five shuffles of two
 // words per round, one block routed 32 tokens over 128 experts in 21.8 us and 64 over 8 in 15.3.)
 template <int NV>
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(256) moe_topk_kernel(const float* __restrict__
                     nullptr);
 }
 
-// Routing of a decode-size batch in ONE launch of one CTA (32 warps; 16 above 256 experts, whose scores take the registers): top-k per token, expert histogram and offsets, the stable
+// Routing of a decode-size batch in ONE launch of one CTA (32 warps; 16 above 512 experts, whose scores take the registers): top-k per token, expert histogram and offsets, the stable
 // permutation that groups (token, slot) pairs by expert, and the grouped GEMM's work list for the local experts [e0, e0 + ne)
 // with `bn` rows per item. It replaces a memset and four launches (moe_topk, moe_sort, moe_items and, where the grouped GEMV reads
 // token rows through `perm`, moe_gather), which cost more than the work at a few hundred pairs. Shared memory: T k + 2 E + ne + 3
@@ -287,19 +288,21 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
 
 // The same grouping for prefill-size batches, in parallel. The single-CTA kernel above walks all T k pairs once per expert (one
 // thread each): 2.5 ms for the 65,536 pairs of an 8,192-token chunk with 128 experts, two thirds of the whole MoE block at prefill.
-// Here the pairs are cut into chunks of kSortChunk: (a) every chunk counts its pairs per expert, (b) one CTA turns the expert
+// Here the pairs are cut into chunks (sort_chunk): (a) every chunk counts its pairs per expert, (b) one CTA turns the expert
 // histogram into offsets and the chunk counts into the first row of every (chunk, expert), (c) one warp per chunk hands out the
 // rows in pair order (__match_any_sync groups the lanes of one expert; the group's first lane advances the running row). The
 // order is the stable one: ascending pair index inside an expert.
-constexpr int kSortChunk = 256;
+// Chunks of 256 pairs spread the ranks over more warps; but one CTA scans the counts of all chunks, with fewer than four threads per expert beyond 256 experts. So those take
+// chunks of 1,024 above 8,192 pairs (all of the routing, 131,072 pairs, two per token: 300 experts 194 us with 256, 106 with 1,024; 512 experts 206 and 109; 128 experts 79 and 48).
+static int sort_chunk(long long pairs, int E) { return E > 256 && pairs > 8192 ? 1024 : 256; }
 constexpr int kSortSerialMaxPairs = 256;  // up to here the single-CTA kernel is used (us there and in the three launches: 260 pairs of 8 experts 12.8 and 8.6, 884 pairs 36.5 and 8.6)
-__global__ void __launch_bounds__(256) moe_chunk_hist_kernel(const int* __restrict__ idx, int P, int E, int* __restrict__ chunk_hist) {
+__global__ void __launch_bounds__(256) moe_chunk_hist_kernel(const int* __restrict__ idx, int P, int E, int chunk, int* __restrict__ chunk_hist) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
   extern __shared__ int hs[];  // [E]
   for (int e = threadIdx.x; e < E; e += blockDim.x) hs[e] = 0;
   __syncthreads();
-  const int p0 = blockIdx.x * kSortChunk, p1 = min(P, p0 + kSortChunk);
+  const int p0 = blockIdx.x * chunk, p1 = min(P, p0 + chunk);
   for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) atomicAdd(&hs[idx[p]], 1);
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) chunk_hist[static_cast<size_t>(blockIdx.x) * E + e] = hs[e];
@@ -362,15 +365,15 @@ __global__ void __launch_bounds__(1024) moe_chunk_scan_kernel(int* __restrict__ 
     }
   }
 }
-__global__ void __launch_bounds__(32) moe_chunk_rank_kernel(const int* __restrict__ idx, int P, int E, const int* __restrict__ chunk_base,
+__global__ void __launch_bounds__(32) moe_chunk_rank_kernel(const int* __restrict__ idx, int P, int E, int chunk, const int* __restrict__ chunk_base,
                                                             int* __restrict__ perm, int* __restrict__ pos) {
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
-  extern __shared__ int rk[];  // [E] running row per expert, then [kSortChunk] the chunk's expert ids
+  extern __shared__ int rk[];  // [E] running row per expert, then [chunk] the chunk's expert ids
   int* run_s = rk;
   int* idx_s = rk + E;
   const int lane = threadIdx.x;
-  const int p0 = blockIdx.x * kSortChunk, n = min(P - p0, kSortChunk);
+  const int p0 = blockIdx.x * chunk, n = min(P - p0, chunk);
   for (int e = lane; e < E; e += 32) run_s[e] = chunk_base[static_cast<size_t>(blockIdx.x) * E + e];
   for (int i = lane; i < n; i += 32) idx_s[i] = idx[p0 + i];
   __syncwarp();
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(const __nv_bfloat16* _
 // Ints of workspace launch_moe_route needs for T tokens (0: none, the single-CTA grouping is used)
 size_t moe_route_workspace_ints(int T, int E, int k) {
   const long long P = static_cast<long long>(T) * k;
-  return P > kSortSerialMaxPairs ? static_cast<size_t>((P + kSortChunk - 1) / kSortChunk) * E : 0;
+  return P > kSortSerialMaxPairs ? static_cast<size_t>((P + sort_chunk(P, E) - 1) / sort_chunk(P, E)) * E : 0;
 }
 void launch_moe_route(const float* logits, int T, int E, int k, const MoeRouting& r, float* w, int* idx, int* counts, int* offsets,
                       int* perm, int* pos, int* ws, cudaStream_t st) {
@@ -473,13 +476,14 @@ void launch_moe_route(const float* logits, int T, int E, int k, const MoeRouting
   int* histogram = chunks ? nullptr : counts;
   if (E <= 128) moe_topk_kernel<4><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   else if (E <= 256) moe_topk_kernel<8><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
+  else if (E <= 512) moe_topk_kernel<16><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   else moe_topk_kernel<32><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   const int P = T * k;
   if (chunks) {
-    const int C = (P + kSortChunk - 1) / kSortChunk;
-    moe_chunk_hist_kernel<<<C, 256, sizeof(int) * E, st>>>(idx, P, E, ws);
+    const int chunk = sort_chunk(P, E), C = (P + chunk - 1) / chunk;
+    moe_chunk_hist_kernel<<<C, 256, sizeof(int) * E, st>>>(idx, P, E, chunk, ws);
     moe_chunk_scan_kernel<<<1, 1024, sizeof(int) * (E + 1 + 1024), st>>>(counts, E, C, offsets, ws);
-    moe_chunk_rank_kernel<<<C, 32, sizeof(int) * (E + kSortChunk), st>>>(idx, P, E, ws, perm, pos);
+    moe_chunk_rank_kernel<<<C, 32, sizeof(int) * (E + chunk), st>>>(idx, P, E, chunk, ws, perm, pos);
     return;
   }
   moe_sort_kernel<<<1, 1024, sizeof(int) * (E + 1), st>>>(idx, counts, T, E, k, offsets, perm, pos);
@@ -495,6 +499,7 @@ bool launch_moe_route_small(const float* logits, int T, int E, int k, const MoeR
   };
   if (E <= 128) return run(moe_route_small_kernel<4, 1024>, 1024);
   if (E <= 256) return run(moe_route_small_kernel<8, 1024>, 1024);
+  if (E <= 512) return run(moe_route_small_kernel<16, 1024>, 1024);
   return run(moe_route_small_kernel<32, 512>, 512);
 }
 void launch_moe_gather(const void* x, const int* perm, int rows, int k, int row_bytes, void* xs, const int* offsets, int e0, int ne,
@@ -515,9 +520,18 @@ __global__ void __launch_bounds__(256) moe_items_kernel(const int* __restrict__ 
   pdl_trigger();  // first: the next kernel may then be set up (and a GEMM prefetch its weights) while this one still waits
   pdl_wait();
   __shared__ int first[1025];
-  for (int e = threadIdx.x; e < ne; e += blockDim.x) first[e] = (offsets[e0 + e + 1] - offsets[e0 + e] + bn - 1) / bn;
-  __syncthreads();
-  if (threadIdx.x < 32) {
+  if (ne <= 32) {  // (a lane per expert, no trip through shared memory)
+    const int lane = threadIdx.x;
+    if (lane < 32) {
+      const int n = lane < ne ? (offsets[e0 + lane + 1] - offsets[e0 + lane] + bn - 1) / bn : 0, incl = warp_incl_scan(n, lane);
+      if (lane < ne) first[lane] = incl - n;
+      if (lane == 31) first[ne] = incl;
+    }
+  } else {
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) first[e] = (offsets[e0 + e + 1] - offsets[e0 + e] + bn - 1) / bn;
+    __syncthreads();
+  }
+  if (ne > 32 && threadIdx.x < 32) {
     const int lane = threadIdx.x, chunk = (ne + 31) / 32, lo = min(ne, lane * chunk), hi = min(ne, lo + chunk);
     int sum = 0;
     for (int e = lo; e < hi; ++e) sum += first[e];
