@@ -359,7 +359,7 @@ class DecoderModel:
         k_cache, v_cache = kv.layer(i)
         local_rope = lw.kind == "sliding" and self.cos_local is not None
         cos, sin = (self.cos_local, self.sin_local) if local_rope else (self.cos, self.sin)
-        inside = (self.rope_in_attention and batch.is_decode and self._sp is None and ops.rope_in_attention(x.device, self.n_heads, self.n_kv, cfg.head_dim) and
+        inside = (self.rope_in_attention and batch.is_decode and self._sp is None and ops.rope_in_attention(x.device, x.shape[0], self.n_heads, self.n_kv, cfg.head_dim) and
                   batch.rows_apart())  # (else every new key is in the cache before any row reads it)
         if inside:  # norm + rotary + cache write in the attention kernel
             with self._stage("causalselfattention.qkv_projection"):

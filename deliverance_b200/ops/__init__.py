@@ -575,10 +575,12 @@ def decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, H, scale, soft
     return o.reshape(B, H * D)
 
 
-def rope_in_attention(device: torch.device, H: int, KV: int, D: int) -> bool:
+def rope_in_attention(device: torch.device, B: int, H: int, KV: int, D: int, sms: int = 148) -> bool:
     """Whether a decode step's norm, rotation and cache write go into the attention kernel (:func:`decode_attention_rope`): heads of 64, whose projection does not do them in
-    its epilogue."""
-    return device.type == "cuda" and D == 64 and H // KV <= 16 and not _MERGE_IN_KERNEL[0]
+    its epilogue, and (sequence, KV head) pairs that are resident at one time, two per SM. With more, every wave waits for the loads in front of its keys: us in two kernels / in one, 32 heads,
+    KV 4, 64 sequences of 40, 300, 1,500 keys 6.2 / 5.0, 10.0 / 8.9, 27.6 / 26.8; KV 8, 64 sequences 7.4 / 7.6, 12.8 / 14.3, 50.2 / 46.9; KV 4, 256 sequences of 300 keys
+    21.6 / 22.9; 12 heads, KV 12, 49.5 / 56.2."""
+    return device.type == "cuda" and D == 64 and H // KV <= 16 and B * KV <= 2 * sms and not _MERGE_IN_KERNEL[0]
 
 
 def decode_attention_rope(qkv, positions, slots, q_norm_w, k_norm_w, cos, sin, k_cache, v_cache, block_tables, ctx_lens, H, scale, softcap=0.0, window=0, splits=1,

@@ -253,6 +253,16 @@ def test_make_batch_long_and_short_sequences():
     assert d.is_decode and d.slots.tolist() == [3 * page + 4] * 3
 
 
+def test_rope_in_attention_rule():
+    """Heads of 64 in groups of up to 16, and no more (sequence, KV head) pairs than two per SM."""
+    from deliverance_b200 import ops
+
+    gpu = torch.device("cuda")
+    assert ops.rope_in_attention(gpu, 1, 32, 4, 64) and ops.rope_in_attention(gpu, 74, 32, 4, 64) and ops.rope_in_attention(gpu, 37, 16, 8, 64)
+    assert not ops.rope_in_attention(gpu, 75, 32, 4, 64) and not ops.rope_in_attention(gpu, 64, 32, 8, 64) and not ops.rope_in_attention(gpu, 1, 17, 1, 64)
+    assert not ops.rope_in_attention(gpu, 1, 32, 4, 128) and not ops.rope_in_attention(torch.device("cpu"), 1, 32, 4, 64)
+
+
 def test_decode_rows_apart():
     """Which decode batches have a row that reads another row's new key: two positions of one sequence, in one page and on either side of a page's end; the same entry twice; a shared
     page that is being filled. Shared full pages, unused entries behind a sequence's last page and prompts of one token are none."""
