@@ -299,7 +299,7 @@ class GemmWeight {
     if (force_splits == 0 && parts(impl, M, out.data_ptr(), out.stride(0), 0, room)) {
       dlv::gemm_parts_run(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), out_f32, bptr, floats(room),
                            scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
-      check_last_error("JQ4 pair gemm launch");
+      check_last_error("pair gemm (cut tiles) launch");
       return out;
     }
     TORCH_CHECK(impl != 4, "shape outside the pair kernel with cut tiles, or no memory for its partial sums");
@@ -368,7 +368,7 @@ class GemmWeight {
         Tensor out = new_out({M, desc_.N / 2}, x.options());
         dlv::gemm_parts_run_act(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), out.data_ptr(), static_cast<int>(out.stride(0)), static_cast<int>(act),
                                  floats(room), scratch_for(x.device().index()).status.data_ptr<int>(), cur_stream());
-        check_last_error("JQ4 pair gemm (gated activation) launch");
+        check_last_error("pair gemm (cut tiles, gated activation) launch");
         return out;
       }
     }
@@ -399,7 +399,7 @@ class GemmWeight {
       dlv::gemm_parts_run_grouped(&desc_, static_cast<int>(n_per_expert), xs.data_ptr(), static_cast<int>(xs.size(0)), static_cast<int>(xs.stride(0)), out.data_ptr(),
                                   static_cast<int>(out.stride(0)), items.data_ptr<int>(), static_cast<int>(items.size(0)), static_cast<int>(item_rows),
                                   static_cast<int>(act), scratch_for(xs.device().index()).status.data_ptr<int>(), cur_stream());
-      check_last_error("JQ4 pair gemm (grouped, gated activation) launch");
+      check_last_error("pair gemm (cut tiles, grouped, gated activation) launch");
       return out;
     }
     if (item_rows != 256 || !dlv::gemm_pair_act_supported(&desc_, static_cast<int>(n_per_expert), nullptr, static_cast<int>(n_per_expert / 2), true)) return Tensor();
@@ -525,7 +525,7 @@ class GemmWeight {
     if (parts(impl, M, q.data_ptr(), q.stride(0), 2, room)) {
       dlv::gemm_parts_run_qkv(&desc_, x.data_ptr(), M, static_cast<int>(x.stride(0)), q.data_ptr(), static_cast<int>(q.stride(0)), bptr, &a, floats(room),
                                s.status.data_ptr<int>(), cur_stream());
-      check_last_error("JQ4 pair gemm (fused q/k/v epilogue) launch");
+      check_last_error("pair gemm (cut tiles, fused q/k/v epilogue) launch");
       return q;
     }
     TORCH_CHECK(impl != 4, "shape outside the pair kernel with cut tiles, or no memory for its partial sums");

@@ -151,6 +151,29 @@ static int cluster_capacity(int size) {
   return cap[size];
 }
 
+// Split-K plan. The CTAs of one output tile form a cluster; cost model (microseconds): every wave of resident clusters
+// pays a fixed prologue/epilogue and its share of the k-blocks, split tiles also pay the cluster reduction.
+template <bool Q4, int BN, int EPI>
+static int choose_splits(int tiles, int kb_total, const GemmTpArgs* tp) {
+  int splits = 1;
+  double best = 1e30;
+  for (int s = 1; s <= 8; ++s) {
+    if (s > 1 && kb_total / s < 2) break;
+    const int cap = cluster_capacity<Q4, BN, EPI>(s);
+    if (cap <= 0) continue;
+    if (tp != nullptr && tp->size > 1 && (tiles > cap || tiles * s > tp->ncta_max)) continue;  // fused all-reduce: one wave
+    const int waves = (tiles + cap - 1) / cap;
+    const int kb = (kb_total + s - 1) / s;
+    const double per_kb = 0.22 * (BN > 64 ? BN / 64.0 : 1.0);
+    const double cost = waves * (3.0 + kb * per_kb + (s > 1 ? 1.0 : 0.0));
+    if (cost < best - 1e-9) {
+      best = cost;
+      splits = s;
+    }
+  }
+  return splits;
+}
+
 template <bool Q4, int BN, int EPI = 0>
 static void run_tc(const GemmWeightDesc* w, const void* x, int M, int ldx, GemmParams p, float* ws, size_t ws_floats, int* counters,
                    int n_counters, int force_splits, cudaStream_t st, const GemmTpArgs* tp) {
@@ -158,29 +181,8 @@ static void run_tc(const GemmWeightDesc* w, const void* x, int M, int ldx, GemmP
   p.n_tiles = (w->N + kGemmBM - 1) / kGemmBM;
   p.m_tiles = (M + BN - 1) / BN;
   const int tiles = p.n_tiles * p.m_tiles;
-  // Split-K plan. The CTAs of one output tile form a cluster; cost model (microseconds): every wave of resident clusters
-  // pays a fixed prologue/epilogue and its share of the k-blocks, split tiles also pay the cluster reduction.
   const bool no_cluster = force_splits < 0;  // negative: that many splits, reduced through the global workspace
-  int splits = 1;
-  if (force_splits != 0) {
-    splits = force_splits < 0 ? -force_splits : force_splits;
-  } else {
-    double best = 1e30;
-    for (int s = 1; s <= 8; ++s) {
-      if (s > 1 && p.kb_total / s < 2) break;
-      const int cap = cluster_capacity<Q4, BN, EPI>(s);
-      if (cap <= 0) continue;
-      if (tp != nullptr && tp->size > 1 && (tiles > cap || tiles * s > tp->ncta_max)) continue;  // fused all-reduce: one wave
-      const int waves = (tiles + cap - 1) / cap;
-      const int kb = (p.kb_total + s - 1) / s;
-      const double per_kb = 0.22 * (BN > 64 ? BN / 64.0 : 1.0);
-      const double cost = waves * (3.0 + kb * per_kb + (s > 1 ? 1.0 : 0.0));
-      if (cost < best - 1e-9) {
-        best = cost;
-        splits = s;
-      }
-    }
-  }
+  int splits = force_splits != 0 ? std::abs(force_splits) : choose_splits<Q4, BN, EPI>(tiles, p.kb_total, tp);
   if (splits > p.kb_total) splits = p.kb_total;
   if (splits < 1) splits = 1;
   p.kb_per_split = (p.kb_total + splits - 1) / splits;
@@ -298,6 +300,37 @@ static int pick_bn_waves(int M, int N) {
   if (t256 <= sms) return 256;  // a single partial wave: measured no gain from smaller tiles (the split-K planner fills the SMs)
   const double c256 = static_cast<double>((t256 + sms - 1) / sms), c128 = static_cast<double>((t128 + sms - 1) / sms) * kCost128;
   return c128 < 0.97 * c256 ? 128 : 256;
+}
+
+// Time of the one-tile kernel for M > 32 rows of a dense weight, in microseconds; `gated`: and of the activation kernel behind it (up to 128 rows). Per kind of weight and
+// token tile: a + waves * (b + k-blocks * c) + r with split tiles, no less than a and the bytes at bw TB/s, + e per million outputs of gate | up. The constants are
+// fitted to 1,500 products (22 shapes of either kind of weight, 512 to 40960 rows, K 512 to 16384, in chains of launches that start early); of single
+// products the estimate is within 8 to 12 % (standard deviation).
+double gemm_tc_estimate(const GemmWeightDesc* w, int M, bool gated) {
+  struct Fit {
+    double a, b, c, r, bw, e;
+  };
+  static const Fit fits[2][2][3] = {{{{0.0, 3.0, 0.67, 1.0, 5.2, 0.0}, {0.9, 3.3, 0.835, 1.5, 4.2, 0.0}, {0.0, 6.2, 1.04, 1.3, 5.0, 0.0}},
+                                     {{4.9, 0.2, 0.37, 2.7, 5.4, 0.7}, {5.5, 0.0, 0.86, 1.5, 5.4, 1.5}, {0.4, 7.9, 0.99, 1.6, 4.1, 0.5}}},
+                                    {{{0.0, 2.7, 0.37, 2.3, 5.0, 0.0}, {0.0, 5.1, 0.36, 1.4, 5.0, 0.0}, {0.0, 7.2, 0.77, 1.1, 5.0, 0.0}},
+                                     {{0.8, 3.3, 0.345, 1.6, 5.2, 2.2}, {3.2, 2.3, 0.363, 1.5, 5.2, 1.8}, {2.3, 4.5, 0.75, 2.6, 4.9, 1.2}}}};
+  const int BN = std::max(64, pick_bn_waves(M, w->N)), n_tiles = (w->N + kGemmBM - 1) / kGemmBM, m_tiles = (M + BN - 1) / BN, tiles = n_tiles * m_tiles;
+  const int kb_total = (w->K + kGemmBK - 1) / kGemmBK, sms = gemm_num_sms();
+  int s = 1, cap = sms;
+  auto plan = [&](auto bn) {
+    constexpr int B = decltype(bn)::value;
+    s = w->is_q4 ? choose_splits<true, B, 0>(tiles, kb_total, nullptr) : choose_splits<false, B, 0>(tiles, kb_total, nullptr);
+    cap = w->is_q4 ? cluster_capacity<true, B, 0>(s) : cluster_capacity<false, B, 0>(s);
+  };
+  if (BN == 64) plan(std::integral_constant<int, 64>());
+  else if (BN == 128) plan(std::integral_constant<int, 128>());
+  else plan(std::integral_constant<int, 256>());
+  const Fit& f = fits[w->is_q4 ? 1 : 0][gated ? 1 : 0][BN == 64 ? 0 : (BN == 128 ? 1 : 2)];
+  const int rest = n_tiles % sms;
+  double waves = (tiles + std::max(cap, 1) - 1) / std::max(cap, 1);
+  if (s == 1 && m_tiles == 1 && kb_total >= 8 && n_tiles > sms && rest > 0 && rest * 8 <= sms) waves -= 0.65;  // (run_tc cuts the few tiles of the last wave)
+  const double n = w->N, m = M, bytes = n * w->K * (w->is_q4 ? 0.625 : 2.0) + m * w->K * 2 + m * n * 2;
+  return std::max(f.a + waves * (f.b + (kb_total + s - 1) / s * f.c) + (s > 1 ? f.r : 0.0), f.a + bytes / (f.bw * 1e6)) + m * n * 1e-6 * f.e;
 }
 
 bool gemm_tp_supported(const GemmWeightDesc* w, int M, const GemmTpArgs* tp) {

@@ -113,6 +113,7 @@ void gemm_tc_run_gathered(const GemmWeightDesc* w, int M, const GemmScatterArgs*
                           const float* bias, float* ws, size_t ws_floats, int* counters, int n_counters, int* status, cudaStream_t st);
 // gemm_pair.cu: prefill-size products on pairs of SMs. `expanded`: device room of gemm_pair_expanded_bytes() for a JQ4 weight's bf16 form.
 bool gemm_pair_preferred(const GemmWeightDesc* w, int M, int n, int merged);  // faster than the one-tile kernel
+double gemm_tc_estimate(const GemmWeightDesc* w, int M, bool gated);  // of the one-tile kernel, gated: and of the activation behind it
 double gemm_pair_estimate(const GemmWeightDesc* w, int M, int n);  // its time in microseconds, the expansion of JQ4 weights included
 extern int g_gemm_pairs;  // most pairs of SMs that a launch takes; 0: the pair kernel is off, < 0: as many as the GPU holds
 bool gemm_pair_supported(const GemmWeightDesc* w, int n, const void* out, int ldo, bool grouped, int epi);
@@ -125,7 +126,7 @@ void gemm_pair_run_qkv(const GemmWeightDesc* w, const void* x, int M, int ldx, v
 bool gemm_pair_qkv_supported(const GemmWeightDesc* w, const void* q_out, int ldo, const GemmQkvArgs* a);
 void gemm_pair_run_grouped(const GemmWeightDesc* w, int n_per_expert, const void* x, int rows, int ldx, void* out, int ldo, const int* items, int max_items,
                            int act, int* status, cudaStream_t st);
-// gemm_parts.cu: JQ4 products of some dozens to some thousand rows, and experts, on pairs of SMs; what whole waves of tiles leave over is cut over k. `sums`: fp32
+// gemm_parts.cu: products of some dozens to some thousand rows, and JQ4 experts, on pairs of SMs; what whole waves of tiles leave over is cut over k. `sums`: fp32
 // room of gemm_parts_room() for what its second kernel finishes. epi: 0 store, 1 gated activation, 2 q | k | v heads.
 bool gemm_parts_supported(const GemmWeightDesc* w, int n, const void* out, int ldo, int epi);
 bool gemm_parts_preferred(const GemmWeightDesc* w, int M, int epi);

@@ -791,7 +791,7 @@ int cut_tiles(const PartPlan& q) { return q.n_tiles * q.m_tiles - q.waves * q.pa
 
 template <bool Q4, int EPI>
 void launch_parts(const GemmWeightDesc* w, const void* x, int rows, int ldx, PartParams p, cudaStream_t st) {
-  if ((static_cast<long long>(p.m_tiles) + 16) * p.n_tiles + p.pairs > 0x7fffffffll) throw std::runtime_error("pair gemm (parts): more tiles than the walk can number");
+  if ((static_cast<long long>(p.m_tiles) + 16) * p.n_tiles + p.pairs > 0x7fffffffll) throw std::runtime_error("pair gemm (cut tiles): more tiles than the walk can number");
   CUtensorMap map_x;
   p.box = (p.bn <= kOneMma ? p.bn : (((p.bn >> 1) + 31) & ~31)) / 2;
   encode_map_kchunks(&map_x, x, static_cast<uint64_t>(rows), static_cast<uint64_t>(w->K), static_cast<uint64_t>(ldx) * 2, p.box, Q4 ? 2 : 1);
@@ -803,7 +803,7 @@ void launch_parts(const GemmWeightDesc* w, const void* x, int rows, int ldx, Par
   p.by_parts.set(p.parts);
   p.by_group.set(8 * p.n_tiles);
   p.x_stages = Q4 ? std::min(kMaxX, kXRoom / (p.box * 256 * (p.bn > kOneMma ? 2 : 1))) : std::min(kMaxX, kStageRoom / (kWStage + p.box * 128 * (p.bn > kOneMma ? 2 : 1)));
-  if (part_pairs<Q4, EPI>() < p.pairs || p.pairs < 1) throw std::runtime_error("pair gemm (parts): no pair of SMs can hold the kernel");
+  if (part_pairs<Q4, EPI>() < p.pairs || p.pairs < 1) throw std::runtime_error("pair gemm (cut tiles): no pair of SMs can hold the kernel");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * p.pairs);
   cfg.blockDim = dim3(kThreads);
@@ -812,7 +812,7 @@ void launch_parts(const GemmWeightDesc* w, const void* x, int rows, int ldx, Par
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_parts_kernel<Q4, EPI>, map_x, map_w, p);
   const int tiles = p.n_tiles * p.m_tiles, second = EPI == 2 ? tiles : (p.parts > 1 ? tiles - p.waves * p.pairs : 0);
   if (e == cudaSuccess && p.items == nullptr && second > 0) e = launch_pdl(gemm_parts_sum_kernel<EPI>, dim3(2 * second, (p.bn + 7) / 8), dim3(128), 0, st, p);
-  if (e != cudaSuccess) throw std::runtime_error(std::string("pair gemm (parts) launch: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) throw std::runtime_error(std::string("pair gemm (cut tiles) launch: ") + cudaGetErrorString(e));
 }
 
 PartParams dense_params(const GemmWeightDesc* w, int M, int epi, float* sums, int* status) {
@@ -845,35 +845,49 @@ bool gemm_parts_supported(const GemmWeightDesc* w, int n, const void* out, int l
   return true;
 }
 
-// Whether this kernel is the faster one for M rows of a dense weight; all times in microseconds, 1.62 thousand cycles of the plan are one.
-// JQ4, below: the one-tile kernel, which may start under the kernel in front and so saves some two microseconds, up to 128 rows, and the gated form (whose
-// activation would be a launch of its own) up to 32: 19456 x 2560, 64 rows 22.4 us against 22.3 and two launches, 128 rows 24.3 against 29.5, 333 rows 38
-// against 51; 6144 x 2560 with heads 333 rows 22 against 38; 2560 x 9728 128 rows 15.4 against 13.0, 333 rows 23 against 27.
-// Above: the pair kernel behind an expansion to bf16, whose drain runs under the next tile; by both kernels' estimated times. The pair kernel's
-// estimate must be a seventh longer: where they are closer than that, prompts of several thousand rows that pull the clock
-// down by their power ran up to a tenth longer here (19456 x 2560, 1536 rows 119 us against 143, 2048 rows 154 against 174, 4096 rows 332 against
-// 322; 2560 x 9728, 2048 rows 68 against 112).
-// bf16, gated: from 33 rows on, against the pair kernel's 1.2 estimates and 8 us (its drain takes longer than the plain one): 28672 x 3584, 48 rows 42.7 against
-// 44.5 in two launches, 128 rows 44.8 against 56.4, 384 rows 69 against 86, 896 rows 137 against 149, but 1280 rows 187 against 179 and 2048 rows 298 against 281; 11264 x 2048, 128 rows 15.1
-// against 20.1, 384 rows 22.9 against 35.5, 1536 rows 54 against 65. Heads: one token tile (64 to 384 rows: every sum goes through the second kernel),
-// 6144 x 4096, 128 rows 18.0 against 22.4, 320 rows 25.2 against 31.6, 512 rows 35.5 against 31.9. Plain: from 193 rows on, against the better of the others (one-tile
-// while gemm_pair_preferred says so): 3584 x 14336, 384 rows 40 against 58, 700 rows 64 against 70, 1024 rows 91 against 79; 2560 x 2048, 256 rows 11.5 against
-// 12.9, 2048 rows 18.1 against 24.9; 2048 x 2048, 256 rows 11.1 against 12.4, 512 rows 13.3 against 12.8.
-// Plain, fewer rows: the one-tile kernel reads weights at some 4.3 TB/s with 65 to 128 rows and 5.8 with 33 to 64, this one at 5.7 and 6.2 and starts some 4 us later:
-// 36 M and some 170 M weights (256000 x 3584, 128 rows 323 us against 429, 64 rows 295 against 317; 3584 x 14336, 128 rows 28.4 against 29.9).
+// Whether this kernel is the faster one for M rows of a dense weight; all times in microseconds, 1.62 thousand cycles of the plan are one. It starts in ordinary order,
+// some two to four microseconds behind a one-tile kernel that starts under the kernel in front, and cut tiles take a second launch; so it has to earn that. The
+// comparisons are by estimates of the kernel that would run instead, where measured shapes (0.8 M to 920 M weights, 40 to 2048 rows, us here against there) fall on either side:
+// JQ4, plain and heads: above 128 rows (2560 x 9728, 128 rows 15.4 against 13.0, 333 rows 22.6 against 27.2; 6144 x 2560 with heads, 128 rows 13.7 against 13.8, 333 rows 22
+// against 38). Plain with at least six tiles of weights: fewer are a chain of cut tiles here and a cluster each there (1024 x 1024, 129 rows 8.9 against 7.6; 896 x 12032 18.2
+// against 15.4; 3200 x 512 6.8 against 7.6). Above 512 rows by the one-tile kernel's estimate (2560 x 4096, 768 rows 21.1 against 20.3, 1024 rows 26.1 against 34.3).
+// JQ4, gated: above 128 rows (0.71 to 0.95 of the other two launches). Below by the estimate, with a fourteenth to spare: expansion bounds a pair's
+// 256 weight rows at 0.59 per 128 k and two one-tile CTAs at 0.35 (28672 x 4096, 40 rows 42.4 against 30.9, 128 rows 42.9 against 38.3; 7552 x 8960, 128 rows 26.5 against 22.1;
+// but 19456 x 2560, whose last wave there is nearly empty, 80 rows 23.8 against 27.1, 128 rows 24.7 against 30.5).
+// JQ4 from 768 rows on also by the pair kernel's estimate (behind an expansion to bf16, its drain under the next tile), which must be a seventh longer: where they are closer than that,
+// prompts of several thousand rows that pull the clock down by their power ran up to a tenth longer here (19456 x 2560, 1536 rows 119 us against 143, 2048 rows 154 against 174,
+// 4096 rows 332 against 322; 2560 x 9728, 2048 rows 68 against 112).
+// bf16, gated: above 128 rows against the pair kernel's 1.2 estimates and 8 us (its drain takes longer than the plain one; 28672 x 3584, 384 rows 69 against 86, 896 rows 137 against 149,
+// but 1280 rows 187 against 179; 11264 x 2048, 384 rows 22.9 against 35.5), below by the one-tile estimate too (65 to 128 rows 0.70 to 1.04; 40 to 64 rows mostly slower:
+// 6144 x 1024, 48 rows 9.6 against 8.3, but 23040 x 2560 29.5 against 32.4).
+// bf16, heads: every sum goes through the second kernel. Up to 128 rows wide weights of 16 M and more (6144 x 4096, 65 rows 18.1 against 21.5; 1536 x 13184 20.3 against 18.0, 1536 x 1024
+// 9.8 against 8.1), to 192 rows not those of 2.3 to 8 M (2816 x 1792, 129 rows 12.8 against 12.2; on either side of them 0.68 to 0.95), to 256 rows where the pair kernel is not the
+// choice there (12288 x 12544, 160 rows 71 against 107, 256 rows 94 against 82), to 384 rows always (0.59 to 0.96), then by its estimate.
+// bf16, plain: from 193 rows on, against the better of the others by their estimates (3584 x 14336, 384 rows 40 against 59, 1024 rows 93 against 78; 2560 x 2048, 256 rows
+// 11.5 against 12.9; 1024 x 1024, 256 rows 9.4 against 8.7). Fewer rows: the one-tile kernel reads weights at some 4.3 TB/s with 65 to 128 rows and 5.8 with 33 to 64, this one at 5.7 and
+// 6.2, which pays from some 36 M and 170 M weights on, where the estimate does not say otherwise (256000 x 3584, 128 rows 323 against 424; 28672 x 8192, 65 rows 89 against 110, 48 rows 90
+// against 81).
 bool gemm_parts_preferred(const GemmWeightDesc* w, int M, int epi) {
   if (M <= 32 || g_gemm_persist || g_gemm_force_bn != 0) return false;  // (the last two: another kernel or tile was asked for)
   const double weights = static_cast<double>(w->N) * w->K;
-  if (w->is_q4 ? (epi != 1 && M <= 128) : (epi == 0 && M <= 192 && weights < (M > 64 ? 36e6 : 170e6))) return false;
+  if (w->is_q4 ? (epi != 1 && M <= 128) || (epi == 0 && w->N <= 1280) : (epi == 0 && M <= 192 && weights < (M > 64 ? 36e6 : 170e6))) return false;
   if (epi == 2 && M <= 64) return false;
   const PartPlan plan = plan_parts(w, M, epi);
   if (plan.pairs == 0) return false;
-  const double pair = gemm_pair_estimate(w, M, w->N);
-  if (w->is_q4) return M < 768 || 2.5 + plan.cost / 1.62 < 0.86 * pair;
-  const double here = 3.0 + plan.cost / 1.62;
-  if (epi == 1) return M < 2048 && here < 0.95 * (1.2 * pair + 8.0);
-  if (epi == 2) return M <= kMaxTokens || here < 0.86 * pair;
-  return M <= 192 || here < (gemm_pair_preferred(w, M, w->N, 0) ? 0.95 : 1.08) * pair;
+  const double pair = gemm_pair_estimate(w, M, w->N), here = (w->is_q4 ? 2.5 : 3.0) + plan.cost / 1.62;
+  const auto one = [&] { return gemm_tc_estimate(w, M, epi == 1); };
+  if (w->is_q4) {
+    if (M >= 768 && here >= 0.86 * pair) return false;
+    if (epi == 1) return M > 128 || here < 0.93 * one();
+    return epi == 2 || M <= 512 || here < one();
+  }
+  if (epi == 1) return M < 2048 && here < 0.9 * (1.2 * pair + 8.0) && (M > 128 || here < 0.95 * one());
+  if (epi == 2) {
+    if (M <= 128) return w->N >= 3400 && weights >= 16e6;
+    if (M <= 192 && weights > 2.3e6 && weights < 8e6) return false;
+    return M <= 256 ? !gemm_pair_preferred(w, M, w->N, 0) : M <= kMaxTokens || here < 0.86 * pair;
+  }
+  return (M <= 192 || here < (gemm_pair_preferred(w, M, w->N, 0) ? 0.95 : 1.08) * pair) && here < (M <= 64 ? 0.92 : 1.0) * one();
 }
 
 // fp32 room for the sums that the second kernel finishes (0: none)
@@ -918,7 +932,7 @@ void gemm_parts_run_qkv(const GemmWeightDesc* w, const void* x, int M, int ldx, 
 // Experts: work items of up to `item_rows` rows (384 at most); act 0: out [rows, n], otherwise act(gate) * up: out [rows, n / 2].
 void gemm_parts_run_grouped(const GemmWeightDesc* w, int n_per_expert, const void* x, int rows, int ldx, void* out, int ldo, const int* items, int max_items,
                             int item_rows, int act, int* status, cudaStream_t st) {
-  if (item_rows < 1 || item_rows > kMaxTokens) throw std::runtime_error("JQ4 pair gemm: work items of 1 to 384 rows");
+  if (item_rows < 1 || item_rows > kMaxTokens) throw std::runtime_error("pair gemm (cut tiles): work items of 1 to 384 rows");
   PartParams p = {};
   p.M = rows;
   p.N = n_per_expert;
