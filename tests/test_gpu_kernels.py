@@ -1084,10 +1084,20 @@ def test_rmsnorm_widths(T, H):
     torch.cuda.synchronize()
     want_res = (res.float() + 0.5 * x.float()).to(torch.bfloat16)
     assert torch.equal(got_res.cpu(), want_res)
+    assert _rel(y.cpu(), ref.rmsnorm(x.double(), w.double(), 1e-6, 1.0)) < 3e-3 and _rel(z.cpu(), ref.rmsnorm(want_res.double(), w.double(), 1e-6)) < 3e-3
+
+
+@pytest.mark.parametrize("T,H", [(1, 8), (7, 8), (1, 1024), (7, 2056), (3, 4104), (1185, 8), (2, 8200)])
+def test_rmsnorm_values(T, H):
+    """Value by value: rows in which nothing averages the roundings out."""
+    x, res = ((torch.randn(T, H) * s).to(torch.bfloat16) for s in (1.0, 3.0))
+    w = (torch.randn(H) * 0.1).to(torch.bfloat16)
+    got_res = res.to(DEV).clone()
+    y, z = ops.rmsnorm(x.to(DEV), w.to(DEV), 1e-6, 1.0).cpu(), ops.add_rmsnorm(x.to(DEV), got_res, w.to(DEV), 1e-6, 0.0, 0.5).cpu()
     # in front of the rounding, in fp32: at most H / 32 squares added up by a thread and ten sums across threads (the root halves their error), then a division, a
     # reciprocal root, the weight's offset and two products
     slack = (H / 64 + 16) * 2.0**-24
-    for got, want in ((y.cpu(), ref.rmsnorm(x.double(), w.double(), 1e-6, 1.0)), (z.cpu(), ref.rmsnorm(want_res.double(), w.double(), 1e-6))):
+    for got, want in ((y, ref.rmsnorm(x.double(), w.double(), 1e-6, 1.0)), (z, ref.rmsnorm(got_res.cpu().double(), w.double(), 1e-6))):
         assert _rounded_once(got, want, slack * want.abs())
 
 
@@ -1102,9 +1112,20 @@ def _row_slack(x, w, bias):
 def test_gemv_bf16_row(N, K, f32):
     w, x = (torch.randn(N, K) * 0.05).to(torch.bfloat16), torch.randn(1, K).to(torch.bfloat16)
     bias = torch.randn(N)
-    y = ops.linear(x.to(DEV), LinearWeight(w, bias).to(DEV, torch.bfloat16), out_f32=f32).cpu()
+    y = ops.linear(x.to(DEV), LinearWeight(w, bias).to(DEV, torch.bfloat16), out_f32=f32)
+    torch.cuda.synchronize()
+    assert _rel(y.cpu(), x.double() @ w.double().t() + bias.double()) < (1e-5 if f32 else 4e-3)
+
+
+@pytest.mark.parametrize("N,K", [(1, 8), (5, 8), (7, 1024), (33, 2056), (300, 3080), (33, 14336), (60000, 1544)])
+def test_gemv_bf16_values(N, K):
+    """Value by value, with bias: single sums that may cancel."""
+    w, x = (torch.randn(N, K) * 0.05).to(torch.bfloat16), torch.randn(1, K).to(torch.bfloat16)
+    bias = torch.randn(N)
+    lw = LinearWeight(w, bias).to(DEV, torch.bfloat16)
+    y, y32 = ops.linear(x.to(DEV), lw).cpu(), ops.linear(x.to(DEV), lw, out_f32=True).cpu()
     want, slack = x.double() @ w.double().t() + bias.double(), _row_slack(x, w, bias)
-    assert bool(((y.double() - want).abs() <= slack).all()) if f32 else _rounded_once(y, want, slack)
+    assert bool(((y32.double() - want).abs() <= slack).all()) and _rounded_once(y, want, slack)
 
 
 # As for the pair kernel: fp32 sums rounded to bf16 once, JQ4 products rounded to bf16 twice on top.
@@ -1118,7 +1139,7 @@ def test_gemv_bf16_pieces(N, K):
     y, y32, again = ops.linear(x, w), ops.linear(x, w, out_f32=True), ops.linear(x, w)
     f = x.double() @ w.w.double().t() + w.bias.double()
     torch.cuda.synchronize()
-    assert bool(((y32.double() - f).abs() <= _row_slack(x, w.w, w.bias)).all()) and torch.equal(y, y32.to(torch.bfloat16)) and torch.equal(y, again)
+    assert _rel(y32, f) < 1e-5 and torch.equal(y, y32.to(torch.bfloat16)) and torch.equal(y, again)
 
 
 def test_first_product_of_a_fresh_weight():
@@ -1269,9 +1290,9 @@ def test_parts_gemm_bf16(M, N, K):
     finally:
         ops.set_bounds_check(False)
     ops.check_status()
-    assert _rel(y.cpu(), f) < 4e-3 and _rel(y32.cpu(), f) < 2e-5 and torch.equal(odd[:, :N], y) and bool((odd[:, N] == 7.0).all())
+    assert _rel(y.cpu(), f) < 3e-3 and _rel(y32.cpu(), f) < 2e-5 and torch.equal(odd[:, :N], y) and bool((odd[:, N] == 7.0).all())
     if N % 16 == 0:
-        assert _rel(h.cpu(), torch.nn.functional.silu(f[:, : N // 2]) * f[:, N // 2 :]) < 4e-3
+        assert _rel(h.cpu(), torch.nn.functional.silu(f[:, : N // 2]) * f[:, N // 2 :]) < 3e-3
     else:
         assert h is None
 
