@@ -305,7 +305,8 @@ static int pick_bn_waves(int M, int N) {
 // Time of the one-tile kernel for M > 32 rows of a dense weight, in microseconds; `gated`: and of the activation kernel behind it (up to 128 rows). Per kind of weight and
 // token tile: a + waves * (b + k-blocks * c) + r with split tiles, no less than a and the bytes at bw TB/s, + e per million outputs of gate | up. The constants are
 // fitted to 1,500 products (22 shapes of either kind of weight, 512 to 40960 rows, K 512 to 16384, in chains of launches that start early); of single
-// products the estimate is within 8 to 12 % (standard deviation).
+// products the estimate is within 8 to 12 % (standard deviation). A wave of split tiles behind the first costs 3 more (JQ4 24576 x 4096, 96 rows in three waves 40.3), and a
+// last wave of a few tiles counts as a whole one, although run_tc cuts them (JQ4 19456 x 2560, 152 tiles on 148 SMs, 64 rows 23.3, 128 rows 31.2).
 double gemm_tc_estimate(const GemmWeightDesc* w, int M, bool gated) {
   struct Fit {
     double a, b, c, r, bw, e;
@@ -326,11 +327,9 @@ double gemm_tc_estimate(const GemmWeightDesc* w, int M, bool gated) {
   else if (BN == 128) plan(std::integral_constant<int, 128>());
   else plan(std::integral_constant<int, 256>());
   const Fit& f = fits[w->is_q4 ? 1 : 0][gated ? 1 : 0][BN == 64 ? 0 : (BN == 128 ? 1 : 2)];
-  const int rest = n_tiles % sms;
-  double waves = (tiles + std::max(cap, 1) - 1) / std::max(cap, 1);
-  if (s == 1 && m_tiles == 1 && kb_total >= 8 && n_tiles > sms && rest > 0 && rest * 8 <= sms) waves -= 0.65;  // (run_tc cuts the few tiles of the last wave)
+  const int waves = (tiles + std::max(cap, 1) - 1) / std::max(cap, 1);
   const double n = w->N, m = M, bytes = n * w->K * (w->is_q4 ? 0.625 : 2.0) + m * w->K * 2 + m * n * 2;
-  return std::max(f.a + waves * (f.b + (kb_total + s - 1) / s * f.c) + (s > 1 ? f.r : 0.0), f.a + bytes / (f.bw * 1e6)) + m * n * 1e-6 * f.e;
+  return std::max(f.a + waves * (f.b + (kb_total + s - 1) / s * f.c) + (s > 1 ? f.r + 3.0 * (waves - 1) : 0.0), f.a + bytes / (f.bw * 1e6)) + m * n * 1e-6 * f.e;
 }
 
 bool gemm_tp_supported(const GemmWeightDesc* w, int M, const GemmTpArgs* tp) {

@@ -849,8 +849,10 @@ bool gemm_parts_supported(const GemmWeightDesc* w, int n, const void* out, int l
 // some two to four microseconds behind a one-tile kernel that starts under the kernel in front, and cut tiles take a second launch; so it has to earn that. The
 // comparisons are by estimates of the kernel that would run instead, where measured shapes (0.8 M to 920 M weights, 40 to 2048 rows, us here against there) fall on either side:
 // JQ4, plain and heads: above 128 rows (2560 x 9728, 128 rows 15.4 against 13.0, 333 rows 22.6 against 27.2; 6144 x 2560 with heads, 128 rows 13.7 against 13.8, 333 rows 22
-// against 38). Plain with at least six tiles of weights: fewer are a chain of cut tiles here and a cluster each there (1024 x 1024, 129 rows 8.9 against 7.6; 896 x 12032 18.2
-// against 15.4; 3200 x 512 6.8 against 7.6). Above 512 rows by the one-tile kernel's estimate (2560 x 4096, 768 rows 21.1 against 20.3, 1024 rows 26.1 against 34.3).
+// against 38). Plain with at least five tiles of weights: fewer are a chain of cut tiles here and a cluster each there (1024 x 1024, 129 rows 9.3 against 7.6; 896 x 4864 13.1
+// against 10.8; 1152 x 896 8.5 against 8.7, 256 rows 8.7 against 10.4), and by the one-tile kernel's estimate (2048 x 5632, 160 rows 15.0 against 14.2, 320 rows 15.7 against
+// 16.4; 2560 x 4096, 160 rows 13.9 against 13.4, 320 rows 14.9 against 16.5, 768 rows 21.6 against 20.2, 1024 rows 26.3 against 34.4). That estimate does not see
+// how full the token tile of 256 is: up to 224 rows it is 2 % long and then 5 % short.
 // JQ4, gated: above 128 rows (0.71 to 0.95 of the other two launches). Below by the estimate, with a fourteenth to spare: expansion bounds a pair's
 // 256 weight rows at 0.59 per 128 k and two one-tile CTAs at 0.35 (28672 x 4096, 40 rows 42.4 against 30.9, 128 rows 42.9 against 38.3; 7552 x 8960, 128 rows 26.5 against 22.1;
 // but 19456 x 2560, whose last wave there is nearly empty, 80 rows 23.8 against 27.1, 128 rows 24.7 against 30.5).
@@ -858,11 +860,11 @@ bool gemm_parts_supported(const GemmWeightDesc* w, int n, const void* out, int l
 // prompts of several thousand rows that pull the clock down by their power ran up to a tenth longer here (19456 x 2560, 1536 rows 119 us against 143, 2048 rows 154 against 174,
 // 4096 rows 332 against 322; 2560 x 9728, 2048 rows 68 against 112).
 // bf16, gated: above 128 rows against the pair kernel's 1.2 estimates and 8 us (its drain takes longer than the plain one; 28672 x 3584, 384 rows 69 against 86, 896 rows 137 against 149,
-// but 1280 rows 187 against 179; 11264 x 2048, 384 rows 22.9 against 35.5), below by the one-tile estimate too (65 to 128 rows 0.70 to 1.04; 40 to 64 rows mostly slower:
-// 6144 x 1024, 48 rows 9.6 against 8.3, but 23040 x 2560 29.5 against 32.4).
-// bf16, heads: every sum goes through the second kernel. Up to 128 rows wide weights of 16 M and more (6144 x 4096, 65 rows 18.1 against 21.5; 1536 x 13184 20.3 against 18.0, 1536 x 1024
-// 9.8 against 8.1), to 192 rows not those of 2.3 to 8 M (2816 x 1792, 129 rows 12.8 against 12.2; on either side of them 0.68 to 0.95), to 256 rows where the pair kernel is not the
-// choice there (12288 x 12544, 160 rows 71 against 107, 256 rows 94 against 82), to 384 rows always (0.59 to 0.96), then by its estimate.
+// but 1280 rows 187 against 179; 18944 x 1536, 1280 rows 61 against 76; 11264 x 2048, 384 rows 22.9 against 35.5), below by the one-tile estimate too (65 to 128 rows 0.70 to 1.04; 40
+// to 64 rows mostly slower: 6144 x 1024, 48 rows 9.6 against 8.3, but 23040 x 2560 29.5 against 32.4).
+// bf16, heads: every sum goes through the second kernel. Up to 128 rows wide weights of 10 M and more (6144 x 4096, 65 rows 18.1 against 21.5; 6144 x 2560, 128 rows 15.1 against 18.5;
+// 1536 x 13184 20.3 against 18.0, 1536 x 1024 9.8 against 8.1), to 192 rows not those of 2.3 to 6 M (2816 x 1792, 129 rows 12.8 against 12.2; on either side of them 0.68 to
+// 0.95), to 256 rows where the pair kernel is not the choice there (12288 x 12544, 160 rows 71 against 107, 256 rows 94 against 82), to 384 rows always (0.59 to 0.96), then by its estimate.
 // bf16, plain: from 193 rows on, against the better of the others by their estimates (3584 x 14336, 384 rows 40 against 59, 1024 rows 93 against 78; 2560 x 2048, 256 rows
 // 11.5 against 12.9; 1024 x 1024, 256 rows 9.4 against 8.7). Fewer rows: the one-tile kernel reads weights at some 4.3 TB/s with 65 to 128 rows and 5.8 with 33 to 64, this one at 5.7 and
 // 6.2, which pays from some 36 M and 170 M weights on, where the estimate does not say otherwise (256000 x 3584, 128 rows 323 against 424; 28672 x 8192, 65 rows 89 against 110, 48 rows 90
@@ -870,7 +872,7 @@ bool gemm_parts_supported(const GemmWeightDesc* w, int n, const void* out, int l
 bool gemm_parts_preferred(const GemmWeightDesc* w, int M, int epi) {
   if (M <= 32 || g_gemm_persist || g_gemm_force_bn != 0) return false;  // (the last two: another kernel or tile was asked for)
   const double weights = static_cast<double>(w->N) * w->K;
-  if (w->is_q4 ? (epi != 1 && M <= 128) || (epi == 0 && w->N <= 1280) : (epi == 0 && M <= 192 && weights < (M > 64 ? 36e6 : 170e6))) return false;
+  if (w->is_q4 ? (epi != 1 && M <= 128) || (epi == 0 && w->N <= 1024) : (epi == 0 && M <= 192 && weights < (M > 64 ? 36e6 : 170e6))) return false;
   if (epi == 2 && M <= 64) return false;
   const PartPlan plan = plan_parts(w, M, epi);
   if (plan.pairs == 0) return false;
@@ -879,12 +881,12 @@ bool gemm_parts_preferred(const GemmWeightDesc* w, int M, int epi) {
   if (w->is_q4) {
     if (M >= 768 && here >= 0.86 * pair) return false;
     if (epi == 1) return M > 128 || here < 0.93 * one();
-    return epi == 2 || M <= 512 || here < one();
+    return epi == 2 || here < (M <= 224 ? 0.98 : (M <= 512 ? 1.05 : 1.0)) * one();
   }
-  if (epi == 1) return M < 2048 && here < 0.9 * (1.2 * pair + 8.0) && (M > 128 || here < 0.95 * one());
+  if (epi == 1) return M < 2048 && here < 0.95 * (1.2 * pair + 8.0) && (M > 128 || here < one());
   if (epi == 2) {
-    if (M <= 128) return w->N >= 3400 && weights >= 16e6;
-    if (M <= 192 && weights > 2.3e6 && weights < 8e6) return false;
+    if (M <= 128) return w->N >= 3400 && weights >= 10e6;
+    if (M <= 192 && weights > 2.3e6 && weights < 6e6) return false;
     return M <= 256 ? !gemm_pair_preferred(w, M, w->N, 0) : M <= kMaxTokens || here < 0.86 * pair;
   }
   return (M <= 192 || here < (gemm_pair_preferred(w, M, w->N, 0) ? 0.95 : 1.08) * pair) && here < (M <= 64 ? 0.92 : 1.0) * one();

@@ -1242,6 +1242,21 @@ def test_parts_gemm_gated_far_below_zero(q4):
     assert bool((want[1] != 0).all()) and _rounded_once(h.cpu(), want, 2.0**-16 * want.abs() + 2.0**-130)
 
 
+@pytest.mark.parametrize("q4,N,K,M,taken", [(True, 19456, 2560, 64, True), (True, 24576, 4096, 96, True), (True, 28672, 4096, 64, False), (True, 11264, 2048, 128, False),
+                                            (True, 11264, 2048, 129, True), (False, 28672, 3584, 128, True), (False, 6144, 2560, 100, True), (False, 3072, 1024, 64, False)])
+def test_parts_gemm_gated_rule(q4, N, K, M, taken):
+    """Where the one kernel takes a gated product and where projection and activation are two launches: a last wave of few one-tile CTAs, a second wave of clusters, narrow and wide
+    weights (each choice the faster one by 5 % or more, but for the first, which is so in a decode step)."""
+    if q4:
+        w = LinearWeight(Q4Tensor(torch.randint(0, 256, (N, K // 2), dtype=torch.uint8), torch.randn(N, K // 32) * 0.01, (N, K))).to(DEV, torch.bfloat16)
+    else:
+        w = LinearWeight((torch.randn(N, K, device=DEV) * 0.02).to(torch.bfloat16))
+    x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    out = w.handle().run_gated(x, 1)
+    torch.cuda.synchronize()
+    assert (out is not None) == taken
+
+
 @pytest.mark.parametrize("M", [1, 129, 400, 2310])
 @pytest.mark.parametrize("heads,kv,norm,rope,bias", [(4, 1, True, True, False), (6, 3, False, True, True), (3, 1, True, False, True)])
 def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
