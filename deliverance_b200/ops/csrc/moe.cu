@@ -76,7 +76,7 @@ __device__ __forceinline__ unsigned order_key(float v) {
   return v != v ? 0u : (u & 0x80000000u ? ~u : u | 0x80000000u);
 }
 
-// NV experts per lane (expert lane + 32 j; 4, 8, 16 or 32: with 32 for all beyond 256, and the half of the warps that its registers leave, one launch took 122 us for 128 tokens x 300
+// NV experts per lane (expert lane + 32 j; 4, 8, 16, 24 or 32: with 32 for all beyond 256, and the half of the warps that its registers leave, one launch took 122 us for 128 tokens x 300
 // experts, and 76 with 16): they stay in registers through all rounds, a round is one warp-wide maximum of their order and one minimum of the index, and
 // lane r keeps what round r chose. (With the chosen ones in arrays of a thread, which a loop of run-time length puts into local memory, and five shuffles of two
 // words per round, one block routed 32 tokens over 128 experts in 21.8 us and 64 over 8 in 15.3.)
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) moe_topk_kernel(const float* __restrict__
                     nullptr);
 }
 
-// Routing of a decode-size batch in ONE launch of one CTA (32 warps; 16 above 512 experts, whose scores take the registers): top-k per token, expert histogram and offsets, the stable
+// Routing of a decode-size batch in ONE launch of one CTA (32 warps; 24 above 512 experts and 16 above 768, whose scores take the registers): top-k per token, expert histogram and offsets, the stable
 // permutation that groups (token, slot) pairs by expert, and the grouped GEMM's work list for the local experts [e0, e0 + ne)
 // with `bn` rows per item. It replaces a memset and four launches (moe_topk, moe_sort, moe_items and, where the grouped GEMV reads
 // token rows through `perm`, moe_gather), which cost more than the work at a few hundred pairs. Shared memory: T k + 2 E + ne + 3
@@ -477,6 +477,7 @@ void launch_moe_route(const float* logits, int T, int E, int k, const MoeRouting
   if (E <= 128) moe_topk_kernel<4><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   else if (E <= 256) moe_topk_kernel<8><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   else if (E <= 512) moe_topk_kernel<16><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
+  else if (E <= 768) moe_topk_kernel<24><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   else moe_topk_kernel<32><<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, r, w, idx, histogram);
   const int P = T * k;
   if (chunks) {
@@ -500,6 +501,7 @@ bool launch_moe_route_small(const float* logits, int T, int E, int k, const MoeR
   if (E <= 128) return run(moe_route_small_kernel<4, 1024>, 1024);
   if (E <= 256) return run(moe_route_small_kernel<8, 1024>, 1024);
   if (E <= 512) return run(moe_route_small_kernel<16, 1024>, 1024);
+  if (E <= 768) return run(moe_route_small_kernel<24, 768>, 768);
   return run(moe_route_small_kernel<32, 512>, 512);
 }
 void launch_moe_gather(const void* x, const int* perm, int rows, int k, int row_bytes, void* xs, const int* offsets, int e0, int ne,

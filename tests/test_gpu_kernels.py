@@ -1379,6 +1379,12 @@ def test_moe_route_choices(T, E, k):
             assert torch.equal(perm.long(), order) and torch.equal(perm[pos.flatten().long()].long(), torch.arange(T * k))
 
 
+@pytest.mark.parametrize("T,E,k", [(25, 512, 8), (49, 513, 2), (128, 768, 1), (30, 768, 8), (17, 769, 15), (1100, 513, 8), (600, 768, 16)])
+def test_moe_route_widths(T, E, k):
+    """The numbers of experts at which a lane keeps more scores and a block has fewer warps, and either size of chunk."""
+    test_moe_route_choices(T, E, k)
+
+
 @pytest.mark.parametrize("T,k,H", [(1, 1, 8), (3, 5, 1032), (9, 8, 2048), (2, 70, 128)])
 def test_moe_combine_slots(T, k, H):
     """Slots that do not fill a group of four, more of them than are looked up ahead, rows of another rank's experts."""
