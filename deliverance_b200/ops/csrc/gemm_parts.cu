@@ -169,7 +169,10 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uin
 
 __device__ __forceinline__ float apply_act(int kind, float g) {
   if (kind == 2) return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
-  return g / (1.f + __expf(-g));  // (as in the other kernels: __fdividef is 0 where the divisor passes 2^126)
+  // Both sides of the quotient at a quarter: __fdividef is 0 for divisors of 2^126 and more, which 1 + exp(-g) reaches in front of the end of its range. Its 2 ulp are a 2^-13th of the
+  // rounding to bf16 behind the product (errors against 64 bits agree to seven digits with those of a division: 1.665046e-3, of the two kernels 3.1e-3); a division, in a drain that the
+  // next tile waits for, took 4.3 us of the 38 of JQ4 19456 x 2560 with 333 rows, this multiplication 0.3 to 1.1.
+  return __fdividef(0.25f * g, 0.25f + 0.25f * __expf(-g));
 }
 
 // What becomes of the sums of one token: a warp holds the token's 128 rows of a CTA's half tile, lane l rows 4 l .. + 3 (EPI 1: gate rows 2 l, 2 l + 1

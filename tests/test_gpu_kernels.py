@@ -1257,6 +1257,20 @@ def test_parts_gemm_gated_rule(q4, N, K, M, taken):
     assert (out is not None) == taken
 
 
+def test_parts_gemm_gated_huge_gates():
+    """Gates of 2^126 and more on either side of zero, and sums that overflow: as they are and nothing, then infinity and not a number, as g / (1 + exp(-g)) has it."""
+    inter, K, M = 64, 64, 3
+    w, x = torch.zeros(2 * inter, K), torch.zeros(M, K)
+    w[:inter, 0], w[inter:, 1] = torch.tensor([2.0**127, -(2.0**127), 2.0**126, -(2.0**126), 1.5 * 2.0**127, -100.0, 0.0, 1.0]).repeat(inter // 8), 2.0**-100
+    x[:, 0], x[:, 1] = torch.tensor([1.0, 1.0, 4.0]), torch.tensor([1.0, -(2.0**90), 1.0])
+    h = LinearWeight(w.to(torch.bfloat16)).to(DEV, torch.bfloat16).handle().run_gated(x.to(torch.bfloat16).to(DEV), 1, 4).float().cpu()
+    ops.check_status()
+    for m, up in ((0, 2.0**-100), (1, -(2.0**-10))):
+        assert torch.equal(h[m, :5], torch.tensor([2.0**127, 0.0, 2.0**126, 0.0, 1.5 * 2.0**127]) * up) and h[m, 6] == 0 and abs(h[m, 5]) < 2.0**-137
+        assert abs(h[m, 7] - 0.7310586 * up) <= abs(up) * 2.0**-8
+    assert bool((h[2, [0, 2, 4]] == math.inf).all()) and bool(torch.isnan(h[2, [1, 3]]).all()) and bool((h[2, [5, 6]] == 0).all())
+
+
 @pytest.mark.parametrize("M", [1, 129, 400, 2310])
 @pytest.mark.parametrize("heads,kv,norm,rope,bias", [(4, 1, True, True, False), (6, 3, False, True, True), (3, 1, True, False, True)])
 def test_parts_gemm_heads(M, heads, kv, norm, rope, bias):
